@@ -346,6 +346,9 @@ __device__ __forceinline__ void hist_ref(uint32_t *H, float4 tlo, float4 thi, fl
 // warp (lane k writes plane k of the three axes) or threads 0..95 of a CTA;
 // the caller syncs before reading.
 constexpr uint32_t kPlanes = 3 * kBins;
+// a warp's scratch for one node: histogram and plane table, or the packed
+// bounds of at most 32 references
+constexpr uint32_t kWarpScratch = kHist + kPlanes;
 __device__ __forceinline__ void node_planes_warp(float *P, float4 blo, float4 bhi) {
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
@@ -770,110 +773,192 @@ __device__ __forceinline__ int32_t exact_label(int axis, float p, float4 blo, fl
 // bounds, upper bounds and flat references' bounds; the lowest cost wins,
 // ties to the lower axis, then the lower plane, as in the oracle's loop.
 // ---------------------------------------------------------------------------
-// sorted ascending across the warp, one value per lane
-__device__ __forceinline__ float warp_sort32(float v) {
-    const uint32_t lane = threadIdx.x & 31u;
+// Nodes of at most 32 references, one warp, one reference per lane. A plane p
+// strictly inside the node needs no clipped bounds (lo < p says the same of
+// the triangle's own bound), and a reference flat on an axis (lo == hi == v)
+// goes below for v <= p and above for v >= p, which the bounds one step
+// outside v say with the plain comparisons. So with lane_bounds' values
+//   below(p) = #(lo < p),  above(p) = #(hi > p)
+// hold for every plane either search costs, and the partition is the same two
+// comparisons.
+__device__ __forceinline__ void lane_bounds(float4 &lo, float4 &hi) {
 #pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1)
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            const float o = __shfl_xor_sync(0xffffffffu, v, j);
-            const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
-            v = keep_min ? (o < v ? o : v) : (o > v ? o : v);
-        }
-    return v;
-}
-
-// #(sorted lane values < p) (LT) or <= p, over the warp's 32 sorted values
-template <bool LE>
-__device__ __forceinline__ uint32_t warp_rank32(float sorted, float p) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t step = 16; step; step >>= 1) {
-        const float v = __shfl_sync(0xffffffffu, sorted, (int)(pos + step - 1));
-        if (LE ? v <= p : v < p) pos += step;
-    }
-    // [0, pos) pass; lane pos is untested only when pos == 31
-    const float v = __shfl_sync(0xffffffffu, sorted, (int)pos);
-    if (LE ? v <= p : v < p) pos += 1;
-    return pos;
-}
-
-// a node of at most 32 references, one warp, registers only: the lanes with
-// have set hold its references' bounds (cnt of them, in any lanes)
-__device__ Decision sah_exact_lanes(bool have, float4 tlo, float4 thi, uint32_t cnt, float4 blo, float4 bhi,
-                                    float ct, float ci) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const float Anode = surf(blo, bhi);
-    float mc = kInf, m_pk = 0.0f;
-    uint32_t m_ax = 3, m_nb = 0, m_na = 0;
-#pragma unroll 1
     for (uint32_t a = 0; a < 3; a++) {
-        const float l = c3(blo, a), h = c3(bhi, a);
-        if (!(__fsub_rn(h, l) > 0.0f)) continue;
-        const float lo = have ? mxf(c3(tlo, a), l) : kInf, hi = have ? mnf(c3(thi, a), h) : kInf;
-        const float slo = warp_sort32(lo), shi = warp_sort32(hi);
-        // references flat on this axis (often none: then no sort, no search)
-        const bool any_flat = __ballot_sync(0xffffffffu, have && lo == hi) != 0u;
-        const float sfl = any_flat ? warp_sort32(lo == hi ? lo : kInf) : kInf;
+        // a NaN bound clips to the node's side
+        const float l = fmaxf(c3(lo, a), -kInf), h = fminf(c3(hi, a), kInf);
+        s3(lo, a, l == h ? nextafterf(l, -kInf) : l);
+        s3(hi, a, l == h ? nextafterf(h, kInf) : h);
+    }
+}
+
+// a warp's scratch: the bounds of a node's references, packed (the set lanes
+// in order), 32 values per axis and side: lane_bounds' values, then the
+// triangles' own (the exact search's candidates)
+constexpr uint32_t kLaneScratch = 12 * 32;
+static_assert(kLaneScratch <= kWarpScratch && kWarpScratch % 4 == 0, "the packed bounds fit a warp's scratch");
+
+// the set lanes' bounds (rank: the lane's place among them, c of them) to S,
+// padded to a multiple of four with references that no plane counts
+template <bool EXACT>
+__device__ __forceinline__ void lanes_pack(float *S, bool in, uint32_t rank, uint32_t c, float4 tlo, float4 thi,
+                                           float4 nlo, float4 nhi) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();   // the previous node's readers are done
+    if (in) {
 #pragma unroll
-        for (int side = 0; side < 2; side++) {
-            const float pk = __fadd_rn(side ? hi : lo, 0.0f);
-            const uint32_t fon = any_flat ? warp_rank32<true>(sfl, pk) - warp_rank32<false>(sfl, pk) : 0u;
-            const uint32_t nb = warp_rank32<false>(slo, pk) + fon;
-            const uint32_t na = (cnt - warp_rank32<true>(shi, pk)) + fon;
-            if (!(have && pk > l && pk < h)) continue;
-            float4 bb = bhi, ba = blo;
-            s3(bb, a, pk);
-            s3(ba, a, pk);
-            const float sb = surf(blo, bb), sa = surf(ba, bhi);
-            const float cost = __fadd_rn(
-                ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
-            if (cost < mc || (cost == mc && a == m_ax && pk < m_pk)) {
-                mc = cost;
-                m_ax = a;
-                m_pk = pk;
-                m_nb = nb;
-                m_na = na;
+        for (uint32_t a = 0; a < 3; a++) {
+            S[(2 * a) * 32 + rank] = c3(nlo, a);
+            S[(2 * a + 1) * 32 + rank] = c3(nhi, a);
+            if (EXACT) {
+                S[(6 + 2 * a) * 32 + rank] = c3(tlo, a);
+                S[(7 + 2 * a) * 32 + rank] = c3(thi, a);
             }
         }
     }
-    float bc = mc, bp = m_pk;
-    uint32_t bax = m_ax, blane = lane;
-    for (int off = 16; off; off >>= 1) {
-        const float oc = __shfl_xor_sync(0xffffffffu, bc, off), op = __shfl_xor_sync(0xffffffffu, bp, off);
-        const uint32_t oax = __shfl_xor_sync(0xffffffffu, bax, off), ol = __shfl_xor_sync(0xffffffffu, blane, off);
-        if (oc < bc || (oc == bc && (oax < bax || (oax == bax && (op < bp || (op == bp && ol < blane)))))) {
-            bc = oc;
-            bp = op;
-            bax = oax;
-            blane = ol;
+    if (lane >= c && lane < ((c + 3u) & ~3u)) {
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            S[(2 * a) * 32 + lane] = kInf;
+            S[(2 * a + 1) * 32 + lane] = -kInf;
         }
     }
-    Decision best{-1, 0.0f, 0, 0, kInf, 0};
-    const uint32_t nb = __shfl_sync(0xffffffffu, m_nb, blane), na = __shfl_sync(0xffffffffu, m_na, blane);
-    if (bc < kInf) {
-        best.axis = (int)bax;
-        best.plane = bp;
-        best.nb = nb;
-        best.na = na;
-        best.cost = bc;
+    __syncwarp();
+}
+
+// cost of the plane pk on axis a of a node with extents ext, surface Anode
+__device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float h, float4 ext, float Anode,
+                                            uint32_t nb, uint32_t na, float ct, float ci) {
+    const float db = __fsub_rn(pk, l), da = __fsub_rn(h, pk);
+    const float bx = a == 0 ? db : ext.x, by = a == 1 ? db : ext.y, bz = a == 2 ? db : ext.z;
+    const float ax = a == 0 ? da : ext.x, ay = a == 1 ? da : ext.y, az = a == 2 ? da : ext.z;
+    const float sb =
+        __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(bx, by), __fmul_rn(bz, by)), __fmul_rn(bx, bz)));
+    const float sa =
+        __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(ax, ay), __fmul_rn(az, ay)), __fmul_rn(ax, az)));
+    return __fadd_rn(
+        ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
+}
+
+// the binned SAH of a packed node: lane k counts and costs plane k of every
+// axis (sah_warp's planes, counts and argmin). Counting c references takes
+// about 14 instructions each; a histogram costs about 350 whatever c is
+// (clearing, bins, atomics, scans), and the subtree pass's nodes hold 9
+// references on average.
+__device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c, float4 blo, float4 bhi, float ct,
+                                                     float ci) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float Anode = surf(blo, bhi);
+    const float4 ext = make_float4(__fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), 0.0f);
+    float pk[3];
+    uint32_t nb[3] = {0, 0, 0}, na[3] = {0, 0, 0};
+#pragma unroll
+    for (uint32_t a = 0; a < 3; a++) pk[a] = plane_k(c3(blo, a), c3(ext, a), lane);
+    for (uint32_t i = 0; i < c; i += 4) {
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            const float4 L = *reinterpret_cast<const float4 *>(S + (2 * a) * 32 + i);
+            const float4 H = *reinterpret_cast<const float4 *>(S + (2 * a + 1) * 32 + i);
+            nb[a] += (L.x < pk[a] ? 1u : 0u) + (L.y < pk[a] ? 1u : 0u) + (L.z < pk[a] ? 1u : 0u) + (L.w < pk[a] ? 1u : 0u);
+            na[a] += (H.x > pk[a] ? 1u : 0u) + (H.y > pk[a] ? 1u : 0u) + (H.z > pk[a] ? 1u : 0u) + (H.w > pk[a] ? 1u : 0u);
+        }
     }
-    if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)cnt))) best.axis = -1;
+    float mc = kInf, m_pk = 0.0f;
+    uint32_t mkey = 0xffffffffu, m_n = 0;
+#pragma unroll
+    for (uint32_t a = 0; a < 3; a++) {
+        const float l = c3(blo, a), h = c3(bhi, a);
+        if (!(c3(ext, a) > 0.0f)) continue;
+        const float pk1 = __shfl_down_sync(0xffffffffu, pk[a], 1);   // plane k + 1 (lane 31: unused)
+        if (!(lane >= 1 && pk[a] > l && pk[a] < h && (lane == 31 || pk[a] < pk1))) continue;
+        const float cost = plane_cost(a, pk[a], l, h, ext, Anode, nb[a], na[a], ct, ci);
+        if (cost < mc) {   // NaN / inf never win; an earlier axis keeps ties
+            mc = cost;
+            mkey = a * 32u + lane;
+            m_n = nb[a] | (na[a] << 16);
+            m_pk = pk[a];
+        }
+    }
+    // as in sah_warp: the least cost, then the least key
+    const uint32_t cbits = __float_as_uint(mc);
+    const uint32_t mbits = __reduce_min_sync(0xffffffffu, cbits);
+    const uint32_t bk = __reduce_min_sync(0xffffffffu, cbits == mbits ? mkey : 0xffffffffu);
+    const float bc = __uint_as_float(mbits);
+    Decision best{-1, 0.0f, 0, 0, kInf, 0};
+    const uint32_t src = bk & 31u;
+    const float p = __shfl_sync(0xffffffffu, m_pk, src);
+    const uint32_t n = __shfl_sync(0xffffffffu, m_n, src);
+    if (bc < kInf) best = Decision{(int)(bk >> 5), p, n & 0xffffu, n >> 16, bc, (int)src};
+    if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)c))) best.axis = -1;
+    return best;
+}
+
+// the exact SAH of a packed node: candidate q of 6 c (axis, side, reference)
+// is taken by lane q % 32, which counts the references below and above it;
+// two sorts per axis and a binary search per candidate and list cost four
+// times as much at the subtree pass's 9 references per node
+__device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, float4 blo, float4 bhi, float ct,
+                                                    float ci) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float Anode = surf(blo, bhi);
+    const float4 ext = make_float4(__fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), 0.0f);
+    float mc = kInf, m_pk = 0.0f;
+    uint32_t m_ax = 3, m_n = 0;
+    for (uint32_t q0 = 0; q0 < 6 * c; q0 += 32) {
+        const uint32_t q = min(q0 + lane, 6 * c - 1);   // (a repeated candidate changes nothing)
+        const uint32_t a = (q >= 2 * c ? 1u : 0u) + (q >= 4 * c ? 1u : 0u), j = q - 2 * a * c;
+        const float x = S[(6 + 2 * a + (j >= c ? 1u : 0u)) * 32 + (j >= c ? j - c : j)];
+        const float pk = __fadd_rn(x, 0.0f);
+        const float l = c3(blo, a), h = c3(bhi, a);
+        uint32_t nb = 0, na = 0;
+        const float *Sl = S + 64 * a, *Sh = Sl + 32;
+        for (uint32_t i = 0; i < c; i += 4) {
+            const float4 L = *reinterpret_cast<const float4 *>(Sl + i);
+            const float4 H = *reinterpret_cast<const float4 *>(Sh + i);
+            nb += (L.x < pk ? 1u : 0u) + (L.y < pk ? 1u : 0u) + (L.z < pk ? 1u : 0u) + (L.w < pk ? 1u : 0u);
+            na += (H.x > pk ? 1u : 0u) + (H.y > pk ? 1u : 0u) + (H.z > pk ? 1u : 0u) + (H.w > pk ? 1u : 0u);
+        }
+        // (an axis without extent has no plane strictly inside)
+        if (!(pk > l && pk < h)) continue;
+        const float cost = plane_cost(a, pk, l, h, ext, Anode, nb, na, ct, ci);
+        if (cost < mc || (cost == mc && a == m_ax && pk < m_pk)) {   // a rises with q
+            mc = cost;
+            m_ax = a;
+            m_pk = pk;
+            m_n = nb | (na << 16);
+        }
+    }
+    // the least (cost, axis, plane); equal keys are the same plane with the
+    // same counts. Costs are +0 .. +inf, so their bits order as they do.
+    const uint32_t mbits = __reduce_min_sync(0xffffffffu, __float_as_uint(mc));
+    bool win = __float_as_uint(mc) == mbits;
+    const uint32_t bax = __reduce_min_sync(0xffffffffu, win ? m_ax : 3u);
+    win = win && m_ax == bax;
+    const uint32_t pb = __float_as_uint(m_pk), po = (pb & 0x80000000u) ? ~pb : (pb | 0x80000000u);
+    const uint32_t bpo = __reduce_min_sync(0xffffffffu, win ? po : 0xffffffffu);
+    const uint32_t src = __ffs(__ballot_sync(0xffffffffu, win && po == bpo)) - 1u;
+    const float bc = __uint_as_float(mbits);
+    Decision best{-1, 0.0f, 0, 0, kInf, 0};
+    const float p = __shfl_sync(0xffffffffu, m_pk, src & 31u);
+    const uint32_t n = __shfl_sync(0xffffffffu, m_n, src & 31u);
+    if (bc < kInf) best = Decision{(int)bax, p, n & 0xffffu, n >> 16, bc, 0};
+    if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)c))) best.axis = -1;
     return best;
 }
 
 // a node of at most 32 references of the level, one per lane
-__device__ Decision sah_exact_warp32(const LevelArgs &A, uint4 info, float4 blo, float4 bhi, float ct, float ci) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const bool have = lane < info.y;
+template <bool EXACT>
+__device__ __forceinline__ Decision sah_warp32(const LevelArgs &A, float *S, uint4 info, float4 blo, float4 bhi) {
+    const uint32_t lane = threadIdx.x & 31u, c = info.y;
     float4 tlo = make_float4(0, 0, 0, 0), thi = tlo;
-    if (have) {
+    if (lane < c) {
         const uint32_t tri = A.refs()[info.x + lane];
         tlo = A.tb_lo[tri];
         thi = A.tb_hi[tri];
     }
-    return sah_exact_lanes(have, tlo, thi, info.y, blo, bhi, ct, ci);
+    float4 nlo = tlo, nhi = thi;
+    lane_bounds(nlo, nhi);
+    lanes_pack<EXACT>(S, lane < c, lane, c, tlo, thi, nlo, nhi);
+    return EXACT ? sah_lanes_exact(S, c, blo, bhi, A.ct, A.ci) : sah_lanes_binned(S, c, blo, bhi, A.ct, A.ci);
 }
 
 // first index in sorted v[0, n) with v[i] >= p (lower) or v[i] > p (upper)
@@ -1202,8 +1287,7 @@ __global__ void __launch_bounds__(256, 3) k_hist(LevelArgs A) {
 // binned decision and histogram features are stored for k_learn, which
 // decides it (a node past the row capacity keeps the binned decision).
 template <bool WARP_EXACT, bool LEARNED>
-__device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*HS)[kHist], float (*PS)[kPlanes],
-                                           Tally &tally) {
+__device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*WS)[kWarpScratch], Tally &tally) {
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nodes = A.lc->nodes;
     const uint32_t ngroups = (nodes + 7) / 8;
@@ -1225,11 +1309,11 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*HS)[kH
         }
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
         Decision d;
-        if (WARP_EXACT && cnt <= kWarpExact) {
-            d = sah_exact_warp32(A, info, blo, bhi, A.ct, A.ci);
+        if (cnt <= kWarpExact) {
+            d = sah_warp32<WARP_EXACT>(A, reinterpret_cast<float *>(WS[wib]), info, blo, bhi);
         } else {
-            uint32_t *Hw = HS[wib];
-            float *Pw = PS[wib];
+            uint32_t *Hw = WS[wib];
+            float *Pw = reinterpret_cast<float *>(WS[wib] + kHist);
             __syncwarp();   // the previous node's readers are done
             {
                 // 288 counters = 72 16-byte stores
@@ -1271,13 +1355,12 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*HS)[kH
 
 template <bool WARP_EXACT, bool LEARNED>
 __global__ void __launch_bounds__(256, 5) k_small(LevelArgs A) {
-    __shared__ __align__(16) uint32_t HS[8][kHist];
-    __shared__ float PS[8][kPlanes];
+    __shared__ __align__(16) uint32_t WS[8][kWarpScratch];
     __shared__ uint32_t s_tally[kTallies];
     wait_prior_grid();
     if (level_aborted(A)) return;
     Tally tally;
-    small_body<WARP_EXACT, LEARNED>(A, HS, PS, tally);
+    small_body<WARP_EXACT, LEARNED>(A, WS, tally);
     tally_flush(A, tally, s_tally);
 }
 
@@ -1286,10 +1369,7 @@ __global__ void __launch_bounds__(256, 5) k_small(LevelArgs A) {
 // (no second stream, no fork and join per level)
 union DecideSmem {
     HistSmem hist;
-    struct {
-        uint32_t HS[8][kHist];
-        float PS[8][kPlanes];
-    } small;
+    uint32_t small[8][kWarpScratch];
 };
 
 __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
@@ -1300,7 +1380,7 @@ __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
     Tally tally;
     hist_body<false>(A, sm.hist, nullptr, tally);
     __syncthreads();
-    small_body<false, false>(A, sm.small.HS, sm.small.PS, tally);
+    small_body<false, false>(A, sm.small, tally);
     tally_flush(A, tally, s_tally);
 }
 
@@ -2382,10 +2462,11 @@ constexpr int kSubWarps = 8;
 // the root, an even count (the per-warp shared-memory regions stay 16-byte
 // aligned)
 __host__ __device__ constexpr uint32_t sub_stack_entries(uint32_t max_depth) { return (max_depth + 3u) & ~1u; }
-// per warp: the binned histograms, the plane table, then the stack (cells lo,
-// hi; meta: lane mask, depth, scratch slot; 6 rope words per entry)
-__host__ __device__ constexpr size_t sub_warp_smem(uint32_t entries) {
-    return kHist * 4 + kPlanes * 4 + (size_t)72 * entries;
+// per warp: the packed bounds (the exact search's candidates too), then the
+// stack (cells lo, hi; meta: lane mask, depth, scratch slot; 6 rope words per
+// entry)
+__host__ __device__ constexpr size_t sub_warp_smem(uint32_t entries, bool exact) {
+    return (exact ? kLaneScratch : kLaneScratch / 2) * 4 + (size_t)72 * entries;
 }
 
 // a scratch entry moved to its place: child pairs and leaf starts shifted by
@@ -2435,10 +2516,9 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
     wait_prior_grid();
     if (sub_aborted(A)) return;
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    unsigned char *wbase = sub_smem + (size_t)wib * sub_warp_smem(E);
-    uint32_t *Hw = reinterpret_cast<uint32_t *>(wbase);
-    float *Pw = reinterpret_cast<float *>(wbase + kHist * 4);
-    float4 *s_lo = reinterpret_cast<float4 *>(wbase + kHist * 4 + kPlanes * 4);
+    unsigned char *wbase = sub_smem + (size_t)wib * sub_warp_smem(E, WARP_EXACT);
+    float *Sw = reinterpret_cast<float *>(wbase);
+    float4 *s_lo = reinterpret_cast<float4 *>(wbase + sub_warp_smem(0, WARP_EXACT));
     float4 *s_hi = s_lo + E;
     uint4 *s_meta = reinterpret_cast<uint4 *>(s_hi + E);
     uint32_t *s_rope = reinterpret_cast<uint32_t *>(s_meta + E);
@@ -2467,6 +2547,8 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
             tlo = A.tb_lo[tri];
             thi = A.tb_hi[tri];
         }
+        float4 nlo = tlo, nhi = thi;
+        lane_bounds(nlo, nhi);
         uint32_t rr = lane < 12 ? A.out_ropes[6 * (size_t)rt.x + f6] : 0u;
         uint32_t mask = cnt0 >= 32 ? 0xffffffffu : ((1u << cnt0) - 1u);
         uint32_t depth = rt.w, slot = kNoSlot, sp = 0, npair = 0, nref = 0;
@@ -2476,20 +2558,8 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
             const uint32_t c = __popc(mask);
             Decision d{-1, 0.0f, 0, 0, kInf, 0};
             if (c > A.leaf_size && depth < A.max_depth) {
-                if (WARP_EXACT) {
-                    d = sah_exact_lanes(in, tlo, thi, c, lo, hi, A.ct, A.ci);
-                } else {
-                    __syncwarp();
-                    uint4 *H4 = reinterpret_cast<uint4 *>(Hw);
-                    H4[lane] = make_uint4(0, 0, 0, 0);
-                    H4[lane + 32] = make_uint4(0, 0, 0, 0);
-                    if (lane < kHist / 4 - 64) H4[lane + 64] = make_uint4(0, 0, 0, 0);
-                    node_planes_warp(Pw, lo, hi);
-                    __syncwarp();
-                    if (in) hist_ref_tab(Hw, tlo, thi, lo, hi, bin_scale(lo, hi), Pw);
-                    __syncwarp();
-                    d = sah_warp(Hw, lo, hi, c, A.ct, A.ci);
-                }
+                lanes_pack<WARP_EXACT>(Sw, in, __popc(mask & ((1u << lane) - 1u)), c, tlo, thi, nlo, nhi);
+                d = WARP_EXACT ? sah_lanes_exact(Sw, c, lo, hi, A.ct, A.ci) : sah_lanes_binned(Sw, c, lo, hi, A.ct, A.ci);
             }
             if (d.axis < 0) {
                 // a leaf: its references in the subtree's next local slots
@@ -2521,12 +2591,9 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
                 if (slot == kNoSlot) root_entry = entry;
                 else if (lane == 0) A.sc_node[slot] = entry;
                 // the partition of the levels (checkPolygonToAAPlane on the
-                // clipped bounds), as lane masks
-                const float l = c3(lo, ax), h = c3(hi, ax);
-                const float clo = mxf(c3(tlo, ax), l), chi = mnf(c3(thi, ax), h);
-                const bool flat_on = (clo == chi) && clo == p;
-                const uint32_t bm = __ballot_sync(0xffffffffu, in && (clo < p || flat_on));
-                const uint32_t am = __ballot_sync(0xffffffffu, in && (chi > p || flat_on));
+                // clipped bounds, see lane_bounds), as lane masks
+                const uint32_t bm = __ballot_sync(0xffffffffu, in && c3(nlo, ax) < p);
+                const uint32_t am = __ballot_sync(0xffffffffu, in && c3(nhi, ax) > p);
                 if (nused + 2 > kScNodeChunk) {
                     sub_close_chunks(A, nbase, nused, kNoSlot, 0);
                     nbase = sub_chunk(&A.ctr->sc_node_ctr, kScNodeChunk, A.cap_sc_nodes);
@@ -3031,7 +3098,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     k_root<<<G, 256, 0, st>>>(A, box, nt);
     const bool exact_small = A.learned || A.exact_max >= kWarpExact;
     const uint32_t sub_E = sub_stack_entries(S.p.max_depth);
-    const size_t sub_smem = kSubWarps * sub_warp_smem(sub_E);
+    const size_t sub_smem = kSubWarps * sub_warp_smem(sub_E, exact_small);
     const bool binned_only = !A.learned && A.exact_max == 0 && S.p.level_streams != 2;
     for (uint32_t L = 0; L <= S.p.max_depth; L++) {
         A.level = L;
