@@ -45,6 +45,38 @@ struct DevBuf {
 
 }  // namespace
 
+// rows whose buffers a context keeps (16,384: 139 MB with the training step's)
+constexpr uint32_t kMlpKeepRows = 16384;
+
+// buffers of the proposer's forward and training calls, kept by the context
+// from one call to the next (allocating and freeing eleven of them took longer
+// than a 4,096-row step's kernels); trim gives large ones back
+struct MlpWork {
+    DevBuf<float> X, H1, H2, H3, Z4, d1, d2, d3, d4, part, loss;
+    DevBuf<int32_t> y;
+    cudaError_t ensure_forward(size_t B) {
+        cudaError_t e = X.ensure(B * kMlpIn);
+        return e == cudaSuccess ? Z4.ensure(B * kMlpOut) : e;
+    }
+    cudaError_t ensure(size_t B) {
+        cudaError_t e = ensure_forward(B);
+        for (DevBuf<float> *h : {&H1, &H2, &H3, &d1, &d2, &d3})
+            if (e == cudaSuccess) e = h->ensure(B * kMlpHid);
+        if (e == cudaSuccess) e = d4.ensure(B * kMlpOut);
+        if (e == cudaSuccess) e = y.ensure(B);
+        if (e == cudaSuccess && grad_splits((int)std::min<size_t>(B, INT32_MAX)) > 1)
+            e = part.ensure((size_t)kMlpGradSplits * kMlpParams);
+        return e == cudaSuccess ? loss.ensure(1) : e;
+    }
+    void release() {
+        for (DevBuf<float> *b : {&X, &H1, &H2, &H3, &Z4, &d1, &d2, &d3, &d4, &part, &loss}) b->release();
+        y.release();
+    }
+    void trim() {
+        if (Z4.cap > (size_t)kMlpKeepRows * kMlpOut) release();
+    }
+};
+
 static void batch_detach(hk_batch *b);
 
 struct hk_ctx {
@@ -120,6 +152,7 @@ struct hk_ctx {
     DevBuf<uint32_t> mlp_w1p, mlp_w2p, mlp_w3p, mlp_w4p;
     DevBuf<unsigned char> mlp_tcw;   // tcgen05 weight chunks
     int mlp_step = 0;
+    MlpWork mlp_work;
     DevBuf<float> rec_X;
     DevBuf<int32_t> rec_y;
     DevBuf<uint32_t> rec_rows;
@@ -256,6 +289,7 @@ hk_status hk_destroy(hk_ctx *c) {
     c->ooc.release();
     c->mlp_params.release(); c->mlp_grads.release(); c->mlp_m.release(); c->mlp_v.release();
     c->mlp_w1p.release(); c->mlp_w2p.release(); c->mlp_w3p.release(); c->mlp_w4p.release(); c->mlp_tcw.release();
+    c->mlp_work.release();
     c->rec_X.release(); c->rec_y.release(); c->rec_rows.release();
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -1800,15 +1834,13 @@ hk_status hk_mlp_forward(hk_ctx *c, const float *X, uint32_t n, float *logits) {
     if (!c || (n && (!X || !logits))) return HK_E_ILLEGAL_INPUT;
     if (!c->learn.have_mlp) return fail(c, HK_E_STATE, "no network");
     cudaSetDevice(c->device);
-    DevBuf<float> dx, dl;
-    HK_CUDA(c, dx.ensure((size_t)n * kMlpIn));
-    HK_CUDA(c, dl.ensure((size_t)n * kMlpOut));
-    HK_CUDA(c, cudaMemcpyAsync(dx.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
-    HK_CUDA(c, mlp_infer(c->learn.mlp, dx.p, nullptr, n, dl.p, c->sm_count, c->stream, c->errw.p));
-    HK_CUDA(c, cudaMemcpyAsync(logits, dl.p, (size_t)n * kMlpOut * 4, cudaMemcpyDeviceToHost, c->stream));
+    MlpWork &W = c->mlp_work;
+    HK_CUDA(c, W.ensure_forward(n));
+    HK_CUDA(c, cudaMemcpyAsync(W.X.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
+    HK_CUDA(c, mlp_infer(c->learn.mlp, W.X.p, nullptr, n, W.Z4.p, c->sm_count, c->stream, c->errw.p));
+    HK_CUDA(c, cudaMemcpyAsync(logits, W.Z4.p, (size_t)n * kMlpOut * 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));
-    dx.release();
-    dl.release();
+    W.trim();
     uint32_t w = 0;
     HK_CUDA(c, cudaMemcpy(&w, c->errw.p, 4, cudaMemcpyDeviceToHost));
     if (w) {
@@ -1819,52 +1851,24 @@ hk_status hk_mlp_forward(hk_ctx *c, const float *X, uint32_t n, float *logits) {
 }
 
 // FP32 forward + backward of rows Xb (device) with labels yb; gradients into
-// c->mlp_grads, summed loss into *dloss (device)
-struct MlpWork {
-    DevBuf<float> H1, H2, H3, Z4, d1, d2, d3, d4, loss;
-    cudaError_t ensure(uint32_t B) {
-        cudaError_t e;
-        if ((e = H1.ensure((size_t)B * kMlpHid)) || (e = H2.ensure((size_t)B * kMlpHid)) ||
-            (e = H3.ensure((size_t)B * kMlpHid)) || (e = Z4.ensure((size_t)B * kMlpOut)) ||
-            (e = d1.ensure((size_t)B * kMlpHid)) || (e = d2.ensure((size_t)B * kMlpHid)) ||
-            (e = d3.ensure((size_t)B * kMlpHid)) || (e = d4.ensure((size_t)B * kMlpOut)) || (e = loss.ensure(1)))
-            return e;
-        return cudaSuccess;
-    }
-    void release() {
-        H1.release(); H2.release(); H3.release(); Z4.release();
-        d1.release(); d2.release(); d3.release(); d4.release(); loss.release();
-    }
-};
-
+// c->mlp_grads, summed loss into *W.loss (device)
 static hk_status mlp_fwd_bwd(hk_ctx *c, MlpWork &W, const float *Xb, const int32_t *yb, int B) {
     const float *P = c->mlp_params.p;
-    float *G = c->mlp_grads.p;
     cudaStream_t s = c->stream;
     const int I = kMlpIn, Hd = kMlpHid, O = kMlpOut;
-    HK_CUDA(c, sgemm(false, false, Xb, P + kOffW1, W.H1.p, P + kOffB1, B, Hd, I, I, Hd, Hd, true, false, s));
-    HK_CUDA(c, sgemm(false, false, W.H1.p, P + kOffW2, W.H2.p, P + kOffB2, B, Hd, Hd, Hd, Hd, Hd, true, false, s));
-    HK_CUDA(c, sgemm(false, false, W.H2.p, P + kOffW3, W.H3.p, P + kOffB3, B, Hd, Hd, Hd, Hd, Hd, true, false, s));
-    HK_CUDA(c, sgemm(false, false, W.H3.p, P + kOffW4, W.Z4.p, P + kOffB4, B, O, Hd, Hd, O, O, false, false, s));
+    HK_CUDA(c, gemm_layer(Xb, P + kOffW1, W.H1.p, P + kOffB1, B, I, Hd, true, s));
+    HK_CUDA(c, gemm_layer(W.H1.p, P + kOffW2, W.H2.p, P + kOffB2, B, Hd, Hd, true, s));
+    HK_CUDA(c, gemm_layer(W.H2.p, P + kOffW3, W.H3.p, P + kOffB3, B, Hd, Hd, true, s));
+    HK_CUDA(c, gemm_layer(W.H3.p, P + kOffW4, W.Z4.p, P + kOffB4, B, Hd, O, false, s));
     HK_CUDA(c, softmax_xent(W.Z4.p, yb, B, W.d4.p, W.loss.p, s));
-    // layer 4
-    HK_CUDA(c, sgemm(true, false, W.H3.p, W.d4.p, G + kOffW4, nullptr, Hd, O, B, Hd, O, O, false, false, s));
-    HK_CUDA(c, colsum(W.d4.p, B, O, G + kOffB4, s));
-    HK_CUDA(c, sgemm(false, true, W.d4.p, P + kOffW4, W.d3.p, nullptr, B, Hd, O, O, O, Hd, false, false, s));
-    HK_CUDA(c, relu_back(W.d3.p, W.H3.p, (size_t)B * Hd, s));
-    // layer 3
-    HK_CUDA(c, sgemm(true, false, W.H2.p, W.d3.p, G + kOffW3, nullptr, Hd, Hd, B, Hd, Hd, Hd, false, false, s));
-    HK_CUDA(c, colsum(W.d3.p, B, Hd, G + kOffB3, s));
-    HK_CUDA(c, sgemm(false, true, W.d3.p, P + kOffW3, W.d2.p, nullptr, B, Hd, Hd, Hd, Hd, Hd, false, false, s));
-    HK_CUDA(c, relu_back(W.d2.p, W.H2.p, (size_t)B * Hd, s));
-    // layer 2
-    HK_CUDA(c, sgemm(true, false, W.H1.p, W.d2.p, G + kOffW2, nullptr, Hd, Hd, B, Hd, Hd, Hd, false, false, s));
-    HK_CUDA(c, colsum(W.d2.p, B, Hd, G + kOffB2, s));
-    HK_CUDA(c, sgemm(false, true, W.d2.p, P + kOffW2, W.d1.p, nullptr, B, Hd, Hd, Hd, Hd, Hd, false, false, s));
-    HK_CUDA(c, relu_back(W.d1.p, W.H1.p, (size_t)B * Hd, s));
-    // layer 1
-    HK_CUDA(c, sgemm(true, false, Xb, W.d1.p, G + kOffW1, nullptr, I, Hd, B, I, Hd, Hd, false, false, s));
-    HK_CUDA(c, colsum(W.d1.p, B, Hd, G + kOffB1, s));
+    HK_CUDA(c, gemm_layer_back(W.d4.p, P + kOffW4, W.d3.p, W.H3.p, B, Hd, O, s));
+    HK_CUDA(c, gemm_layer_back(W.d3.p, P + kOffW3, W.d2.p, W.H2.p, B, Hd, Hd, s));
+    HK_CUDA(c, gemm_layer_back(W.d2.p, P + kOffW2, W.d1.p, W.H1.p, B, Hd, Hd, s));
+    const MlpGradArgs a{{{Xb, W.d1.p, I, Hd, kOffW1},
+                         {W.H1.p, W.d2.p, Hd, Hd, kOffW2},
+                         {W.H2.p, W.d3.p, Hd, Hd, kOffW3},
+                         {W.H3.p, W.d4.p, Hd, O, kOffW4}}};
+    HK_CUDA(c, mlp_grad_weights(a, B, W.part.p, c->mlp_grads.p, s));
     return HK_OK;
 }
 
@@ -1874,25 +1878,19 @@ hk_status hk_mlp_grad(hk_ctx *c, const float *X, const int32_t *y, uint32_t n, f
     for (uint32_t i = 0; i < n; i++)
         if (y[i] < 0 || y[i] >= kMlpOut) return fail(c, HK_E_ILLEGAL_INPUT, "label out of range");
     cudaSetDevice(c->device);
-    DevBuf<float> dx;
-    DevBuf<int32_t> dy;
-    MlpWork W;
-    HK_CUDA(c, dx.ensure((size_t)n * kMlpIn));
-    HK_CUDA(c, dy.ensure(n));
+    MlpWork &W = c->mlp_work;
     HK_CUDA(c, W.ensure(n));
-    HK_CUDA(c, cudaMemcpyAsync(dx.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
-    HK_CUDA(c, cudaMemcpyAsync(dy.p, y, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
+    HK_CUDA(c, cudaMemcpyAsync(W.X.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
+    HK_CUDA(c, cudaMemcpyAsync(W.y.p, y, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
     HK_CUDA(c, cudaMemsetAsync(W.loss.p, 0, 4, c->stream));
-    hk_status st = mlp_fwd_bwd(c, W, dx.p, dy.p, (int)n);
+    hk_status st = mlp_fwd_bwd(c, W, W.X.p, W.y.p, (int)n);
     if (st != HK_OK) return st;
     float ls = 0;
     HK_CUDA(c, cudaMemcpyAsync(grads, c->mlp_grads.p, kMlpParams * 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaMemcpyAsync(&ls, W.loss.p, 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (loss) *loss = ls / (float)n;
-    dx.release();
-    dy.release();
-    W.release();
+    W.trim();
     return HK_OK;
 }
 
@@ -1952,12 +1950,8 @@ hk_status hk_mlp_train(hk_ctx *c, uint32_t epochs, uint32_t batch, float lr, uin
     if (st != HK_OK) return st;
     if (rows < batch) return fail(c, HK_E_STATE, "fewer recorded rows than one batch");
     DevBuf<uint32_t> perm;
-    DevBuf<float> Xb;
-    DevBuf<int32_t> yb;
-    MlpWork W;
+    MlpWork &W = c->mlp_work;
     HK_CUDA(c, perm.ensure(rows));
-    HK_CUDA(c, Xb.ensure((size_t)batch * kMlpIn));
-    HK_CUDA(c, yb.ensure(batch));
     HK_CUDA(c, W.ensure(batch));
     std::vector<uint32_t> idx(rows);
     std::mt19937_64 rng(seed);
@@ -1968,9 +1962,9 @@ hk_status hk_mlp_train(hk_ctx *c, uint32_t epochs, uint32_t batch, float lr, uin
         HK_CUDA(c, cudaMemsetAsync(W.loss.p, 0, 4, c->stream));
         uint32_t nb = rows / batch;
         for (uint32_t b = 0; b < nb; b++) {
-            HK_CUDA(c, gather_rows(c->rec_X.p, c->rec_y.p, perm.p + (size_t)b * batch, (int)batch, Xb.p, yb.p,
+            HK_CUDA(c, gather_rows(c->rec_X.p, c->rec_y.p, perm.p + (size_t)b * batch, (int)batch, W.X.p, W.y.p,
                                    c->stream));
-            st = mlp_fwd_bwd(c, W, Xb.p, yb.p, (int)batch);
+            st = mlp_fwd_bwd(c, W, W.X.p, W.y.p, (int)batch);
             if (st != HK_OK) return st;
             c->mlp_step++;
             HK_CUDA(c, adam(c->mlp_params.p, c->mlp_grads.p, c->mlp_m.p, c->mlp_v.p, kMlpParams, lr, c->mlp_step,
@@ -1982,9 +1976,7 @@ hk_status hk_mlp_train(hk_ctx *c, uint32_t epochs, uint32_t batch, float lr, uin
         if (epoch_loss) epoch_loss[e] = ls / (float)(nb * batch);
     }
     perm.release();
-    Xb.release();
-    yb.release();
-    W.release();
+    W.trim();
     return mlp_pack(c);
 }
 

@@ -4,9 +4,9 @@
 // * Inference: BF16 weights and activations on the tensor cores, FP32
 //   accumulate, 64-row tiles (hk_mlp_tile.cuh, shared with the builder);
 //   weights are packed once into the per-lane B-fragment order.
-// * Training: FP32 master weights; hand-written tiled SGEMM (with transposed
-//   operands), bias / ReLU epilogues, softmax cross-entropy, ReLU backward,
-//   column sums and Adam. Gradients are checked against a CPU FP32 reference.
+// * Training: FP32 master weights; hand-written tiled FP32 GEMMs with bias,
+//   ReLU and ReLU-backward epilogues, weight and bias gradients of all layers
+//   in one launch, softmax cross-entropy and Adam. Gradients are checked against a CPU FP32 reference.
 #include <cmath>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -22,69 +22,194 @@
 namespace hk {
 
 // ---------------------------------------------------------------------------
-// tiled FP32 GEMM: C[M x N] = op(A) op(B) (+ bias, ReLU); row-major storage
-//   op(A)(m, k) = TA ? A[k * lda + m] : A[m * lda + k]
-//   op(B)(k, n) = TB ? B[n * ldb + k] : B[k * ldb + n]
+// FP32 GEMMs of the training step, one 64 x 64 tile of C per 256-thread CTA,
+// 4 x 4 outputs per thread, K in steps of 16 through two shared-memory buffers
+// (the next step's tiles are loaded into registers while this one is
+// multiplied). Every operand's leading dimension and every row or column range
+// along which it is contiguous is a multiple of 4 (the network's 200, 256 and
+// 96), so all global loads are 16 bytes wide.
+//   A_COL: A(m, k) = A[k * lda + m], else A[m * lda + k]
+//   B_COL: B(k, n) = B[n * ldb + k], else B[k * ldb + n]
 // ---------------------------------------------------------------------------
-constexpr int GT = 64, GK = 16;
+constexpr int GT = 64, GK = 16, GS = GT + 4;
+// smallest K range of one CTA of the weight gradients
+constexpr int kGradSplitRows = 128;
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_sgemm(const float *__restrict__ A, const float *__restrict__ B,
-                                               float *__restrict__ C, const float *__restrict__ bias, int M, int N,
-                                               int K, int lda, int ldb, int ldc, int relu, int accumulate) {
-    __shared__ float As[GK][GT + 1];
-    __shared__ float Bs[GK][GT + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int i = threadIdx.x; i < GK * GT; i += 256) {
-            int kk = i / GT, mm = i % GT;
-            int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? (TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]) : 0.0f;
-            int n = n0 + mm;
-            Bs[kk][mm] = (n < N && k < K) ? (TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n]) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                a[i] = As[kk][ty * 4 + i];
-                b[i] = Bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            float v = acc[i][j];
-            if (accumulate) v += C[(size_t)m * ldc + n];
-            if (bias) v += bias[n];
-            if (relu) v = v > 0.0f ? v : 0.0f;
-            C[(size_t)m * ldc + n] = v;
-        }
+struct GemmSmem {
+    float As[2][GK][GS];
+    float Bs[2][GK][GS];
+};
+
+// a 16 x 64 tile (k x m) from a matrix contiguous along m (COL) or along k:
+// this thread's 4 values, zero past the ends
+template <bool COL>
+__device__ __forceinline__ float4 gemm_load(const float *__restrict__ A, int ld, int m0, int M, int k0, int K) {
+    const int t = threadIdx.x;
+    const int k = COL ? k0 + t / 16 : k0 + (t % 4) * 4, m = COL ? m0 + (t % 16) * 4 : m0 + t / 4;
+    if (k >= K || m >= M) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return *reinterpret_cast<const float4 *>(COL ? A + (size_t)k * ld + m : A + (size_t)m * ld + k);
+}
+template <bool COL>
+__device__ __forceinline__ void gemm_store(float (*S)[GS], float4 v) {
+    const int t = threadIdx.x;
+    if (COL) {
+        *reinterpret_cast<float4 *>(&S[t / 16][(t % 16) * 4]) = v;
+    } else {
+        const int k = (t % 4) * 4, m = t / 4;
+        S[k][m] = v.x;
+        S[k + 1][m] = v.y;
+        S[k + 2][m] = v.z;
+        S[k + 3][m] = v.w;
     }
 }
 
-cudaError_t sgemm(bool ta, bool tb, const float *A, const float *B, float *C, const float *bias, int M, int N, int K,
-                  int lda, int ldb, int ldc, bool relu, bool accumulate, cudaStream_t s) {
-    dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
-    if (!ta && !tb) k_sgemm<false, false><<<grid, 256, 0, s>>>(A, B, C, bias, M, N, K, lda, ldb, ldc, relu, accumulate);
-    else if (ta && !tb) k_sgemm<true, false><<<grid, 256, 0, s>>>(A, B, C, bias, M, N, K, lda, ldb, ldc, relu, accumulate);
-    else if (!ta && tb) k_sgemm<false, true><<<grid, 256, 0, s>>>(A, B, C, bias, M, N, K, lda, ldb, ldc, relu, accumulate);
-    else k_sgemm<true, true><<<grid, 256, 0, s>>>(A, B, C, bias, M, N, K, lda, ldb, ldc, relu, accumulate);
+// acc += the tile's product over k in [kb, ke); colsum: thread t < 64 also adds
+// column t of B
+template <bool A_COL, bool B_COL, bool COLSUM>
+__device__ __forceinline__ void gemm_tile(GemmSmem &S, const float *__restrict__ A, int lda, int m0, int M,
+                                          const float *__restrict__ B, int ldb, int n0, int N, int kb, int ke,
+                                          float (&acc)[4][4], float &colsum) {
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    float4 a4 = gemm_load<A_COL>(A, lda, m0, M, kb, ke), b4 = gemm_load<!B_COL>(B, ldb, n0, N, kb, ke);
+    int buf = 0;
+    for (int k0 = kb; k0 < ke; k0 += GK, buf ^= 1) {
+        gemm_store<A_COL>(S.As[buf], a4);
+        gemm_store<!B_COL>(S.Bs[buf], b4);
+        __syncthreads();
+        if (k0 + GK < ke) {
+            a4 = gemm_load<A_COL>(A, lda, m0, M, k0 + GK, ke);
+            b4 = gemm_load<!B_COL>(B, ldb, n0, N, k0 + GK, ke);
+        }
+#pragma unroll
+        for (int kk = 0; kk < GK; kk++) {
+            const float4 a = *reinterpret_cast<const float4 *>(&S.As[buf][kk][ty * 4]);
+            const float4 b = *reinterpret_cast<const float4 *>(&S.Bs[buf][kk][tx * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (COLSUM && threadIdx.x < GT)
+#pragma unroll
+            for (int kk = 0; kk < GK; kk++) colsum += S.Bs[buf][kk][threadIdx.x];
+    }
+}
+
+// C = A B^(T) (+ bias, ReLU); mask (with B_COL: the input gradient of a layer
+// behind a ReLU): C = 0 where mask, the ReLU's output, is not positive
+template <bool B_COL>
+__global__ void __launch_bounds__(256) k_gemm(const float *__restrict__ A, const float *__restrict__ B,
+                                              float *__restrict__ C, const float *__restrict__ bias,
+                                              const float *__restrict__ mask, int M, int N, int K, int relu) {
+    __shared__ __align__(16) GemmSmem S;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
+    float acc[4][4] = {}, cs = 0.0f;
+    gemm_tile<false, B_COL, false>(S, A, K, m0, M, B, B_COL ? K : N, n0, N, 0, K, acc, cs);
+    const int n = n0 + tx * 4;
+    if (n >= N) return;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int m = m0 + ty * 4 + i;
+        if (m >= M) continue;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[j] = acc[i][j];
+            if (bias) v[j] += bias[n + j];
+            if (relu) v[j] = v[j] > 0.0f ? v[j] : 0.0f;
+        }
+        if (mask) {
+            const float4 h = *reinterpret_cast<const float4 *>(mask + (size_t)m * N + n);
+            v[0] = h.x > 0.0f ? v[0] : 0.0f;
+            v[1] = h.y > 0.0f ? v[1] : 0.0f;
+            v[2] = h.z > 0.0f ? v[2] : 0.0f;
+            v[3] = h.w > 0.0f ? v[3] : 0.0f;
+        }
+        *reinterpret_cast<float4 *>(C + (size_t)m * N + n) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+cudaError_t gemm_layer(const float *X, const float *W, float *Y, const float *bias, int rows, int in, int out,
+                       bool relu, cudaStream_t s) {
+    const dim3 grid((out + GT - 1) / GT, (rows + GT - 1) / GT);
+    k_gemm<false><<<grid, 256, 0, s>>>(X, W, Y, bias, nullptr, rows, out, in, relu);
+    return cudaGetLastError();
+}
+
+cudaError_t gemm_layer_back(const float *dY, const float *W, float *dX, const float *X, int rows, int in, int out,
+                            cudaStream_t s) {
+    const dim3 grid((in + GT - 1) / GT, (rows + GT - 1) / GT);
+    k_gemm<true><<<grid, 256, 0, s>>>(dY, W, dX, nullptr, X, rows, in, out, 0);
+    return cudaGetLastError();
+}
+
+// Weight and bias gradients of all four layers in one launch: dW = X^T dY, db =
+// the column sums of dY (added up by the CTAs of each column's first tile from
+// the tiles they load anyway). A layer has at most 16 tiles, so the rows are
+// split over blockIdx.y, each split into its own copy of the parameter vector
+// (out + split * kMlpParams), which k_grad_sum adds up in order. One CTA per
+// tile and no split kept 16 of 148 SMs busy: 4,096 rows took 2,963 us and the
+// four column sums 943 us.
+__global__ void __launch_bounds__(256) k_grad_w(MlpGradArgs a, int rows, int per, float *__restrict__ out) {
+    __shared__ __align__(16) GemmSmem S;
+    int tile = blockIdx.x, l = 0;
+    int nt = (a.layer[0].out + GT - 1) / GT, mt = (a.layer[0].in + GT - 1) / GT;
+    while (tile >= nt * mt) {
+        tile -= nt * mt;
+        l++;
+        nt = (a.layer[l].out + GT - 1) / GT;
+        mt = (a.layer[l].in + GT - 1) / GT;
+    }
+    const MlpGradArgs::Layer L = a.layer[l];
+    const int m0 = (tile / nt) * GT, n0 = (tile % nt) * GT;
+    const int kb = blockIdx.y * per, ke = min(rows, kb + per);
+    float acc[4][4] = {}, cs = 0.0f;
+    if (m0 == 0) gemm_tile<true, false, true>(S, L.X, L.in, m0, L.in, L.dY, L.out, n0, L.out, kb, ke, acc, cs);
+    else gemm_tile<true, false, false>(S, L.X, L.in, m0, L.in, L.dY, L.out, n0, L.out, kb, ke, acc, cs);
+    float *W = out + (size_t)blockIdx.y * kMlpParams + L.off;
+    const int n = n0 + (threadIdx.x % 16) * 4;
+    if (n < L.out) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int m = m0 + (threadIdx.x / 16) * 4 + i;
+            if (m < L.in)
+                *reinterpret_cast<float4 *>(W + (size_t)m * L.out + n) =
+                    make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+    }
+    if (m0 == 0 && threadIdx.x < GT && n0 + (int)threadIdx.x < L.out)
+        W[(size_t)L.in * L.out + n0 + threadIdx.x] = cs;
+}
+
+__global__ void k_grad_sum(const float4 *__restrict__ part, int splits, float4 *__restrict__ G) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (int)(kMlpParams / 4)) return;
+    float4 s = part[i];
+    for (int k = 1; k < splits; k++) {
+        const float4 v = part[(size_t)k * (kMlpParams / 4) + i];
+        s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+    }
+    G[i] = s;
+}
+static_assert(kMlpParams % 4 == 0 && kOffW2 % 4 == 0 && kOffW3 % 4 == 0 && kOffW4 % 4 == 0,
+              "16-byte loads of the parameters");
+
+int grad_splits(int rows) {
+    // 56 tiles x 16 splits are six CTAs per SM
+    return std::max(1, std::min(kMlpGradSplits, rows / kGradSplitRows));
+}
+
+cudaError_t mlp_grad_weights(const MlpGradArgs &a, int rows, float *part, float *G, cudaStream_t s) {
+    const int splits = grad_splits(rows);
+    const int per = ((rows + splits - 1) / splits + GK - 1) / GK * GK;
+    int tiles = 0;
+    for (const auto &l : a.layer) tiles += ((l.in + GT - 1) / GT) * ((l.out + GT - 1) / GT);
+    k_grad_w<<<dim3(tiles, splits), 256, 0, s>>>(a, rows, per, splits > 1 ? part : G);
+    if (splits > 1)
+        k_grad_sum<<<(int)(kMlpParams / 4 + 127) / 128, 128, 0, s>>>(reinterpret_cast<const float4 *>(part), splits,
+                                                                    reinterpret_cast<float4 *>(G));
     return cudaGetLastError();
 }
 
@@ -118,19 +243,6 @@ __global__ void k_softmax_xent(const float *__restrict__ Z, const int32_t *__res
     }
 }
 
-__global__ void k_relu_back(float *__restrict__ dH, const float *__restrict__ H, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (!(H[i] > 0.0f)) dH[i] = 0.0f;
-}
-
-__global__ void k_colsum(const float *__restrict__ dZ, int rows, int cols, float *__restrict__ db) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (int r = 0; r < rows; r++) s += dZ[(size_t)r * cols + c];
-    db[c] = s;
-}
-
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                        size_t n, float lr, float b1, float b2, float eps, float c1, float c2) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -145,14 +257,6 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
 
 cudaError_t softmax_xent(const float *Z, const int32_t *y, int rows, float *dZ, float *loss, cudaStream_t s) {
     if (rows) k_softmax_xent<<<(rows * 32 + 255) / 256, 256, 0, s>>>(Z, y, rows, dZ, loss);
-    return cudaGetLastError();
-}
-cudaError_t relu_back(float *dH, const float *H, size_t n, cudaStream_t s) {
-    if (n) k_relu_back<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(dH, H, n);
-    return cudaGetLastError();
-}
-cudaError_t colsum(const float *dZ, int rows, int cols, float *db, cudaStream_t s) {
-    k_colsum<<<(cols + 127) / 128, 128, 0, s>>>(dZ, rows, cols, db);
     return cudaGetLastError();
 }
 cudaError_t adam(float *p, const float *g, float *m, float *v, size_t n, float lr, int step, cudaStream_t s) {

@@ -29,11 +29,26 @@ struct MlpDevice {
     const unsigned char *tcw;                // tcgen05 weight chunks (pack_umma)
 };
 
-cudaError_t sgemm(bool ta, bool tb, const float *A, const float *B, float *C, const float *bias, int M, int N, int K,
-                  int lda, int ldb, int ldc, bool relu, bool accumulate, cudaStream_t s);
+// Y = X W + bias (ReLU), X rows x in, W in x out
+cudaError_t gemm_layer(const float *X, const float *W, float *Y, const float *bias, int rows, int in, int out,
+                       bool relu, cudaStream_t s);
+// dX = dY W^T where X (the layer's input, a ReLU's output) is positive, else 0
+cudaError_t gemm_layer_back(const float *dY, const float *W, float *dX, const float *X, int rows, int in, int out,
+                            cudaStream_t s);
+// weight and bias gradients of the four layers into G (the flat parameter
+// order); part: kMlpGradSplits x kMlpParams floats (unused when
+// grad_splits(rows) is 1)
+constexpr int kMlpGradSplits = 16;
+struct MlpGradArgs {
+    struct Layer {
+        const float *X, *dY;   // rows x in, rows x out
+        int in, out;
+        size_t off;            // of the layer's weights in the parameter vector
+    } layer[4];
+};
+int grad_splits(int rows);
+cudaError_t mlp_grad_weights(const MlpGradArgs &a, int rows, float *part, float *G, cudaStream_t s);
 cudaError_t softmax_xent(const float *Z, const int32_t *y, int rows, float *dZ, float *loss, cudaStream_t s);
-cudaError_t relu_back(float *dH, const float *H, size_t n, cudaStream_t s);
-cudaError_t colsum(const float *dZ, int rows, int cols, float *db, cudaStream_t s);
 cudaError_t adam(float *p, const float *g, float *m, float *v, size_t n, float lr, int step, cudaStream_t s);
 cudaError_t pack_b(const float *W, int K, int N, uint32_t *out, cudaStream_t s);
 // all four layers (flat FP32 parameters P) into the tcgen05 chunk layout
