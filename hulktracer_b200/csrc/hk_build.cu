@@ -598,9 +598,16 @@ __device__ __forceinline__ bool decidable(const LevelArgs &A, uint32_t cnt) {
 
 // classes of a splittable node by its reference count: small (one warp,
 // k_small), medium (exact SAH, one CTA, when exact_max reaches it) and large
-// (chunked binned histograms, or the proposer)
-__device__ __forceinline__ bool is_medium(const LevelArgs &A, uint32_t c) {
+// (chunked binned histograms, or the proposer). is_exact: above a warp's 32
+// references and within exact_max
+__device__ __forceinline__ bool is_exact(const LevelArgs &A, uint32_t c) {
     return A.exact_max >= kWarpExact && c > kWarpExact && c <= A.exact_max;
+}
+// (nodes of up to kExactWarp references are one warp's work too, unless
+// training rows are recorded, which the CTA does)
+constexpr uint32_t kExactWarp = 128;
+__device__ __forceinline__ bool is_medium(const LevelArgs &A, uint32_t c) {
+    return is_exact(A, c) && (c > kExactWarp || A.record);
 }
 // learned mode: a proposer row (33..1024 references)
 __device__ __forceinline__ bool is_learn(const LevelArgs &A, uint32_t c) {
@@ -609,7 +616,7 @@ __device__ __forceinline__ bool is_learn(const LevelArgs &A, uint32_t c) {
 // large: k_hist's chunked histograms (in learned mode the proposer rows too, so
 // that the proposer's chain needs nothing from k_small)
 __device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c) {
-    return (c > kSmall || is_learn(A, c)) && !is_medium(A, c);
+    return (c > kSmall || is_learn(A, c)) && !is_exact(A, c);
 }
 // a decidable node of 2..A.defer references roots a deferred subtree
 constexpr uint32_t kDeferMax = 32;   // one reference per lane
@@ -825,10 +832,10 @@ __device__ __forceinline__ void lanes_pack(float *S, bool in, uint32_t rank, uin
     __syncwarp();
 }
 
-// cost of the plane pk on axis a of a node with extents ext, surface Anode
-__device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float h, float4 ext, float Anode,
-                                            uint32_t nb, uint32_t na, float ct, float ci) {
-    const float db = __fsub_rn(pk, l), da = __fsub_rn(h, pk);
+// cost of nb references in a below cell that is db long on axis a and na in an
+// above cell that is da long, of a node with extents ext and surface Anode
+__device__ __forceinline__ float bounds_cost(uint32_t a, float db, float da, float4 ext, float Anode, uint32_t nb,
+                                             uint32_t na, float ct, float ci) {
     const float bx = a == 0 ? db : ext.x, by = a == 1 ? db : ext.y, bz = a == 2 ? db : ext.z;
     const float ax = a == 0 ? da : ext.x, ay = a == 1 ? da : ext.y, az = a == 2 ? da : ext.z;
     const float sb =
@@ -837,6 +844,11 @@ __device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float
         __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(ax, ay), __fmul_rn(az, ay)), __fmul_rn(ax, az)));
     return __fadd_rn(
         ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
+}
+// ... split at the plane pk
+__device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float h, float4 ext, float Anode,
+                                            uint32_t nb, uint32_t na, float ct, float ci) {
+    return bounds_cost(a, __fsub_rn(pk, l), __fsub_rn(h, pk), ext, Anode, nb, na, ct, ci);
 }
 
 // the binned SAH of a packed node: lane k counts and costs plane k of every
@@ -892,6 +904,18 @@ __device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c,
     return best;
 }
 
+// the lane of the warp with the least (cost, axis, plane); costs are +0 ..
+// +inf, so their bits order as they do
+__device__ __forceinline__ uint32_t warp_argmin(float cost, uint32_t ax, float pk) {
+    const uint32_t mbits = __reduce_min_sync(0xffffffffu, __float_as_uint(cost));
+    bool win = __float_as_uint(cost) == mbits;
+    const uint32_t bax = __reduce_min_sync(0xffffffffu, win ? ax : 0xffffffffu);
+    win = win && ax == bax;
+    const uint32_t pb = __float_as_uint(pk), po = (pb & 0x80000000u) ? ~pb : (pb | 0x80000000u);
+    const uint32_t bpo = __reduce_min_sync(0xffffffffu, win ? po : 0xffffffffu);
+    return (__ffs(__ballot_sync(0xffffffffu, win && po == bpo)) - 1u) & 31u;
+}
+
 // the exact SAH of a packed node: candidate q of 6 c (axis, side, reference)
 // is taken by lane q % 32, which counts the references below and above it;
 // two sorts per axis and a binary search per candidate and list cost four
@@ -927,20 +951,14 @@ __device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, 
             m_n = nb | (na << 16);
         }
     }
-    // the least (cost, axis, plane); equal keys are the same plane with the
-    // same counts. Costs are +0 .. +inf, so their bits order as they do.
-    const uint32_t mbits = __reduce_min_sync(0xffffffffu, __float_as_uint(mc));
-    bool win = __float_as_uint(mc) == mbits;
-    const uint32_t bax = __reduce_min_sync(0xffffffffu, win ? m_ax : 3u);
-    win = win && m_ax == bax;
-    const uint32_t pb = __float_as_uint(m_pk), po = (pb & 0x80000000u) ? ~pb : (pb | 0x80000000u);
-    const uint32_t bpo = __reduce_min_sync(0xffffffffu, win ? po : 0xffffffffu);
-    const uint32_t src = __ffs(__ballot_sync(0xffffffffu, win && po == bpo)) - 1u;
-    const float bc = __uint_as_float(mbits);
+    // (equal keys are the same plane with the same counts)
+    const uint32_t src = warp_argmin(mc, m_ax, m_pk);
+    mc = __shfl_sync(0xffffffffu, mc, src);
+    m_ax = __shfl_sync(0xffffffffu, m_ax, src);
+    m_pk = __shfl_sync(0xffffffffu, m_pk, src);
+    m_n = __shfl_sync(0xffffffffu, m_n, src);
     Decision best{-1, 0.0f, 0, 0, kInf, 0};
-    const float p = __shfl_sync(0xffffffffu, m_pk, src & 31u);
-    const uint32_t n = __shfl_sync(0xffffffffu, m_n, src & 31u);
-    if (bc < kInf) best = Decision{(int)bax, p, n & 0xffffu, n >> 16, bc, 0};
+    if (mc < kInf) best = Decision{(int)m_ax, m_pk, m_n & 0xffffu, m_n >> 16, mc, 0};
     if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)c))) best.axis = -1;
     return best;
 }
@@ -981,89 +999,227 @@ __device__ __forceinline__ uint32_t upper_bound_f(const float *v, uint32_t n, fl
     return lo;
 }
 
-// Exact SAH of a medium node (33..1024 references), one CTA: the same
-// algorithm with the three sorts (bitonic, shared memory) and the candidates
-// spread over the CTA, then a CTA argmin over (cost, axis, plane).
-struct ExactCtaSmem {
-    float lo[kChunk], hi[kChunk], fl[kChunk];
-    uint32_t nflat;
-    float w_cost[8], w_pk[8];
-    uint32_t w_ax[8], w_nb[8], w_na[8], w_key[8];
+// Exact SAH of a node of more than 32 references by a group of NT threads (a
+// warp: up to 128 references; a CTA of 256: up to 1024), without sorting.
+//   1. every clipped bound strictly inside the node goes to its bin's bucket
+//      (32 bins per axis, a counting sort on the bins); bounds at the node's
+//      sides only count;
+//   2. a bin's candidates cannot cost less than its lower bound: the count
+//      below and the below surface at the bin's lower edge, the count above
+//      and the above surface at its upper edge. Every operation of the cost
+//      is monotonic in these four, rounded or not, so the bound holds for the
+//      rounded costs exactly;
+//   3. the candidates of each axis's bin of least bound are costed (each
+//      counts the bounds of its own bin's two buckets), then those of every
+//      bin whose bound is not above the cost found.
+// A 200k-triangle frame's 25,000 such nodes cost two rounds of few candidates
+// each instead of three sorts and 6 binary searches per reference: 2,358 us of
+// bitonic sorts (one CTA per node) before.
+// A bound flat on its axis is kept one step outside its value (lane_bounds)
+// and flagged; a flat bound equal to a bin's edge lies in another bin's bucket
+// and is added from `on`.
+template <uint32_t NT>
+struct ExactSmem {
+    static constexpr uint32_t kCap = 4 * NT;
+    // bin counts, then the buckets' cursors ([axis * 64 + side * 32 + bin]),
+    // then the candidates of the selected bins before each bin (97)
+    uint32_t H[196];
+    uint32_t S[6 * 33];        // per axis and side: bounds in the bins before
+    uint32_t on[3 * 32];       // flat bounds on the bin's lower plane
+    float P[3 * 32];           // planes
+    uint32_t clip[6];          // bounds at (or past) the node's side
+    uint32_t best;             // least cost so far (bits)
+    uint32_t flat[6 * kCap / 32];
+    float B[6 * kCap];         // buckets
+    uint32_t w_cost[NT / 32], w_ax[NT / 32], w_nb[NT / 32], w_na[NT / 32];
+    float w_pk[NT / 32];
 };
 
-__device__ Decision sah_exact_cta(const LevelArgs &A, uint4 info, float4 blo, float4 bhi, float ct, float ci,
-                                  ExactCtaSmem &S) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+template <uint32_t NT>
+__device__ __forceinline__ void group_sync() {
+    if (NT == 32) __syncwarp();
+    else __syncthreads();
+}
+
+__device__ __forceinline__ bool refine_better(float c, uint32_t a, float p, float bc, uint32_t ba, float bp) {
+    return c < bc || (c == bc && (a < ba || (a == ba && p < bp)));
+}
+
+template <uint32_t NT>
+__device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, float4 bhi, ExactSmem<NT> &S) {
+    constexpr uint32_t kCap = ExactSmem<NT>::kCap;
+    const uint32_t lane = threadIdx.x & 31u, tid = NT == 32 ? lane : threadIdx.x;
     const uint32_t cnt = info.y;
-    uint32_t n2 = 1;
-    while (n2 < cnt) n2 <<= 1;
     const float Anode = surf(blo, bhi);
+    const float4 ext = make_float4(__fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), 0.0f);
+    group_sync<NT>();   // the previous node's readers are done
+    for (uint32_t i = tid; i < 192; i += NT) S.H[i] = 0;
+    for (uint32_t i = tid; i < 96; i += NT) {
+        const uint32_t a = i >> 5;
+        S.on[i] = 0;
+        S.P[i] = plane_k(c3(blo, a), c3(ext, a), i & 31u);
+    }
+    for (uint32_t i = tid; i < 6 * kCap / 32; i += NT) S.flat[i] = 0;
+    if (tid < 6) S.clip[tid] = 0;
+    if (tid == 6) S.best = __float_as_uint(kInf);
+    // the thread's references, all loads issued together
+    float4 tlo[4], thi[4];
+    uint32_t tri[4], bins[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t r = tid + NT * k;
+        tri[k] = r < cnt ? A.refs()[info.x + r] : 0xffffffffu;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (tri[k] != 0xffffffffu) {
+            tlo[k] = A.tb_lo[tri[k]];
+            thi[k] = A.tb_hi[tri[k]];
+        }
+    group_sync<NT>();
+    // 1. bins (5 bits each, lo then hi per axis), counts
+    const float4 inv3 = bin_scale(blo, bhi);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (NT * k >= cnt) break;   // uniform
+        const bool have = tri[k] != 0xffffffffu;
+        uint32_t w = 0;
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            const float l = c3(blo, a), h = c3(bhi, a);
+            if (!(c3(ext, a) > 0.0f)) continue;   // uniform
+            const float lo = have ? mxf(c3(tlo[k], a), l) : kInf, hi = have ? mnf(c3(thi[k], a), h) : -kInf;
+            int b, c;
+            bool on;
+            bin_interval_tab(lo, hi, l, c3(inv3, a), S.P + a * 32, b, c, on);
+            w |= ((uint32_t)b << (10 * a)) | ((uint32_t)c << (10 * a + 5));
+            const uint32_t ml = __ballot_sync(0xffffffffu, have && !(lo > l));
+            const uint32_t mh = __ballot_sync(0xffffffffu, have && !(hi < h));
+            if (lane == 0) {
+                if (ml) atomicAdd(&S.clip[2 * a], (uint32_t)__popc(ml));
+                if (mh) atomicAdd(&S.clip[2 * a + 1], (uint32_t)__popc(mh));
+            }
+            if (have && lo > l) atomicAdd(&S.H[a * 64 + b], 1u);
+            if (have && hi < h) atomicAdd(&S.H[a * 64 + 32 + c], 1u);
+            if (have && on) atomicAdd(&S.on[a * 32 + b], 1u);
+        }
+        bins[k] = w;
+    }
+    group_sync<NT>();
+    // the buckets' places
+    for (uint32_t r = NT == 32 ? 0u : (tid >> 5); r < 6; r += NT / 32) {
+        const uint32_t v = S.H[r * 32 + lane];
+        uint32_t inc = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, d);
+            if ((int)lane >= d) inc += u;
+        }
+        S.S[r * 33 + lane] = S.H[r * 32 + lane] = inc - v;
+        if (lane == 31) S.S[r * 33 + 32] = inc;
+    }
+    group_sync<NT>();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (tri[k] == 0xffffffffu) continue;
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            const float l = c3(blo, a), h = c3(bhi, a);
+            if (!(c3(ext, a) > 0.0f)) continue;
+            const float lo = mxf(c3(tlo[k], a), l), hi = mnf(c3(thi[k], a), h);
+            const bool fl = lo == hi;
+            if (lo > l) {
+                const uint32_t pos = atomicAdd(&S.H[a * 64 + ((bins[k] >> (10 * a)) & 31u)], 1u);
+                S.B[2 * a * kCap + pos] = fl ? nextafterf(lo, -kInf) : lo;
+                if (fl) atomicOr(&S.flat[(2 * a * kCap + pos) >> 5], 1u << (pos & 31u));
+            }
+            if (hi < h) {
+                const uint32_t pos = atomicAdd(&S.H[a * 64 + 32 + ((bins[k] >> (10 * a + 5)) & 31u)], 1u);
+                S.B[(2 * a + 1) * kCap + pos] = fl ? nextafterf(hi, kInf) : hi;
+                if (fl) atomicOr(&S.flat[((2 * a + 1) * kCap + pos) >> 5], 1u << (pos & 31u));
+            }
+        }
+    }
+    group_sync<NT>();
+    // 2. the bins' lower bounds (one warp, lane = bin)
+    float lb[3];
+    uint32_t nc[3], taken = 0;
     float mc = kInf, m_pk = 0.0f;
     uint32_t m_ax = 3, m_nb = 0, m_na = 0;
-    for (uint32_t a = 0; a < 3; a++) {
-        const float l = c3(blo, a), h = c3(bhi, a);
-        if (!(__fsub_rn(h, l) > 0.0f)) continue;
-        if (tid == 0) S.nflat = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < n2; i += blockDim.x) {
-            float lo = kInf, hi = kInf;
-            if (i < cnt) {
-                const uint32_t tri = A.refs()[info.x + i];
-                lo = mxf(c3(A.tb_lo[tri], a), l);
-                hi = mnf(c3(A.tb_hi[tri], a), h);
-                if (lo == hi) S.fl[atomicAdd(&S.nflat, 1u)] = lo;   // flat references, any order
-            }
-            S.lo[i] = lo;
-            S.hi[i] = hi;
+    if (tid < 32) {
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            const float l = c3(blo, a), h = c3(bhi, a);
+            const uint32_t *Sl = S.S + 2 * a * 33, *Sh = Sl + 33;
+            nc[a] = Sl[lane + 1] - Sl[lane] + Sh[lane + 1] - Sh[lane];
+            const float e0 = lane == 0 ? l : S.P[a * 32 + lane], e1 = lane == 31 ? h : S.P[a * 32 + lane + 1];
+            lb[a] = bounds_cost(a, __fsub_rn(e0, l), __fsub_rn(h, e1), ext, Anode, S.clip[2 * a] + Sl[lane],
+                                S.clip[2 * a + 1] + Sh[32] - Sh[lane + 1], A.ct, A.ci);
         }
-        __syncthreads();
-        const uint32_t nfl = S.nflat;
-        uint32_t nf2 = nfl ? 1u : 0u;
-        while (nf2 < nfl) nf2 <<= 1;
-        for (uint32_t i = nfl + tid; i < nf2; i += blockDim.x) S.fl[i] = kInf;
-        __syncthreads();
-        for (uint32_t k = 2; k <= n2; k <<= 1)
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = tid; i < n2; i += blockDim.x) {
-                    const uint32_t ixj = i ^ j;
-                    if (ixj > i) {
-                        const bool up = (i & k) == 0;
-                        float x = S.lo[i], y = S.lo[ixj];
-                        if ((x > y) == up) {
-                            S.lo[i] = y;
-                            S.lo[ixj] = x;
-                        }
-                        x = S.hi[i];
-                        y = S.hi[ixj];
-                        if ((x > y) == up) {
-                            S.hi[i] = y;
-                            S.hi[ixj] = x;
-                        }
-                        if (i < nf2 && ixj < nf2 && k <= nf2) {
-                            x = S.fl[i];
-                            y = S.fl[ixj];
-                            if ((x > y) == up) {
-                                S.fl[i] = y;
-                                S.fl[ixj] = x;
-                            }
-                        }
-                    }
+    }
+    // 3. two rounds
+    for (int round = 0; round < 2; round++) {
+        if (tid < 32) {
+            uint32_t base = 0;
+            const float limit = __uint_as_float(S.best);
+#pragma unroll
+            for (uint32_t a = 0; a < 3; a++) {
+                bool sel = nc[a] != 0;
+                if (round == 0) {
+                    // the least bound of the axis (bounds are not negative)
+                    const uint32_t bits = sel ? __float_as_uint(lb[a]) : 0xffffffffu;
+                    const uint32_t m = __reduce_min_sync(0xffffffffu, bits);
+                    sel = sel && bits == m;
+                    if (sel) taken |= 1u << a;
+                } else {
+                    sel = sel && !((taken >> a) & 1u) && !(lb[a] > limit);
                 }
-                __syncthreads();
+                const uint32_t v = sel ? nc[a] : 0u;
+                uint32_t inc = v;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, d);
+                    if ((int)lane >= d) inc += u;
+                }
+                S.H[a * 32 + lane] = base + inc - v;
+                base += __shfl_sync(0xffffffffu, inc, 31);
             }
-        for (uint32_t q = tid; q < 2 * cnt; q += blockDim.x) {
-            const float pk = __fadd_rn(q < cnt ? S.lo[q] : S.hi[q - cnt], 0.0f);
+            if (lane == 0) S.H[96] = base;
+        }
+        group_sync<NT>();
+        const uint32_t M = S.H[96];
+        for (uint32_t q = tid; q < M; q += NT) {
+            uint32_t i = 0, n = 96;   // the last bin with H[i] <= q
+            while (n > 1) {
+                const uint32_t m = n >> 1;
+                if (S.H[i + m] <= q) i += m;
+                n -= m;
+            }
+            const uint32_t a = i >> 5, j = i & 31u;
+            const uint32_t *Sl = S.S + 2 * a * 33, *Sh = Sl + 33;
+            const uint32_t l0 = Sl[j], l1 = Sl[j + 1], h0 = Sh[j], h1 = Sh[j + 1];
+            const float *Bl = S.B + 2 * a * kCap, *Bh = Bl + kCap;
+            const uint32_t t = q - S.H[i];
+            const bool side = t >= l1 - l0;
+            const uint32_t pos = side ? h0 + t - (l1 - l0) : l0 + t;
+            float x = side ? Bh[pos] : Bl[pos];
+            if ((S.flat[((2 * a + (side ? 1u : 0u)) * kCap + pos) >> 5] >> (pos & 31u)) & 1u)
+                x = nextafterf(x, side ? -kInf : kInf);
+            const float pk = __fadd_rn(x, 0.0f), l = c3(blo, a), h = c3(bhi, a);
             if (!(pk > l && pk < h)) continue;
-            const uint32_t fon = nfl ? upper_bound_f(S.fl, nfl, pk) - lower_bound_f(S.fl, nfl, pk) : 0u;
-            const uint32_t nb = lower_bound_f(S.lo, cnt, pk) + fon;
-            const uint32_t na = (cnt - upper_bound_f(S.hi, cnt, pk)) + fon;
-            float4 bb = bhi, ba = blo;
-            s3(bb, a, pk);
-            s3(ba, a, pk);
-            const float sb = surf(blo, bb), sa = surf(ba, bhi);
-            const float cost = __fadd_rn(
-                ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
-            if (cost < mc || (cost == mc && a == m_ax && pk < m_pk)) {
+            uint32_t nb = S.clip[2 * a] + l0, na = S.clip[2 * a + 1] + Sh[32] - h1;
+            for (uint32_t k = l0; k < l1; k++) nb += Bl[k] < pk ? 1u : 0u;
+            for (uint32_t k = h0; k < h1; k++) na += Bh[k] > pk ? 1u : 0u;
+            const float *Pa = S.P + a * 32;
+            if (!side) {
+                if (j >= 1 && pk == Pa[j]) na += S.on[a * 32 + j];
+            } else if (j < 31 && pk == Pa[j + 1]) {
+                uint32_t b = j + 1;   // the bin whose bucket holds lower bounds equal to pk
+                while (b < 31 && Pa[b + 1] <= pk) b++;
+                nb += S.on[a * 32 + b];
+            }
+            const float cost = plane_cost(a, pk, l, h, ext, Anode, nb, na, A.ct, A.ci);
+            if (refine_better(cost, a, pk, mc, m_ax, m_pk)) {
                 mc = cost;
                 m_ax = a;
                 m_pk = pk;
@@ -1071,57 +1227,38 @@ __device__ Decision sah_exact_cta(const LevelArgs &A, uint4 info, float4 blo, fl
                 m_na = na;
             }
         }
+        __syncwarp();
+        const uint32_t wb = __reduce_min_sync(0xffffffffu, __float_as_uint(mc));
+        if (lane == 0) atomicMin(&S.best, wb);
+        group_sync<NT>();
+    }
+    uint32_t src = warp_argmin(mc, m_ax, m_pk);
+    if (NT > 32) {
+        if (lane == src) {
+            const uint32_t w = tid >> 5;
+            S.w_cost[w] = __float_as_uint(mc);
+            S.w_ax[w] = m_ax;
+            S.w_pk[w] = m_pk;
+            S.w_nb[w] = m_nb;
+            S.w_na[w] = m_na;
+        }
         __syncthreads();
-    }
-    // argmin over (cost, axis, plane): warps, then warp 0 over the warps
-    float bc = mc, bp = m_pk;
-    uint32_t bax = m_ax, bkey = tid;
-    for (int off = 16; off; off >>= 1) {
-        const float oc = __shfl_xor_sync(0xffffffffu, bc, off), op = __shfl_xor_sync(0xffffffffu, bp, off);
-        const uint32_t oax = __shfl_xor_sync(0xffffffffu, bax, off), ok = __shfl_xor_sync(0xffffffffu, bkey, off);
-        if (oc < bc || (oc == bc && (oax < bax || (oax == bax && (op < bp || (op == bp && ok < bkey)))))) {
-            bc = oc;
-            bp = op;
-            bax = oax;
-            bkey = ok;
-        }
-    }
-    if (lane == 0) {
-        S.w_cost[wid] = bc;
-        S.w_pk[wid] = bp;
-        S.w_ax[wid] = bax;
-        S.w_key[wid] = bkey;
-    }
-    // the winning thread of each warp publishes its counts
-    if (tid == bkey) {
-        S.w_nb[wid] = m_nb;
-        S.w_na[wid] = m_na;
-    }
-    __syncthreads();
-    const uint32_t nw = blockDim.x >> 5;
-    float fc = S.w_cost[0], fp = S.w_pk[0];
-    uint32_t fax = S.w_ax[0], fw = 0;
-    for (uint32_t w = 1; w < nw; w++) {
-        const float oc = S.w_cost[w], op = S.w_pk[w];
-        const uint32_t oax = S.w_ax[w];
-        if (oc < fc || (oc == fc && (oax < fax || (oax == fax && op < fp)))) {
-            fc = oc;
-            fp = op;
-            fax = oax;
-            fw = w;
-        }
+        const uint32_t w = min(lane, NT / 32 - 1);
+        mc = __uint_as_float(S.w_cost[w]);
+        m_ax = S.w_ax[w];
+        m_pk = S.w_pk[w];
+        m_nb = S.w_nb[w];
+        m_na = S.w_na[w];
+        src = warp_argmin(mc, m_ax, m_pk);
     }
     Decision best{-1, 0.0f, 0, 0, kInf, 0};
-    if (fc < kInf) {
-        best.axis = (int)fax;
-        best.plane = fp;
-        best.nb = S.w_nb[fw];
-        best.na = S.w_na[fw];
-        best.cost = fc;
-        best.bin = 0;
-    }
-    if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)cnt))) best.axis = -1;
-    __syncthreads();
+    mc = __shfl_sync(0xffffffffu, mc, src);
+    m_ax = __shfl_sync(0xffffffffu, m_ax, src);
+    m_pk = __shfl_sync(0xffffffffu, m_pk, src);
+    m_nb = __shfl_sync(0xffffffffu, m_nb, src);
+    m_na = __shfl_sync(0xffffffffu, m_na, src);
+    if (mc < kInf) best = Decision{(int)m_ax, m_pk, m_nb, m_na, mc, 0};
+    if (best.axis >= 0 && !(best.cost < __fmul_rn(A.ci, (float)cnt))) best.axis = -1;
     return best;
 }
 
@@ -1165,7 +1302,7 @@ struct HistSmem {
 // k_hist's work for one level (every CTA of the grid calls it): the chunks of
 // the large nodes and, with MEDIUM, the medium nodes (exact SAH, XS)
 template <bool MEDIUM>
-__device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, ExactCtaSmem *XSp, Tally &tally) {
+__device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, ExactSmem<256> *XSp, Tally &tally) {
     uint32_t *H = SH.H;
     int &s_last = SH.last;
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -1179,7 +1316,7 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
             if (s >= nodes) continue;
             const uint4 info = A.n_info()[s];
             const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
-            const Decision d = sah_exact_cta(A, info, blo, bhi, A.ct, A.ci, *XSp);
+            const Decision d = sah_exact_group<256>(A, info, blo, bhi, *XSp);
             if (threadIdx.x == 0) {
                 write_decision(A, s, d);
                 tally.add(d, info.y);
@@ -1269,15 +1406,32 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
     }
 }
 
+// (the exact search's registers and shared memory only where a level can have
+// medium nodes)
+template <bool MEDIUM>
 __global__ void __launch_bounds__(256, 3) k_hist(LevelArgs A) {
     __shared__ HistSmem SH;
-    __shared__ ExactCtaSmem XS;
+    __shared__ std::conditional_t<MEDIUM, ExactSmem<256>, uint32_t> XS;
     __shared__ uint32_t s_tally[kTallies];
     if (level_aborted(A)) return;
     Tally tally;
-    hist_body<true>(A, SH, &XS, tally);
+    if constexpr (MEDIUM) hist_body<true>(A, SH, &XS, tally);
+    else hist_body<false>(A, SH, nullptr, tally);
     tally_flush(A, tally, s_tally);
 }
+
+// a small-node warp's shared memory (16-byte aligned in an array of them: the
+// scratch is cleared and read 16 bytes at a time)
+template <bool EXACT>
+union alignas(16) WarpSmem {
+    uint32_t scratch[kWarpScratch];
+};
+template <>
+union alignas(16) WarpSmem<true> {
+    uint32_t scratch[kWarpScratch];
+    ExactSmem<32> exact;
+};
+static_assert(sizeof(WarpSmem<false>) % 16 == 0 && sizeof(WarpSmem<true>) % 16 == 0, "16-byte accesses");
 
 // Small nodes (not splittable, or splittable and neither medium nor large):
 // one warp per node; the exact SAH in registers for nodes of at most 32
@@ -1287,7 +1441,7 @@ __global__ void __launch_bounds__(256, 3) k_hist(LevelArgs A) {
 // binned decision and histogram features are stored for k_learn, which
 // decides it (a node past the row capacity keeps the binned decision).
 template <bool WARP_EXACT, bool LEARNED>
-__device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*WS)[kWarpScratch], Tally &tally) {
+__device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXACT && !LEARNED> *WSp, Tally &tally) {
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nodes = A.lc->nodes;
     const uint32_t ngroups = (nodes + 7) / 8;
@@ -1310,10 +1464,12 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*WS)[kW
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
         Decision d;
         if (cnt <= kWarpExact) {
-            d = sah_warp32<WARP_EXACT>(A, reinterpret_cast<float *>(WS[wib]), info, blo, bhi);
+            d = sah_warp32<WARP_EXACT>(A, reinterpret_cast<float *>(WSp[wib].scratch), info, blo, bhi);
+        } else if (WARP_EXACT && !LEARNED && is_exact(A, cnt)) {
+            if constexpr (WARP_EXACT && !LEARNED) d = sah_exact_group<32>(A, info, blo, bhi, WSp[wib].exact);
         } else {
-            uint32_t *Hw = WS[wib];
-            float *Pw = reinterpret_cast<float *>(WS[wib] + kHist);
+            uint32_t *Hw = WSp[wib].scratch;
+            float *Pw = reinterpret_cast<float *>(WSp[wib].scratch + kHist);
             __syncwarp();   // the previous node's readers are done
             {
                 // 288 counters = 72 16-byte stores
@@ -1354,8 +1510,8 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, uint32_t (*WS)[kW
 }
 
 template <bool WARP_EXACT, bool LEARNED>
-__global__ void __launch_bounds__(256, 5) k_small(LevelArgs A) {
-    __shared__ __align__(16) uint32_t WS[8][kWarpScratch];
+__global__ void __launch_bounds__(256, WARP_EXACT && !LEARNED ? 4 : 5) k_small(LevelArgs A) {
+    __shared__ __align__(16) WarpSmem<WARP_EXACT && !LEARNED> WS[8];
     __shared__ uint32_t s_tally[kTallies];
     wait_prior_grid();
     if (level_aborted(A)) return;
@@ -1369,7 +1525,7 @@ __global__ void __launch_bounds__(256, 5) k_small(LevelArgs A) {
 // (no second stream, no fork and join per level)
 union DecideSmem {
     HistSmem hist;
-    uint32_t small[8][kWarpScratch];
+    WarpSmem<false> small[8];
 };
 
 __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
@@ -1620,10 +1776,6 @@ constexpr size_t kRefineWarpSmem = (size_t)kRefineRowWarps * kLearnScratch * 4; 
 // k_refine_warp's grid in CTAs per SM: more than are resident (two, by its
 // registers), so that CTAs finishing early are replaced by new ones
 constexpr int kRefineWarpGrid = 3;
-
-__device__ __forceinline__ bool refine_better(float c, uint32_t a, float p, float bc, uint32_t ba, float bp) {
-    return c < bc || (c == bc && (a < ba || (a == ba && p < bp)));
-}
 
 __global__ void __launch_bounds__(kRefineThreads) k_refine_cta(LevelArgs A) {
     extern __shared__ __align__(16) float refine_smem[];
@@ -3117,7 +3269,9 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         // binned histograms, or the proposer's features, inference and costing
         cudaEventRecord(S.ev_fork, st);
         cudaStreamWaitEvent(S.aux, S.ev_fork, 0);
-        k_hist<<<S.sm_count * 3, 256, 0, S.aux>>>(A);   // one wave: three CTAs per SM resident
+        // one wave: three CTAs per SM resident
+        if (A.exact_max >= kWarpExact) k_hist<true><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
+        else k_hist<false><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
         if (A.learned) {
             // the proposer's chain on the second stream after the histograms
             // (every proposer row comes from k_hist), beside the small nodes
@@ -3136,7 +3290,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         if (A.learned) {
             launch_pdl(k_small<true, true>, S.sm_count * 5, 256, 0, st, A);
         } else if (A.exact_max >= kWarpExact) {
-            launch_pdl(k_small<true, false>, S.sm_count * 5, 256, 0, st, A);
+            launch_pdl(k_small<true, false>, S.sm_count * 4, 256, 0, st, A);
         } else {
             launch_pdl(k_small<false, false>, S.sm_count * 5, 256, 0, st, A);
         }
