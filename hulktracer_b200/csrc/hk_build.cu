@@ -173,6 +173,29 @@ constexpr uint32_t kErrAbort = 4u | 8u | 16u | kErrTensorWait;
 // writes visible. Without the launch attribute it returns at once.
 __device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// One window of a look-back (a warp, lane k at the tile k before): poll()
+// gives the lane's status (0: not published yet). The window is complete once
+// every tile up to the nearest inclusive one has published, whatever the tiles
+// behind it do: waiting for all 32 held every tile of a level until its 32
+// predecessors had loaded their references (7 of a level's 20 us). Returns that
+// nearest lane (32: none in the window); a wait that runs out sets error bit 4
+// and ends the look-back at the first tile without a value.
+template <class Poll>
+__device__ __forceinline__ int lookback_window(const Poll &poll, uint32_t *err, uint32_t spin_limit) {
+    for (uint32_t spins = 0;; spins++) {
+        const uint32_t st = poll();
+        const uint32_t m2 = __ballot_sync(0xffffffffu, st == 2u), m0 = __ballot_sync(0xffffffffu, st == 0u);
+        const int stop = m2 ? __ffs(m2) - 1 : 32;
+        const uint32_t need = stop >= 31 ? 0xffffffffu : (2u << stop) - 1u;
+        if (!(m0 & need)) return stop;
+        if (spins >= spin_limit) {
+            if ((threadIdx.x & 31u) == 0) atomicOr(err, 4u);
+            return __ffs(m0) - 1;
+        }
+        __nanosleep(32);
+    }
+}
+
 template <class T>
 __device__ T lookback(const uint32_t *flags, const T *aggs, const T *incls, uint32_t tile, uint32_t tag,
                       uint32_t *err, uint32_t spin_limit) {
@@ -182,32 +205,56 @@ __device__ T lookback(const uint32_t *flags, const T *aggs, const T *incls, uint
     for (;;) {
         const int32_t q = p - lane;
         uint32_t st = 2;    // before tile 0: an inclusive prefix of zero
-        bool have = false;
-        if (q >= 0) {
-            have = true;
-            for (uint32_t spins = 0;; spins++) {
-                const uint32_t f = __ldcv(flags + q);
-                if ((f >> 2) == tag && (f & 3u)) {
-                    st = f & 3u;
-                    break;
+        const int stop = lookback_window(
+            [&] {
+                if (q >= 0) {
+                    const uint32_t f = __ldcv(flags + q);
+                    st = (f >> 2) == tag ? f & 3u : 0u;
                 }
-                if (spins >= spin_limit) {
-                    atomicOr(err, 4u);
-                    have = false;
-                    st = 2;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
+                return st;
+            },
+            err, spin_limit);
         __threadfence();
-        const uint32_t m2 = __ballot_sync(0xffffffffu, st == 2);
-        const int stop = m2 ? __ffs(m2) - 1 : 32;
         T v = vzero<T>();
-        if (have && lane <= stop) v = lane == stop ? ldcg(incls + q) : ldcg(aggs + q);
+        if (q >= 0 && lane <= stop && st) v = lane == stop ? ldcg(incls + q) : ldcg(aggs + q);
         for (int o = 16; o; o >>= 1) v = vadd(v, shfl_xor(v, o));
         excl = vadd(excl, v);
-        if (m2) break;
+        if (stop < 32) break;
+        p -= 32;
+    }
+    return excl;
+}
+
+// The reference tiles' flags carry their values: two 64-bit words, each with
+// the flag in its upper half and a count (below, above) in its lower half, so
+// one load gives both and no fence stands between them. A word is read whole;
+// two words that differ in their flags are a record between two writes.
+__device__ __forceinline__ void ref_publish(ulonglong2 *rec, uint32_t flag, uint2 v) {
+    const unsigned long long f = (unsigned long long)flag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(rec), "l"(f | v.x), "l"(f | v.y) : "memory");
+}
+__device__ __forceinline__ uint32_t ref_poll(const ulonglong2 *rec, uint32_t tag, uint2 &v) {
+    unsigned long long x, y;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(rec) : "memory");
+    v = make_uint2((uint32_t)x, (uint32_t)y);
+    const uint32_t f = (uint32_t)(x >> 32);
+    return f == (uint32_t)(y >> 32) && (f >> 2) == tag ? f & 3u : 0u;
+}
+
+__device__ __forceinline__ uint2 ref_lookback(const ulonglong2 *recs, uint32_t tile, uint32_t tag, uint32_t *err,
+                                              uint32_t spin_limit) {
+    const int lane = threadIdx.x & 31;
+    uint2 excl = make_uint2(0, 0);
+    int32_t p = (int32_t)tile - 1;
+    for (;;) {
+        const int32_t q = p - lane;
+        uint2 v = make_uint2(0, 0);
+        uint32_t st = 2;    // before tile 0: zero
+        const int stop = lookback_window([&] { return q >= 0 ? st = ref_poll(recs + q, tag, v) : st; }, err, spin_limit);
+        if (lane > stop || !st) v = make_uint2(0, 0);
+        excl.x += __reduce_add_sync(0xffffffffu, v.x);
+        excl.y += __reduce_add_sync(0xffffffffu, v.y);
+        if (stop < 32) break;
         p -= 32;
     }
     return excl;
@@ -419,12 +466,15 @@ __device__ Decision sah_warp(HistPtr H, float4 blo, float4 bhi, uint32_t cnt, fl
     float mc = kInf;
     uint32_t mkey = 0xffffffffu, m_nb = 0, m_na = 0;
     float m_pk = 0.0f;
+    uint32_t hist[9];   // every counter of the lane loaded together
+#pragma unroll
+    for (uint32_t k = 0; k < 9; k++) hist[k] = H[k * 32 + lane];
 #pragma unroll
     for (uint32_t a = 0; a < 3; a++) {
         const float l = c3(blo, a), h = c3(bhi, a);
         const float ext = __fsub_rn(h, l);
         if (!(ext > 0.0f)) continue;
-        const uint32_t hlo = H[a * 96 + lane], hhi = H[a * 96 + 32 + lane];
+        const uint32_t hlo = hist[3 * a], hhi = hist[3 * a + 1];
         uint32_t slo, shi;
         if (packed) {
             uint32_t v = hlo | (hhi << 16);
@@ -447,7 +497,7 @@ __device__ Decision sah_warp(HistPtr H, float4 blo, float4 bhi, uint32_t cnt, fl
         }
         const uint32_t below = slo - hlo;          // sum_{b < k} hlo[b]
         const uint32_t above = cnt - (shi - hhi);  // sum_{c >= k} hhi[c]
-        const uint32_t on = H[a * 96 + 64 + lane];
+        const uint32_t on = hist[3 * a + 2];
         const float pk = plane_k(l, ext, lane);
         const float pk1 = __shfl_down_sync(0xffffffffu, pk, 1);   // plane k + 1 (lane 31: unused)
         const bool valid = lane >= 1 && pk > l && pk < h && (lane == 31 || pk < pk1);
@@ -494,7 +544,9 @@ __device__ Decision sah_warp(HistPtr H, float4 blo, float4 bhi, uint32_t cnt, fl
 // kernels
 // ---------------------------------------------------------------------------
 struct LevelArgs {
-    const float4 *tb_lo, *tb_hi;
+    // triangle bounds, 32 bytes (one memory sector) each: {lo.x, hi.x, lo.y,
+    // hi.y}, {lo.z, hi.z, -, -}
+    const float4 *tb;
     // the level's nodes and references, ping-pong by level parity: level L
     // reads buffer L & 1 and writes the other (the accessors below)
     float4 *lo_buf[2], *hi_buf[2];
@@ -505,8 +557,7 @@ struct LevelArgs {
     uint2 *cnt;
     float4 *split;          // per node: axis (int bits, -1 = leaf), plane, node min / max on the axis
     uint4 *scat;            // per node: where its references go (written by the plan scan)
-    uint2 *chunks;          // (large rank, chunk index within the node)
-    uint32_t *large_slot;
+    uint4 *chunks;          // large rank, node slot, first reference, end
     uint32_t *medium_slot;
     uint32_t *hist;
     uint32_t *done;
@@ -582,14 +633,24 @@ __device__ __forceinline__ bool level_aborted(const LevelArgs &A) {
     return s_abort != 0;
 }
 
-__global__ void k_tri_bounds(const float4 *__restrict__ V, const uint4 *__restrict__ T, uint32_t nt, float4 *lo,
-                             float4 *hi) {
+__global__ void k_tri_bounds(const float4 *__restrict__ V, const uint4 *__restrict__ T, uint32_t nt, float4 *tb) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
     uint4 t = T[i];
     float4 a = V[t.x], b = V[t.y], c = V[t.z];
-    lo[i] = make_float4(mnf(mnf(a.x, b.x), c.x), mnf(mnf(a.y, b.y), c.y), mnf(mnf(a.z, b.z), c.z), 0.0f);
-    hi[i] = make_float4(mxf(mxf(a.x, b.x), c.x), mxf(mxf(a.y, b.y), c.y), mxf(mxf(a.z, b.z), c.z), 0.0f);
+    tb[2 * (size_t)i] = make_float4(mnf(mnf(a.x, b.x), c.x), mxf(mxf(a.x, b.x), c.x), mnf(mnf(a.y, b.y), c.y),
+                                    mxf(mxf(a.y, b.y), c.y));
+    tb[2 * (size_t)i + 1] = make_float4(mnf(mnf(a.z, b.z), c.z), mxf(mxf(a.z, b.z), c.z), 0.0f, 0.0f);
+}
+
+__device__ __forceinline__ void load_bounds(const LevelArgs &A, uint32_t tri, float4 &lo, float4 &hi) {
+    const float4 a = A.tb[2 * (size_t)tri], b = A.tb[2 * (size_t)tri + 1];
+    lo = make_float4(a.x, a.z, b.x, 0.0f);
+    hi = make_float4(a.y, a.w, b.y, 0.0f);
+}
+// one axis: (lo, hi)
+__device__ __forceinline__ float2 load_bounds_axis(const LevelArgs &A, uint32_t tri, uint32_t axis) {
+    return reinterpret_cast<const float2 *>(A.tb)[4 * (size_t)tri + axis];
 }
 
 __device__ __forceinline__ bool decidable(const LevelArgs &A, uint32_t cnt) {
@@ -642,7 +703,6 @@ __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
         l0->n_large = large ? 1u : 0u;
         l0->n_chunks = nch;
         l0->n_medium = medium ? 1u : 0u;
-        if (large) A.large_slot[0] = 0;
         if (medium) A.medium_slot[0] = 0;
         // level 0's node buffers (A.level is 0)
         A.n_lo()[0] = make_float4(box[0], box[1], box[2], 0.0f);
@@ -660,7 +720,7 @@ __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
         A.ref_node()[i] = 0;
     }
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nch; k += gridDim.x * blockDim.x)
-        A.chunks[k] = make_uint2(0, k);
+        A.chunks[k] = make_uint4(0, 0, k * kChunk, min(nt, (k + 1) * kChunk));
 }
 
 
@@ -970,8 +1030,7 @@ __device__ __forceinline__ Decision sah_warp32(const LevelArgs &A, float *S, uin
     float4 tlo = make_float4(0, 0, 0, 0), thi = tlo;
     if (lane < c) {
         const uint32_t tri = A.refs()[info.x + lane];
-        tlo = A.tb_lo[tri];
-        thi = A.tb_hi[tri];
+        load_bounds(A, tri, tlo, thi);
     }
     float4 nlo = tlo, nhi = thi;
     lane_bounds(nlo, nhi);
@@ -1072,10 +1131,7 @@ __device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, 
     }
 #pragma unroll
     for (int k = 0; k < 4; k++)
-        if (tri[k] != 0xffffffffu) {
-            tlo[k] = A.tb_lo[tri[k]];
-            thi[k] = A.tb_hi[tri[k]];
-        }
+        if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
     group_sync<NT>();
     // 1. bins (5 bits each, lo then hi per axis), counts
     const float4 inv3 = bin_scale(blo, bhi);
@@ -1329,7 +1385,9 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
                 const float4 inv3 = bin_scale(blo, bhi);
                 for (uint32_t r = info.x + threadIdx.x; r < info.x + info.y; r += blockDim.x) {
                     const uint32_t tri = A.refs()[r];
-                    hist_ref(H, A.tb_lo[tri], A.tb_hi[tri], blo, bhi, inv3);
+                    float4 tlo, thi;
+                    load_bounds(A, tri, tlo, thi);
+                    hist_ref(H, tlo, thi, blo, bhi, inv3);
                 }
                 __syncthreads();
                 if (wib == 0) {
@@ -1345,14 +1403,11 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
             }
             continue;
         }
-        const uint2 ck = A.chunks[item];
-        const uint32_t rank = ck.x;
-        if (rank >= A.cap_large) continue;  // uniform per CTA
-        const uint32_t s = A.large_slot[rank];
-        if (s >= nodes) continue;
+        const uint4 ck = A.chunks[item];
+        const uint32_t rank = ck.x, s = ck.y, r0 = ck.z, r1 = ck.w;
+        if (rank >= A.cap_large || s >= nodes) continue;   // uniform per CTA
         const uint4 info = A.n_info()[s];
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
-        const uint32_t r0 = info.x + ck.y * kChunk, r1 = min(info.x + info.y, r0 + kChunk);
         for (uint32_t i = threadIdx.x; i < kHist; i += blockDim.x) H[i] = 0;
         node_planes_cta(SH.P, blo, bhi);
         __syncthreads();
@@ -1369,10 +1424,7 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
             }
 #pragma unroll
             for (int k = 0; k < kPer; k++)
-                if (tri[k] != 0xffffffffu) {
-                    tlo[k] = A.tb_lo[tri[k]];
-                    thi[k] = A.tb_hi[tri[k]];
-                }
+                if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
 #pragma unroll
             for (int k = 0; k < kPer; k++)
                 if (tri[k] != 0xffffffffu) hist_ref_tab(H, tlo[k], thi[k], blo, bhi, inv3, SH.P);
@@ -1436,16 +1488,15 @@ static_assert(sizeof(WarpSmem<false>) % 16 == 0 && sizeof(WarpSmem<true>) % 16 =
 // Small nodes (not splittable, or splittable and neither medium nor large):
 // one warp per node; the exact SAH in registers for nodes of at most 32
 // references when exact_max >= 32 or in learned mode (the WARP_EXACT
-// instantiations), else a warp-private histogram + the binned SAH. In learned
-// mode (LEARNED) a node of 33..1024 references becomes a proposer row: its
-// binned decision and histogram features are stored for k_learn, which
-// decides it (a node past the row capacity keeps the binned decision).
+// instantiations), else counts per plane up to 32 references and a
+// warp-private histogram + the binned SAH above.
 template <bool WARP_EXACT, bool LEARNED>
-__device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXACT && !LEARNED> *WSp, Tally &tally) {
+__device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXACT && !LEARNED> *WSp, Tally &tally,
+                                           uint32_t cta) {
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nodes = A.lc->nodes;
     const uint32_t ngroups = (nodes + 7) / 8;
-    for (uint32_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    for (uint32_t g = cta; g < ngroups; g += gridDim.x) {
         const uint32_t s = g * 8 + wib;
         if (s >= nodes) continue;
         const uint4 info = A.n_info()[s];
@@ -1463,7 +1514,8 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
         }
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
         Decision d;
-        if (cnt <= kWarpExact) {
+        if (LEARNED || cnt <= kWarpExact) {
+            // (learned mode: larger nodes are k_hist's)
             d = sah_warp32<WARP_EXACT>(A, reinterpret_cast<float *>(WSp[wib].scratch), info, blo, bhi);
         } else if (WARP_EXACT && !LEARNED && is_exact(A, cnt)) {
             if constexpr (WARP_EXACT && !LEARNED) d = sah_exact_group<32>(A, info, blo, bhi, WSp[wib].exact);
@@ -1481,25 +1533,29 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
             node_planes_warp(Pw, blo, bhi);
             __syncwarp();
             const float4 inv3 = bin_scale(blo, bhi);
-            for (uint32_t r = info.x + lane; r < info.x + cnt; r += 32) {
-                const uint32_t tri = A.refs()[r];
-                hist_ref_tab(Hw, A.tb_lo[tri], A.tb_hi[tri], blo, bhi, inv3, Pw);
+            // four references per lane and pass, their loads issued together
+            // (the exact instantiation, which has few nodes here and no
+            // registers to spare: one)
+            constexpr int kPass = WARP_EXACT ? 1 : 4;
+            for (uint32_t base = 0; base < cnt; base += 32 * kPass) {
+                uint32_t tri[kPass];
+                float4 tlo[kPass], thi[kPass];
+#pragma unroll
+                for (int k = 0; k < kPass; k++) {
+                    const uint32_t r = base + 32u * k + lane;
+                    tri[k] = r < cnt ? A.refs()[info.x + r] : 0xffffffffu;
+                }
+#pragma unroll
+                for (int k = 0; k < kPass; k++)
+                    if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
+#pragma unroll
+                for (int k = 0; k < kPass; k++) {
+                    if (base + 32u * k >= cnt) break;   // uniform across the warp
+                    if (tri[k] != 0xffffffffu) hist_ref_tab(Hw, tlo[k], thi[k], blo, bhi, inv3, Pw);
+                }
             }
             __syncwarp();
             d = sah_warp(Hw, blo, bhi, cnt, A.ct, A.ci);
-            if (LEARNED && is_learn(A, cnt)) {
-                uint32_t row = 0;
-                if (lane == 0) row = atomicAdd(&A.lc->n_learn, 1u);
-                row = __shfl_sync(0xffffffffu, row, 0);
-                if (row < A.cap_learn) {
-                    if (lane == 0) {
-                        A.learn_slot[row] = s;
-                        A.learn_bin[row] = LearnBin{d.cost, d.plane, d.axis, d.nb, d.na, {info.y, 0, 0}};
-                    }
-                    hist_features(Hw, cnt, blo, bhi, A.level, A.max_depth, A.feat + (size_t)row * 200);
-                    continue;   // decided and tallied by k_learn
-                }
-            }
         }
         if (lane == 0) {
             write_decision(A, s, d, blo, bhi);
@@ -1510,13 +1566,13 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
 }
 
 template <bool WARP_EXACT, bool LEARNED>
-__global__ void __launch_bounds__(256, WARP_EXACT && !LEARNED ? 4 : 5) k_small(LevelArgs A) {
+__global__ void __launch_bounds__(256, LEARNED ? 5 : 4) k_small(LevelArgs A) {
     __shared__ __align__(16) WarpSmem<WARP_EXACT && !LEARNED> WS[8];
     __shared__ uint32_t s_tally[kTallies];
     wait_prior_grid();
     if (level_aborted(A)) return;
     Tally tally;
-    small_body<WARP_EXACT, LEARNED>(A, WS, tally);
+    small_body<WARP_EXACT, LEARNED>(A, WS, tally, blockIdx.x);
     tally_flush(A, tally, s_tally);
 }
 
@@ -1536,7 +1592,8 @@ __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
     Tally tally;
     hist_body<false>(A, sm.hist, nullptr, tally);
     __syncthreads();
-    small_body<false, false>(A, sm.small, tally);
+    // the last CTAs take the first node groups: the first ones have the chunks
+    small_body<false, false>(A, sm.small, tally, gridDim.x - 1 - blockIdx.x);
     tally_flush(A, tally, s_tally);
 }
 
@@ -1827,8 +1884,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_refine_cta(LevelArgs A) {
             float4 tlo = make_float4(0, 0, 0, 0), thi = tlo;
             if (have) {
                 const uint32_t tri = A.refs()[info.x + base + tid];
-                tlo = A.tb_lo[tri];
-                thi = A.tb_hi[tri];
+                load_bounds(A, tri, tlo, thi);
             }
 #pragma unroll
             for (int i = 0; i < kLearnMaxK; i++) {
@@ -2023,8 +2079,8 @@ __global__ void __launch_bounds__(256) k_refine_warp(LevelArgs A) {
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                tlo[u] = have[u] ? A.tb_lo[tri[u]] : make_float4(0, 0, 0, 0);
-                thi[u] = have[u] ? A.tb_hi[tri[u]] : make_float4(0, 0, 0, 0);
+                tlo[u] = thi[u] = make_float4(0, 0, 0, 0);
+                if (have[u]) load_bounds(A, tri[u], tlo[u], thi[u]);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -2153,9 +2209,9 @@ __device__ __forceinline__ bool level_over(const LevelArgs &A) {
            (uint64_t)l->nodes_total + 2 * splits > A.cap_nodes || l->t_next > A.cap_level;
 }
 
-// a child of count c in next-level slot ns: large nodes take a rank and
+// a child of count c (from reference start) in next-level slot ns: large nodes take a rank and
 // their chunks (few per level, so plain atomics)
-__device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t c) {
+__device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t start, uint32_t c) {
     const bool dec = c > A.leaf_size && A.level + 1 < A.max_depth;
     if (dec && is_medium(A, c)) {
         const uint32_t m = atomicAdd(&A.nlc->n_medium, 1u);
@@ -2171,8 +2227,8 @@ __device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t c) {
         atomicOr(A.err, 2u);
         return;
     }
-    A.large_slot[rank] = ns;
-    for (uint32_t k = 0; k < nch; k++) A.chunks[first + k] = make_uint2(rank, k);
+    for (uint32_t k = 0; k < nch; k++)
+        A.chunks[first + k] = make_uint4(rank, ns, start + k * kChunk, start + min(c, (k + 1) * kChunk));
 }
 
 struct PlanCtx {
@@ -2318,7 +2374,7 @@ struct PlanOp {
             A.nx_lo()[ns] = lo;
             A.nx_hi()[ns] = h2;
             A.nx_info()[ns] = make_uint4(co, ct.x, pair, 0);
-            child_setup(A, ns, ct.x);
+            child_setup(A, ns, co, ct.x);
             ns++;
         } else {
             A.out_nodes[pair] = make_uint2(kLeafTag, 0);
@@ -2329,7 +2385,7 @@ struct PlanOp {
             A.nx_lo()[ns] = l2;
             A.nx_hi()[ns] = hi;
             A.nx_info()[ns] = make_uint4(co + ct.x, ct.y, pair + 1, 0);
-            child_setup(A, ns, ct.y);
+            child_setup(A, ns, co + ct.x, ct.y);
         } else {
             A.out_nodes[pair + 1] = make_uint2(kLeafTag, 0);
         }
@@ -2347,28 +2403,43 @@ struct RefItem {
 };
 
 struct RefOp {
-    using T = uint2;
     using Item = RefItem;
     using Ctx = uint32_t;   // the level stopped splitting
     static constexpr int kItems = 4;
     LevelArgs A;
-    __device__ uint32_t count() const { return A.lc->refs; }
-    __device__ uint32_t tag() const { return level_tag(A); }
-    __device__ uint32_t *err() const { return A.err; }
-    __device__ Ctx ctx() const { return A.lc->stop; }
-    __device__ Item load(uint32_t r, const Ctx &stop) const {
-        if (r == 0xffffffffu) return Item{make_uint2(0, 0), 0, 0};
-        const uint32_t s = A.ref_node()[r];
-        const uint32_t tri = A.refs()[r];
-        const float4 sp = A.split[s];
-        const int ax = stop ? -1 : __float_as_int(sp.x);
-        if (ax < 0) return Item{make_uint2(0, 0), s, tri};
-        const float p = sp.y, l = sp.z, h = sp.w;
-        const float lo = mxf(c3(A.tb_lo[tri], ax), l), hi = mnf(c3(A.tb_hi[tri], ax), h);
-        const bool flat_on = (lo == hi) && lo == p;
-        return Item{make_uint2((lo < p || flat_on) ? 1u : 0u, (hi > p || flat_on) ? 1u : 0u), s, tri};
+    // kItems consecutive references from `base` (a multiple of kItems), those
+    // before n: the indices in two 16-byte loads, then every gather together
+    __device__ void load(uint32_t base, uint32_t n, const Ctx &stop, Item (&it)[kItems]) const {
+        uint32_t node[4] = {0, 0, 0, 0}, tri[4] = {0, 0, 0, 0};
+        if (base + 4 <= n) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(A.ref_node() + base);
+            const uint4 b = *reinterpret_cast<const uint4 *>(A.refs() + base);
+            node[0] = a.x; node[1] = a.y; node[2] = a.z; node[3] = a.w;
+            tri[0] = b.x; tri[1] = b.y; tri[2] = b.z; tri[3] = b.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < kItems; k++)
+                if (base + k < n) {
+                    node[k] = A.ref_node()[base + k];
+                    tri[k] = A.refs()[base + k];
+                }
+        }
+        float4 sp[kItems];
+#pragma unroll
+        for (int k = 0; k < kItems; k++)
+            sp[k] = base + k < n ? A.split[node[k]] : make_float4(__int_as_float(-1), 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < kItems; k++) {
+            const int ax = stop ? -1 : __float_as_int(sp[k].x);
+            it[k] = Item{make_uint2(0, 0), node[k], tri[k]};
+            if (ax < 0) continue;
+            const float p = sp[k].y, l = sp[k].z, h = sp[k].w;
+            const float2 b = load_bounds_axis(A, tri[k], (uint32_t)ax);
+            const float lo = mxf(b.x, l), hi = mnf(b.y, h);
+            const bool flat_on = (lo == hi) && lo == p;
+            it[k].f = make_uint2((lo < p || flat_on) ? 1u : 0u, (hi > p || flat_on) ? 1u : 0u);
+        }
     }
-    __device__ T value(const Item &it) const { return it.f; }
     // R: the reference's rank among its node's below / above references
     __device__ void apply(uint32_t r, uint2 R, const Item &it, const Ctx &) const {
         const uint4 sc = __ldcg(A.scat + it.s);   // written by a plan tile of this launch
@@ -2417,29 +2488,35 @@ struct RefTileSmem {
     SegV w_tot[kScanThreads / 32];
     uint32_t w_last[kScanThreads / 32];   // node of each warp's last reference
     uint2 carry;                          // the tile's first segment: flags in earlier tiles
+    uint32_t first_node, last_node;       // nodes of the tile's references
+    uint32_t wait_ok;
 };
 
 // One reference tile (kTile references, kScanItems per thread). The scan is
 // segmented by node: a tile in which a node starts publishes its last
 // segment's counts as complete (status 2) at once; only its first segment,
 // when it continues a node of earlier tiles, needs the look-back, which ends at
-// the tile where that node starts. wait_plan() runs (all threads) before the
-// scatter.
+// the tile where that node starts. One warp looks back while another waits
+// (wait_plan(first, last node)) for the plan tiles of the tile's nodes; the
+// scatter follows both.
 template <class Wait>
-__device__ void ref_tile(const RefOp &R, uint32_t rt, uint32_t nr, uint32_t tag, uint32_t stop, uint32_t *flags,
-                         uint2 *aggs, uint2 *incls, RefTileSmem &sh, const Wait &wait_plan) {
+__device__ void ref_tile(const RefOp &R, uint32_t rt, uint32_t nr, uint32_t tag, uint32_t stop, ulonglong2 *recs,
+                         RefTileSmem &sh, const Wait &wait_plan) {
     const LevelArgs &A = R.A;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint32_t r0 = rt * kTile;
     const uint32_t base = r0 + threadIdx.x * kScanItems;
+    const uint32_t first_prev = (threadIdx.x == 0 && r0 > 0) ? A.ref_node()[r0 - 1] : 0xffffffffu;
     RefItem it[kScanItems];
     bool hd[kScanItems];
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) it[k] = R.load(base + k < nr ? base + k : 0xffffffffu, stop);
+    R.load(base, nr, stop, it);
     // node of the reference before this thread's first one
     uint32_t prev = __shfl_up_sync(0xffffffffu, it[kScanItems - 1].s, 1);
     if (lane == 31) sh.w_last[wid] = it[kScanItems - 1].s;
-    const uint32_t first_prev = (threadIdx.x == 0 && r0 > 0) ? A.ref_node()[r0 - 1] : 0xffffffffu;
+    if (threadIdx.x == 0) sh.first_node = it[0].s;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++)
+        if (base + k == min(nr, r0 + kTile) - 1) sh.last_node = it[k].s;
     __syncthreads();
     if (lane == 0) prev = wid ? sh.w_last[wid - 1] : first_prev;
     SegV t{make_uint2(0, 0), 0u};
@@ -2465,30 +2542,23 @@ __device__ void ref_tile(const RefOp &R, uint32_t rt, uint32_t nr, uint32_t tag,
         tot = seg_join(tot, sh.w_tot[w]);
     }
     ex = seg_join(wp, ex);
-    // the tile's first reference starts a node: no earlier tile matters
-    const bool starts = r0 == 0 || first_prev != it[0].s;
-    if (threadIdx.x == 0) {
-        if (tot.h) incls[rt] = tot.v;
-        else aggs[rt] = tot.v;
-        __threadfence();
-        *reinterpret_cast<volatile uint32_t *>(flags + rt) = (tag << 2) | (tot.h ? 2u : 1u);
-    }
-    if (threadIdx.x < 32) {
-        // the tile-0 rule is kept for the look-back: before tile 0 is zero
-        const uint2 c = (rt && !__shfl_sync(0xffffffffu, starts ? 1u : 0u, 0))
-                            ? lookback(flags, aggs, incls, rt, tag, A.err, A.spin_limit)
-                            : make_uint2(0, 0);
+    if (threadIdx.x == 0) ref_publish(recs + rt, (tag << 2) | (tot.h ? 2u : 1u), tot.v);
+    if (wid == 0) {
+        // the tile's first reference starts a node: no earlier tile matters
+        const bool starts = r0 == 0 || first_prev != it[0].s;
+        const uint2 c = __shfl_sync(0xffffffffu, starts ? 1u : 0u, 0)
+                            ? make_uint2(0, 0)
+                            : ref_lookback(recs, rt, tag, A.err, A.spin_limit);
         if (threadIdx.x == 0) {
-            if (!tot.h) {
-                incls[rt] = vadd(c, tot.v);
-                __threadfence();
-                *reinterpret_cast<volatile uint32_t *>(flags + rt) = (tag << 2) | 2u;
-            }
+            if (!tot.h) ref_publish(recs + rt, (tag << 2) | 2u, vadd(c, tot.v));
             sh.carry = c;
         }
+    } else if (wid == 1) {
+        const bool ok = wait_plan(sh.first_node, sh.last_node);
+        if (lane == 0) sh.wait_ok = ok ? 1u : 0u;
     }
     __syncthreads();
-    if (!wait_plan()) return;   // uniform: the scatter needs the plan's destinations
+    if (!sh.wait_ok) return;   // uniform: the scatter needs the plan's destinations
     uint2 run = ex.h ? ex.v : vadd(ex.v, sh.carry);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
@@ -2513,17 +2583,13 @@ struct PlanSmem {
     U7 shp[kScanThreads / 32 + 1];
     U7 sxp;
     RefTileSmem shr_seg;
-    uint32_t tile, wait_ok;
+    uint32_t tile;
 };
 
 __device__ __forceinline__ void plan_refs_body(const LevelArgs &A, PlanSmem &SM, uint32_t *pflags, U7 *paggs,
-                                               U7 *pincls, uint32_t *rflags, uint2 *raggs, uint2 *rincls,
-                                               uint32_t *pdone, uint32_t *ticket) {
-    U7 *shp = SM.shp;
-    U7 &sxp = SM.sxp;
-    RefTileSmem &shr_seg = SM.shr_seg;
-    uint32_t &s_tile = SM.tile;
-    uint32_t &s_wait_ok = SM.wait_ok;
+                                               U7 *pincls, ulonglong2 *rrecs, uint32_t *pdone, uint32_t *ticket) {
+    // the first ticket, on its way while the level's counters are read
+    if (threadIdx.x == 0) SM.tile = atomicAdd(ticket, 1u);
     const PlanOp P{A};
     const RefOp R{A};
     const uint32_t tag = level_tag(A);
@@ -2533,58 +2599,59 @@ __device__ __forceinline__ void plan_refs_body(const LevelArgs &A, PlanSmem &SM,
     const uint32_t ntn = (nn + kPlanTile - 1) / kPlanTile;
     const uint32_t ntr = (nr + kTile - 1) / kTile;
     for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
         __syncthreads();
-        const uint32_t t = s_tile;
+        const uint32_t t = SM.tile;
         if (t < ntn) {
             // the done flag follows the tile's reference destinations; the
             // rest of its emission overlaps the reference tiles' scatter
-            scan_tile(P, t, nn, tag, pc, pflags, paggs, pincls, shp, sxp, [&] {
+            scan_tile(P, t, nn, tag, pc, pflags, paggs, pincls, SM.shp, SM.sxp, [&] {
                 __threadfence();
                 __syncthreads();
                 if (threadIdx.x == 0 && !(t == 0 && A.level == A.withhold_level))
                     *reinterpret_cast<volatile uint32_t *>(pdone + t) = tag;
             });
         } else if (t < ntn + ntr) {
-            const uint32_t rt = t - ntn;
-            // true when every plan tile of this tile's nodes has published
-            // its reference destinations; a wait that runs out leaves the
-            // tile's scatter undone (error bit 4, the build reports failure)
-            auto wait_plan = [&]() -> bool {
-                if (threadIdx.x == 0) {
-                    uint32_t ok = 1;
-                    const uint32_t r0 = rt * kTile, r1 = min(nr, r0 + kTile) - 1;
-                    const uint32_t k0 = A.ref_node()[r0] / kPlanTile, k1 = A.ref_node()[r1] / kPlanTile;
-                    for (uint32_t k = k0; k <= k1 && k < ntn && ok; k++) {
-                        for (uint32_t spins = 0; __ldcv(pdone + k) != tag; spins++) {
-                            if (spins >= A.spin_limit) {
-                                atomicOr(A.err, 4u);
-                                ok = 0;
-                                break;
-                            }
-                            __nanosleep(32);
-                        }
+            // true when every plan tile of the tile's nodes has published its
+            // reference destinations (one warp, lane k at the k-th such plan
+            // tile: a tile's references span at most kTile nodes); a wait that
+            // runs out leaves the tile's scatter undone (error bit 4, the
+            // build reports failure)
+            static_assert(kTile / kPlanTile + 2 <= 32, "one lane per plan tile of a reference tile");
+            auto wait_plan = [&](uint32_t first, uint32_t last) -> bool {
+                const uint32_t k = first / kPlanTile + (threadIdx.x & 31u);
+                const bool mine = k <= last / kPlanTile && k < ntn;
+                for (uint32_t spins = 0;; spins++) {
+                    const bool ready = !mine || __ldcv(pdone + k) == tag;
+                    if (__ballot_sync(0xffffffffu, !ready) == 0) break;
+                    if (spins >= A.spin_limit) {
+                        if (!ready) atomicOr(A.err, 4u);
+                        return false;
                     }
-                    __threadfence();
-                    s_wait_ok = ok;
+                    __nanosleep(32);
                 }
-                __syncthreads();
-                return s_wait_ok != 0;
+                __threadfence();
+                return true;
             };
-            ref_tile(R, rt, nr, tag, stop, rflags, raggs, rincls, shr_seg, wait_plan);
+            ref_tile(R, t - ntn, nr, tag, stop, rrecs, SM.shr_seg, wait_plan);
         } else {
             break;
         }
+        if (threadIdx.x == 0) SM.tile = atomicAdd(ticket, 1u);
     }
 }
 
-__global__ void __launch_bounds__(kScanThreads, 6) k_plan_refs(LevelArgs A, uint32_t *pflags, U7 *paggs, U7 *pincls,
-                                                            uint32_t *rflags, uint2 *raggs, uint2 *rincls,
-                                                            uint32_t *pdone, uint32_t *ticket) {
+// Four CTAs per SM, one resident wave: 64 registers keep the four references
+// of a thread in flight without spills, and fewer CTAs take fewer tickets (six
+// per SM, 40 registers: a 200k-triangle frame 1,950 us; five 1,930; four 1,905;
+// three and two 1,930 and 1,923, and the 1M-triangle frame 3,290 and 3,407
+// against 3,205).
+constexpr int kPlanGrid = 4;
+__global__ void __launch_bounds__(kScanThreads, kPlanGrid) k_plan_refs(LevelArgs A, uint32_t *pflags, U7 *paggs, U7 *pincls,
+                                                               ulonglong2 *rrecs, uint32_t *pdone, uint32_t *ticket) {
     __shared__ PlanSmem SM;
     wait_prior_grid();
     if (level_aborted(A)) return;
-    plan_refs_body(A, SM, pflags, paggs, pincls, rflags, raggs, rincls, pdone, ticket);
+    plan_refs_body(A, SM, pflags, paggs, pincls, rrecs, pdone, ticket);
 }
 
 // ---------------------------------------------------------------------------
@@ -2696,8 +2763,7 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
         float4 tlo = make_float4(0, 0, 0, 0), thi = tlo;
         if (lane < cnt0) {
             tri = A.defer_refs[rt.y + lane];
-            tlo = A.tb_lo[tri];
-            thi = A.tb_hi[tri];
+            load_bounds(A, tri, tlo, thi);
         }
         float4 nlo = tlo, nhi = thi;
         lane_bounds(nlo, nhi);
@@ -2981,13 +3047,13 @@ void build_release(BuildState &S) {
         if (p) cudaFree((void *)p);
         p = nullptr;
     };
-    f(S.tb_lo); f(S.tb_hi);
+    f(S.tb);
     for (int k = 0; k < 2; k++) {
         f(S.n_lo[k]); f(S.n_hi[k]); f(S.n_info[k]); f(S.refs[k]); f(S.ref_node[k]);
     }
     f(S.d_axis); f(S.d_plane); f(S.d_cnt); f(S.d_split); f(S.d_scat);
     f(S.chunks); f(S.hist); f(S.done); f(S.medium_slot); f(S.learn_slot); f(S.learn_bin); f(S.learn_prop); f(S.feat); f(S.prop_log);
-    f(S.plan_flags); f(S.ref_flags); f(S.plan_done); f(S.plan_agg); f(S.plan_incl); f(S.ref_agg); f(S.ref_incl); f(S.epoch);
+    f(S.plan_flags); f(S.ref_recs); f(S.plan_done); f(S.plan_agg); f(S.plan_incl); f(S.epoch);
     f(S.ctr); f(S.err);
     f(S.out_nodes); f(S.out_refs); f(S.out_ropes); f(S.out_cbox);
     f(S.d_root); f(S.d_lo); f(S.d_hi); f(S.defer_refs);
@@ -3044,8 +3110,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     }
     S.sub_tiles = S.cap_defer / kTile + 2;
     bool bad = false;
-    bad |= dalloc(S.tb_lo, nt) != cudaSuccess;
-    bad |= dalloc(S.tb_hi, nt) != cudaSuccess;
+    bad |= dalloc(S.tb, 2 * (size_t)nt) != cudaSuccess;
     for (int k = 0; k < 2; k++) {
         bad |= dalloc(S.n_lo[k], S.cap_level) != cudaSuccess;
         bad |= dalloc(S.n_hi[k], S.cap_level) != cudaSuccess;
@@ -3058,7 +3123,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     bad |= dalloc(S.d_cnt, S.cap_level) != cudaSuccess;
     bad |= dalloc(S.d_split, S.cap_level) != cudaSuccess;
     bad |= dalloc(S.d_scat, S.cap_level) != cudaSuccess;
-    bad |= dalloc(S.chunks, S.cap_chunks + S.cap_large) != cudaSuccess;  // tail holds large_slot
+    bad |= dalloc(S.chunks, S.cap_chunks) != cudaSuccess;
     bad |= dalloc(S.hist, (size_t)S.cap_large * kHist) != cudaSuccess;
     bad |= dalloc(S.done, S.cap_large) != cudaSuccess;
     bad |= dalloc(S.medium_slot, S.cap_medium) != cudaSuccess;
@@ -3068,7 +3133,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     bad |= dalloc(S.feat, (size_t)S.cap_learn * kMlpIn) != cudaSuccess;
     if (p.prop_log) bad |= dalloc(S.prop_log, (size_t)cap_nodes * 8) != cudaSuccess;
     bad |= dalloc(S.plan_flags, S.plan_tiles) != cudaSuccess;
-    bad |= dalloc(S.ref_flags, S.ref_tiles) != cudaSuccess;
+    bad |= dalloc(S.ref_recs, S.ref_tiles) != cudaSuccess;
     bad |= dalloc(S.plan_done, S.plan_tiles) != cudaSuccess;
     {
         U7 *pa = nullptr, *pi = nullptr;
@@ -3077,8 +3142,6 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
         S.plan_agg = pa;
         S.plan_incl = pi;
     }
-    bad |= dalloc(S.ref_agg, S.ref_tiles) != cudaSuccess;
-    bad |= dalloc(S.ref_incl, S.ref_tiles) != cudaSuccess;
     bad |= dalloc(S.epoch, 1) != cudaSuccess;
     bad |= dalloc(S.ctr, 1) != cudaSuccess;
     bad |= dalloc(S.err, 1) != cudaSuccess;
@@ -3116,7 +3179,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     cudaMemset(S.hist, 0, (size_t)S.cap_large * kHist * sizeof(uint32_t));
     cudaMemset(S.done, 0, (size_t)S.cap_large * sizeof(uint32_t));
     cudaMemset(S.plan_flags, 0, (size_t)S.plan_tiles * 4);
-    cudaMemset(S.ref_flags, 0, (size_t)S.ref_tiles * 4);
+    cudaMemset(S.ref_recs, 0, (size_t)S.ref_tiles * sizeof(ulonglong2));
     cudaMemset(S.plan_done, 0, (size_t)S.plan_tiles * 4);
     cudaMemset(S.sub_flags, 0, (size_t)S.sub_tiles * 4);
 
@@ -3160,15 +3223,13 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     const int G = S.sm_count * 4;
     LevelArgs A;
     memset(&A, 0, sizeof(A));
-    A.tb_lo = S.tb_lo;
-    A.tb_hi = S.tb_hi;
+    A.tb = S.tb;
     A.axis = S.d_axis;
     A.plane = S.d_plane;
     A.cnt = S.d_cnt;
     A.split = S.d_split;
     A.scat = S.d_scat;
     A.chunks = S.chunks;
-    A.large_slot = reinterpret_cast<uint32_t *>(S.chunks + S.cap_chunks);
     A.hist = S.hist;
     A.done = S.done;
     A.out_nodes = S.out_nodes;
@@ -3238,7 +3299,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     // the per-rank histograms and done counters are zero here: zeroed at
     // allocation, cleaned by the kernel that used them, and zeroed again by
     // build_read_stats after a build that stopped on an error
-    if (nt) k_tri_bounds<<<(nt + 255) / 256, 256, 0, st>>>(verts, tris, nt, S.tb_lo, S.tb_hi);
+    if (nt) k_tri_bounds<<<(nt + 255) / 256, 256, 0, st>>>(verts, tris, nt, S.tb);
     for (int k = 0; k < 2; k++) {
         A.lo_buf[k] = S.n_lo[k];
         A.hi_buf[k] = S.n_hi[k];
@@ -3259,9 +3320,9 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         if (binned_only) {
             // one wave (four CTAs per SM resident), grid-stride over the work
             launch_pdl(k_decide, S.sm_count * 4, 256, 0, st, A);
-            launch_pdl(k_plan_refs, S.sm_count * 6, kScanThreads, 0, st, A, S.plan_flags,
-                       static_cast<U7 *>(S.plan_agg), static_cast<U7 *>(S.plan_incl), S.ref_flags, S.ref_agg,
-                       S.ref_incl, S.plan_done, &A.lc->plan_ticket);
+            launch_pdl(k_plan_refs, S.sm_count * kPlanGrid, kScanThreads, 0, st, A, S.plan_flags,
+                       static_cast<U7 *>(S.plan_agg), static_cast<U7 *>(S.plan_incl), S.ref_recs, S.plan_done,
+                       &A.lc->plan_ticket);
             continue;
         }
         // large (and medium) nodes on the second stream, beside the small
@@ -3292,13 +3353,12 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         } else if (A.exact_max >= kWarpExact) {
             launch_pdl(k_small<true, false>, S.sm_count * 4, 256, 0, st, A);
         } else {
-            launch_pdl(k_small<false, false>, S.sm_count * 5, 256, 0, st, A);
+            launch_pdl(k_small<false, false>, S.sm_count * 4, 256, 0, st, A);
         }
         cudaStreamWaitEvent(st, S.ev_join, 0);
         if (A.learned) cudaStreamWaitEvent(st, S.ev_join2, 0);
-        launch_pdl(k_plan_refs, S.sm_count * 6, kScanThreads, 0, st, A, S.plan_flags, static_cast<U7 *>(S.plan_agg),
-                   static_cast<U7 *>(S.plan_incl), S.ref_flags, S.ref_agg, S.ref_incl, S.plan_done,
-                   &A.lc->plan_ticket);
+        launch_pdl(k_plan_refs, S.sm_count * kPlanGrid, kScanThreads, 0, st, A, S.plan_flags, static_cast<U7 *>(S.plan_agg),
+                   static_cast<U7 *>(S.plan_incl), S.ref_recs, S.plan_done, &A.lc->plan_ticket);
     }
     if (A.defer) {
         // every subtree (roots 0 .. the last level's total, tickets of level

@@ -107,7 +107,7 @@ struct BuildState {
     uint32_t last_err = 0;      // error bits of the last build: 2 arena capacity, 4 scan wait ran
                                 // out, 8 partition / decision count mismatch, 16 plan bounds
     // per-triangle bounds
-    float4 *tb_lo = nullptr, *tb_hi = nullptr;
+    float4 *tb = nullptr;   // triangle bounds, 2 per triangle (LevelArgs::tb)
     // level nodes (ping-pong)
     float4 *n_lo[2] = {nullptr, nullptr}, *n_hi[2] = {nullptr, nullptr};
     uint4 *n_info[2] = {nullptr, nullptr};      // start, count, cidx, -
@@ -117,18 +117,19 @@ struct BuildState {
     uint2 *d_cnt = nullptr;                      // below, above
     float4 *d_split = nullptr;                   // axis bits, plane, node min / max on the axis
     uint4 *d_scat = nullptr;                     // reference destinations (plan scan)
-    uint2 *chunks = nullptr;                     // (large rank, chunk index); tail: large_slot
+    uint4 *chunks = nullptr;                     // large rank, node slot, first reference, end
     uint32_t *hist = nullptr;                    // per large node 3 x 96
     uint32_t *done = nullptr;                    // per large node: chunks finished
     uint32_t *medium_slot = nullptr;             // exact-SAH medium nodes of the level
     // references (ping-pong)
     uint32_t *refs[2] = {nullptr, nullptr};
     uint32_t *ref_node[2] = {nullptr, nullptr};
-    // single-pass scan tile states (flags, aggregates, inclusive prefixes)
-    uint32_t *plan_flags = nullptr, *ref_flags = nullptr;
+    // single-pass scan tile states (flags, aggregates, inclusive prefixes; the
+    // reference tiles' in one record each)
+    uint32_t *plan_flags = nullptr;
+    ulonglong2 *ref_recs = nullptr;
     uint32_t *plan_done = nullptr;               // per plan tile: emitted (tag of the level)
     void *plan_agg = nullptr, *plan_incl = nullptr;
-    uint2 *ref_agg = nullptr, *ref_incl = nullptr;
     uint32_t plan_tiles = 0, ref_tiles = 0;
     uint32_t *epoch = nullptr;                   // build counter (scan flag tags)
     // second stream: large-node histograms run beside the small-node work;
