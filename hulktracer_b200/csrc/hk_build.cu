@@ -65,7 +65,8 @@ namespace hk {
 
 constexpr uint32_t kBins = 32;
 constexpr uint32_t kSmall = 256;     // nodes with <= kSmall refs: one warp per node
-constexpr uint32_t kChunk = 1024;    // refs per histogram CTA of a large node (4 per thread)
+constexpr uint32_t kChunk = 1024;    // most refs per histogram CTA of a large node (4 per thread)
+constexpr uint32_t kChunkMin = 256;
 constexpr uint32_t kWarpExact = 32;  // exact-SAH nodes up to this size: one warp, in registers
 constexpr uint32_t kLearnMax = 1024; // learned mode: nodes of kWarpExact + 1 .. kLearnMax refs are proposer rows
 constexpr uint32_t kHist = 3 * 3 * kBins;
@@ -624,13 +625,10 @@ struct LevelArgs {
 
 // true (on every thread of the CTA alike) when an earlier kernel of this build
 // hit an error after which its data may be inconsistent; the kernel then does
-// nothing. Called after wait_prior_grid by every thread.
+// nothing. Called after wait_prior_grid by every thread. (Loads that a kernel
+// issues before it overlap the error word's.)
 __device__ __forceinline__ bool level_aborted(const LevelArgs &A) {
-    __shared__ uint32_t s_abort;
-    __syncthreads();
-    if (threadIdx.x == 0) s_abort = __ldcg(A.err) & kErrAbort;
-    __syncthreads();
-    return s_abort != 0;
+    return __syncthreads_or((int)(__ldcg(A.err) & kErrAbort)) != 0;
 }
 
 __global__ void k_tri_bounds(const float4 *__restrict__ V, const uint4 *__restrict__ T, uint32_t nt, float4 *tb) {
@@ -679,6 +677,18 @@ __device__ __forceinline__ bool is_learn(const LevelArgs &A, uint32_t c) {
 __device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c) {
     return (c > kSmall || is_learn(A, c)) && !is_exact(A, c);
 }
+// References per chunk of a node of more than kChunk references, in a level
+// of `refs` references: small enough that the level's chunks fill k_decide's
+// one wave of four CTAs per SM (148 SMs), since a chunk of 256 takes 1.5 us less
+// than one of 1024 and the levels of small scenes have few of them. A node of
+// up to kChunk is one chunk: it then needs no sum in global memory.
+__device__ __forceinline__ uint32_t chunk_refs(uint32_t refs) {
+    const uint32_t per = refs / (4u * 148u);
+    return per <= kChunkMin ? kChunkMin : (per <= 2 * kChunkMin ? 2 * kChunkMin : kChunk);
+}
+__device__ __forceinline__ uint32_t node_chunks(uint32_t c, uint32_t per) {
+    return c <= kChunk ? 1u : (c + per - 1) / per;
+}
 // a decidable node of 2..A.defer references roots a deferred subtree
 constexpr uint32_t kDeferMax = 32;   // one reference per lane
 constexpr int kDeferAxis = -2;       // the decision that records a deferred root
@@ -692,7 +702,7 @@ __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
     const bool dec = nt > A.leaf_size && A.max_depth > 0;
     const bool medium = dec && is_medium(A, nt);
     const bool large = dec && is_large(A, nt);
-    const uint32_t nch = large ? (nt + kChunk - 1) / kChunk : 0u;
+    const uint32_t per = nt <= kChunk ? kChunk : chunk_refs(nt), nch = large ? node_chunks(nt, per) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *A.epoch += 1u;
         LevelCounters *l0 = &A.ctr->lvl[0];
@@ -720,7 +730,7 @@ __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
         A.ref_node()[i] = 0;
     }
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nch; k += gridDim.x * blockDim.x)
-        A.chunks[k] = make_uint4(0, 0, k * kChunk, min(nt, (k + 1) * kChunk));
+        A.chunks[k] = make_uint4(0, 0, k * per, min(nt, (k + 1) * per));
 }
 
 
@@ -1357,14 +1367,25 @@ struct HistSmem {
 
 // k_hist's work for one level (every CTA of the grid calls it): the chunks of
 // the large nodes and, with MEDIUM, the medium nodes (exact SAH, XS)
+// what a CTA's large-node work starts from, loaded before the kernel's first
+// barrier (the record of its first chunk is read whether the level has it or not)
+struct HistStart {
+    uint4 ck;
+    uint32_t nch, nmed, nodes;
+};
 template <bool MEDIUM>
-__device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, ExactSmem<256> *XSp, Tally &tally) {
+__device__ __forceinline__ HistStart hist_start(const LevelArgs &A) {
+    return HistStart{__ldcg(A.chunks + min(blockIdx.x, A.cap_chunks - 1)), min(__ldcg(&A.lc->n_chunks), A.cap_chunks),
+                     MEDIUM ? min(__ldcg(&A.lc->n_medium), A.cap_medium) : 0u, __ldcg(&A.lc->nodes)};
+}
+
+template <bool MEDIUM>
+__device__ __forceinline__ void hist_body(const LevelArgs &A, const HistStart &hs, HistSmem &SH, ExactSmem<256> *XSp,
+                                          Tally &tally) {
     uint32_t *H = SH.H;
     int &s_last = SH.last;
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t nch = min(A.lc->n_chunks, A.cap_chunks);
-    const uint32_t nmed = MEDIUM ? min(A.lc->n_medium, A.cap_medium) : 0u;
-    const uint32_t nodes = A.lc->nodes;
+    const uint32_t nch = hs.nch, nmed = hs.nmed, nodes = hs.nodes;
     for (uint32_t item = blockIdx.x; item < nch + nmed; item += gridDim.x) {
         if (MEDIUM && item >= nch) {
             // a medium node: the exact SAH in this CTA
@@ -1403,7 +1424,7 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
             }
             continue;
         }
-        const uint4 ck = A.chunks[item];
+        const uint4 ck = item == blockIdx.x ? hs.ck : A.chunks[item];
         const uint32_t rank = ck.x, s = ck.y, r0 = ck.z, r1 = ck.w;
         if (rank >= A.cap_large || s >= nodes) continue;   // uniform per CTA
         const uint4 info = A.n_info()[s];
@@ -1442,7 +1463,7 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, HistSmem &SH, Exac
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) {
-            const uint32_t nchunks = (info.y + kChunk - 1) / kChunk;
+            const uint32_t nchunks = node_chunks(info.y, chunk_refs(A.lc->refs));
             s_last = (atomicAdd(&A.done[rank], 1u) == nchunks - 1) ? 1 : 0;
         }
         __syncthreads();
@@ -1465,10 +1486,11 @@ __global__ void __launch_bounds__(256, 3) k_hist(LevelArgs A) {
     __shared__ HistSmem SH;
     __shared__ std::conditional_t<MEDIUM, ExactSmem<256>, uint32_t> XS;
     __shared__ uint32_t s_tally[kTallies];
+    const HistStart hs = hist_start<MEDIUM>(A);
     if (level_aborted(A)) return;
     Tally tally;
-    if constexpr (MEDIUM) hist_body<true>(A, SH, &XS, tally);
-    else hist_body<false>(A, SH, nullptr, tally);
+    if constexpr (MEDIUM) hist_body<true>(A, hs, SH, &XS, tally);
+    else hist_body<false>(A, hs, SH, nullptr, tally);
     tally_flush(A, tally, s_tally);
 }
 
@@ -1500,6 +1522,7 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
         const uint32_t s = g * 8 + wib;
         if (s >= nodes) continue;
         const uint4 info = A.n_info()[s];
+        const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];   // (with the record: one round trip)
         const uint32_t cnt = info.y;
         const bool dec = decidable(A, cnt);
         if (dec && (is_large(A, cnt) || is_medium(A, cnt))) continue;   // k_hist
@@ -1512,7 +1535,6 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
             }
             continue;
         }
-        const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
         Decision d;
         if (LEARNED || cnt <= kWarpExact) {
             // (learned mode: larger nodes are k_hist's)
@@ -1588,9 +1610,10 @@ __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
     __shared__ __align__(16) DecideSmem sm;
     __shared__ uint32_t s_tally[kTallies];
     wait_prior_grid();
+    const HistStart hs = hist_start<false>(A);
     if (level_aborted(A)) return;
     Tally tally;
-    hist_body<false>(A, sm.hist, nullptr, tally);
+    hist_body<false>(A, hs, sm.hist, nullptr, tally);
     __syncthreads();
     // the last CTAs take the first node groups: the first ones have the chunks
     small_body<false, false>(A, sm.small, tally, gridDim.x - 1 - blockIdx.x);
@@ -2220,7 +2243,7 @@ __device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t start, uin
         return;
     }
     if (!(dec && is_large(A, c))) return;
-    const uint32_t nch = (c + kChunk - 1) / kChunk;
+    const uint32_t per = c <= kChunk ? kChunk : chunk_refs(A.lc->t_childrefs), nch = node_chunks(c, per);
     const uint32_t rank = atomicAdd(&A.nlc->n_large, 1u);
     const uint32_t first = atomicAdd(&A.nlc->n_chunks, nch);
     if (rank >= A.cap_large || first + nch > A.cap_chunks) {
@@ -2228,7 +2251,7 @@ __device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t start, uin
         return;
     }
     for (uint32_t k = 0; k < nch; k++)
-        A.chunks[first + k] = make_uint4(rank, ns, start + k * kChunk, start + min(c, (k + 1) * kChunk));
+        A.chunks[first + k] = make_uint4(rank, ns, start + k * per, start + min(c, (k + 1) * per));
 }
 
 struct PlanCtx {
@@ -2251,21 +2274,24 @@ struct PlanOp {
     __device__ uint32_t tag() const { return level_tag(A); }
     __device__ uint32_t *err() const { return A.err; }
     __device__ Ctx ctx() const {
+        const LevelCounters *l = A.lc;
+        return Ctx{level_over(A) ? 1u : 0u, l->nodes_total, l->leafrefs_total, l->defer_refs_total,
+                   l->defer_nodes_total};
+    }
+    // the next level's counters (one thread of the launch)
+    __device__ void next_level(const Ctx &cx) const {
         LevelCounters *l = A.lc, *nx = A.nlc;
-        const bool over = level_over(A);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            l->stop = over ? 1u : 0u;
-            if (over) A.ctr->capacity_hit = 1;
-            nx->nodes = over ? 0u : l->t_next;
-            nx->refs = over ? 0u : l->t_childrefs;
-            nx->nodes_total = l->nodes_total + (over ? 0u : 2u * l->t_splits);
-            nx->leafrefs_total = l->leafrefs_total + (over ? l->refs : l->t_leafrefs);
-            nx->defer_refs_total = l->defer_refs_total + (over ? 0u : l->t_deferrefs);
-            nx->defer_nodes_total = l->defer_nodes_total + (over ? 0u : l->t_defernodes);
-            A.ctr->leaves += over ? l->nodes : l->t_leafnodes;
-            if (!over && l->t_next) A.ctr->depth = A.level + 1;
-        }
-        return Ctx{over ? 1u : 0u, l->nodes_total, l->leafrefs_total, l->defer_refs_total, l->defer_nodes_total};
+        const bool over = cx.stop != 0;
+        l->stop = over ? 1u : 0u;
+        if (over) A.ctr->capacity_hit = 1;
+        nx->nodes = over ? 0u : l->t_next;
+        nx->refs = over ? 0u : l->t_childrefs;
+        nx->nodes_total = cx.nodes_total + (over ? 0u : 2u * l->t_splits);
+        nx->leafrefs_total = cx.leafrefs_total + (over ? l->refs : l->t_leafrefs);
+        nx->defer_refs_total = cx.defer_refs_total + (over ? 0u : l->t_deferrefs);
+        nx->defer_nodes_total = cx.defer_nodes_total + (over ? 0u : l->t_defernodes);
+        A.ctr->leaves += over ? l->nodes : l->t_leafnodes;
+        if (!over && l->t_next) A.ctr->depth = A.level + 1;
     }
     __device__ Item load(uint32_t s, const Ctx &) const {
         if (s == 0xffffffffu) return Item{make_uint4(0, 0, 0, 0), make_uint2(0, 0), -1};
@@ -2588,16 +2614,21 @@ struct PlanSmem {
 
 __device__ __forceinline__ void plan_refs_body(const LevelArgs &A, PlanSmem &SM, uint32_t *pflags, U7 *paggs,
                                                U7 *pincls, ulonglong2 *rrecs, uint32_t *pdone, uint32_t *ticket) {
-    // the first ticket, on its way while the level's counters are read
-    if (threadIdx.x == 0) SM.tile = atomicAdd(ticket, 1u);
     const PlanOp P{A};
     const RefOp R{A};
+    // (the level's counters, read while the error word is)
     const uint32_t tag = level_tag(A);
-    const PlanCtx pc = P.ctx();                 // block 0 also writes the next level's counters
+    const PlanCtx pc = P.ctx();
     const uint32_t stop = pc.stop;              // the guard, decided from the tallies by every CTA
     const uint32_t nn = A.lc->nodes, nr = A.lc->refs;
+    if (level_aborted(A)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.next_level(pc);
     const uint32_t ntn = (nn + kPlanTile - 1) / kPlanTile;
     const uint32_t ntr = (nr + kTile - 1) / kTile;
+    // with a CTA per tile every CTA takes one ticket and the others none
+    const bool single = ntn + ntr <= gridDim.x;
+    if (single && blockIdx.x >= ntn + ntr) return;
+    if (threadIdx.x == 0) SM.tile = atomicAdd(ticket, 1u);
     for (;;) {
         __syncthreads();
         const uint32_t t = SM.tile;
@@ -2636,6 +2667,7 @@ __device__ __forceinline__ void plan_refs_body(const LevelArgs &A, PlanSmem &SM,
         } else {
             break;
         }
+        if (single) break;
         if (threadIdx.x == 0) SM.tile = atomicAdd(ticket, 1u);
     }
 }
@@ -2650,7 +2682,6 @@ __global__ void __launch_bounds__(kScanThreads, kPlanGrid) k_plan_refs(LevelArgs
                                                                ulonglong2 *rrecs, uint32_t *pdone, uint32_t *ticket) {
     __shared__ PlanSmem SM;
     wait_prior_grid();
-    if (level_aborted(A)) return;
     plan_refs_body(A, SM, pflags, paggs, pincls, rrecs, pdone, ticket);
 }
 
@@ -3092,7 +3123,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     S.alloc_depth = p.max_depth;
     S.cap_level = std::min(cap_refs, cap_nodes) + 1;
     S.cap_large = cap_refs / (kWarpExact + 1) + 2;   // learned mode: every node above 32 references
-    S.cap_chunks = cap_refs / kChunk + S.cap_large + 2;
+    S.cap_chunks = cap_refs / kChunkMin + S.cap_large + 2;
     S.cap_medium = cap_refs / (kWarpExact + 1) + 2;
     S.cap_learn = cap_refs / (kWarpExact + 1) + 2;
     S.plan_tiles = S.cap_level / kPlanTile + 2;
