@@ -1003,8 +1003,8 @@ static hk_status trace_enqueue(hk_ctx *c, const float4 *d_rays, uint32_t n, cons
     if (trace_smem_bytes(L.variant, c->cfg.block_size, L.stack_depth, false, occlusion, L.count) > kTraceMaxSmem)
         return fail(c, HK_E_ILLEGAL_INPUT,
                     "shared memory of this traversal exceeds 48 KB (short_stack x block_size x 12 + block_size x 8)");
-    int per_sm = c->cfg.blocks_per_sm ? (int)c->cfg.blocks_per_sm : std::max(1, 2048 / L.block);
-    L.grid = c->sm_count * per_sm;
+    L.grid = c->sm_count * (int)c->cfg.blocks_per_sm;   // 0: one resident wave
+    L.sm_count = c->sm_count;
     if (c->counting) HK_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 24, c->stream));
     HK_CUDA(c, launch_trace(L, c->stream));
     return HK_OK;
@@ -1529,8 +1529,8 @@ hk_status hk_batch_trace_device(hk_batch *b, const float *d_rays8, const uint32_
     L.variant = (int)v;
     L.count = c->counting;
     L.block = (int)c->cfg.block_size;
-    int per_sm = c->cfg.blocks_per_sm ? (int)c->cfg.blocks_per_sm : std::max(1, 2048 / L.block);
-    L.grid = c->sm_count * per_sm;
+    L.grid = c->sm_count * (int)c->cfg.blocks_per_sm;   // 0: one resident wave
+    L.sm_count = c->sm_count;
     L.scenes = b->table.p;
     L.ray_offsets = b->offsets.p;
     L.nscenes = nscenes;

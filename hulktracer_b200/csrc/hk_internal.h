@@ -42,7 +42,9 @@ struct TraceLaunch {
     bool count;
     bool occlusion;             // shadow rays: origin w = light distance, stop at the first hit closer than it
     uint32_t *leaf_out;         // ropes: per ray, the leaf its traversal ended in (a start hint), or nullptr
-    int grid, block;
+    int block;
+    int grid;                   // blocks, or 0: one resident wave on sm_count SMs
+    int sm_count;
     // ropes
     const uint32_t *ropes;      // 6 per node
     const float4 *cbox;         // 2 per node (min, max)
@@ -69,6 +71,12 @@ constexpr size_t kTraceMaxSmem = 48 * 1024;
 // closest-hit kernel. The kernel and the launcher both use this.
 __host__ __device__ constexpr bool trace_coop_slots(int variant, bool batch, bool any) {
     return variant != HK_TRACE_BRUTE && !batch && !any;
+}
+
+// Blocks of kTraceMaxBlock threads that an instantiation is compiled to keep
+// resident on an SM (its __launch_bounds__; smaller blocks in proportion).
+__host__ __device__ constexpr uint32_t trace_resident_blocks(int variant, bool batch, bool any) {
+    return batch ? 4u : ((variant != HK_TRACE_BRUTE && !any) ? 5u : 6u);
 }
 
 // dynamic shared memory of one trace launch: the shared-memory ring of

@@ -154,7 +154,7 @@ extern "C" hk_status hk_render_noalloc(const uint32_t *d_nodes2, const uint32_t 
     L.variant = (int)variant;
     L.count = false;
     L.block = 128;
-    L.grid = sm * 16;
+    L.sm_count = sm;
     HK_TRY(launch_camera_rays(cam, w, h, rays, s));
     L.rays = rays;
     L.hits = hits;

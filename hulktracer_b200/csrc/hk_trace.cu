@@ -8,6 +8,8 @@
 // "child 0" sentinel, strict < between hits in leaf order); see the comments
 // at each variant. Closest-hit single-scene launches test the leaves of a
 // whole warp together (coop_leaf), which keeps the same hits bit for bit.
+#include <algorithm>
+
 #include "hk_common.cuh"
 #include "hk_internal.h"
 
@@ -82,21 +84,19 @@ __device__ __forceinline__ float comp(float3 v, uint32_t a) { return a == 0 ? v.
 
 // child selection result: node index (0 = the reference's "no child", i.e.
 // the root) and the node itself
-__device__ __forceinline__ void pick_child(const uint2 *nodes, uint32_t pair, bool take_below,
+__device__ __forceinline__ void pick_child(uint2 nb, uint2 na, uint32_t pair, bool take_below,
                                            uint32_t &idx, uint2 &node, uint2 root) {
-    uint32_t c = take_below ? pair : pair + 1;
-    uint2 n = nodes[c];
+    const uint2 n = take_below ? nb : na;
     if (is_leaf(n) && n.y == 0) {
         idx = 0;
         node = root;
     } else {
-        idx = c;
+        idx = take_below ? pair : pair + 1;
         node = n;
     }
 }
 
-__device__ __forceinline__ uint32_t sentinel_to_root(const uint2 *nodes, uint32_t c) {
-    uint2 n = nodes[c];
+__device__ __forceinline__ uint32_t sentinel_to_root(uint2 n, uint32_t c) {
     return (is_leaf(n) && n.y == 0) ? 0u : c;
 }
 
@@ -168,16 +168,17 @@ __device__ __forceinline__ bool leg_shortstack(const TraceArgs &A, const SceneVi
             return true;
         }
         uint32_t axis = L.node.x & 3u, pair = L.node.x >> 2;
+            const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
         float pl = __int_as_float(L.node.y);
         float rs = comp(L.o, axis), dc = comp(L.d, axis);
         float split = __fmul_rn(__fsub_rn(pl, rs), comp(L.inv, axis));
         bool below_first = (rs < pl) || (rs == pl && dc <= 0.0f);
         if (split >= L.tmax || split <= 0.0f) {
-            pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, below_first, L.cur, L.node, root);
         } else if (split <= L.tmin) {
-            pick_child(V.nodes, pair, !below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, !below_first, L.cur, L.node, root);
         } else {
-            uint32_t second = sentinel_to_root(V.nodes, below_first ? pair + 1 : pair);
+            uint32_t second = sentinel_to_root(below_first ? na : nb, below_first ? pair + 1 : pair);
             if (SMEM) {
                 s_s[L.idx * stride + tid] = split;
                 s_e[L.idx * stride + tid] = L.tmax;
@@ -190,7 +191,7 @@ __device__ __forceinline__ bool leg_shortstack(const TraceArgs &A, const SceneVi
             L.idx = (L.idx + 1) % (int)D;
             L.size++;
             L.size = L.size > (int)D ? (int)D : L.size;
-            pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, below_first, L.cur, L.node, root);
             L.tmax = split;
         }
         if (L.cur == 0) break;
@@ -234,23 +235,24 @@ __device__ __forceinline__ bool leg_fullstack(const TraceArgs &A, const SceneVie
             tested = true;
         } else {
             uint32_t axis = L.node.x & 3u, pair = L.node.x >> 2;
+            const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
             float pl = __int_as_float(L.node.y);
             float rs = comp(L.o, axis), dc = comp(L.d, axis);
             float split = __fmul_rn(__fsub_rn(pl, rs), comp(L.inv, axis));
             bool below_first = (rs < pl) || (rs == pl && dc <= 0.0f);
             if (split > L.tmax || split <= 0.0f) {
-                pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+                pick_child(nb, na, pair, below_first, L.cur, L.node, root);
             } else if (split < L.tmin) {
-                pick_child(V.nodes, pair, !below_first, L.cur, L.node, root);
+                pick_child(nb, na, pair, !below_first, L.cur, L.node, root);
             } else {
-                uint32_t second = sentinel_to_root(V.nodes, below_first ? pair + 1 : pair);
+                uint32_t second = sentinel_to_root(below_first ? na : nb, below_first ? pair + 1 : pair);
                 if (second != 0 && L.size < max_stack) {
                     st_n[L.size] = second;
                     st_s[L.size] = split;
                     st_e[L.size] = L.tmax;
                     L.size++;
                 }
-                pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+                pick_child(nb, na, pair, below_first, L.cur, L.node, root);
                 L.tmax = split;
             }
         }
@@ -286,16 +288,17 @@ __device__ __forceinline__ bool leg_restart(const TraceArgs &A, const SceneView 
             return true;
         }
         uint32_t axis = L.node.x & 3u, pair = L.node.x >> 2;
+            const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
         float pl = __int_as_float(L.node.y);
         float rs = comp(L.o, axis), dc = comp(L.d, axis);
         float split = __fmul_rn(__fsub_rn(pl, rs), comp(L.inv, axis));
         bool below_first = (rs < pl) || (rs == pl && dc <= 0.0f);
         if (split >= L.tmax || split <= 0.0f) {
-            pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, below_first, L.cur, L.node, root);
         } else if (split <= L.tmin) {
-            pick_child(V.nodes, pair, !below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, !below_first, L.cur, L.node, root);
         } else {
-            pick_child(V.nodes, pair, below_first, L.cur, L.node, root);
+            pick_child(nb, na, pair, below_first, L.cur, L.node, root);
             L.tmax = split;
         }
         if (L.cur == 0) break;
@@ -312,86 +315,11 @@ __device__ __forceinline__ bool leg_restart(const TraceArgs &A, const SceneView 
     return false;
 }
 
-// one leg of the ropes traversal (no reference counterpart; restated in the
-// oracle's search_ropes): locate the leaf cell holding o + d*tentry from the
-// current node (ties on a plane go to the side the ray moves into), test it,
-// stop when the closest hit precedes the cell's exit, else follow the rope of
-// the exit face. Legs are bounded by 4 * nodes + 8. ropes_locate does the
-// descent and the exit face (true = the leg bound ran out), the leaf test
-// follows, ropes_advance decides and follows the rope (true = finished).
-template <bool COUNT>
-__device__ __forceinline__ bool ropes_locate(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
-                                             uint32_t &lstart, uint32_t &lcnt, float &texit, int &face) {
-    if (++L.size > (int)legs_max) return true;
-    float p[3] = {__fadd_rn(L.o.x, __fmul_rn(L.d.x, L.tmin)), __fadd_rn(L.o.y, __fmul_rn(L.d.y, L.tmin)),
-                  __fadd_rn(L.o.z, __fmul_rn(L.d.z, L.tmin))};
-    uint2 node = A.nodes[L.cur];
-    while (!is_leaf(node)) {
-        if (COUNT) c_nodes++;
-        uint32_t axis = node.x & 3u, pair = node.x >> 2;
-        float pl = __int_as_float(node.y);
-        float pc = axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2]);
-        bool below = (pc < pl) || (pc == pl && comp(L.d, axis) <= 0.0f);
-        L.cur = below ? pair : pair + 1;
-        node = A.nodes[L.cur];
-    }
-    const float4 blo = A.cbox[2 * (size_t)L.cur], bhi = A.cbox[2 * (size_t)L.cur + 1];
+// the distance at which the ray leaves the cell (at most te) and the face it
+// leaves by (2 axis + side; -1: none before te)
+constexpr uint32_t kNoRope = 0xffffffffu;
+__device__ __forceinline__ int cell_exit(const LaneState &L, float4 blo, float4 bhi, float &texit) {
     texit = L.te;
-    face = -1;
-    const float o3[3] = {L.o.x, L.o.y, L.o.z}, d3[3] = {L.d.x, L.d.y, L.d.z}, i3[3] = {L.inv.x, L.inv.y, L.inv.z};
-    const float lo3[3] = {blo.x, blo.y, blo.z}, hi3[3] = {bhi.x, bhi.y, bhi.z};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        if (d3[k] > 0.0f) {
-            float tt = __fmul_rn(__fsub_rn(hi3[k], o3[k]), i3[k]);
-            if (tt < texit) {
-                texit = tt;
-                face = 2 * k + 1;
-            }
-        } else if (d3[k] < 0.0f) {
-            float tt = __fmul_rn(__fsub_rn(lo3[k], o3[k]), i3[k]);
-            if (tt < texit) {
-                texit = tt;
-                face = 2 * k;
-            }
-        }
-    }
-    if (COUNT) c_nodes++;
-    lstart = node.x >> 2;
-    lcnt = node.y;
-    return false;
-}
-
-template <bool ANY>
-__device__ __forceinline__ bool ropes_advance(const SceneView &A, LaneState &L, uint32_t lcnt, float texit, int face) {
-    if (lcnt && (L.best < texit || (ANY && L.best < L.lim))) return true;
-    if (face < 0) return true;
-    uint32_t r = A.ropes[6 * (size_t)L.cur + face];
-    if (r == 0xffffffffu) return true;
-    L.tmin = texit > L.tmin ? texit : L.tmin;
-    L.cur = r;
-    return false;
-}
-
-// the whole leg with the in-order leaf test (occlusion rays, batches)
-template <bool COUNT, bool ANY>
-__device__ __forceinline__ bool leg_ropes(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
-                                          uint32_t &c_refs) {
-    if (++L.size > (int)legs_max) return true;
-    float p[3] = {__fadd_rn(L.o.x, __fmul_rn(L.d.x, L.tmin)), __fadd_rn(L.o.y, __fmul_rn(L.d.y, L.tmin)),
-                  __fadd_rn(L.o.z, __fmul_rn(L.d.z, L.tmin))};
-    uint2 node = A.nodes[L.cur];
-    while (!is_leaf(node)) {
-        if (COUNT) c_nodes++;
-        uint32_t axis = node.x & 3u, pair = node.x >> 2;
-        float pl = __int_as_float(node.y);
-        float pc = axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2]);
-        bool below = (pc < pl) || (pc == pl && comp(L.d, axis) <= 0.0f);
-        L.cur = below ? pair : pair + 1;
-        node = A.nodes[L.cur];
-    }
-    const float4 blo = A.cbox[2 * (size_t)L.cur], bhi = A.cbox[2 * (size_t)L.cur + 1];
-    float texit = L.te;
     int face = -1;
     const float o3[3] = {L.o.x, L.o.y, L.o.z}, d3[3] = {L.d.x, L.d.y, L.d.z}, i3[3] = {L.inv.x, L.inv.y, L.inv.z};
     const float lo3[3] = {blo.x, blo.y, blo.z}, hi3[3] = {bhi.x, bhi.y, bhi.z};
@@ -411,17 +339,61 @@ __device__ __forceinline__ bool leg_ropes(const SceneView &A, LaneState &L, uint
             }
         }
     }
-    if (COUNT) c_nodes++;
-    if (node.y) {
-        test_leaf<COUNT, ANY>(A, node, L.o, L.d, L.best, L.best_id, c_refs, L.lim);
-        if (L.best < texit || (ANY && L.best < L.lim)) return true;
+    return face;
+}
+
+// one leg of the ropes traversal (no reference counterpart; restated in the
+// oracle's search_ropes): locate the leaf cell holding o + d*tentry from the
+// current node (ties on a plane go to the side the ray moves into), test it,
+// stop when the closest hit precedes the cell's exit, else follow the rope of
+// the exit face. Legs are bounded by 4 * nodes + 8. ropes_locate does the
+// descent and the exit face (true = the leg bound ran out), the leaf test
+// follows, ropes_advance decides and follows the rope (true = finished).
+template <bool COUNT>
+__device__ __forceinline__ bool ropes_locate(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
+                                             uint32_t &lstart, uint32_t &lcnt, float &texit, uint32_t &rope) {
+    if (++L.size > (int)legs_max) return true;
+    float p[3] = {__fadd_rn(L.o.x, __fmul_rn(L.d.x, L.tmin)), __fadd_rn(L.o.y, __fmul_rn(L.d.y, L.tmin)),
+                  __fadd_rn(L.o.z, __fmul_rn(L.d.z, L.tmin))};
+    uint2 node = A.nodes[L.cur];
+    while (!is_leaf(node)) {
+        if (COUNT) c_nodes++;
+        uint32_t axis = node.x & 3u, pair = node.x >> 2;
+        const uint2 nb = A.nodes[pair], na = A.nodes[pair + 1];
+        float pl = __int_as_float(node.y);
+        float pc = axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2]);
+        bool below = (pc < pl) || (pc == pl && comp(L.d, axis) <= 0.0f);
+        L.cur = below ? pair : pair + 1;
+        node = below ? nb : na;
     }
-    if (face < 0) return true;
-    uint32_t r = A.ropes[6 * (size_t)L.cur + face];
-    if (r == 0xffffffffu) return true;
-    L.tmin = texit > L.tmin ? texit : L.tmin;
-    L.cur = r;
+    const float4 blo = A.cbox[2 * (size_t)L.cur], bhi = A.cbox[2 * (size_t)L.cur + 1];
+    const int face = cell_exit(L, blo, bhi, texit);
+    if (COUNT) c_nodes++;
+    // the node across the exit face, on its way while the leaf is tested
+    rope = face >= 0 ? A.ropes[6 * (size_t)L.cur + face] : kNoRope;
+    lstart = node.x >> 2;
+    lcnt = node.y;
     return false;
+}
+
+template <bool ANY>
+__device__ __forceinline__ bool ropes_advance(LaneState &L, uint32_t lcnt, float texit, uint32_t rope) {
+    if (lcnt && (L.best < texit || (ANY && L.best < L.lim))) return true;
+    if (rope == kNoRope) return true;
+    L.tmin = texit > L.tmin ? texit : L.tmin;
+    L.cur = rope;
+    return false;
+}
+
+// the whole leg with the in-order leaf test (occlusion rays, batches)
+template <bool COUNT, bool ANY>
+__device__ __forceinline__ bool leg_ropes(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
+                                          uint32_t &c_refs) {
+    uint32_t lstart, lcnt, rope;
+    float texit;
+    if (ropes_locate<COUNT>(A, L, legs_max, c_nodes, lstart, lcnt, texit, rope)) return true;
+    if (lcnt) test_leaf<COUNT, ANY>(A, make_uint2(lstart << 2, lcnt), L.o, L.d, L.best, L.best_id, c_refs, L.lim);
+    return ropes_advance<ANY>(L, lcnt, texit, rope);
 }
 
 // The leaf tests of a whole warp shared out over its 32 lanes (all lanes call
@@ -506,8 +478,7 @@ __device__ __forceinline__ uint32_t scene_of(const uint32_t *off, uint32_t nscen
 // traversal's, so "some hit closer than the light" is found exactly when the
 // closest-hit traversal's answer is closer than the light, in every variant.
 template <int VARIANT, bool COUNT, bool BATCH, bool ANY>
-__global__ void __launch_bounds__(kTraceMaxBlock, BATCH ? 4 : ((VARIANT != HK_TRACE_BRUTE && !ANY) ? 5 : 6))
-    k_trace(TraceArgs A) {
+__global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT, BATCH, ANY)) k_trace(TraceArgs A) {
     extern __shared__ float smem[];
     const bool smem_ring = (VARIANT == HK_TRACE_SMEMSTACK);
     float *s_s = smem;
@@ -534,6 +505,11 @@ __global__ void __launch_bounds__(kTraceMaxBlock, BATCH ? 4 : ((VARIANT != HK_TR
         __syncwarp();
     }
     const uint32_t n = A.n_dev ? *A.n_dev : A.n;
+    // Fewer rays than lanes: every warp takes an even share on its first lanes,
+    // so that the rays spread over all warps, a warp waits for fewer of them at
+    // each step, and its other lanes only share the leaf tests.
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const bool takes = lane < max(1u, min(32u, (n + warps - 1) / warps));
     if (BATCH && threadIdx.x == 0) atomicMin(A.start_ns, global_ns());
     // scene arrays: launch-uniform for one scene, per lane in a batch
     SceneView V{A.nodes, A.refs, A.tris, A.ropes, A.cbox};
@@ -558,14 +534,14 @@ __global__ void __launch_bounds__(kTraceMaxBlock, BATCH ? 4 : ((VARIANT != HK_TR
     uint32_t steps = 0;
     while (true) {
         // refill idle lanes
-        uint32_t idle = __ballot_sync(0xffffffffu, !active);
+        uint32_t idle = __ballot_sync(0xffffffffu, !active && takes);
         if (idle && !drained) {
             uint32_t want = __popc(idle);
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(A.fetch, want);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (base + want >= n) drained = true;
-            if (!active) {
+            if (!active && takes) {
                 uint32_t rid = base + __popc(idle & lt_mask);
                 if (rid < n) {
                     if (BATCH) {
@@ -644,14 +620,14 @@ __global__ void __launch_bounds__(kTraceMaxBlock, BATCH ? 4 : ((VARIANT != HK_TR
             // every lane takes part in the warp's leaf tests
             uint32_t lstart = 0, lcnt = 0;
             float texit = 0.0f;
-            int face = -1;
+            uint32_t rope = kNoRope;
             bool fin = false;
-            if (active) fin = ropes_locate<COUNT>(V, L, legs_max, c_nodes, lstart, lcnt, texit, face);
+            if (active) fin = ropes_locate<COUNT>(V, L, legs_max, c_nodes, lstart, lcnt, texit, rope);
             const uint32_t work = (active && !fin) ? lcnt : 0u;
             coop_leaf(V, L, lstart, work, slot);
             if (COUNT) c_refs += work;
             if (!active) continue;
-            if (fin || ropes_advance<ANY>(V, L, lcnt, texit, face)) {
+            if (fin || ropes_advance<ANY>(L, lcnt, texit, rope)) {
                 A.hits[L.ray] = hk_hit{L.best, L.best_id};
                 if (A.leaf_out) A.leaf_out[L.ray] = L.cur;
                 active = false;
@@ -802,7 +778,13 @@ cudaError_t launch_trace(const TraceLaunch &L, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (L.n == 0 && L.n_dev == nullptr) return cudaSuccess;
     int block = L.block;
-    int grid = L.grid;
+    // one resident wave: a warp beyond it would find no rays left (batches keep
+    // more than their bound's threads resident at 128 a block: as many as an SM
+    // has)
+    const uint32_t threads =
+        L.scenes ? 2048u : trace_resident_blocks(L.variant, false, L.occlusion && !L.count) * kTraceMaxBlock;
+    const int wave = L.sm_count * (int)std::max(1u, threads / (uint32_t)std::max(block, 32));
+    int grid = L.grid > 0 ? L.grid : wave;
     const size_t smem =
         trace_smem_bytes(L.variant, (uint32_t)block, L.stack_depth, L.scenes != nullptr, L.occlusion, L.count);
     if (block < 32 || (uint32_t)block > kTraceMaxBlock || smem > kTraceMaxSmem) return cudaErrorInvalidConfiguration;
