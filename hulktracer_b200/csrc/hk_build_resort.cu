@@ -27,6 +27,13 @@
 //            a split node; a stable partition (scans) writes the next level's
 //            lists in the reference's list order, below child then above
 //
+// A level is nine launches (more while segments are long enough for the radix
+// sort): every scan is one single-pass kernel that computes what it sums (the
+// candidate counts, the group heads, the decisions, the classification) as it
+// loads it, sizes that the host needs for the next level come back in one
+// read, and launches in between take theirs from device memory. Three launches
+// per scan and two reads per level took 5.1 ms for 59,280 triangles.
+//
 // The output is the compact tree the traversal kernels read (child pairs in
 // breadth-first order: below, above; an absent child is an empty leaf cell),
 // with the ropes and cell boxes of every cell. It is the tree of the
@@ -37,6 +44,7 @@
 
 #include "hk_common.cuh"
 #include "hk_resort.h"
+#include "hk_scan.cuh"
 
 namespace hk {
 
@@ -86,113 +94,72 @@ cudaError_t grow_keep(RBuf<T> &b, size_t n, size_t keep, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------- scans ----
-constexpr int kSB = 512;  // threads per scan block
-constexpr int kSI = 8;    // elements per thread
+constexpr int kScanNT = 256;    // threads per scan tile
+constexpr int kScanItems = 4;   // elements per thread
+constexpr uint32_t kScanTile = kScanNT * kScanItems;
+constexpr uint32_t kScanSpins = 1u << 22;   // polls before a wait gives up (error word)
 
-template <class T>
-__device__ __forceinline__ T warp_incl(T v) {
-    const int lane = threadIdx.x & 31;
+// tile states of a scan and its ticket; every scan of a build has a tag and a
+// ticket of its own
+struct ScanPtrs {
+    uint32_t *flags, *ticket, *err;
+    uint4 *aggs, *incls;   // uint2 scans use their first half
+    uint32_t tag;
+};
+
+// one scan: op.count() elements, op.load(i) -> Item, op.value(Item) -> T,
+// op.apply(i, exclusive prefix, Item), op.finish(total) by one thread
+template <class Op>
+__global__ void __launch_bounds__(kScanNT) k_r_scan(Op op, ScanPtrs sp) {
+    using T = typename Op::T;
+    __shared__ T sw[kScanNT / 32];
+    __shared__ T s_excl;
+    __shared__ uint32_t s_tile;
+    const uint32_t n = op.count();
+    const uint32_t ntiles = n ? (n + kScanTile - 1) / kScanTile : 1u;
+    T *aggs = reinterpret_cast<T *>(sp.aggs), *incls = reinterpret_cast<T *>(sp.incls);
+    for (;;) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(sp.ticket, 1u);
+        __syncthreads();
+        const uint32_t tile = s_tile;
+        if (tile >= ntiles) break;
+        const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
+        typename Op::Item it[kScanItems];
+        T v[kScanItems], s = vzero<T>();
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += y;
-    }
-    return v;
-}
-
-// exclusive block scan; *total (if given) receives the block's sum
-template <class T>
-__device__ T block_excl(T v, T *sw, T *total) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const T inc = warp_incl(v);
-    if (lane == 31) sw[w] = inc;
-    __syncthreads();
-    if (w == 0) {
-        T s = lane < nw ? sw[lane] : T(0);
-        s = warp_incl(s);
-        sw[lane] = s;
-    }
-    __syncthreads();
-    const T base = w ? sw[w - 1] : T(0);
-    if (total) *total = sw[nw - 1];
-    __syncthreads();
-    return base + inc - v;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kSB) k_scan_reduce(const T *__restrict__ in, uint32_t n, T *part) {
-    __shared__ T sw[32];
-    const size_t base = (size_t)blockIdx.x * kSB * kSI;
-    T s = 0;
-#pragma unroll
-    for (int k = 0; k < kSI; k++) {
-        const size_t i = base + (size_t)k * kSB + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    T tot;
-    block_excl(s, sw, &tot);
-    if (threadIdx.x == 0) part[blockIdx.x] = tot;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kSB) k_scan_part(T *part, uint32_t nb) {
-    __shared__ T sw[32];
-    T carry = 0;
-    for (uint32_t b0 = 0; b0 < nb; b0 += kSB) {
-        const uint32_t i = b0 + threadIdx.x;
-        const T v = i < nb ? part[i] : T(0);
+        for (int k = 0; k < kScanItems; k++) {
+            v[k] = vzero<T>();
+            if (base + k < n) {
+                it[k] = op.load(base + k);
+                v[k] = op.value(it[k]);
+            }
+            s = vadd(s, v[k]);
+        }
         T tot;
-        const T e = block_excl(v, sw, &tot);
-        if (i < nb) part[i] = carry + e;
-        carry += tot;
-    }
-    if (threadIdx.x == 0) part[nb] = carry;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kSB) k_scan_down(const T *in, uint32_t n, const T *__restrict__ part, T *out) {
-    __shared__ T sw[32];
-    const size_t base = (size_t)blockIdx.x * kSB * kSI + (size_t)threadIdx.x * kSI;
-    T v[kSI];
-    T s = 0;
+        const T ex = block_excl<kScanNT>(s, sw, tot);
+        tile_prefix(tile, tot, sp.tag, sp.flags, aggs, incls, &s_excl, sp.err, kScanSpins);
+        T pre = vadd(s_excl, ex);
 #pragma unroll
-    for (int k = 0; k < kSI; k++) {
-        const size_t i = base + k;
-        v[k] = i < n ? in[i] : T(0);
-        s += v[k];
+        for (int k = 0; k < kScanItems; k++) {
+            if (base + k < n) op.apply(base + k, pre, it[k]);
+            pre = vadd(pre, v[k]);
+        }
+        if (tile == ntiles - 1 && threadIdx.x == 0) op.finish(vadd(s_excl, tot));
+        __syncthreads();
     }
-    T e = block_excl(s, sw, (T *)nullptr) + part[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kSI; k++) {
-        const size_t i = base + k;
-        if (i < n) out[i] = e;
-        e += v[k];
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = part[gridDim.x];
-}
-
-// out[0..n] = exclusive prefix sums of in[0..n) and the total; out may be in
-template <class T>
-cudaError_t scan_excl(const T *in, T *out, uint32_t n, RBuf<T> &part, cudaStream_t st) {
-    const uint32_t per = (uint32_t)(kSB * kSI);
-    uint32_t nb = (n + per - 1) / per;
-    if (nb == 0) nb = 1;
-    cudaError_t e = part.ensure(nb + 1);
-    if (e != cudaSuccess) return e;
-    k_scan_reduce<T><<<nb, kSB, 0, st>>>(in, n, part.p);
-    k_scan_part<T><<<1, kSB, 0, st>>>(part.p, nb);
-    k_scan_down<T><<<nb, kSB, 0, st>>>(in, n, part.p, out);
-    return cudaGetLastError();
 }
 
 // ----------------------------------------------------------- radix sort ----
 constexpr int kRT = 256;                     // threads per sort tile
-constexpr int kRI = 16;                      // keys per thread
-constexpr uint32_t kTile = kRT * kRI;        // 4096 keys per tile
+constexpr int kRI = 4;                       // keys per thread
+// 1024 keys per tile: the levels that need this sort have few keys per SM, and
+// a tile's rounds follow one another (4096 keys: 22 us a pass for 70,000 keys)
+constexpr uint32_t kTile = kRT * kRI;
 
-__global__ void __launch_bounds__(kRT) k_rs_hist(const u64 *__restrict__ keys, uint32_t n, int shift,
-                                                 uint32_t ntiles, uint32_t *hist) {
+__global__ void __launch_bounds__(kRT) k_rs_hist(const u64 *__restrict__ keys, const uint32_t *__restrict__ nkeys,
+                                                 int shift, uint32_t ntiles, uint32_t *hist) {
     __shared__ uint32_t h[256];
+    const uint32_t n = *nkeys;
     h[threadIdx.x] = 0;
     __syncthreads();
     const size_t base = (size_t)blockIdx.x * kTile;
@@ -204,13 +171,27 @@ __global__ void __launch_bounds__(kRT) k_rs_hist(const u64 *__restrict__ keys, u
     hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
+// exclusive prefix of the tiles' counts, digit by digit
+struct RsScanOp {
+    using T = uint2;
+    using Item = uint32_t;
+    uint32_t *hist;
+    uint32_t n;
+    __device__ uint32_t count() const { return n; }
+    __device__ Item load(uint32_t i) const { return hist[i]; }
+    __device__ T value(const Item &it) const { return make_uint2(it, 0); }
+    __device__ void apply(uint32_t i, T pre, const Item &) const { hist[i] = pre.x; }
+    __device__ void finish(T) const {}
+};
+
 // stable scatter: within a tile keys are ranked in index order (rounds of
 // 256 consecutive keys; warps in order; lanes by __match_any_sync)
-__global__ void __launch_bounds__(kRT) k_rs_scatter(const u64 *__restrict__ in, u64 *__restrict__ out, uint32_t n,
-                                                    int shift, uint32_t ntiles, const uint32_t *__restrict__ offs) {
+__global__ void __launch_bounds__(kRT) k_rs_scatter(const u64 *__restrict__ in, u64 *__restrict__ out,
+                                                    const uint32_t *__restrict__ nkeys, int shift, uint32_t ntiles,
+                                                    const uint32_t *__restrict__ offs) {
     __shared__ uint32_t run[256];
     __shared__ uint32_t wc[kRT / 32][256];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, n = *nkeys;
     run[threadIdx.x] = 0;
     const size_t base = (size_t)blockIdx.x * kTile;
     for (int r = 0; r < kRI; r++) {
@@ -267,6 +248,10 @@ __device__ __forceinline__ float key_value(u64 k) { return o2f((uint32_t)(k >> 2
 __device__ __forceinline__ uint32_t lo32(u64 x) { return (uint32_t)x; }
 __device__ __forceinline__ uint32_t hi32(u64 x) { return (uint32_t)(x >> 32); }
 
+// sizes that a level leaves for the host (and, SK_MAXCNT, the next level's
+// largest node that has candidates)
+enum { SK_JUNCTIONS = 0, SK_REFS, SK_LEAFREFS, SK_MAXCNT, SK_ERR, SK_WORDS };
+
 struct LevelPtrs {
     // this level
     uint32_t n;
@@ -274,10 +259,12 @@ struct LevelPtrs {
     const float *surf;
     const uint32_t *off, *cnt, *ropes, *refs, *ref_node;
     // scratch
-    uint32_t *nkeys, *koff, *jflag, *jrank, *leafcnt, *loff, *efirst, *decision, *gfirst;
+    uint32_t *koff, *jrank, *loff, *efirst, *decision, *gfirst;
     float *plane, *surf_lo, *surf_hi;
-    u64 *best, *keys, *f1, *f2, *rflag, *rscan;
-    uint32_t *maxseg;   // longest candidate segment of the level
+    u64 *best, *keys;
+    uint4 *sweep;       // per key: begins and co-planars, co-planars, ends, groups before it
+    uint2 *rscan;       // per reference: references that go below / above before it
+    uint32_t *sizes;    // SK_*
     // next level
     float4 *nlo, *nhi;
     float *nsurf;
@@ -291,25 +278,31 @@ struct LevelPtrs {
     uint32_t depth;
 };
 
-__device__ __forceinline__ bool forced_leaf(const LevelPtrs &L, uint32_t c) {
-    return c == 0 || c <= L.p.leaf_size || L.depth >= L.p.max_depth;
+__device__ __forceinline__ bool forced_leaf(const LevelPtrs &L, uint32_t c, uint32_t depth) {
+    return c == 0 || c <= L.p.leaf_size || depth >= L.p.max_depth;
 }
 
-__global__ void k_r_init(LevelPtrs L) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
-    const uint32_t c = L.cnt[i];
-    const uint32_t s = forced_leaf(L, c) ? 0u : (c + L.p.sample - 1) / L.p.sample;
-    L.nkeys[i] = 6u * s;
-    if (s) atomicMax(L.maxseg, 2u * s);
-    L.best[i] = ~0ull;
-    L.efirst[3 * i] = L.efirst[3 * i + 1] = L.efirst[3 * i + 2] = 0;
-}
+// candidate slots of every node: six per sampled polygon
+struct InitOp {
+    using T = uint2;
+    using Item = uint32_t;
+    LevelPtrs L;
+    __device__ uint32_t count() const { return L.n; }
+    __device__ Item load(uint32_t i) const {
+        const uint32_t c = L.cnt[i];
+        L.best[i] = ~0ull;
+        L.efirst[3 * (size_t)i] = L.efirst[3 * (size_t)i + 1] = L.efirst[3 * (size_t)i + 2] = 0;
+        return forced_leaf(L, c, L.depth) ? 0u : 6u * ((c + L.p.sample - 1) / L.p.sample);
+    }
+    __device__ T value(const Item &it) const { return make_uint2(it, 0); }
+    __device__ void apply(uint32_t i, T pre, const Item &) const { L.koff[i] = pre.x; }
+    __device__ void finish(T tot) const { L.koff[L.n] = tot.x; }
+};
 
 // KDTreeSAH.cpp:51-82: candidates of the sampled polygons
-__global__ void k_r_emit(LevelPtrs L, uint32_t Q, const float4 *__restrict__ V, const uint4 *__restrict__ T) {
+__global__ void k_r_emit(LevelPtrs L, const float4 *__restrict__ V, const uint4 *__restrict__ T) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= Q) return;
+    if (q >= L.koff[L.n] / 6u) return;
     uint32_t a = 0, b = L.n;   // node: koff[i] / 6 <= q < koff[i + 1] / 6
     while (a < b) {
         const uint32_t m = (a + b) >> 1;
@@ -442,53 +435,55 @@ __global__ void __launch_bounds__(256) k_seg_sort_cta(LevelPtrs L, uint32_t nseg
     }
 }
 
-// group heads and the counters the sweep accumulates:
-//   f1 = [begin or co-planar] | [co-planar] << 32, f2 = [end] | [head] << 32
-__global__ void k_r_heads(LevelPtrs L, uint32_t K) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= K) return;
-    const u64 k = L.keys[p];
-    const uint32_t m = (uint32_t)k & 3u;
-    const bool real = m != kNone;
-    bool head = false;
-    if (real) {
+// group heads and the counters the sweep accumulates
+struct SweepOp {
+    using T = uint4;
+    using Item = uint4;
+    LevelPtrs L;
+    __device__ uint32_t count() const { return L.koff[L.n]; }
+    __device__ Item load(uint32_t p) const {
+        const u64 k = L.keys[p];
+        const uint32_t m = (uint32_t)k & 3u;
+        if (m == kNone) return make_uint4(0, 0, 0, 0);
         uint32_t i, ax, s0, s1;
         seg_range(L, (uint32_t)(k >> 34), i, ax, s0, s1);
         const float v = key_value(k);
-        head = p == s0 || !(key_value(L.keys[p - 1]) == v);
+        const bool head = p == s0 || !(key_value(L.keys[p - 1]) == v);
         // ends in the segment's first group are never subtracted (:164-169)
         if (m == 2 && key_value(L.keys[s0]) == v) atomicAdd(&L.efirst[(uint32_t)(k >> 34)], 1u);
+        return make_uint4(m != 2 ? 1u : 0u, m == 1 ? 1u : 0u, m == 2 ? 1u : 0u, head ? 1u : 0u);
     }
-    L.f1[p] = (u64)(real && m != 2) | ((u64)(real && m == 1) << 32);
-    L.f2[p] = (u64)(real && m == 2) | ((u64)head << 32);
-}
-
-__global__ void k_r_gfirst(LevelPtrs L, uint32_t K) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) L.gfirst[hi32(L.f2[K])] = K;   // f2 holds the scan: total groups
-    if (p >= K) return;
-    const u64 a = L.f2[p], b = L.f2[p + 1];
-    if (hi32(b) != hi32(a)) L.gfirst[hi32(a)] = p;
-}
+    __device__ T value(const Item &it) const { return it; }
+    __device__ void apply(uint32_t p, T pre, const Item &it) const {
+        L.sweep[p] = pre;
+        if (it.w) L.gfirst[pre.w] = p;
+    }
+    __device__ void finish(T tot) const {
+        const uint32_t K = L.koff[L.n];
+        L.sweep[K] = tot;
+        L.gfirst[tot.w] = K;
+    }
+};
 
 // (cost, key position) of the group that starts at key p, or ~0 when p
 // starts no group or its cost is not below FLT_MAX
 __device__ u64 r_group_cost(const LevelPtrs &L, uint32_t p) {
-    const u64 g2 = L.f2[p], g2n = L.f2[p + 1];
-    if (hi32(g2n) == hi32(g2)) return ~0ull;   // not a group head
-    const uint32_t g = hi32(g2);
+    const uint4 at = L.sweep[p];
+    const uint32_t g = at.w;
+    if (L.sweep[p + 1].w == g) return ~0ull;   // not a group head
     const u64 k = L.keys[p];
     const uint32_t seg = (uint32_t)(k >> 34);
     uint32_t i, ax, s0, s1;
     seg_range(L, seg, i, ax, s0, s1);
-    const uint32_t real_end = s0 + (lo32(L.f1[s1]) - lo32(L.f1[s0])) + (lo32(L.f2[s1]) - lo32(L.f2[s0]));
+    const uint4 first = L.sweep[s0], last = L.sweep[s1];
+    const uint32_t real_end = s0 + (last.x - first.x) + (last.z - first.z);
     const uint32_t nxt = L.gfirst[g + 1];
     const uint32_t l1 = nxt < real_end ? nxt : real_end;
-    const uint32_t cop_here = hi32(L.f1[l1]) - hi32(L.f1[p]);
-    const uint32_t cop = p == s0 ? cop_here : hi32(L.f1[p]) - hi32(L.f1[L.gfirst[g - 1]]);
-    const uint32_t below = lo32(L.f1[p]) - lo32(L.f1[s0]);
+    const uint4 end = L.sweep[l1];
+    const uint32_t cop = p == s0 ? end.y - at.y : at.y - L.sweep[L.gfirst[g - 1]].y;
+    const uint32_t below = at.x - first.x;
     const uint32_t N = L.cnt[i] / L.p.sample;
-    const uint32_t above = N - (hi32(L.f1[l1]) - hi32(L.f1[s0])) - ((lo32(L.f2[l1]) - lo32(L.f2[s0])) - L.efirst[seg]);
+    const uint32_t above = N - (end.y - first.y) - ((end.z - first.z) - L.efirst[seg]);
     const float v = key_value(k);
     const float4 bl = L.lo[i], bh = L.hi[i];
     const float dim[3] = {__fsub_rn(bh.x, bl.x), __fsub_rn(bh.y, bl.y), __fsub_rn(bh.z, bl.z)};
@@ -507,8 +502,8 @@ __device__ u64 r_group_cost(const LevelPtrs &L, uint32_t p) {
 // the SAH of every group (KDTreeSAH.cpp:147-175); the node's minimum of
 // (cost, position) is taken over the warp first (keys are sorted by node, so
 // a warp's lanes span few nodes), then with one atomicMin per node and warp
-__global__ void k_r_cost(LevelPtrs L, uint32_t K) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_r_cost(LevelPtrs L) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, K = L.koff[L.n];
     const uint32_t lane = threadIdx.x & 31u;
     u64 packed = ~0ull;
     uint32_t node = 0xffffffffu;
@@ -529,65 +524,84 @@ __global__ void k_r_cost(LevelPtrs L, uint32_t K) {
 }
 
 
-// leaf test (KDTreeSAH.cpp:186-191) and the split's child surfaces
-__global__ void k_r_decide(LevelPtrs L) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
-    const uint32_t c = L.cnt[i];
-    const u64 b = L.best[i];
-    bool leaf = forced_leaf(L, c) || b == ~0ull;
-    if (!leaf) {
-        const float score = o2f(hi32(b));
-        const float leafcost = __fmul_rn(L.p.ci, (float)(c / L.p.sample));
-        leaf = score >= leafcost;
+// leaf test (KDTreeSAH.cpp:186-191) and the split's child surfaces; ranks of
+// the junctions and the leaves' places
+struct DecideOp {
+    using T = uint2;
+    using Item = uint2;   // (junction, leaf references)
+    LevelPtrs L;
+    __device__ uint32_t count() const { return L.n; }
+    __device__ Item load(uint32_t i) const {
+        const uint32_t c = L.cnt[i];
+        const u64 b = L.best[i];
+        bool leaf = forced_leaf(L, c, L.depth) || b == ~0ull;
+        if (!leaf) {
+            const float score = o2f(hi32(b));
+            const float leafcost = __fmul_rn(L.p.ci, (float)(c / L.p.sample));
+            leaf = score >= leafcost;
+        }
+        if (leaf) {
+            L.decision[i] = kDecLeaf;
+            return make_uint2(0, c);
+        }
+        const u64 k = L.keys[lo32(b)];
+        const uint32_t ax = (uint32_t)(k >> 34) % 3u;
+        const float v = key_value(k);
+        const float4 bl = L.lo[i], bh = L.hi[i];
+        const float dim[3] = {__fsub_rn(bh.x, bl.x), __fsub_rn(bh.y, bl.y), __fsub_rn(bh.z, bl.z)};
+        const float x = dim[(ax + 1) % 3], y = dim[(ax + 2) % 3];
+        const float xpy = __fadd_rn(x, y), area = __fmul_rn(x, y);
+        L.surf_hi[i] = __fadd_rn(area, __fmul_rn(__fsub_rn(c3(bh, ax), v), xpy));
+        L.surf_lo[i] = __fadd_rn(area, __fmul_rn(__fsub_rn(v, c3(bl, ax)), xpy));
+        L.plane[i] = v;
+        L.decision[i] = ax;
+        return make_uint2(1, 0);
     }
-    if (leaf) {
-        L.decision[i] = kDecLeaf;
-        L.jflag[i] = 0;
-        L.leafcnt[i] = c;
-        return;
+    __device__ T value(const Item &it) const { return it; }
+    __device__ void apply(uint32_t i, T pre, const Item &) const {
+        L.jrank[i] = pre.x;
+        L.loff[i] = pre.y;
     }
-    const u64 k = L.keys[lo32(b)];
-    const uint32_t ax = (uint32_t)(k >> 34) % 3u;
-    const float v = key_value(k);
-    const float4 bl = L.lo[i], bh = L.hi[i];
-    const float dim[3] = {__fsub_rn(bh.x, bl.x), __fsub_rn(bh.y, bl.y), __fsub_rn(bh.z, bl.z)};
-    const float x = dim[(ax + 1) % 3], y = dim[(ax + 2) % 3];
-    const float xpy = __fadd_rn(x, y), area = __fmul_rn(x, y);
-    L.surf_hi[i] = __fadd_rn(area, __fmul_rn(__fsub_rn(c3(bh, ax), v), xpy));
-    L.surf_lo[i] = __fadd_rn(area, __fmul_rn(__fsub_rn(v, c3(bl, ax)), xpy));
-    L.plane[i] = v;
-    L.decision[i] = ax;
-    L.jflag[i] = 1;
-    L.leafcnt[i] = 0;
-}
+    __device__ void finish(T tot) const {
+        L.sizes[SK_JUNCTIONS] = tot.x;
+        L.sizes[SK_LEAFREFS] = tot.y;
+        L.sizes[SK_MAXCNT] = 0;   // k_r_nodes takes the maximum
+    }
+};
 
 // KDTreeCPU::checkPolygonToAAPlane (KDTreeCPU.cpp:450-477) on the polygons of
-// split nodes: rflag = [goes below] | [goes above] << 32
-__global__ void k_r_classify(LevelPtrs L, uint32_t R, const float4 *__restrict__ V, const uint4 *__restrict__ T) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= R) return;
-    const uint32_t i = L.ref_node[q];
-    const uint32_t d = L.decision[i];
-    if (d == kDecLeaf) {
-        L.rflag[q] = 0;
-        return;
+// split nodes: (goes below, goes above)
+struct ClassifyOp {
+    using T = uint2;
+    using Item = uint2;
+    LevelPtrs L;
+    uint32_t R;
+    const float4 *V;
+    const uint4 *Tr;
+    __device__ uint32_t count() const { return R; }
+    __device__ Item load(uint32_t q) const {
+        const uint32_t i = L.ref_node[q];
+        const uint32_t d = L.decision[i];
+        if (d == kDecLeaf) return make_uint2(0, 0);
+        const float v = L.plane[i];
+        const uint4 t = Tr[L.refs[q]];
+        const float a = c3(V[t.x], d), b = c3(V[t.y], d), c = c3(V[t.z], d);
+        const bool cop = (a == v) & (b == v) & (c == v);
+        const bool above = (a >= v) & (b >= v) & (c >= v);
+        const bool below = (a <= v) & (b <= v) & (c <= v);
+        // below, intersecting, co-planar; above, intersecting, co-planar
+        return make_uint2(cop || !above ? 1u : 0u, cop || above || !below ? 1u : 0u);
     }
-    const float v = L.plane[i];
-    const uint4 t = T[L.refs[q]];
-    const float a = c3(V[t.x], d), b = c3(V[t.y], d), c = c3(V[t.z], d);
-    const bool cop = (a == v) & (b == v) & (c == v);
-    const bool above = (a >= v) & (b >= v) & (c >= v);
-    const bool below = (a <= v) & (b <= v) & (c <= v);
-    const bool goA = cop || above || !below;   // above, intersecting, co-planar
-    const bool goB = cop || !above;            // below, intersecting, co-planar
-    L.rflag[q] = (u64)goB | ((u64)goA << 32);
-}
+    __device__ T value(const Item &it) const { return it; }
+    __device__ void apply(uint32_t q, T pre, const Item &) const { L.rscan[q] = pre; }
+    __device__ void finish(T tot) const {
+        L.rscan[R] = tot;
+        L.sizes[SK_REFS] = tot.x + tot.y;
+    }
+};
 
 // cells of this level, and the next level's nodes
-__global__ void k_r_nodes(LevelPtrs L) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
+__device__ __forceinline__ uint32_t r_node(const LevelPtrs &L, uint32_t i) {
     const uint32_t cell = L.cbase + i;
     const uint32_t c = L.cnt[i], d = L.decision[i];
     const float4 bl = L.lo[i], bh = L.hi[i];
@@ -596,14 +610,14 @@ __global__ void k_r_nodes(LevelPtrs L) {
     L.out_cbox[2 * (size_t)cell + 1] = make_float4(bh.x, bh.y, bh.z, 0.0f);
     if (d == kDecLeaf) {
         L.nodes[cell] = c ? make_uint2(((L.rbase + L.loff[i]) << 2) | kLeafTag, c) : make_uint2(kLeafTag, 0u);
-        return;
+        return 0;
     }
     const uint32_t k = L.jrank[i], pair = L.nbase + 2 * k;
     const float v = L.plane[i];
     L.nodes[cell] = make_uint2((pair << 2) | d, __float_as_uint(v));
-    const u64 r0 = L.rscan[L.off[i]], r1 = L.rscan[L.off[i] + c];
-    const uint32_t cB = lo32(r1) - lo32(r0), cA = hi32(r1) - hi32(r0);
-    const uint32_t oB = lo32(r0) + hi32(r0);
+    const uint2 r0 = L.rscan[L.off[i]], r1 = L.rscan[L.off[i] + c];
+    const uint32_t cB = r1.x - r0.x, cA = r1.y - r0.y;
+    const uint32_t oB = r0.x + r0.y;
     // below child (pair), above child (pair + 1)
     float4 hB = bh, lA = bl;
     s3(hB, d, v);
@@ -625,6 +639,15 @@ __global__ void k_r_nodes(LevelPtrs L) {
     }
     L.nropes[12 * (size_t)k + 2 * d + 1] = pair + 1;
     L.nropes[12 * (size_t)k + 6 + 2 * d] = pair;
+    const uint32_t sB = forced_leaf(L, cB, L.depth + 1) ? 0u : cB, sA = forced_leaf(L, cA, L.depth + 1) ? 0u : cA;
+    return max(sB, sA);
+}
+
+__global__ void k_r_nodes(LevelPtrs L) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the largest child with candidates
+    const uint32_t m = __reduce_max_sync(0xffffffffu, i < L.n ? r_node(L, i) : 0u);
+    if (m && (threadIdx.x & 31u) == 0) atomicMax(&L.sizes[SK_MAXCNT], m);
 }
 
 // leaf references out; split references into the next level (stable)
@@ -638,40 +661,49 @@ __global__ void k_r_scatter(LevelPtrs L, uint32_t R) {
         return;
     }
     const uint32_t k = L.jrank[i];
-    const u64 f = L.rflag[q], rq = L.rscan[q], r0 = L.rscan[L.off[i]], r1 = L.rscan[L.off[i] + L.cnt[i]];
-    const uint32_t oB = lo32(r0) + hi32(r0), cB = lo32(r1) - lo32(r0);
-    if (lo32(f)) {
-        const uint32_t dst = oB + (lo32(rq) - lo32(r0));
+    const uint2 rq = L.rscan[q], rn = L.rscan[q + 1], r0 = L.rscan[L.off[i]], r1 = L.rscan[L.off[i] + L.cnt[i]];
+    const uint32_t oB = r0.x + r0.y, cB = r1.x - r0.x;
+    if (rn.x != rq.x) {
+        const uint32_t dst = oB + (rq.x - r0.x);
         L.nrefs[dst] = ref;
         L.nref_node[dst] = 2 * k;
     }
-    if (hi32(f)) {
-        const uint32_t dst = oB + cB + (hi32(rq) - hi32(r0));
+    if (rn.y != rq.y) {
+        const uint32_t dst = oB + cB + (rq.y - r0.y);
         L.nrefs[dst] = ref;
         L.nref_node[dst] = 2 * k + 1;
     }
 }
 
-__global__ void k_r_iota(uint32_t *refs, uint32_t *ref_node, uint32_t n) {
+// level 0: the root over every polygon (its box and half surface, getHalfBox-
+// Surface, SharedFunctions.hpp:40-44, from the host), and the padding cell 1
+struct RootPtrs {
+    float4 *lo, *hi;
+    float *surf;
+    uint32_t *off, *cnt, *ropes, *refs, *ref_node;
+    uint2 *nodes;
+    uint32_t *out_ropes;
+    float4 *out_cbox;
+};
+__global__ void k_r_root(RootPtrs P, float4 lo, float4 hi, float half, uint32_t nt) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        refs[i] = i;
-        ref_node[i] = 0;
+    if (i < nt) {
+        P.refs[i] = i;
+        P.ref_node[i] = 0;
     }
-}
-
-__global__ void k_r_pad(uint2 *nodes, uint32_t *ropes, float4 *cbox) {
-    const int f = threadIdx.x;
-    if (f == 0) nodes[1] = make_uint2(kLeafTag, 0u);
-    if (f < 6) ropes[6 + f] = 0xffffffffu;
-    if (f < 2) cbox[2 + f] = make_float4(0, 0, 0, 0);
-}
-
-__global__ void k_r_copy3(const uint32_t *a, const u64 *b, uint32_t ia, uint32_t ib, const uint32_t *c, uint32_t ic,
-                          uint32_t *out) {
-    out[0] = a[ia];
-    out[1] = lo32(b[ib]) + hi32(b[ib]);
-    out[2] = c[ic];
+    if (i < 6) {
+        P.ropes[i] = 0xffffffffu;
+        P.out_ropes[6 + i] = 0xffffffffu;
+    }
+    if (i < 2) P.out_cbox[2 + i] = make_float4(0, 0, 0, 0);
+    if (i == 0) {
+        P.lo[0] = lo;
+        P.hi[0] = hi;
+        P.surf[0] = half;
+        P.off[0] = 0;
+        P.cnt[0] = nt;
+        P.nodes[1] = make_uint2(kLeafTag, 0u);
+    }
 }
 
 inline unsigned blocks(uint32_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t) ? (unsigned)((n + t - 1) / t) : 1u; }
@@ -690,11 +722,8 @@ void ResortState::release() {
         ref_node[b].release();
         keys[b].release();
     }
-    nkeys.release();
     koff.release();
-    jflag.release();
     jrank.release();
-    leafcnt.release();
     loff.release();
     efirst.release();
     decision.release();
@@ -702,15 +731,17 @@ void ResortState::release() {
     surf_lo.release();
     surf_hi.release();
     best.release();
-    kscan_a.release();
-    kscan_b.release();
+    sweep.release();
     rscan.release();
-    rflag.release();
     hist.release();
     gfirst.release();
-    scan_part.release();
-    scan_part64.release();
-    dev_u32.release();
+    scan_flags.release();
+    scan_agg.release();
+    scan_incl.release();
+    tickets.release();
+    sizes.release();
+    if (host_sizes) cudaFreeHost(host_sizes);
+    host_sizes = nullptr;
     nodes.release();
     out_refs.release();
     out_ropes.release();
@@ -726,6 +757,33 @@ void ResortState::release() {
         }                                                           \
     } while (0)
 
+// the tile states of a scan of up to n elements, and its tag and ticket
+static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t &next_ticket, ScanPtrs &sp, cudaStream_t st) {
+    const size_t tiles = n / kScanTile + 2;
+    if (tiles > S.scan_flags.cap) {
+        cudaError_t e = S.scan_flags.ensure(tiles);
+        if (e == cudaSuccess) e = S.scan_agg.ensure(tiles);
+        if (e == cudaSuccess) e = S.scan_incl.ensure(tiles);
+        if (e == cudaSuccess) e = cudaMemsetAsync(S.scan_flags.p, 0, S.scan_flags.cap * 4, st);
+        if (e != cudaSuccess) return e;
+    }
+    S.scan_tag = (S.scan_tag + 1u) & 0x3fffffffu;
+    sp = ScanPtrs{S.scan_flags.p, S.tickets.p + next_ticket++, S.sizes.p + SK_ERR, S.scan_agg.p, S.scan_incl.p,
+                  S.scan_tag};
+    return cudaSuccess;
+}
+
+template <class Op>
+static cudaError_t scan(ResortState &S, const Op &op, size_t n, uint32_t &next_ticket, cudaStream_t st) {
+    ScanPtrs sp;
+    cudaError_t e = scan_begin(S, n, next_ticket, sp, st);
+    if (e != cudaSuccess) return e;
+    // a CTA per tile up to four per SM
+    const unsigned grid = (unsigned)std::min<size_t>(n / kScanTile + 1, 148u * 4u);
+    k_r_scan<Op><<<grid, kScanNT, 0, st>>>(op, sp);
+    return cudaGetLastError();
+}
+
 hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *verts, const uint4 *tris, uint32_t nt,
                        const float *hbox, cudaStream_t st, std::string *err) {
     if (p.sample == 0 || p.max_depth > 64) {
@@ -735,6 +793,8 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
     // level 0: the root (cell 0) over every polygon; cell 1 is padding
     // cells [cbase, cbase + n) hold the current level; `written` cells exist
     uint32_t n = 1, R = nt, cbase = 0, rbase = 0, written = 2, depth = 0;
+    // four scans a level and at most eight radix passes (34 + 30 key bits)
+    constexpr uint32_t kTickets = 66 * 12;
     RS_CHECK(S.lo[0].ensure(1));
     RS_CHECK(S.hi[0].ensure(1));
     RS_CHECK(S.surf[0].ensure(1));
@@ -743,48 +803,62 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
     RS_CHECK(S.ropes[0].ensure(6));
     RS_CHECK(S.refs[0].ensure(R));
     RS_CHECK(S.ref_node[0].ensure(R));
-    RS_CHECK(S.dev_u32.ensure(4));
+    RS_CHECK(S.sizes.ensure(SK_WORDS));
+    RS_CHECK(S.tickets.ensure(kTickets));
     RS_CHECK(grow_keep(S.nodes, 2, 0, st));
     RS_CHECK(grow_keep(S.out_ropes, 12, 0, st));
     RS_CHECK(grow_keep(S.out_cbox, 4, 0, st));
     RS_CHECK(grow_keep(S.out_refs, 1, 0, st));
+    if (!S.host_sizes) RS_CHECK(cudaHostAlloc((void **)&S.host_sizes, SK_WORDS * 4, cudaHostAllocDefault));
+    RS_CHECK(cudaMemsetAsync(S.sizes.p, 0, SK_WORDS * 4, st));
+    RS_CHECK(cudaMemsetAsync(S.tickets.p, 0, kTickets * 4, st));
+    uint32_t next_ticket = 0;
     {
-        // root box and half surface (getHalfBoxSurface, SharedFunctions.hpp:40-44)
-        const float4 lo = make_float4(hbox[0], hbox[1], hbox[2], hbox[3]);
-        const float4 hi = make_float4(hbox[4], hbox[5], hbox[6], hbox[7]);
         const float sx = hbox[4] - hbox[0], sy = hbox[5] - hbox[1], sz = hbox[6] - hbox[2];
-        const float half = sx * sy + sz * sy + sx * sz;
-        const uint32_t zero = 0, ropes[6] = {~0u, ~0u, ~0u, ~0u, ~0u, ~0u};
-        RS_CHECK(cudaMemcpyAsync(S.lo[0].p, &lo, sizeof lo, cudaMemcpyHostToDevice, st));
-        RS_CHECK(cudaMemcpyAsync(S.hi[0].p, &hi, sizeof hi, cudaMemcpyHostToDevice, st));
-        RS_CHECK(cudaMemcpyAsync(S.surf[0].p, &half, sizeof half, cudaMemcpyHostToDevice, st));
-        RS_CHECK(cudaMemcpyAsync(S.off[0].p, &zero, sizeof zero, cudaMemcpyHostToDevice, st));
-        RS_CHECK(cudaMemcpyAsync(S.cnt[0].p, &nt, sizeof nt, cudaMemcpyHostToDevice, st));
-        RS_CHECK(cudaMemcpyAsync(S.ropes[0].p, ropes, sizeof ropes, cudaMemcpyHostToDevice, st));
-        if (R) k_r_iota<<<blocks(R), 256, 0, st>>>(S.refs[0].p, S.ref_node[0].p, R);
-        k_r_pad<<<1, 32, 0, st>>>(S.nodes.p, S.out_ropes.p, S.out_cbox.p);
-        RS_CHECK(cudaStreamSynchronize(st));
+        const RootPtrs P{S.lo[0].p, S.hi[0].p, S.surf[0].p, S.off[0].p, S.cnt[0].p, S.ropes[0].p,
+                         S.refs[0].p, S.ref_node[0].p, S.nodes.p, S.out_ropes.p, S.out_cbox.p};
+        k_r_root<<<blocks(std::max<uint32_t>(R, 6)), 256, 0, st>>>(
+            P, make_float4(hbox[0], hbox[1], hbox[2], hbox[3]), make_float4(hbox[4], hbox[5], hbox[6], hbox[7]),
+            sx * sy + sz * sy + sx * sz, nt);
     }
+    // the largest node with candidates (forced_leaf)
+    uint32_t maxcnt = (nt <= p.leaf_size || p.max_depth == 0) ? 0u : nt;
     for (uint32_t level = 0; n > 0; level++) {
         const int cur = level & 1, nxt = cur ^ 1;
         depth = level;
         // per-node scratch
-        RS_CHECK(S.nkeys.ensure(n));
-        RS_CHECK(S.koff.ensure(n + 1));
-        RS_CHECK(S.jflag.ensure(n));
-        RS_CHECK(S.jrank.ensure(n + 1));
-        RS_CHECK(S.leafcnt.ensure(n));
-        RS_CHECK(S.loff.ensure(n + 1));
+        RS_CHECK(S.koff.ensure((size_t)n + 1));
+        RS_CHECK(S.jrank.ensure(n));
+        RS_CHECK(S.loff.ensure(n));
         RS_CHECK(S.efirst.ensure(3 * (size_t)n));
         RS_CHECK(S.decision.ensure(n));
         RS_CHECK(S.plane.ensure(n));
         RS_CHECK(S.surf_lo.ensure(n));
         RS_CHECK(S.surf_hi.ensure(n));
         RS_CHECK(S.best.ensure(n));
-        // this level's cells in the output
+        RS_CHECK(S.rscan.ensure((size_t)R + 1));
+        // candidate slots: six per sampled polygon, at least one per node
+        const uint64_t Q = maxcnt ? (uint64_t)R / p.sample + std::min(n, R) : 0u;
+        if (6 * Q >= 0xfffffff0ull) {
+            if (err) *err = "more candidate slots than 32 bits index";
+            return HK_E_CAPACITY;
+        }
+        const uint32_t K = (uint32_t)(6 * Q);   // at most; the actual count stays on the device
+        RS_CHECK(S.keys[0].ensure(K ? K : 1));
+        RS_CHECK(S.keys[1].ensure(K ? K : 1));
+        RS_CHECK(S.sweep.ensure((size_t)K + 1));
+        RS_CHECK(S.gfirst.ensure((size_t)K + 2));
+        // this level's cells in the output; the next level has at most 2 n nodes
         RS_CHECK(grow_keep(S.nodes, (size_t)cbase + n, written, st));
         RS_CHECK(grow_keep(S.out_ropes, 6 * ((size_t)cbase + n), 6 * (size_t)written, st));
         RS_CHECK(grow_keep(S.out_cbox, 2 * ((size_t)cbase + n), 2 * (size_t)written, st));
+        const size_t n2max = std::min<size_t>(2 * (size_t)n, 2 * (size_t)R);
+        RS_CHECK(S.lo[nxt].ensure(n2max));
+        RS_CHECK(S.hi[nxt].ensure(n2max));
+        RS_CHECK(S.surf[nxt].ensure(n2max));
+        RS_CHECK(S.off[nxt].ensure(n2max));
+        RS_CHECK(S.cnt[nxt].ensure(n2max));
+        RS_CHECK(S.ropes[nxt].ensure(6 * n2max));
         LevelPtrs L;
         memset(&L, 0, sizeof L);
         L.n = n;
@@ -796,11 +870,8 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
         L.ropes = S.ropes[cur].p;
         L.refs = S.refs[cur].p;
         L.ref_node = S.ref_node[cur].p;
-        L.nkeys = S.nkeys.p;
         L.koff = S.koff.p;
-        L.jflag = S.jflag.p;
         L.jrank = S.jrank.p;
-        L.leafcnt = S.leafcnt.p;
         L.loff = S.loff.p;
         L.efirst = S.efirst.p;
         L.decision = S.decision.p;
@@ -808,32 +879,32 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
         L.surf_lo = S.surf_lo.p;
         L.surf_hi = S.surf_hi.p;
         L.best = S.best.p;
+        L.sweep = S.sweep.p;
+        L.gfirst = S.gfirst.p;
+        L.rscan = S.rscan.p;
+        L.sizes = S.sizes.p;
+        L.nlo = S.lo[nxt].p;
+        L.nhi = S.hi[nxt].p;
+        L.nsurf = S.surf[nxt].p;
+        L.noff = S.off[nxt].p;
+        L.ncnt = S.cnt[nxt].p;
+        L.nropes = S.ropes[nxt].p;
+        L.nodes = S.nodes.p;
+        L.out_ropes = S.out_ropes.p;
+        L.out_cbox = S.out_cbox.p;
         L.p = p;
         L.depth = level;
         L.cbase = cbase;
         L.nbase = level == 0 ? 2u : cbase + n;   // the next level's first cell
         L.rbase = rbase;
         // 1. candidates
-        L.maxseg = S.dev_u32.p + 3;
-        RS_CHECK(cudaMemsetAsync(L.maxseg, 0, 4, st));
-        k_r_init<<<blocks(n), 256, 0, st>>>(L);
-        RS_CHECK(scan_excl<uint32_t>(S.nkeys.p, S.koff.p, n, S.scan_part, st));
-        uint32_t K = 0, maxseg = 0;
-        RS_CHECK(cudaMemcpyAsync(&K, S.koff.p + n, 4, cudaMemcpyDeviceToHost, st));
-        RS_CHECK(cudaMemcpyAsync(&maxseg, L.maxseg, 4, cudaMemcpyDeviceToHost, st));
-        RS_CHECK(cudaStreamSynchronize(st));
-        RS_CHECK(S.keys[0].ensure(K ? K : 1));
-        RS_CHECK(S.keys[1].ensure(K ? K : 1));
-        RS_CHECK(S.kscan_a.ensure((size_t)K + 1));
-        RS_CHECK(S.kscan_b.ensure((size_t)K + 1));
-        RS_CHECK(S.gfirst.ensure((size_t)K + 2));
-        RS_CHECK(S.rscan.ensure((size_t)R + 1));
-        RS_CHECK(S.rflag.ensure(R ? R : 1));
         int kc = 0;
         L.keys = S.keys[kc].p;
+        RS_CHECK(scan(S, InitOp{L}, n, next_ticket, st));
         if (K) {
-            k_r_emit<<<blocks(K / 6), 256, 0, st>>>(L, K / 6, verts, tris);
+            k_r_emit<<<blocks(K / 6), 256, 0, st>>>(L, verts, tris);
             // 2. sort by (segment, value, marker)
+            const uint32_t maxseg = 2 * ((maxcnt + p.sample - 1) / p.sample);
             if (maxseg <= kSegCtaMax) {
                 const uint32_t nseg = 3 * n;
                 k_seg_sort_warp<<<(unsigned)(((size_t)nseg * 32 + 255) / 256), 256, 0, st>>>(L, nseg);
@@ -843,70 +914,46 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
                 while (segbits < 30 && (1ull << segbits) < 3ull * n) segbits++;
                 const int nbits = 34 + (int)segbits;
                 const uint32_t ntiles = (K + kTile - 1) / kTile;
-                RS_CHECK(S.hist.ensure(256 * (size_t)ntiles + 1));
+                RS_CHECK(S.hist.ensure(256 * (size_t)ntiles));
                 for (int shift = 0; shift < nbits; shift += 8) {
-                    k_rs_hist<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, K, shift, ntiles, S.hist.p);
-                    RS_CHECK(scan_excl<uint32_t>(S.hist.p, S.hist.p, 256 * ntiles, S.scan_part, st));
-                    k_rs_scatter<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, S.keys[kc ^ 1].p, K, shift, ntiles,
+                    k_rs_hist<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, L.koff + n, shift, ntiles, S.hist.p);
+                    RS_CHECK(scan(S, RsScanOp{S.hist.p, 256 * ntiles}, 256 * (size_t)ntiles, next_ticket, st));
+                    k_rs_scatter<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, S.keys[kc ^ 1].p, L.koff + n, shift, ntiles,
                                                          S.hist.p);
                     kc ^= 1;
                 }
             }
             L.keys = S.keys[kc].p;
             // 3. sweep
-            L.f1 = S.kscan_a.p;
-            L.f2 = S.kscan_b.p;
-            L.gfirst = S.gfirst.p;
-            k_r_heads<<<blocks(K), 256, 0, st>>>(L, K);
-            RS_CHECK(scan_excl<u64>(S.kscan_a.p, S.kscan_a.p, K, S.scan_part64, st));
-            RS_CHECK(scan_excl<u64>(S.kscan_b.p, S.kscan_b.p, K, S.scan_part64, st));
-            k_r_gfirst<<<blocks(K), 256, 0, st>>>(L, K);
-            k_r_cost<<<blocks(K), 256, 0, st>>>(L, K);
+            RS_CHECK(scan(S, SweepOp{L}, K, next_ticket, st));
+            k_r_cost<<<blocks(K), 256, 0, st>>>(L);
         }
-        // 4. decisions, ranks, leaf offsets
-        k_r_decide<<<blocks(n), 256, 0, st>>>(L);
-        RS_CHECK(scan_excl<uint32_t>(S.jflag.p, S.jrank.p, n, S.scan_part, st));
-        RS_CHECK(scan_excl<uint32_t>(S.leafcnt.p, S.loff.p, n, S.scan_part, st));
-        // 5. classification and stable partition
-        L.rflag = S.rflag.p;
-        L.rscan = S.rscan.p;
-        k_r_classify<<<blocks(R), 256, 0, st>>>(L, R, verts, tris);
-        RS_CHECK(scan_excl<u64>(L.rflag, S.rscan.p, R, S.scan_part64, st));
-        k_r_copy3<<<1, 1, 0, st>>>(S.jrank.p, S.rscan.p, n, R, S.loff.p, n, S.dev_u32.p);
-        uint32_t h3[3];
-        RS_CHECK(cudaMemcpyAsync(h3, S.dev_u32.p, sizeof h3, cudaMemcpyDeviceToHost, st));
+        // 4. decisions, ranks, leaf offsets; classification; cells and nodes
+        RS_CHECK(scan(S, DecideOp{L}, n, next_ticket, st));
+        RS_CHECK(scan(S, ClassifyOp{L, R, verts, tris}, R, next_ticket, st));
+        k_r_nodes<<<blocks(n), 256, 0, st>>>(L);
+        RS_CHECK(cudaGetLastError());
+        RS_CHECK(cudaMemcpyAsync(S.host_sizes, S.sizes.p, SK_WORDS * 4, cudaMemcpyDeviceToHost, st));
         RS_CHECK(cudaStreamSynchronize(st));
-        const uint32_t J = h3[0], R2 = h3[1], Lrefs = h3[2];
-        const uint32_t n2 = 2 * J;
-        // 6. emit cells, next level
+        if (S.host_sizes[SK_ERR]) {
+            if (err) *err = "a scan's wait ran out";
+            return HK_E_DEVICE_TIMEOUT;
+        }
+        const uint32_t J = S.host_sizes[SK_JUNCTIONS], R2 = S.host_sizes[SK_REFS], Lrefs = S.host_sizes[SK_LEAFREFS];
+        maxcnt = S.host_sizes[SK_MAXCNT];
+        // 5. leaf references, the next level's lists
         RS_CHECK(grow_keep(S.out_refs, (size_t)rbase + Lrefs, rbase, st));
-        RS_CHECK(S.lo[nxt].ensure(n2));
-        RS_CHECK(S.hi[nxt].ensure(n2));
-        RS_CHECK(S.surf[nxt].ensure(n2));
-        RS_CHECK(S.off[nxt].ensure(n2));
-        RS_CHECK(S.cnt[nxt].ensure(n2));
-        RS_CHECK(S.ropes[nxt].ensure(6 * (size_t)n2));
         RS_CHECK(S.refs[nxt].ensure(R2));
         RS_CHECK(S.ref_node[nxt].ensure(R2));
-        L.nodes = S.nodes.p;
         L.out_refs = S.out_refs.p;
-        L.out_ropes = S.out_ropes.p;
-        L.out_cbox = S.out_cbox.p;
-        L.nlo = S.lo[nxt].p;
-        L.nhi = S.hi[nxt].p;
-        L.nsurf = S.surf[nxt].p;
-        L.noff = S.off[nxt].p;
-        L.ncnt = S.cnt[nxt].p;
-        L.nropes = S.ropes[nxt].p;
         L.nrefs = S.refs[nxt].p;
         L.nref_node = S.ref_node[nxt].p;
-        k_r_nodes<<<blocks(n), 256, 0, st>>>(L);
         k_r_scatter<<<blocks(R), 256, 0, st>>>(L, R);
         RS_CHECK(cudaGetLastError());
         written = L.nbase;
         cbase = L.nbase;
         rbase += Lrefs;
-        n = n2;
+        n = 2 * J;
         R = R2;
     }
     RS_CHECK(cudaStreamSynchronize(st));
@@ -921,5 +968,6 @@ template struct RBuf<float>;
 template struct RBuf<uint32_t>;
 template struct RBuf<u64>;
 template struct RBuf<uint2>;
+template struct RBuf<uint4>;
 
 }  // namespace hk

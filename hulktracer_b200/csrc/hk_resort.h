@@ -33,14 +33,21 @@ struct ResortState {
     // per reference of the current / next level
     RBuf<uint32_t> refs[2], ref_node[2];
     // per node scratch
-    RBuf<uint32_t> nkeys, koff, jflag, jrank, leafcnt, loff, efirst, decision;
+    RBuf<uint32_t> koff, jrank, loff, efirst, decision;
     RBuf<float> plane, surf_lo, surf_hi;
     RBuf<unsigned long long> best;
     // keys, sort and sweep scratch
-    RBuf<unsigned long long> keys[2], kscan_a, kscan_b, rscan, rflag;
-    RBuf<uint32_t> hist, gfirst, scan_part;
-    RBuf<unsigned long long> scan_part64;
-    RBuf<uint32_t> dev_u32;   // small device scalars read back per level
+    RBuf<unsigned long long> keys[2];
+    RBuf<uint4> sweep;
+    RBuf<uint2> rscan;
+    RBuf<uint32_t> hist, gfirst;
+    // single-pass scans: tile states, tickets of one build
+    RBuf<uint32_t> scan_flags, tickets;
+    RBuf<uint4> scan_agg, scan_incl;
+    uint32_t scan_tag = 0;
+    // sizes of a level, and their pinned host copy
+    RBuf<uint32_t> sizes;
+    uint32_t *host_sizes = nullptr;
     // output tree (compact layout, see hk_api.cu)
     RBuf<uint2> nodes;
     RBuf<uint32_t> out_refs, out_ropes;
