@@ -962,7 +962,8 @@ static hk_status ensure_imported_ropes(hk_ctx *c) {
 }
 
 static hk_status trace_enqueue(hk_ctx *c, const float4 *d_rays, uint32_t n, const uint32_t *n_dev, hk_variant v,
-                               hk_hit *d_hits, bool occlusion = false, uint32_t *leaf_out = nullptr) {
+                               hk_hit *d_hits, bool occlusion = false, uint32_t *leaf_out = nullptr,
+                               uint32_t refill = 0) {
     if ((int)v < HK_TRACE_FULLSTACK || (int)v > HK_TRACE_BRUTE) return fail(c, HK_E_ILLEGAL_INPUT, "variant");
     if (!c->rec_valid) return fail(c, HK_E_STATE, "no triangle cache (hk_precompute or hk_cache_import)");
     if (v != HK_TRACE_BRUTE && !c->tree_valid) return fail(c, HK_E_STATE, "no tree");
@@ -998,6 +999,7 @@ static hk_status trace_enqueue(hk_ctx *c, const float4 *d_rays, uint32_t n, cons
     L.variant = (int)v;
     L.count = c->counting;
     L.occlusion = occlusion;
+    L.refill = refill;
     L.leaf_out = v == HK_TRACE_ROPES ? leaf_out : nullptr;
     L.block = (int)c->cfg.block_size;
     if (trace_smem_bytes(L.variant, c->cfg.block_size, L.stack_depth, false, occlusion, L.count) > kTraceMaxSmem)
@@ -1150,7 +1152,8 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
     HK_CUDA(c, launch_camera_rays(c->cam.p, w, h, c->rays.p, c->stream, tiled, row0, full_h));
     // ropes: each pixel's last leaf, where its shadow rays may start
     const bool hint = v == HK_TRACE_ROPES && shade != HK_SHADE_PICTURE;
-    hk_status s = trace_enqueue(c, c->rays.p, npix, nullptr, v, c->hits.p, false, hint ? c->hleaf.p : nullptr);
+    hk_status s = trace_enqueue(c, c->rays.p, npix, nullptr, v, c->hits.p, false, hint ? c->hleaf.p : nullptr,
+                                kRefillCoherent);
     if (s != HK_OK) return s;
     if (shade == HK_SHADE_PICTURE) {
         HK_CUDA(c, launch_hit4(c->hits.p, c->rec.p, npix, c->hit4.p, c->stream));
@@ -1163,7 +1166,7 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
         // one mirror bounce: reflected rays, traced, merged into the shading rays
         HK_CUDA(c, launch_mirror_rays(c->rays.p, c->hits.p, c->rec.p, c->mirror.p, npix, c->mrays.p, c->mslot.p,
                                       c->mcount.p, c->stream));
-        s = trace_enqueue(c, c->mrays.p, 0, c->mcount.p, v, c->mhits.p);
+        s = trace_enqueue(c, c->mrays.p, 0, c->mcount.p, v, c->mhits.p, false, nullptr, kRefillMirror);
         if (s != HK_OK) return s;
         HK_CUDA(c, launch_mirror_merge(c->rays.p, c->hits.p, c->mslot.p, c->mrays.p, c->mhits.p, npix, c->prays.p,
                                        c->phits.p, c->stream));
@@ -1173,7 +1176,7 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
     HK_CUDA(c, launch_shadow_rays(shade_rays, shade_hits, c->rec.p, npix, c->lights.p, nl,
                                   hint ? c->hleaf.p : nullptr, c->srays.p, c->slot.p, c->spix.p, c->scount.p,
                                   c->stream));
-    s = trace_enqueue(c, c->srays.p, 0, c->scount.p, v, c->shits.p, true);
+    s = trace_enqueue(c, c->srays.p, 0, c->scount.p, v, c->shits.p, true, nullptr, kRefillCoherent);
     if (s != HK_OK) return s;
     HK_CUDA(c, launch_shade_cpu(shade_rays, shade_hits, c->rec.p, npix, c->lights.p, nl, c->slot.p, c->shits.p,
                                 d_rgba, c->stream, w, tiled));

@@ -42,6 +42,7 @@ struct TraceLaunch {
     bool count;
     bool occlusion;             // shadow rays: origin w = light distance, stop at the first hit closer than it
     uint32_t *leaf_out;         // ropes: per ray, the leaf its traversal ended in (a start hint), or nullptr
+    uint32_t refill;            // idle lanes before a warp takes new rays (0: kRefillBatch / kRefillRays)
     int block;
     int grid;                   // blocks, or 0: one resident wave on sm_count SMs
     int sm_count;
@@ -65,18 +66,33 @@ struct TraceLaunch {
 constexpr uint32_t kTraceMaxBlock = 256;
 constexpr size_t kTraceMaxSmem = 48 * 1024;
 
+// Idle lanes that a warp gathers before it takes new rays. A fresh ray descends
+// from the root while its neighbours follow ropes a step or two, so lanes
+// refilled one by one hold the others at nearly every step; idle lanes still
+// share the leaf tests meanwhile. Camera and shadow rays come in tiles that run
+// alike: a warp finishes all 32 first (six-light frame 2,095 us at one, 1,974 at
+// 8, 1,929 at 16, 1,883 at 32). Rays of unknown order: 8 (a million incoherent
+// rays 710 us at one, 677 at 8, 683 at 16, 820 at 32); batches, whose lanes
+// also wait for memory longer: 4.
+constexpr uint32_t kRefillRays = 8, kRefillBatch = 4, kRefillCoherent = 32, kRefillMirror = 24;
+
 // Whether an instantiation shares its warp's leaf tests (coop_leaf, one
-// 8-byte slot per thread): the closest-hit single-scene kernels of every
-// variant but brute force. Counting launches of occlusion rays take the
-// closest-hit kernel. The kernel and the launcher both use this.
+// 8-byte slot per thread): every closest-hit kernel but brute force and the
+// batches' shared-memory stack, whose ring may fill the shared memory alone;
+// occlusion rays of the stack variants too (a 24,576-triangle frame's take 45
+// us less), not of ropes, where stopping at the first hit closer than the light
+// saves more (a six-light frame's would take 145 us more). Counting launches
+// of occlusion rays take the closest-hit kernel. The kernel and the launcher
+// both use this.
 __host__ __device__ constexpr bool trace_coop_slots(int variant, bool batch, bool any) {
-    return variant != HK_TRACE_BRUTE && !batch && !any;
+    if (variant == HK_TRACE_BRUTE) return false;
+    return batch ? variant != HK_TRACE_SMEMSTACK : !(any && variant == HK_TRACE_ROPES);
 }
 
 // Blocks of kTraceMaxBlock threads that an instantiation is compiled to keep
 // resident on an SM (its __launch_bounds__; smaller blocks in proportion).
 __host__ __device__ constexpr uint32_t trace_resident_blocks(int variant, bool batch, bool any) {
-    return batch ? 4u : ((variant != HK_TRACE_BRUTE && !any) ? 5u : 6u);
+    return batch ? 4u : (trace_coop_slots(variant, batch, any) ? 5u : 6u);
 }
 
 // dynamic shared memory of one trace launch: the shared-memory ring of

@@ -6,8 +6,8 @@
 // count and uneven ray batches balance themselves. Traversal semantics follow
 // the reference kernels exactly (comparison operators, near/far rule, the
 // "child 0" sentinel, strict < between hits in leaf order); see the comments
-// at each variant. Closest-hit single-scene launches test the leaves of a
-// whole warp together (coop_leaf), which keeps the same hits bit for bit.
+// at each variant. Most launches test the leaves of a whole warp together
+// (coop_leaf), which keeps the same hits bit for bit.
 #include <algorithm>
 
 #include "hk_common.cuh"
@@ -30,6 +30,7 @@ struct TraceArgs {
     uint32_t *err;            // error word (bounded loops)
     uint32_t stack_depth;     // ring depth for the short-stack variants
     uint32_t max_steps;       // per-ray iteration bound
+    uint32_t refill;          // idle lanes before a warp takes new rays
     const uint32_t *ropes;    // ropes variant: 6 per node
     const float4 *cbox;       // ropes variant: cell min, max per node
     uint32_t rope_nn;         // compact node count (legs bound 4 n + 8) ...
@@ -106,10 +107,10 @@ __device__ __forceinline__ uint32_t sentinel_to_root(uint2 n, uint32_t c) {
 // Every lane keeps its ray's traversal state across iterations of the warp
 // loop. One iteration runs one "leg" per active lane: pop (or restart at the
 // root), descend to a leaf, test it. A lane whose ray is finished writes its
-// hit and takes a new ray at the next iteration: the warp counts its idle
-// lanes with __ballot_sync, lane 0 takes that many rays with one atomicAdd
-// and each idle lane picks its own by rank. Rays of different cost therefore
-// no longer hold a warp hostage until the slowest of 32 finishes.
+// hit and idles until the warp has as many idle lanes as the launch asks for
+// (kRefill*): lane 0 then takes that many rays with one atomicAdd and each idle
+// lane picks its own by rank, so rays of different cost do not hold a warp
+// until the slowest of 32 finishes.
 // ---------------------------------------------------------------------------
 struct LaneState {
     float3 o, d, inv;
@@ -405,8 +406,10 @@ __device__ __forceinline__ bool leg_ropes(const SceneView &A, LaneState &L, uint
 // t does not depend on the best hit it is tested against (that only culls),
 // so this is the hit the in-order loop keeps -- the closest, the first in
 // leaf order among equal t -- bit for bit.
-__device__ __forceinline__ void coop_leaf(const SceneView &V, LaneState &L, uint32_t start, uint32_t cnt,
-                                          unsigned long long *slot) {
+// In a batch a pair's scene is its owner's.
+template <bool BATCH>
+__device__ __forceinline__ void coop_leaf(const SceneView &V, const SceneDesc *scenes, uint32_t scene, LaneState &L,
+                                          uint32_t start, uint32_t cnt, unsigned long long *slot) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t P = cnt;   // inclusive prefix of the counts over the lanes
 #pragma unroll
@@ -434,9 +437,16 @@ __device__ __forceinline__ void coop_leaf(const SceneView &V, LaneState &L, uint
         const float3 d = make_float3(__shfl_sync(0xffffffffu, L.d.x, owner), __shfl_sync(0xffffffffu, L.d.y, owner),
                                      __shfl_sync(0xffffffffu, L.d.z, owner));
         const float best = __shfl_sync(0xffffffffu, L.best, owner);
+        const uint32_t *refs = V.refs;
+        const TriRec *tris = V.tris;
+        if (BATCH) {
+            const SceneDesc &D = scenes[__shfl_sync(0xffffffffu, scene, owner)];   // (idle lanes: scene 0)
+            refs = D.refs;
+            tris = D.tris;
+        }
         if (w < W) {
-            const uint32_t tri = __ldg(&V.refs[st + j]);
-            const float t = isect_tri(&V.tris[tri], o, d, best);
+            const uint32_t tri = __ldg(&refs[st + j]);
+            const float t = isect_tri(&tris[tri], o, d, best);
             if (t < best) {
                 const uint32_t tb = __float_as_uint(t);
                 const unsigned long long key =
@@ -490,10 +500,8 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t c_nodes = 0, c_refs = 0;
-    // single-scene closest-hit ropes: leaf tests shared out over the warp
-    // (coop_leaf), one 8-byte slot per lane in dynamic shared memory. Occlusion
-    // rays keep the in-order test, which stops at the first hit closer than
-    // the light.
+    // leaf tests shared out over the warp (coop_leaf), one 8-byte slot per lane
+    // in dynamic shared memory
     constexpr bool COOP = VARIANT == HK_TRACE_ROPES && trace_coop_slots(VARIANT, BATCH, ANY);
     // the stack variants defer their leaf test to the same warp-wide pass
     constexpr bool COOP_LEG = VARIANT != HK_TRACE_ROPES && trace_coop_slots(VARIANT, BATCH, ANY);
@@ -530,12 +538,21 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
         L.o = L.d = make_float3(0.0f, 0.0f, 0.0f);
         L.best = kInf;
     }
+    // a batch lane's scene arrays, looked up at every leg (L1-resident) rather
+    // than kept
+    auto look_up = [&] {
+        const SceneDesc &D = A.scenes[scene];
+        V = SceneView{D.nodes, D.refs, D.tris, D.ropes, D.cbox};
+        legs_max = 4u * D.nn + 8u;
+        ntris = D.ntris;
+        if (VARIANT != HK_TRACE_ROPES && VARIANT != HK_TRACE_BRUTE) root = V.nodes[0];
+    };
     bool active = false, drained = false;
     uint32_t steps = 0;
     while (true) {
         // refill idle lanes
         uint32_t idle = __ballot_sync(0xffffffffu, !active && takes);
-        if (idle && !drained) {
+        if (idle && !drained && (__popc(idle) >= (int)A.refill || __ballot_sync(0xffffffffu, active) == 0)) {
             uint32_t want = __popc(idle);
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(A.fetch, want);
@@ -622,15 +639,19 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
             float texit = 0.0f;
             uint32_t rope = kNoRope;
             bool fin = false;
-            if (active) fin = ropes_locate<COUNT>(V, L, legs_max, c_nodes, lstart, lcnt, texit, rope);
+            if (active) {
+                if (BATCH) look_up();
+                fin = ropes_locate<COUNT>(V, L, legs_max, c_nodes, lstart, lcnt, texit, rope);
+            }
             const uint32_t work = (active && !fin) ? lcnt : 0u;
-            coop_leaf(V, L, lstart, work, slot);
+            coop_leaf<BATCH>(V, A.scenes, scene, L, lstart, work, slot);
             if (COUNT) c_refs += work;
             if (!active) continue;
             if (fin || ropes_advance<ANY>(L, lcnt, texit, rope)) {
                 A.hits[L.ray] = hk_hit{L.best, L.best_id};
-                if (A.leaf_out) A.leaf_out[L.ray] = L.cur;
+                if (!BATCH && A.leaf_out) A.leaf_out[L.ray] = L.cur;
                 active = false;
+                if (BATCH && atomicSub(&A.remaining[scene], 1u) == 1u) A.done_ns[scene] = global_ns();
             }
             continue;
         }
@@ -640,6 +661,7 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
             Defer df{0u, 0u, kNoTest};
             bool fin = false;
             if (active) {
+                if (BATCH) look_up();
                 if (VARIANT == HK_TRACE_FULLSTACK)
                     fin = leg_fullstack<COUNT, ANY, true>(A, V, L, root, l_s, l_e, l_n, kLocal, c_nodes, c_refs,
                                                           steps, &df);
@@ -652,22 +674,18 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
                                                                       c_nodes, c_refs, steps, &df);
             }
             const uint32_t work = (active && df.after != kNoTest) ? df.cnt : 0u;
-            coop_leaf(V, L, df.start, work, slot);
+            coop_leaf<BATCH>(V, A.scenes, scene, L, df.start, work, slot);
             if (COUNT) c_refs += work;
             if (!active) continue;
-            if (fin || df.after == kDone || (df.after == kDoneIfCloser && L.best < L.tmax)) {
+            if (fin || df.after == kDone || (df.after == kDoneIfCloser && L.best < L.tmax) ||
+                (ANY && df.after != kNoTest && L.best < L.lim)) {
                 A.hits[L.ray] = hk_hit{L.best, L.best_id};
                 active = false;
+                if (BATCH && atomicSub(&A.remaining[scene], 1u) == 1u) A.done_ns[scene] = global_ns();
             }
             continue;
         }
-        if (BATCH) {
-            const SceneDesc &D = A.scenes[scene];
-            V = SceneView{D.nodes, D.refs, D.tris, D.ropes, D.cbox};
-            legs_max = 4u * D.nn + 8u;
-            ntris = D.ntris;
-            if (VARIANT != HK_TRACE_ROPES && VARIANT != HK_TRACE_BRUTE) root = V.nodes[0];
-        }
+        if (BATCH) look_up();
         bool done;
         if (VARIANT == HK_TRACE_BRUTE) {
             // GPUTrace_bruteforce.cl:30-42: every triangle in index order
@@ -763,6 +781,7 @@ cudaError_t launch_trace(const TraceLaunch &L, cudaStream_t s) {
     a.err = L.err;
     a.stack_depth = L.stack_depth;
     a.max_steps = L.max_steps;
+    a.refill = L.refill ? L.refill : (L.scenes ? kRefillBatch : kRefillRays);
     a.ropes = L.ropes;
     a.cbox = L.cbox;
     a.rope_nn = L.rope_nn;
