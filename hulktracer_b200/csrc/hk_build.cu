@@ -545,20 +545,22 @@ __device__ __forceinline__ bool decidable(const LevelArgs &A, uint32_t cnt) {
 __device__ __forceinline__ bool is_exact(const LevelArgs &A, uint32_t c) {
     return A.exact_max >= kWarpExact && c > kWarpExact && c <= A.exact_max;
 }
-// (nodes of up to kExactWarp references are one warp's work too, unless
-// training rows are recorded, which the CTA does)
-constexpr uint32_t kExactWarp = 128;
-__device__ __forceinline__ bool is_medium(const LevelArgs &A, uint32_t c) {
-    return is_exact(A, c) && (c > kExactWarp || A.record);
-}
 // learned mode: a proposer row (33..1024 references)
 __device__ __forceinline__ bool is_learn(const LevelArgs &A, uint32_t c) {
     return A.learned && c > kWarpExact && c <= kLearnMax;
 }
+// ... whose histogram one warp builds (in the medium list; larger ones are chunks)
+__device__ __forceinline__ bool is_row_warp(const LevelArgs &A, uint32_t c) { return is_learn(A, c) && c <= kSmall; }
+// (nodes of up to kExactWarp references are one warp's work too, unless
+// training rows are recorded, which the CTA does)
+constexpr uint32_t kExactWarp = 128;
+__device__ __forceinline__ bool is_medium(const LevelArgs &A, uint32_t c) {
+    return (is_exact(A, c) && (c > kExactWarp || A.record)) || is_row_warp(A, c);
+}
 // large: k_hist's chunked histograms (in learned mode the proposer rows too, so
 // that the proposer's chain needs nothing from k_small)
 __device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c) {
-    return (c > kSmall || is_learn(A, c)) && !is_exact(A, c);
+    return (c > kSmall || is_learn(A, c)) && !is_exact(A, c) && !is_row_warp(A, c);
 }
 // References per chunk of a node of more than kChunk references, in a level
 // of `refs` references: small enough that the level's chunks fill k_decide's
@@ -931,26 +933,6 @@ __device__ __forceinline__ Decision sah_warp32(const LevelArgs &A, float *S, uin
     return EXACT ? sah_lanes_exact(S, c, blo, bhi, A.ct, A.ci) : sah_lanes_binned(S, c, blo, bhi, A.ct, A.ci);
 }
 
-// first index in sorted v[0, n) with v[i] >= p (lower) or v[i] > p (upper)
-__device__ __forceinline__ uint32_t lower_bound_f(const float *v, uint32_t n, float p) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t m = (lo + hi) >> 1;
-        if (v[m] < p) lo = m + 1;
-        else hi = m;
-    }
-    return lo;
-}
-__device__ __forceinline__ uint32_t upper_bound_f(const float *v, uint32_t n, float p) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t m = (lo + hi) >> 1;
-        if (v[m] <= p) lo = m + 1;
-        else hi = m;
-    }
-    return lo;
-}
-
 // Exact SAH of a node of more than 32 references by a group of NT threads (a
 // warp: up to 128 references; a CTA of 256: up to 1024), without sorting.
 //   1. every clipped bound strictly inside the node goes to its bin's bucket
@@ -995,6 +977,38 @@ __device__ __forceinline__ void group_sync() {
 
 __device__ __forceinline__ bool refine_better(float c, uint32_t a, float p, float bc, uint32_t ba, float bp) {
     return c < bc || (c == bc && (a < ba || (a == ba && p < bp)));
+}
+
+// the group's least (cost, axis, plane) with its counts, on every thread (S:
+// shared memory with the arrays w_cost .. w_pk)
+template <uint32_t NT, class Smem>
+__device__ __forceinline__ void group_argmin(Smem &S, float &mc, uint32_t &m_ax, float &m_pk, uint32_t &m_nb,
+                                             uint32_t &m_na) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t src = warp_argmin(mc, m_ax, m_pk);
+    if (NT > 32) {
+        if (lane == src) {
+            const uint32_t w = threadIdx.x >> 5;
+            S.w_cost[w] = __float_as_uint(mc);
+            S.w_ax[w] = m_ax;
+            S.w_pk[w] = m_pk;
+            S.w_nb[w] = m_nb;
+            S.w_na[w] = m_na;
+        }
+        __syncthreads();
+        const uint32_t w = min(lane, NT / 32 - 1);
+        mc = __uint_as_float(S.w_cost[w]);
+        m_ax = S.w_ax[w];
+        m_pk = S.w_pk[w];
+        m_nb = S.w_nb[w];
+        m_na = S.w_na[w];
+        src = warp_argmin(mc, m_ax, m_pk);
+    }
+    mc = __shfl_sync(0xffffffffu, mc, src);
+    m_ax = __shfl_sync(0xffffffffu, m_ax, src);
+    m_pk = __shfl_sync(0xffffffffu, m_pk, src);
+    m_nb = __shfl_sync(0xffffffffu, m_nb, src);
+    m_na = __shfl_sync(0xffffffffu, m_na, src);
 }
 
 template <uint32_t NT>
@@ -1181,31 +1195,8 @@ __device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, 
         if (lane == 0) atomicMin(&S.best, wb);
         group_sync<NT>();
     }
-    uint32_t src = warp_argmin(mc, m_ax, m_pk);
-    if (NT > 32) {
-        if (lane == src) {
-            const uint32_t w = tid >> 5;
-            S.w_cost[w] = __float_as_uint(mc);
-            S.w_ax[w] = m_ax;
-            S.w_pk[w] = m_pk;
-            S.w_nb[w] = m_nb;
-            S.w_na[w] = m_na;
-        }
-        __syncthreads();
-        const uint32_t w = min(lane, NT / 32 - 1);
-        mc = __uint_as_float(S.w_cost[w]);
-        m_ax = S.w_ax[w];
-        m_pk = S.w_pk[w];
-        m_nb = S.w_nb[w];
-        m_na = S.w_na[w];
-        src = warp_argmin(mc, m_ax, m_pk);
-    }
+    group_argmin<NT>(S, mc, m_ax, m_pk, m_nb, m_na);
     Decision best{-1, 0.0f, 0, 0, kInf, 0};
-    mc = __shfl_sync(0xffffffffu, mc, src);
-    m_ax = __shfl_sync(0xffffffffu, m_ax, src);
-    m_pk = __shfl_sync(0xffffffffu, m_pk, src);
-    m_nb = __shfl_sync(0xffffffffu, m_nb, src);
-    m_na = __shfl_sync(0xffffffffu, m_na, src);
     if (mc < kInf) best = Decision{(int)m_ax, m_pk, m_nb, m_na, mc, 0};
     if (best.axis >= 0 && !(best.cost < __fmul_rn(A.ci, (float)cnt))) best.axis = -1;
     return best;
@@ -1241,6 +1232,56 @@ __device__ __forceinline__ void finish_large(const LevelArgs &A, uint32_t s, con
     }
 }
 
+// a small-node warp's shared memory (16-byte aligned in an array of them: the
+// scratch is cleared and read 16 bytes at a time)
+template <bool EXACT>
+union alignas(16) WarpSmem {
+    uint32_t scratch[kWarpScratch];
+};
+template <>
+union alignas(16) WarpSmem<true> {
+    uint32_t scratch[kWarpScratch];
+    ExactSmem<32> exact;
+};
+static_assert(sizeof(WarpSmem<false>) % 16 == 0 && sizeof(WarpSmem<true>) % 16 == 0, "16-byte accesses");
+
+// the binned histogram of a node by one warp: kPass references per lane and
+// pass, their loads issued together
+template <int kPass>
+__device__ __forceinline__ void warp_hist(const LevelArgs &A, uint32_t *Hw, float *Pw, uint4 info, float4 blo,
+                                          float4 bhi) {
+    const uint32_t lane = threadIdx.x & 31u, cnt = info.y;
+    __syncwarp();   // the previous node's readers are done
+    {
+        // 288 counters = 72 16-byte stores
+        uint4 *H4 = reinterpret_cast<uint4 *>(Hw);
+        H4[lane] = make_uint4(0, 0, 0, 0);
+        H4[lane + 32] = make_uint4(0, 0, 0, 0);
+        if (lane < kHist / 4 - 64) H4[lane + 64] = make_uint4(0, 0, 0, 0);
+    }
+    node_planes_warp(Pw, blo, bhi);
+    __syncwarp();
+    const float4 inv3 = bin_scale(blo, bhi);
+    for (uint32_t base = 0; base < cnt; base += 32 * kPass) {
+        uint32_t tri[kPass];
+        float4 tlo[kPass], thi[kPass];
+#pragma unroll
+        for (int k = 0; k < kPass; k++) {
+            const uint32_t r = base + 32u * k + lane;
+            tri[k] = r < cnt ? A.refs()[info.x + r] : 0xffffffffu;
+        }
+#pragma unroll
+        for (int k = 0; k < kPass; k++)
+            if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
+#pragma unroll
+        for (int k = 0; k < kPass; k++) {
+            if (base + 32u * k >= cnt) break;   // uniform across the warp
+            if (tri[k] != 0xffffffffu) hist_ref_tab(Hw, tlo[k], thi[k], blo, bhi, inv3, Pw);
+        }
+    }
+    __syncwarp();
+}
+
 // shared memory of a CTA's large-node work
 struct HistSmem {
     uint32_t H[kHist];
@@ -1250,6 +1291,7 @@ struct HistSmem {
 
 // k_hist's work for one level (every CTA of the grid calls it): the chunks of
 // the large nodes and, with MEDIUM, the medium nodes (exact SAH, XS)
+enum : int { kHistChunks = 0, kHistExact = 1, kHistRows = 2 };
 // what a CTA's large-node work starts from, loaded before the kernel's first
 // barrier (the record of its first chunk is read whether the level has it or not)
 struct HistStart {
@@ -1362,33 +1404,38 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, const HistStart &h
     }
 }
 
-// (the exact search's registers and shared memory only where a level can have
-// medium nodes)
-template <bool MEDIUM>
-__global__ void __launch_bounds__(256, 3) k_hist(LevelArgs A) {
-    __shared__ HistSmem SH;
-    __shared__ std::conditional_t<MEDIUM, ExactSmem<256>, uint32_t> XS;
+// k_hist: the chunks alone, with the exact search of the medium nodes, or (learned
+// mode) with the proposer rows of up to 256 references, a warp each, the CTAs
+// without chunks first
+template <int MODE>
+__global__ void __launch_bounds__(256, MODE == kHistRows ? 4 : 3) k_hist(LevelArgs A) {
+    union Smem {
+        HistSmem hist;
+        std::conditional_t<MODE == kHistRows, WarpSmem<false>, uint32_t> rows[8];
+    };
+    __shared__ __align__(16) Smem SH;
+    __shared__ std::conditional_t<MODE == kHistExact, ExactSmem<256>, uint32_t> XS;
     __shared__ uint32_t s_tally[kTallies];
-    const HistStart hs = hist_start<MEDIUM>(A);
+    const HistStart hs = hist_start<MODE != kHistChunks>(A);
     if (level_aborted(A)) return;
     Tally tally;
-    if constexpr (MEDIUM) hist_body<true>(A, hs, SH, &XS, tally);
-    else hist_body<false>(A, hs, SH, nullptr, tally);
+    if constexpr (MODE == kHistExact) hist_body<true>(A, hs, SH.hist, &XS, tally);
+    else hist_body<false>(A, HistStart{hs.ck, hs.nch, 0u, hs.nodes}, SH.hist, nullptr, tally);
+    if constexpr (MODE == kHistRows) {
+        __syncthreads();
+        const uint32_t wib = threadIdx.x >> 5;
+        for (uint32_t k = (gridDim.x - 1 - blockIdx.x) * 8 + wib; k < hs.nmed; k += gridDim.x * 8) {
+            const uint32_t s = A.medium_slot[k];
+            if (s >= hs.nodes) continue;
+            const uint4 info = A.n_info()[s];
+            const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
+            uint32_t *Hw = SH.rows[wib].scratch;
+            warp_hist<4>(A, Hw, reinterpret_cast<float *>(Hw + kHist), info, blo, bhi);
+            finish_large(A, s, info, blo, bhi, Hw, tally);
+        }
+    }
     tally_flush(A, tally, s_tally);
 }
-
-// a small-node warp's shared memory (16-byte aligned in an array of them: the
-// scratch is cleared and read 16 bytes at a time)
-template <bool EXACT>
-union alignas(16) WarpSmem {
-    uint32_t scratch[kWarpScratch];
-};
-template <>
-union alignas(16) WarpSmem<true> {
-    uint32_t scratch[kWarpScratch];
-    ExactSmem<32> exact;
-};
-static_assert(sizeof(WarpSmem<false>) % 16 == 0 && sizeof(WarpSmem<true>) % 16 == 0, "16-byte accesses");
 
 // Small nodes (not splittable, or splittable and neither medium nor large):
 // one warp per node; the exact SAH in registers for nodes of at most 32
@@ -1425,41 +1472,10 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
         } else if (WARP_EXACT && !LEARNED && is_exact(A, cnt)) {
             if constexpr (WARP_EXACT && !LEARNED) d = sah_exact_group<32>(A, info, blo, bhi, WSp[wib].exact);
         } else {
+            // (one reference per lane and pass in the exact instantiation, which
+            // has few nodes here and no registers to spare)
             uint32_t *Hw = WSp[wib].scratch;
-            float *Pw = reinterpret_cast<float *>(WSp[wib].scratch + kHist);
-            __syncwarp();   // the previous node's readers are done
-            {
-                // 288 counters = 72 16-byte stores
-                uint4 *H4 = reinterpret_cast<uint4 *>(Hw);
-                H4[lane] = make_uint4(0, 0, 0, 0);
-                H4[lane + 32] = make_uint4(0, 0, 0, 0);
-                if (lane < kHist / 4 - 64) H4[lane + 64] = make_uint4(0, 0, 0, 0);
-            }
-            node_planes_warp(Pw, blo, bhi);
-            __syncwarp();
-            const float4 inv3 = bin_scale(blo, bhi);
-            // four references per lane and pass, their loads issued together
-            // (the exact instantiation, which has few nodes here and no
-            // registers to spare: one)
-            constexpr int kPass = WARP_EXACT ? 1 : 4;
-            for (uint32_t base = 0; base < cnt; base += 32 * kPass) {
-                uint32_t tri[kPass];
-                float4 tlo[kPass], thi[kPass];
-#pragma unroll
-                for (int k = 0; k < kPass; k++) {
-                    const uint32_t r = base + 32u * k + lane;
-                    tri[k] = r < cnt ? A.refs()[info.x + r] : 0xffffffffu;
-                }
-#pragma unroll
-                for (int k = 0; k < kPass; k++)
-                    if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
-#pragma unroll
-                for (int k = 0; k < kPass; k++) {
-                    if (base + 32u * k >= cnt) break;   // uniform across the warp
-                    if (tri[k] != 0xffffffffu) hist_ref_tab(Hw, tlo[k], thi[k], blo, bhi, inv3, Pw);
-                }
-            }
-            __syncwarp();
+            warp_hist<WARP_EXACT ? 1 : 4>(A, Hw, reinterpret_cast<float *>(Hw + kHist), info, blo, bhi);
             d = sah_warp(Hw, blo, bhi, cnt, A.ct, A.ci);
         }
         if (lane == 0) {
@@ -1505,7 +1521,6 @@ __global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
 
 constexpr int kLearnMaxK = 8;
 constexpr uint32_t kLearnScratch = 2048;   // floats of list space per warp
-constexpr size_t kRefineSmem = (size_t)kLearnScratch * 4;   // the lists of one row, 8 KB
 
 // list capacity per (proposal, list): the largest power of two with 3 k of
 // them in one warp's space (128 for k = 4), so a list sorts in place
@@ -1514,105 +1529,6 @@ __host__ __device__ constexpr uint32_t learn_list_cap(uint32_t K) {
     while (2 * c * 3 * K <= kLearnScratch) c *= 2;
     return c;
 }
-// lists of up to 32 x kLearnSortRegs values sort in registers (every list
-// with k >= 4 proposals); longer ones in shared memory
-constexpr int kLearnSortRegs = 4;
-
-// warp-aggregated append of val (where pred) to list[n ..); n counts past cap
-__device__ __forceinline__ void list_append(float *list, uint32_t cap, uint32_t &n, bool pred, float val) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t m = __ballot_sync(0xffffffffu, pred);
-    if (pred) {
-        const uint32_t pos = n + __popc(m & ((1u << lane) - 1u));
-        if (pos < cap) list[pos] = val;
-    }
-    n += __popc(m);
-}
-
-// ascending bitonic sort of v[0, n) in shared memory by one warp; the list's
-// capacity is a power of two >= n, the padding up to the next power of two
-// is filled with +inf
-__device__ __forceinline__ void warp_sort_smem(float *v, uint32_t n) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (uint32_t i = n + lane; i < n2; i += 32) v[i] = kInf;
-    __syncwarp();
-    for (uint32_t k = 2; k <= n2; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = lane; i < n2; i += 32) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const bool up = (i & k) == 0;
-                    const float x = v[i], y = v[ixj];
-                    if ((x > y) == up) {
-                        v[i] = y;
-                        v[ixj] = x;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-}
-
-// ascending bitonic sort of v[0, n) by one warp, done in registers: element
-// r * 32 + lane of the list padded with +inf to the next power of two in x[r]
-// of that lane (R registers, up to 32 R elements), every compare-exchange a
-// shuffle (partner in another lane) or a swap between two of the lane's
-// registers; the sorted list is written back to v[0, n)
-template <int R>
-__device__ __forceinline__ void warp_sort_regs(float *v, uint32_t n) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    const uint32_t nr = (n2 + 31u) >> 5;
-    float x[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const uint32_t i = (uint32_t)r * 32u + lane;
-        x[r] = i < n ? v[i] : kInf;
-    }
-    for (uint32_t k = 2; k <= n2; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (j >= 32) {
-                const uint32_t rj = j >> 5;
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    if ((uint32_t)r >= nr || ((uint32_t)r & rj)) continue;
-                    const int r2 = r | (int)rj;
-                    const bool up = (((uint32_t)r * 32u + lane) & k) == 0;
-                    const float a = x[r], b = x[r2];
-                    if ((a > b) == up) {
-                        x[r] = b;
-                        x[r2] = a;
-                    }
-                }
-            } else {
-                const bool lower = (lane & j) == 0;
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    if ((uint32_t)r >= nr) continue;
-                    const float p = __shfl_xor_sync(0xffffffffu, x[r], (int)j);
-                    const bool up = (((uint32_t)r * 32u + lane) & k) == 0;
-                    const float mn = x[r] < p ? x[r] : p, mx = x[r] < p ? p : x[r];
-                    x[r] = (lower == up) ? mn : mx;
-                }
-            }
-        }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const uint32_t i = (uint32_t)r * 32u + lane;
-        if (i < n) v[i] = x[r];
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void warp_sort_list(float *v, uint32_t n) {
-    if (n <= 32u * kLearnSortRegs) warp_sort_regs<kLearnSortRegs>(v, n);
-    else warp_sort_smem(v, n);
-}
-
 // ---------------------------------------------------------------------------
 // learned split search (no reference counterpart), two launches per level.
 // k_learn: the network on the level's proposer rows (tcgen05: 128-row tiles,
@@ -1708,220 +1624,190 @@ __global__ void __launch_bounds__(256, 1) k_learn(LevelArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// k_refine_cta: one CTA per proposer row of more than kRefineWarpMax
-// references, grid-striding over the level's rows (k_refine_warp takes the
-// others).
-//   1. the 256 threads pass over the node's references once: per proposed bin
-//      (axis a, bin b, the closed interval [P0, P1] = [p_b, p_{b+1}] with p_0
-//      the node's minimum and p_32 its maximum) the references whose clipped
-//      lower bound lies below P0 and those whose clipped upper bound lies
-//      above P1 are counted, and the lower bounds, upper bounds and flat
-//      references inside [P0, P1] are listed in shared memory (slots taken
-//      per warp with one shared atomic: the order of a list is arbitrary, its
-//      contents are not);
-//   2. each warp sorts some of the lists (in registers);
-//   3. every listed bound p strictly inside the node is a candidate -- the
+// k_refine_warp, k_refine_cta: the exact search of a proposer row's proposed
+// bins by a group of NT threads -- a warp for rows of up to kRefineWarpMax
+// references, a CTA for larger ones, each kernel grid-striding over the level's
+// rows and leaving the other's.
+//   1. per proposed bin (axis a, bin b, the closed interval [P0, P1] =
+//      [p_b, p_{b+1}] with p_0 the node's minimum and p_32 its maximum) the
+//      references whose clipped lower bound lies below P0 and those whose
+//      clipped upper bound lies above P1 are counted, and the lower and upper
+//      bounds inside are listed in shared memory (in any order; a bound flat
+//      on its axis one step outside its value and flagged, lane_bounds);
+//   2. every listed bound p strictly inside the node is a candidate -- the
 //      exact SAH's candidates that fall in the bin -- with
-//        below = #(lo < P0) + #(listed lo < p) + #(listed flat at p),
-//        above = #(hi > P1) + #(listed hi > p) + #(listed flat at p)
-//      (binary searches in the sorted lists), the exact SAH's own counts; the
-//      threads share the candidates and the cheapest by (cost, axis, plane)
-//      wins (equal keys are the same plane with the same counts);
-//   4. that plane is taken unless it costs more than fallback_ratio x the
-//      binned optimum k_small found for the node (then the binned plane); the
-//      usual leaf test follows.
+//        below = #(lo < P0) + #(listed lo < p),
+//        above = #(hi > P1) + #(listed hi > p),
+//      the exact SAH's own counts; the threads share the candidates, each
+//      counts its bin's two lists, and the cheapest by (cost, axis, plane) wins
+//      (equal keys are the same plane with the same counts). The lists hold a
+//      32nd of the node's bounds: sorting them and searching the sorted lists
+//      took 650 + 524 us of a 200k-triangle learned build;
+//   3. that plane is taken unless it costs more than fallback_ratio x the
+//      binned optimum found for the node (then the binned plane); the usual
+//      leaf test follows.
 // A bin whose lists overflow their capacity (learn_list_cap) is not costed.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kRefineThreads = 256;
 constexpr uint32_t kRefineWarpMax = 128;   // rows up to this many references: one warp each
-constexpr uint32_t kRefineRowWarps = 8;
-constexpr size_t kRefineWarpSmem = (size_t)kRefineRowWarps * kLearnScratch * 4;   // 64 KB
-// k_refine_warp's grid in CTAs per SM: more than are resident (two, by its
-// registers), so that CTAs finishing early are replaced by new ones
-constexpr int kRefineWarpGrid = 3;
+constexpr uint32_t kRefineLists = 1280;    // most floats in the lists: 2 K learn_list_cap(K), K = 5
+static_assert(2 * 1 * learn_list_cap(1) <= kRefineLists && 2 * 2 * learn_list_cap(2) <= kRefineLists &&
+                  2 * 3 * learn_list_cap(3) <= kRefineLists && 2 * 4 * learn_list_cap(4) <= kRefineLists &&
+                  2 * 5 * learn_list_cap(5) <= kRefineLists && 2 * 6 * learn_list_cap(6) <= kRefineLists &&
+                  2 * 7 * learn_list_cap(7) <= kRefineLists && 2 * 8 * learn_list_cap(8) <= kRefineLists,
+              "the lists of every K fit");
 
-__global__ void __launch_bounds__(kRefineThreads) k_refine_cta(LevelArgs A) {
-    extern __shared__ __align__(16) float refine_smem[];
+template <uint32_t NT>
+struct RefineSmem {
+    uint32_t n[2 * kLearnMaxK];                 // listed lower, upper bounds per proposal
+    uint32_t bl[kLearnMaxK], ab[kLearnMaxK];    // references below P0, above P1
+    uint32_t flat[kRefineLists / 32];
+    float lists[kRefineLists];
+    uint32_t w_cost[NT / 32], w_ax[NT / 32], w_nb[NT / 32], w_na[NT / 32];
+    float w_pk[NT / 32];
+};
+
+// the group's row: its decision, and whether the proposal was taken
+template <uint32_t NT>
+__device__ __forceinline__ Decision refine_group(const LevelArgs &A, uint32_t row, const LearnBin &lb, uint32_t s,
+                                                 uint4 info, float4 blo, float4 bhi, RefineSmem<NT> &S, bool &take) {
+    const uint32_t lane = threadIdx.x & 31u, tid = NT == 32 ? lane : threadIdx.x;
+    const uint32_t cnt = info.y;
+    const uint32_t K = A.topk < (uint32_t)kLearnMaxK ? (A.topk ? A.topk : 1u) : (uint32_t)kLearnMaxK;
+    const uint32_t cap = learn_list_cap(K);
+    const uint2 pp = A.learn_prop[row];
+    const float4 ext = make_float4(__fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), 0.0f);
+    const float Anode = surf(blo, bhi);
+    // (axis << 5) | bin of proposal i, or 0xff: none (no later one either)
+    auto proposal = [&](uint32_t i) { return i < K ? ((i < 4 ? pp.x : pp.y) >> (8u * (i & 3u))) & 0xffu : 0xffu; };
+    group_sync<NT>();   // the previous row's readers are done
+    if (tid < 2 * kLearnMaxK) S.n[tid] = 0;
+    if (tid < kLearnMaxK) S.bl[tid] = S.ab[tid] = 0;
+    for (uint32_t i = tid; i < kRefineLists / 32; i += NT) S.flat[i] = 0;
+    // the thread's references, all loads issued together
+    float4 tlo[4], thi[4];
+    uint32_t tri[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t r = tid + NT * k;
+        tri[k] = r < cnt ? A.refs()[info.x + r] : 0xffffffffu;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (tri[k] != 0xffffffffu) load_bounds(A, tri[k], tlo[k], thi[k]);
+    group_sync<NT>();
+    // 1. counts and lists
+    for (uint32_t i = 0; i < (uint32_t)kLearnMaxK; i++) {
+        const uint32_t b8 = proposal(i);
+        if (b8 == 0xffu) break;
+        const uint32_t a = b8 >> 5, b = b8 & 31u;
+        const float l = c3(blo, a), h = c3(bhi, a);
+        const float p0 = b == 0 ? l : plane_k(l, c3(ext, a), b);
+        const float p1 = b == kBins - 1 ? h : plane_k(l, c3(ext, a), b + 1);
+        float *Ls = S.lists + 2 * i * cap, *Hs = Ls + cap;
+        uint32_t bl = 0, ab = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (tri[k] == 0xffffffffu) continue;
+            const float lo = mxf(c3(tlo[k], a), l), hi = mnf(c3(thi[k], a), h);
+            bl += lo < p0 ? 1u : 0u;
+            ab += hi > p1 ? 1u : 0u;
+            const bool fl = lo == hi;
+            if (p0 <= lo && lo <= p1) {
+                const uint32_t pos = atomicAdd(&S.n[2 * i], 1u);
+                if (pos < cap) {
+                    Ls[pos] = fl ? nextafterf(lo, -kInf) : lo;
+                    if (fl) atomicOr(&S.flat[(2 * i * cap + pos) >> 5], 1u << ((2 * i * cap + pos) & 31u));
+                }
+            }
+            if (p0 <= hi && hi <= p1) {
+                const uint32_t pos = atomicAdd(&S.n[2 * i + 1], 1u);
+                if (pos < cap) {
+                    Hs[pos] = fl ? nextafterf(hi, kInf) : hi;
+                    if (fl) atomicOr(&S.flat[((2 * i + 1) * cap + pos) >> 5], 1u << (((2 * i + 1) * cap + pos) & 31u));
+                }
+            }
+        }
+        bl = __reduce_add_sync(0xffffffffu, bl);
+        ab = __reduce_add_sync(0xffffffffu, ab);
+        if (lane == 0) {
+            if (bl) atomicAdd(&S.bl[i], bl);
+            if (ab) atomicAdd(&S.ab[i], ab);
+        }
+    }
+    group_sync<NT>();
+    // 2. the candidates of every proposal that did not overflow, numbered
+    // proposal by proposal
+    float mc = kInf, m_pk = 0.0f;
+    uint32_t m_ax = 3, m_nb = 0, m_na = 0;
+    for (uint32_t q = tid;; q += NT) {
+        uint32_t i = 0, t = q, nl = 0, nh = 0, b8 = 0xffu;
+        for (; i < (uint32_t)kLearnMaxK; i++) {
+            b8 = proposal(i);
+            if (b8 == 0xffu) break;
+            nl = S.n[2 * i];
+            nh = S.n[2 * i + 1];
+            if (nl > cap || nh > cap) continue;   // not costed
+            if (t < nl + nh) break;
+            t -= nl + nh;
+        }
+        if (i == (uint32_t)kLearnMaxK || b8 == 0xffu) break;
+        const uint32_t a = b8 >> 5;
+        const float l = c3(blo, a), h = c3(bhi, a);
+        const float *Ls = S.lists + 2 * i * cap, *Hs = Ls + cap;
+        const bool side = t >= nl;
+        const uint32_t at = 2 * i * cap + (side ? cap + t - nl : t);
+        float x = S.lists[at];
+        if ((S.flat[at >> 5] >> (at & 31u)) & 1u) x = nextafterf(x, side ? -kInf : kInf);
+        if (!(x > l && x < h)) continue;
+        const float pk = __fadd_rn(x, 0.0f);
+        uint32_t nb = S.bl[i], na = S.ab[i];
+        for (uint32_t k = 0; k < nl; k++) nb += Ls[k] < pk ? 1u : 0u;
+        for (uint32_t k = 0; k < nh; k++) na += Hs[k] > pk ? 1u : 0u;
+        const float cost = plane_cost(a, pk, l, h, ext, Anode, nb, na, A.ct, A.ci);
+        if (refine_better(cost, a, pk, mc, m_ax, m_pk)) {
+            mc = cost;
+            m_ax = a;
+            m_pk = pk;
+            m_nb = nb;
+            m_na = na;
+        }
+    }
+    __syncwarp();
+    group_argmin<NT>(S, mc, m_ax, m_pk, m_nb, m_na);
+    // 3. the proposal's plane, or the binned optimum
+    take = mc < kInf && mc <= __fmul_rn(A.fallback_ratio, lb.cost);
+    if (!take) return Decision{lb.axis, lb.plane, lb.nb, lb.na, lb.cost, 0};
+    Decision d{(int)m_ax, m_pk, m_nb, m_na, mc, 0};
+    if (!(mc < __fmul_rn(A.ci, (float)cnt))) d.axis = -1;
+    return d;
+}
+
+template <uint32_t NT>
+__device__ __forceinline__ void refine_rows(const LevelArgs &A, RefineSmem<NT> *SM) {
     __shared__ uint32_t s_tally[kTallies];
     __shared__ uint32_t s_stat[2];
-    __shared__ uint32_t s_n[3 * kLearnMaxK], s_bl[kLearnMaxK], s_ab[kLearnMaxK];
-    __shared__ float s_wc[kRefineThreads / 32], s_wp[kRefineThreads / 32];
-    __shared__ uint32_t s_wa[kRefineThreads / 32], s_wnb[kRefineThreads / 32], s_wna[kRefineThreads / 32];
-    wait_prior_grid();
     if (level_aborted(A)) return;
     Tally tally;
     uint32_t n_learned = 0, n_fallback = 0;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, wib = tid >> 5;
-    constexpr uint32_t kWarps = kRefineThreads / 32;
+    constexpr uint32_t kGroups = 256 / NT;
+    const uint32_t g = threadIdx.x / NT;
     const uint32_t rows = min(A.lc->n_learn, A.cap_learn);
-    const uint32_t K = A.topk < (uint32_t)kLearnMaxK ? (A.topk ? A.topk : 1u) : (uint32_t)kLearnMaxK;
-    const uint32_t cap = learn_list_cap(K);
-    for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
+    for (uint32_t row = blockIdx.x * kGroups + g; row < rows; row += gridDim.x * kGroups) {
         const LearnBin lb = A.learn_bin[row];
-        if (lb.pad[0] <= kRefineWarpMax) continue;   // k_refine_warp's row (uniform over the CTA)
+        if ((lb.pad[0] <= kRefineWarpMax) != (NT == 32)) continue;   // the other kernel's row (uniform over the group)
         const uint32_t s = A.learn_slot[row];
         const uint4 info = A.n_info()[s];
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
-        const uint32_t cnt = info.y;
-        const uint2 pp = A.learn_prop[row];
-        uint32_t pax[kLearnMaxK];
-        float p0[kLearnMaxK], p1[kLearnMaxK];
-        uint32_t np = 0;
-#pragma unroll
-        for (int r = 0; r < kLearnMaxK; r++) {
-            const uint32_t b8 = ((r < 4 ? pp.x : pp.y) >> (8 * (r & 3))) & 0xffu;
-            if (b8 == 0xffu || (uint32_t)r >= K) break;
-            const uint32_t a = b8 >> 5, b = b8 & 31u;
-            const float l = c3(blo, a), h = c3(bhi, a), ext = __fsub_rn(h, l);
-            pax[r] = a;
-            p0[r] = b == 0 ? l : plane_k(l, ext, b);
-            p1[r] = b == kBins - 1 ? h : plane_k(l, ext, b + 1);
-            np++;
-        }
-        if (tid < 3 * kLearnMaxK) s_n[tid] = 0;
-        if (tid < kLearnMaxK) s_bl[tid] = s_ab[tid] = 0;
-        __syncthreads();
-        // 1. counts and lists over the node's references
-        uint32_t bl[kLearnMaxK], ab[kLearnMaxK];
-#pragma unroll
-        for (int i = 0; i < kLearnMaxK; i++) bl[i] = ab[i] = 0;
-        for (uint32_t base = 0; base < cnt; base += kRefineThreads) {
-            const bool have = base + tid < cnt;
-            float4 tlo = make_float4(0, 0, 0, 0), thi = tlo;
-            if (have) {
-                const uint32_t tri = A.refs()[info.x + base + tid];
-                load_bounds(A, tri, tlo, thi);
-            }
-#pragma unroll
-            for (int i = 0; i < kLearnMaxK; i++) {
-                if ((uint32_t)i >= np) break;
-                const uint32_t a = pax[i];
-                const float l = c3(blo, a), h = c3(bhi, a);
-                const float lo = mxf(c3(tlo, a), l), hi = mnf(c3(thi, a), h);
-                bl[i] += (have && lo < p0[i]) ? 1u : 0u;
-                ab[i] += (have && hi > p1[i]) ? 1u : 0u;
-                const bool inL = have && p0[i] <= lo && lo <= p1[i];
-                const bool inH = have && p0[i] <= hi && hi <= p1[i];
-                const bool inF = inL && lo == hi;
-                float *Ls = refine_smem + (size_t)i * 3 * cap;
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    const bool pred = q == 0 ? inL : (q == 1 ? inH : inF);
-                    const uint32_t m = __ballot_sync(0xffffffffu, pred);
-                    if (!m) continue;
-                    uint32_t pos0 = 0;
-                    if (lane == (uint32_t)(__ffs(m) - 1)) pos0 = atomicAdd(&s_n[3 * i + q], (uint32_t)__popc(m));
-                    pos0 = __shfl_sync(0xffffffffu, pos0, __ffs(m) - 1);
-                    if (pred) {
-                        const uint32_t pos = pos0 + __popc(m & ((1u << lane) - 1u));
-                        if (pos < cap) Ls[(size_t)q * cap + pos] = q == 1 ? hi : lo;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kLearnMaxK; i++) {
-            if ((uint32_t)i >= np) break;
-            uint32_t b0 = bl[i], a0 = ab[i];
-            for (int o = 16; o; o >>= 1) {
-                b0 += __shfl_xor_sync(0xffffffffu, b0, o);
-                a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            }
-            if (lane == 0) {
-                if (b0) atomicAdd(&s_bl[i], b0);
-                if (a0) atomicAdd(&s_ab[i], a0);
-            }
-        }
-        __syncthreads();
-        // 2. sort the lists of the bins that did not overflow
-        for (uint32_t j = wib; j < 3 * np; j += kWarps) {
-            const uint32_t i = j / 3;
-            if (s_n[3 * i] > cap || s_n[3 * i + 1] > cap || s_n[3 * i + 2] > cap) continue;
-            const uint32_t n = s_n[j];
-            if (n > 1) warp_sort_list(refine_smem + (size_t)j * cap, n);
-        }
-        __syncthreads();
-        // 3. exact costs of the listed candidates
-        const float Anode = surf(blo, bhi);
-        float mc = kInf, m_pk = 0.0f;
-        uint32_t m_ax = 3, m_nb = 0, m_na = 0;
-        for (uint32_t i = 0; i < np; i++) {
-            const uint32_t nl = s_n[3 * i], nh = s_n[3 * i + 1], nf = s_n[3 * i + 2];
-            if (nl > cap || nh > cap || nf > cap) continue;   // overflowed: not costed
-            const uint32_t a = pax[i], b0 = s_bl[i], a0 = s_ab[i];
-            const float l = c3(blo, a), h = c3(bhi, a);
-            const float *Ls = refine_smem + (size_t)i * 3 * cap, *Hs = Ls + cap, *Fs = Ls + 2 * cap;
-            for (uint32_t q = tid; q < nl + nh; q += kRefineThreads) {
-                const float x = q < nl ? Ls[q] : Hs[q - nl];
-                if (!(x > l && x < h)) continue;
-                const float pk = __fadd_rn(x, 0.0f);
-                const uint32_t fon = nf ? upper_bound_f(Fs, nf, pk) - lower_bound_f(Fs, nf, pk) : 0u;
-                const uint32_t nb = b0 + lower_bound_f(Ls, nl, pk) + fon;
-                const uint32_t na = a0 + (nh - upper_bound_f(Hs, nh, pk)) + fon;
-                float4 bb = bhi, ba = blo;
-                s3(bb, a, pk);
-                s3(ba, a, pk);
-                const float sb = surf(blo, bb), sa = surf(ba, bhi);
-                const float cost = __fadd_rn(
-                    A.ct,
-                    __fmul_rn(A.ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
-                if (refine_better(cost, a, pk, mc, m_ax, m_pk)) {
-                    mc = cost;
-                    m_ax = a;
-                    m_pk = pk;
-                    m_nb = nb;
-                    m_na = na;
-                }
-            }
-        }
-        // 4. the cheapest over the CTA
-        for (int off = 16; off; off >>= 1) {
-            const float oc = __shfl_xor_sync(0xffffffffu, mc, off), op = __shfl_xor_sync(0xffffffffu, m_pk, off);
-            const uint32_t oa = __shfl_xor_sync(0xffffffffu, m_ax, off);
-            const uint32_t onb = __shfl_xor_sync(0xffffffffu, m_nb, off), ona = __shfl_xor_sync(0xffffffffu, m_na, off);
-            if (refine_better(oc, oa, op, mc, m_ax, m_pk)) {
-                mc = oc;
-                m_pk = op;
-                m_ax = oa;
-                m_nb = onb;
-                m_na = ona;
-            }
-        }
-        if (lane == 0) {
-            s_wc[wib] = mc;
-            s_wp[wib] = m_pk;
-            s_wa[wib] = m_ax;
-            s_wnb[wib] = m_nb;
-            s_wna[wib] = m_na;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            float bc = s_wc[0], bp = s_wp[0];
-            uint32_t bax = s_wa[0], nb = s_wnb[0], na = s_wna[0];
-            for (uint32_t w = 1; w < kWarps; w++)
-                if (refine_better(s_wc[w], s_wa[w], s_wp[w], bc, bax, bp)) {
-                    bc = s_wc[w];
-                    bp = s_wp[w];
-                    bax = s_wa[w];
-                    nb = s_wnb[w];
-                    na = s_wna[w];
-                }
-            // 5. the proposal's plane, or the binned optimum
-            const bool take = bc < kInf && bc <= __fmul_rn(A.fallback_ratio, lb.cost);
-            Decision d;
-            if (take) {
-                d = Decision{(int)bax, bp, nb, na, bc, 0};
-                if (!(bc < __fmul_rn(A.ci, (float)cnt))) d.axis = -1;
-            } else {
-                d = Decision{lb.axis, lb.plane, lb.nb, lb.na, lb.cost, 0};
-            }
+        bool take;
+        const Decision d = refine_group<NT>(A, row, lb, s, info, blo, bhi, SM[g], take);
+        if (threadIdx.x % NT == 0) {
             write_decision(A, s, d, blo, bhi);
-            tally.add(d, cnt);
+            tally.add(d, info.y);
             if (take) n_learned++;
             else n_fallback++;
         }
-        __syncthreads();
     }
+    __syncthreads();
     if (threadIdx.x < 2) s_stat[threadIdx.x] = 0;
     __syncthreads();
     if (n_learned) atomicAdd(&s_stat[0], n_learned);
@@ -1932,164 +1818,16 @@ __global__ void __launch_bounds__(kRefineThreads) k_refine_cta(LevelArgs A) {
     tally_flush(A, tally, s_tally);
 }
 
-// rows of at most kRefineWarpMax references: one warp per row, eight rows per
-// CTA, the same three steps with the lists in the warp's own shared memory
-__global__ void __launch_bounds__(256) k_refine_warp(LevelArgs A) {
-    extern __shared__ __align__(16) float refine_smem[];
-    __shared__ uint32_t s_tally[kTallies];
-    __shared__ uint32_t s_stat[2];
+__global__ void __launch_bounds__(256, 3) k_refine_cta(LevelArgs A) {
+    __shared__ RefineSmem<256> S;
     wait_prior_grid();
-    if (level_aborted(A)) return;
-    Tally tally;
-    uint32_t n_learned = 0, n_fallback = 0;
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t rows = min(A.lc->n_learn, A.cap_learn);
-    const uint32_t K = A.topk < (uint32_t)kLearnMaxK ? (A.topk ? A.topk : 1u) : (uint32_t)kLearnMaxK;
-    const uint32_t cap = learn_list_cap(K);
-    float *scratch = refine_smem + (size_t)wib * kLearnScratch;
-    for (uint32_t row = blockIdx.x * kRefineRowWarps + wib; row < rows; row += gridDim.x * kRefineRowWarps) {
-        const LearnBin lb = A.learn_bin[row];
-        if (lb.pad[0] > kRefineWarpMax) continue;   // k_refine_cta's row
-        const uint32_t s = A.learn_slot[row];
-        const uint4 info = A.n_info()[s];
-        const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];
-        const uint32_t cnt = info.y;
-        const uint2 pp = A.learn_prop[row];
-        uint32_t pax[kLearnMaxK];
-        float p0[kLearnMaxK], p1[kLearnMaxK];
-        uint32_t np = 0;
-#pragma unroll
-        for (int r = 0; r < kLearnMaxK; r++) {
-            const uint32_t b8 = ((r < 4 ? pp.x : pp.y) >> (8 * (r & 3))) & 0xffu;
-            if (b8 == 0xffu || (uint32_t)r >= K) break;
-            const uint32_t a = b8 >> 5, b = b8 & 31u;
-            const float l = c3(blo, a), h = c3(bhi, a), ext = __fsub_rn(h, l);
-            pax[r] = a;
-            p0[r] = b == 0 ? l : plane_k(l, ext, b);
-            p1[r] = b == kBins - 1 ? h : plane_k(l, ext, b + 1);
-            np++;
-        }
-        // 1. counts and lists over the node's references
-        uint32_t bl[kLearnMaxK], ab[kLearnMaxK], nL[kLearnMaxK], nH[kLearnMaxK], nF[kLearnMaxK];
-#pragma unroll
-        for (int i = 0; i < kLearnMaxK; i++) bl[i] = ab[i] = nL[i] = nH[i] = nF[i] = 0;
-        // four references per lane per pass: their loads are issued together
-        for (uint32_t base = 0; base < cnt; base += 128) {
-            float4 tlo[4], thi[4];
-            bool have[4];
-            uint32_t tri[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                have[u] = base + 32u * u + lane < cnt;
-                tri[u] = have[u] ? A.refs()[info.x + base + 32u * u + lane] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                tlo[u] = thi[u] = make_float4(0, 0, 0, 0);
-                if (have[u]) load_bounds(A, tri[u], tlo[u], thi[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (base + 32u * u >= cnt) break;   // uniform across the warp
-#pragma unroll
-                for (int i = 0; i < kLearnMaxK; i++) {
-                    if ((uint32_t)i >= np) break;
-                    const uint32_t a = pax[i];
-                    const float l = c3(blo, a), h = c3(bhi, a);
-                    const float lo = mxf(c3(tlo[u], a), l), hi = mnf(c3(thi[u], a), h);
-                    bl[i] += (have[u] && lo < p0[i]) ? 1u : 0u;
-                    ab[i] += (have[u] && hi > p1[i]) ? 1u : 0u;
-                    const bool inL = have[u] && p0[i] <= lo && lo <= p1[i];
-                    const bool inH = have[u] && p0[i] <= hi && hi <= p1[i];
-                    float *Ls = scratch + (size_t)i * 3 * cap;
-                    list_append(Ls, cap, nL[i], inL, lo);
-                    list_append(Ls + cap, cap, nH[i], inH, hi);
-                    list_append(Ls + 2 * cap, cap, nF[i], inL && lo == hi, lo);
-                }
-            }
-        }
-        __syncwarp();
-        // 2. exact costs of the listed candidates
-        const float Anode = surf(blo, bhi);
-        float mc = kInf, m_pk = 0.0f;
-        uint32_t m_ax = 3, m_nb = 0, m_na = 0;
-#pragma unroll
-        for (int i = 0; i < kLearnMaxK; i++) {
-            if ((uint32_t)i >= np) break;
-            uint32_t b0 = bl[i], a0 = ab[i];
-            for (int o = 16; o; o >>= 1) {
-                b0 += __shfl_xor_sync(0xffffffffu, b0, o);
-                a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            }
-            if (nL[i] > cap || nH[i] > cap || nF[i] > cap) continue;   // overflowed: not costed
-            const uint32_t a = pax[i];
-            const float l = c3(blo, a), h = c3(bhi, a);
-            float *Ls = scratch + (size_t)i * 3 * cap, *Hs = Ls + cap, *Fs = Ls + 2 * cap;
-            const uint32_t nl = nL[i], nh = nH[i], nf = nF[i];
-            warp_sort_list(Ls, nl);
-            warp_sort_list(Hs, nh);
-            if (nf) warp_sort_list(Fs, nf);
-            for (uint32_t q = lane; q < nl + nh; q += 32) {
-                const float x = q < nl ? Ls[q] : Hs[q - nl];
-                if (!(x > l && x < h)) continue;
-                const float pk = __fadd_rn(x, 0.0f);
-                const uint32_t fon = nf ? upper_bound_f(Fs, nf, pk) - lower_bound_f(Fs, nf, pk) : 0u;
-                const uint32_t nb = b0 + lower_bound_f(Ls, nl, pk) + fon;
-                const uint32_t na = a0 + (nh - upper_bound_f(Hs, nh, pk)) + fon;
-                float4 bb = bhi, ba = blo;
-                s3(bb, a, pk);
-                s3(ba, a, pk);
-                const float sb = surf(blo, bb), sa = surf(ba, bhi);
-                const float cost = __fadd_rn(
-                    A.ct,
-                    __fmul_rn(A.ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
-                if (cost < mc || (cost == mc && (a < m_ax || (a == m_ax && pk < m_pk)))) {
-                    mc = cost;
-                    m_ax = a;
-                    m_pk = pk;
-                    m_nb = nb;
-                    m_na = na;
-                }
-            }
-        }
-        float bc = mc, bp = m_pk;
-        uint32_t bax = m_ax, blane = lane;
-        for (int off = 16; off; off >>= 1) {
-            const float oc = __shfl_xor_sync(0xffffffffu, bc, off), op = __shfl_xor_sync(0xffffffffu, bp, off);
-            const uint32_t oax = __shfl_xor_sync(0xffffffffu, bax, off), ol = __shfl_xor_sync(0xffffffffu, blane, off);
-            if (oc < bc || (oc == bc && (oax < bax || (oax == bax && (op < bp || (op == bp && ol < blane)))))) {
-                bc = oc;
-                bp = op;
-                bax = oax;
-                blane = ol;
-            }
-        }
-        const uint32_t nb = __shfl_sync(0xffffffffu, m_nb, blane), na = __shfl_sync(0xffffffffu, m_na, blane);
-        // 3. the proposal's plane, or the binned optimum
-        const bool take = bc < kInf && bc <= __fmul_rn(A.fallback_ratio, lb.cost);
-        Decision d;
-        if (take) {
-            d = Decision{(int)bax, bp, nb, na, bc, 0};
-            if (!(bc < __fmul_rn(A.ci, (float)cnt))) d.axis = -1;
-        } else {
-            d = Decision{lb.axis, lb.plane, lb.nb, lb.na, lb.cost, 0};
-        }
-        if (lane == 0) {
-            write_decision(A, s, d, blo, bhi);
-            tally.add(d, cnt);
-            if (take) n_learned++;
-            else n_fallback++;
-        }
-        __syncwarp();
-    }
-    if (threadIdx.x < 2) s_stat[threadIdx.x] = 0;
-    __syncthreads();
-    if (n_learned) atomicAdd(&s_stat[0], n_learned);
-    if (n_fallback) atomicAdd(&s_stat[1], n_fallback);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_stat[0]) atomicAdd(&A.ctr->learned_nodes, s_stat[0]);
-    if (threadIdx.x == 1 && s_stat[1]) atomicAdd(&A.ctr->fallback_nodes, s_stat[1]);
-    tally_flush(A, tally, s_tally);
+    refine_rows<256>(A, &S);
+}
+
+__global__ void __launch_bounds__(256, 3) k_refine_warp(LevelArgs A) {
+    __shared__ RefineSmem<32> S[8];
+    wait_prior_grid();
+    refine_rows<32>(A, S);
 }
 
 // ---------------------------------------------------------------------------
@@ -3122,10 +2860,6 @@ cudaError_t build_learn_setup() {
         e = cudaFuncSetAttribute(k_learn<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_learn<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_refine_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRefineSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_refine_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRefineWarpSmem);
         if (e != cudaSuccess) return e;
         if (dev < 64) attr_set |= 1ull << dev;
     }
@@ -3244,9 +2978,10 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         // binned histograms, or the proposer's features, inference and costing
         cudaEventRecord(S.ev_fork, st);
         cudaStreamWaitEvent(S.aux, S.ev_fork, 0);
-        // one wave: three CTAs per SM resident
-        if (A.exact_max >= kWarpExact) k_hist<true><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
-        else k_hist<false><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
+        // one wave: three (four) CTAs per SM resident
+        if (A.learned) k_hist<kHistRows><<<S.sm_count * 4, 256, 0, S.aux>>>(A);
+        else if (A.exact_max >= kWarpExact) k_hist<kHistExact><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
+        else k_hist<kHistChunks><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
         if (A.learned) {
             // the proposer's chain on the second stream after the histograms
             // (every proposer row comes from k_hist), beside the small nodes
@@ -3257,9 +2992,9 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
             // stream, beside the CTA-costed ones
             cudaEventRecord(S.ev_learn, S.aux);
             cudaStreamWaitEvent(S.aux2, S.ev_learn, 0);
-            k_refine_warp<<<S.sm_count * kRefineWarpGrid, 256, kRefineWarpSmem, S.aux2>>>(A);
+            k_refine_warp<<<S.sm_count * 3, 256, 0, S.aux2>>>(A);
             cudaEventRecord(S.ev_join2, S.aux2);
-            launch_pdl(k_refine_cta, S.sm_count * 8, kRefineThreads, kRefineSmem, S.aux, A);
+            launch_pdl(k_refine_cta, S.sm_count * 3, 256, 0, S.aux, A);
         }
         cudaEventRecord(S.ev_join, S.aux);
         if (A.learned) {

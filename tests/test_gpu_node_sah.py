@@ -49,3 +49,24 @@ def test_small_nodes_identical_to_oracle(hk, oracle, exact_max, subtree_max, sub
                                       defer_margin=subtree_depth)
         assert np.array_equal(cn, on) and np.array_equal(cr, orf), n
     ctx.close()
+
+
+@pytest.mark.parametrize("topk", [1, 2, 3, 5, 6, 8])
+def test_learned_nodes_identical_to_oracle(hk, oracle, topk):
+    """Learned builds (untrained network) around the sizes where a proposer row
+    changes kernel, replayed by the oracle from the logged proposals."""
+    ctx = hk.Context(topk=topk, subtree_depth=0)
+    ctx.mlp_init(topk)
+    ctx.set_proposal_log(True)
+    for n in (33, 64, 127, 128, 129, 255, 256, 257, 700, 1023, 1024, 1025, 2500):
+        V, T = mixed_scene(n, 1000 * topk + n)
+        box = scenes.scene_box(V)
+        ctx.upload(V, T)
+        ctx.set_box(box)
+        ctx.precompute()
+        ctx.build(hk.BUILD_LEARNED)
+        cn, cr = ctx.export_compact()
+        on, orf = oracle.build_binned(V, T, box, proposals=ctx.proposal_log(), topk=topk, fallback_ratio=1.0, defer=32,
+                                      defer_margin=0)
+        assert np.array_equal(cn, on) and np.array_equal(cr, orf), n
+    ctx.close()
