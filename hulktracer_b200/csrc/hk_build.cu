@@ -484,9 +484,7 @@ struct LevelArgs {
     float4 *d_lo, *d_hi;
     uint32_t *defer_refs;
     uint32_t cap_defer;
-    uint2 *sc_key, *sc_node;   // subtree scratch node slots: (subtree, local index), entry
-    float4 *sc_cbox;           // 2 per node slot
-    uint32_t *sc_rope;         // 6 per node slot
+    uint32_t *sc_rec;          // subtree scratch node slots, 16 words each (SubWord)
     uint4 *sc_ref;             // subtree scratch reference slots: (subtree, local index, triangle, -)
     uint32_t cap_sc_nodes, cap_sc_refs;
     uint2 *st_cnt, *st_root, *st_base;   // per subtree: (nodes, refs), root entry, place
@@ -789,21 +787,27 @@ __device__ __forceinline__ void lanes_pack(float *S, bool in, uint32_t rank, uin
 
 // cost of nb references in a below cell that is db long on axis a and na in an
 // above cell that is da long, of a node with extents ext and surface Anode
-__device__ __forceinline__ float bounds_cost(uint32_t a, float db, float da, float4 ext, float Anode, uint32_t nb,
-                                             uint32_t na, float ct, float ci) {
+__device__ __forceinline__ float bounds_cost(uint32_t a, float db, float da, float4 ext, float Anode, float nb,
+                                             float na, float ct, float ci) {
     const float bx = a == 0 ? db : ext.x, by = a == 1 ? db : ext.y, bz = a == 2 ? db : ext.z;
     const float ax = a == 0 ? da : ext.x, ay = a == 1 ? da : ext.y, az = a == 2 ? da : ext.z;
     const float sb =
         __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(bx, by), __fmul_rn(bz, by)), __fmul_rn(bx, bz)));
     const float sa =
         __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(ax, ay), __fmul_rn(az, ay)), __fmul_rn(ax, az)));
-    return __fadd_rn(
-        ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, (float)nb), __fmul_rn(sa, (float)na)), Anode)));
+    return __fadd_rn(ct, __fmul_rn(ci, __fdiv_rn(__fadd_rn(__fmul_rn(sb, nb), __fmul_rn(sa, na)), Anode)));
 }
 // ... split at the plane pk
-__device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float h, float4 ext, float Anode,
-                                            uint32_t nb, uint32_t na, float ct, float ci) {
+__device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float h, float4 ext, float Anode, float nb,
+                                            float na, float ct, float ci) {
     return bounds_cost(a, __fsub_rn(pk, l), __fsub_rn(h, pk), ext, Anode, nb, na, ct, ci);
+}
+
+// 1 where a < b, else 0
+__device__ __forceinline__ float f_less(float a, float b) {
+    float r;
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
 // the binned SAH of a packed node: lane k counts and costs plane k of every
@@ -811,13 +815,15 @@ __device__ __forceinline__ float plane_cost(uint32_t a, float pk, float l, float
 // about 14 instructions each; a histogram costs about 350 whatever c is
 // (clearing, bins, atomics, scans), and the subtree pass's nodes hold 9
 // references on average.
+// (COUNTS: also the winner's counts, which the subtree pass does not need; the
+// counts are kept as floats, which hold them exactly and cost needs)
+template <bool COUNTS>
 __device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c, float4 blo, float4 bhi, float ct,
                                                      float ci) {
     const uint32_t lane = threadIdx.x & 31u;
     const float Anode = surf(blo, bhi);
     const float4 ext = make_float4(__fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), 0.0f);
-    float pk[3];
-    uint32_t nb[3] = {0, 0, 0}, na[3] = {0, 0, 0};
+    float pk[3], nb[3] = {0, 0, 0}, na[3] = {0, 0, 0};
 #pragma unroll
     for (uint32_t a = 0; a < 3; a++) pk[a] = plane_k(c3(blo, a), c3(ext, a), lane);
     for (uint32_t i = 0; i < c; i += 4) {
@@ -825,8 +831,14 @@ __device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c,
         for (uint32_t a = 0; a < 3; a++) {
             const float4 L = *reinterpret_cast<const float4 *>(S + (2 * a) * 32 + i);
             const float4 H = *reinterpret_cast<const float4 *>(S + (2 * a + 1) * 32 + i);
-            nb[a] += (L.x < pk[a] ? 1u : 0u) + (L.y < pk[a] ? 1u : 0u) + (L.z < pk[a] ? 1u : 0u) + (L.w < pk[a] ? 1u : 0u);
-            na[a] += (H.x > pk[a] ? 1u : 0u) + (H.y > pk[a] ? 1u : 0u) + (H.z > pk[a] ? 1u : 0u) + (H.w > pk[a] ? 1u : 0u);
+            nb[a] += f_less(L.x, pk[a]);
+            na[a] += f_less(pk[a], H.x);
+            nb[a] += f_less(L.y, pk[a]);
+            na[a] += f_less(pk[a], H.y);
+            nb[a] += f_less(L.z, pk[a]);
+            na[a] += f_less(pk[a], H.z);
+            nb[a] += f_less(L.w, pk[a]);
+            na[a] += f_less(pk[a], H.w);
         }
     }
     float mc = kInf, m_pk = 0.0f;
@@ -841,7 +853,7 @@ __device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c,
         if (cost < mc) {   // NaN / inf never win; an earlier axis keeps ties
             mc = cost;
             mkey = a * 32u + lane;
-            m_n = nb[a] | (na[a] << 16);
+            if (COUNTS) m_n = (uint32_t)nb[a] | ((uint32_t)na[a] << 16);
             m_pk = pk[a];
         }
     }
@@ -853,7 +865,7 @@ __device__ __forceinline__ Decision sah_lanes_binned(const float *S, uint32_t c,
     Decision best{-1, 0.0f, 0, 0, kInf, 0};
     const uint32_t src = bk & 31u;
     const float p = __shfl_sync(0xffffffffu, m_pk, src);
-    const uint32_t n = __shfl_sync(0xffffffffu, m_n, src);
+    const uint32_t n = COUNTS ? __shfl_sync(0xffffffffu, m_n, src) : 0u;
     if (bc < kInf) best = Decision{(int)(bk >> 5), p, n & 0xffffu, n >> 16, bc, (int)src};
     if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)c))) best.axis = -1;
     return best;
@@ -875,6 +887,7 @@ __device__ __forceinline__ uint32_t warp_argmin(float cost, uint32_t ax, float p
 // is taken by lane q % 32, which counts the references below and above it;
 // two sorts per axis and a binary search per candidate and list cost four
 // times as much at the subtree pass's 9 references per node
+template <bool COUNTS>
 __device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, float4 blo, float4 bhi, float ct,
                                                     float ci) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -888,13 +901,19 @@ __device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, 
         const float x = S[(6 + 2 * a + (j >= c ? 1u : 0u)) * 32 + (j >= c ? j - c : j)];
         const float pk = __fadd_rn(x, 0.0f);
         const float l = c3(blo, a), h = c3(bhi, a);
-        uint32_t nb = 0, na = 0;
+        float nb = 0.0f, na = 0.0f;
         const float *Sl = S + 64 * a, *Sh = Sl + 32;
         for (uint32_t i = 0; i < c; i += 4) {
             const float4 L = *reinterpret_cast<const float4 *>(Sl + i);
             const float4 H = *reinterpret_cast<const float4 *>(Sh + i);
-            nb += (L.x < pk ? 1u : 0u) + (L.y < pk ? 1u : 0u) + (L.z < pk ? 1u : 0u) + (L.w < pk ? 1u : 0u);
-            na += (H.x > pk ? 1u : 0u) + (H.y > pk ? 1u : 0u) + (H.z > pk ? 1u : 0u) + (H.w > pk ? 1u : 0u);
+            nb += f_less(L.x, pk);
+            na += f_less(pk, H.x);
+            nb += f_less(L.y, pk);
+            na += f_less(pk, H.y);
+            nb += f_less(L.z, pk);
+            na += f_less(pk, H.z);
+            nb += f_less(L.w, pk);
+            na += f_less(pk, H.w);
         }
         // (an axis without extent has no plane strictly inside)
         if (!(pk > l && pk < h)) continue;
@@ -903,7 +922,7 @@ __device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, 
             mc = cost;
             m_ax = a;
             m_pk = pk;
-            m_n = nb | (na << 16);
+            if (COUNTS) m_n = (uint32_t)nb | ((uint32_t)na << 16);
         }
     }
     // (equal keys are the same plane with the same counts)
@@ -911,7 +930,7 @@ __device__ __forceinline__ Decision sah_lanes_exact(const float *S, uint32_t c, 
     mc = __shfl_sync(0xffffffffu, mc, src);
     m_ax = __shfl_sync(0xffffffffu, m_ax, src);
     m_pk = __shfl_sync(0xffffffffu, m_pk, src);
-    m_n = __shfl_sync(0xffffffffu, m_n, src);
+    if (COUNTS) m_n = __shfl_sync(0xffffffffu, m_n, src);
     Decision best{-1, 0.0f, 0, 0, kInf, 0};
     if (mc < kInf) best = Decision{(int)m_ax, m_pk, m_n & 0xffffu, m_n >> 16, mc, 0};
     if (best.axis >= 0 && !(best.cost < __fmul_rn(ci, (float)c))) best.axis = -1;
@@ -930,7 +949,8 @@ __device__ __forceinline__ Decision sah_warp32(const LevelArgs &A, float *S, uin
     float4 nlo = tlo, nhi = thi;
     lane_bounds(nlo, nhi);
     lanes_pack<EXACT>(S, lane < c, lane, c, tlo, thi, nlo, nhi);
-    return EXACT ? sah_lanes_exact(S, c, blo, bhi, A.ct, A.ci) : sah_lanes_binned(S, c, blo, bhi, A.ct, A.ci);
+    return EXACT ? sah_lanes_exact<true>(S, c, blo, bhi, A.ct, A.ci)
+                 : sah_lanes_binned<true>(S, c, blo, bhi, A.ct, A.ci);
 }
 
 // Exact SAH of a node of more than 32 references by a group of NT threads (a
@@ -1116,8 +1136,9 @@ __device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, 
             const uint32_t *Sl = S.S + 2 * a * 33, *Sh = Sl + 33;
             nc[a] = Sl[lane + 1] - Sl[lane] + Sh[lane + 1] - Sh[lane];
             const float e0 = lane == 0 ? l : S.P[a * 32 + lane], e1 = lane == 31 ? h : S.P[a * 32 + lane + 1];
-            lb[a] = bounds_cost(a, __fsub_rn(e0, l), __fsub_rn(h, e1), ext, Anode, S.clip[2 * a] + Sl[lane],
-                                S.clip[2 * a + 1] + Sh[32] - Sh[lane + 1], A.ct, A.ci);
+            lb[a] = bounds_cost(a, __fsub_rn(e0, l), __fsub_rn(h, e1), ext, Anode,
+                                (float)(S.clip[2 * a] + Sl[lane]),
+                                (float)(S.clip[2 * a + 1] + Sh[32] - Sh[lane + 1]), A.ct, A.ci);
         }
     }
     // 3. two rounds
@@ -1181,7 +1202,7 @@ __device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, 
                 while (b < 31 && Pa[b + 1] <= pk) b++;
                 nb += S.on[a * 32 + b];
             }
-            const float cost = plane_cost(a, pk, l, h, ext, Anode, nb, na, A.ct, A.ci);
+            const float cost = plane_cost(a, pk, l, h, ext, Anode, (float)nb, (float)na, A.ct, A.ci);
             if (refine_better(cost, a, pk, mc, m_ax, m_pk)) {
                 mc = cost;
                 m_ax = a;
@@ -1763,7 +1784,7 @@ __device__ __forceinline__ Decision refine_group(const LevelArgs &A, uint32_t ro
         uint32_t nb = S.bl[i], na = S.ab[i];
         for (uint32_t k = 0; k < nl; k++) nb += Ls[k] < pk ? 1u : 0u;
         for (uint32_t k = 0; k < nh; k++) na += Hs[k] > pk ? 1u : 0u;
-        const float cost = plane_cost(a, pk, l, h, ext, Anode, nb, na, A.ct, A.ci);
+        const float cost = plane_cost(a, pk, l, h, ext, Anode, (float)nb, (float)na, A.ct, A.ci);
         if (refine_better(cost, a, pk, mc, m_ax, m_pk)) {
             mc = cost;
             m_ax = a;
@@ -2314,8 +2335,8 @@ __global__ void __launch_bounds__(kScanThreads, kPlanGrid) k_plan_refs(LevelArgs
 // histograms, or the exact search in registers). Nodes are numbered locally:
 // a split takes the next pair of local indices (below, above); the below
 // child is built next and the above child waits on a stack in shared memory.
-// Entries, cells and ropes go to scratch slots keyed (subtree, local index),
-// references to slots keyed (subtree, local index); slots are handed out per
+// Nodes go to 64-byte scratch records (cell, ropes, entry, subtree and local
+// index) and references to slots keyed (subtree, local index), handed out per
 // warp in chunks. A single-pass scan over the subtrees' sizes places subtree
 // i after the levels' nodes and leaf references and after subtrees 0 .. i-1,
 // and the last pass moves every slot to its place. When the subtrees do not
@@ -2333,11 +2354,23 @@ constexpr int kSubWarps = 8;
 // the root, an even count (the per-warp shared-memory regions stay 16-byte
 // aligned)
 __host__ __device__ constexpr uint32_t sub_stack_entries(uint32_t max_depth) { return (max_depth + 3u) & ~1u; }
+// the words of a scratch record; on the stack of waiting children the record
+// holds the child's lane mask, depth and scratch slot instead of the words
+// after the slashes
+enum SubWord : uint32_t {
+    kWLo = 0,        // cell minimum, 3 words
+    kWSub = 3,       // subtree / lane mask
+    kWHi = 4,        // cell maximum, 3 words
+    kWIndex = 7,     // local index / depth
+    kWRope = 8,      // 6 words
+    kWEntry = 14,    // the node's entry, 2 words / scratch slot
+    kWords = 16
+};
+
 // per warp: the packed bounds (the exact search's candidates too), then the
-// stack (cells lo, hi; meta: lane mask, depth, scratch slot; 6 rope words per
-// entry)
+// stack
 __host__ __device__ constexpr size_t sub_warp_smem(uint32_t entries, bool exact) {
-    return (exact ? kLaneScratch : kLaneScratch / 2) * 4 + (size_t)72 * entries;
+    return (exact ? kLaneScratch : kLaneScratch / 2) * 4 + (size_t)kWords * 4 * entries;
 }
 
 // a scratch entry moved to its place: child pairs and leaf starts shifted by
@@ -2352,7 +2385,8 @@ __device__ __forceinline__ void sub_close_chunks(const LevelArgs &A, uint32_t nb
                                                  uint32_t rused) {
     const uint32_t lane = threadIdx.x & 31u;
     if (nbase != kNoSlot)
-        for (uint32_t k = nused + lane; k < kScNodeChunk; k += 32) A.sc_key[nbase + k] = make_uint2(kNoSlot, 0);
+        for (uint32_t k = nused + lane; k < kScNodeChunk; k += 32)
+            A.sc_rec[(size_t)(nbase + k) * kWords + kWSub] = kNoSlot;
     if (rbase != kNoSlot)
         for (uint32_t k = rused + lane; k < kScRefChunk; k += 32) A.sc_ref[rbase + k] = make_uint4(kNoSlot, 0, 0, 0);
 }
@@ -2378,9 +2412,11 @@ __device__ __forceinline__ bool sub_aborted(const LevelArgs &A) {
 
 // The subtrees of roots A.lc->defer_nodes_total .. A.nlc->defer_nodes_total,
 // one warp per subtree taken by ticket from A.lc (E stack entries per warp).
-// Lane r holds reference r of the root; lanes 0..11 hold the current node's
-// ropes, word lane % 6, so a child's cell, ropes and stack entry are written
-// by parallel lanes.
+// Lane r holds reference r of the root. The current node's record is spread
+// over the lanes too, word lane % 16 in each half of the warp: a split changes
+// two words of each child's record (its cell's cut side, its rope across the
+// plane), so the pair's records are one 128-byte store, the lower half's the
+// below child, and the above child's stack entry one shared-memory store.
 template <bool WARP_EXACT>
 __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint32_t E) {
     extern __shared__ __align__(16) unsigned char sub_smem[];
@@ -2389,13 +2425,10 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     unsigned char *wbase = sub_smem + (size_t)wib * sub_warp_smem(E, WARP_EXACT);
     float *Sw = reinterpret_cast<float *>(wbase);
-    float4 *s_lo = reinterpret_cast<float4 *>(wbase + sub_warp_smem(0, WARP_EXACT));
-    float4 *s_hi = s_lo + E;
-    uint4 *s_meta = reinterpret_cast<uint4 *>(s_hi + E);
-    uint32_t *s_rope = reinterpret_cast<uint32_t *>(s_meta + E);
+    uint32_t *stack = reinterpret_cast<uint32_t *>(wbase + sub_warp_smem(0, WARP_EXACT));
     const uint32_t r0 = min(A.lc->defer_nodes_total, A.cap_defer);
     const uint32_t r1 = min(A.nlc->defer_nodes_total, A.cap_defer);
-    const uint32_t f6 = lane % 6u, child6 = lane / 6u;   // rope word; child of a pair (lanes 0..11)
+    const uint32_t word = lane & 15u, child = lane >> 4;
     uint32_t nbase = kNoSlot, nused = kScNodeChunk, rbase = kNoSlot, rused = kScRefChunk;
     uint32_t leaves = 0, maxdepth = 0;
     bool dead = false;
@@ -2419,23 +2452,32 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
         }
         float4 nlo = tlo, nhi = thi;
         lane_bounds(nlo, nhi);
-        uint32_t rr = lane < 12 ? A.out_ropes[6 * (size_t)rt.x + f6] : 0u;
+        // the root's record words (cell and ropes)
+        uint32_t rec = 0;
+        if (word >= kWRope && word < kWRope + 6) rec = A.out_ropes[6 * (size_t)rt.x + word - kWRope];
+        if (word < 3) rec = __float_as_uint(c3(lo, word));
+        if (word >= kWHi && word < kWHi + 3) rec = __float_as_uint(c3(hi, word - kWHi));
         uint32_t mask = cnt0 >= 32 ? 0xffffffffu : ((1u << cnt0) - 1u);
         uint32_t depth = rt.w, slot = kNoSlot, sp = 0, npair = 0, nref = 0;
         uint2 root_entry = make_uint2(kLeafTag, 0);
+        // a node's entry, written by the lanes that wrote its record
+        auto put_entry = [&](uint2 entry) {
+            if (slot == kNoSlot) root_entry = entry;
+            else if ((lane | 1u) == ((slot & 1u) ? 31u : 15u))
+                A.sc_rec[(size_t)slot * kWords + word] = (lane & 1u) ? entry.y : entry.x;
+        };
         for (;;) {
             const bool in = (mask >> lane) & 1u;
             const uint32_t c = __popc(mask);
             Decision d{-1, 0.0f, 0, 0, kInf, 0};
             if (c > A.leaf_size && depth < A.max_depth) {
                 lanes_pack<WARP_EXACT>(Sw, in, __popc(mask & ((1u << lane) - 1u)), c, tlo, thi, nlo, nhi);
-                d = WARP_EXACT ? sah_lanes_exact(Sw, c, lo, hi, A.ct, A.ci) : sah_lanes_binned(Sw, c, lo, hi, A.ct, A.ci);
+                d = WARP_EXACT ? sah_lanes_exact<false>(Sw, c, lo, hi, A.ct, A.ci)
+                               : sah_lanes_binned<false>(Sw, c, lo, hi, A.ct, A.ci);
             }
             if (d.axis < 0) {
                 // a leaf: its references in the subtree's next local slots
-                const uint2 entry = make_uint2((nref << 2) | kLeafTag, c);
-                if (slot == kNoSlot) root_entry = entry;
-                else if (lane == 0) A.sc_node[slot] = entry;
+                put_entry(make_uint2((nref << 2) | kLeafTag, c));
                 if (rused + c > kScRefChunk) {
                     sub_close_chunks(A, kNoSlot, 0, rbase, rused);
                     rbase = sub_chunk(&A.ctr->sc_ref_ctr, kScRefChunk, A.cap_sc_refs);
@@ -2457,9 +2499,7 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
                 const float p = d.plane;
                 const uint32_t pair = npair;
                 npair += 2;
-                const uint2 entry = make_uint2((pair << 2) | ax, __float_as_uint(p));
-                if (slot == kNoSlot) root_entry = entry;
-                else if (lane == 0) A.sc_node[slot] = entry;
+                put_entry(make_uint2((pair << 2) | ax, __float_as_uint(p)));
                 // the partition of the levels (checkPolygonToAAPlane on the
                 // clipped bounds, see lane_bounds), as lane masks
                 const uint32_t bm = __ballot_sync(0xffffffffu, in && c3(nlo, ax) < p);
@@ -2473,62 +2513,55 @@ __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint
                         break;
                     }
                 }
-                const uint32_t sb = nbase + nused;
+                const uint32_t sb = nbase + nused;   // even: chunks and pairs are
                 nused += 2;
-                float4 bhi = hi, alo = lo;
-                s3(bhi, ax, p);
-                s3(alo, ax, p);
-                // the pair's scratch slots: keys (lanes 0, 1; an empty child is
-                // an empty leaf, a non-empty one's entry is written when it is
-                // decided), cells (lane = 2 child + corner), ropes (lane = 6
-                // child + face: the parent's, with the face on the plane
-                // pointing at the sibling)
-                if (lane < 2) {
-                    A.sc_key[sb + lane] = make_uint2(i, pair + lane);
-                    if ((lane ? am : bm) == 0) A.sc_node[sb + lane] = make_uint2(kLeafTag, 0);
-                }
-                if (lane < 4) {
-                    const float4 v = lane == 0 ? lo : (lane == 1 ? bhi : (lane == 2 ? alo : hi));
-                    A.sc_cbox[2 * (size_t)sb + lane] = v;
-                }
-                uint32_t rb = rr, ra = rr;
-                if (f6 == 2 * ax + 1) rb = kLocalRope | (pair + 1);
-                if (f6 == 2 * ax) ra = kLocalRope | pair;
-                if (lane < 12) A.sc_rope[6 * (size_t)sb + lane] = child6 ? ra : rb;
+                // the children's records: the parent's, cut on the split's
+                // side, with the rope across the plane at the sibling (the
+                // entry of a child is that of an empty cell until it is decided)
+                const uint32_t cut = __float_as_uint(p);
+                const uint32_t recB =
+                    word == kWHi + ax ? cut : (word == kWRope + 1 + 2 * ax ? kLocalRope | (pair + 1) : rec);
+                const uint32_t recA = word == kWLo + ax ? cut : (word == kWRope + 2 * ax ? kLocalRope | pair : rec);
+                const uint32_t mine = child ? recA : recB;
+                uint32_t w = mine;
+                if (word == kWSub) w = i;
+                if (word == kWIndex) w = pair + child;
+                if (word >= kWEntry) w = word == kWEntry ? kLeafTag : 0u;
+                A.sc_rec[(size_t)sb * kWords + lane] = w;
                 if (bm | am) maxdepth = max(maxdepth, depth + 1);
                 if (am) {
                     if (sp >= E) {
                         dead = true;
                         break;
                     }
-                    if (lane == 0) {
-                        s_lo[sp] = alo;
-                        s_hi[sp] = hi;
-                        s_meta[sp] = make_uint4(am, depth + 1, sb + 1, 0);
-                    }
-                    if (lane < 6) s_rope[6 * sp + lane] = ra;
+                    w = mine;
+                    if (word == kWSub) w = am;
+                    if (word == kWIndex) w = depth + 1;
+                    if (word == kWEntry) w = sb + 1;
+                    if (child) stack[sp * kWords + word] = w;
                     sp++;
                 }
                 if (bm) {
                     mask = bm;
-                    hi = bhi;
+                    s3(hi, ax, p);
                     depth++;
                     slot = sb;
-                    rr = rb;
+                    rec = recB;
                     continue;
                 }
             }
             if (sp == 0) break;
             __syncwarp();
             sp--;
-            lo = s_lo[sp];
-            hi = s_hi[sp];
-            const uint4 m = s_meta[sp];
-            rr = lane < 12 ? s_rope[6 * sp + f6] : 0u;
+            const uint32_t *e = stack + sp * kWords;
+            const uint4 e0 = *reinterpret_cast<const uint4 *>(e), e1 = *reinterpret_cast<const uint4 *>(e + kWHi);
+            slot = e[kWEntry];
+            rec = e[word];
             __syncwarp();
-            mask = m.x;
-            depth = m.y;
-            slot = m.z;
+            lo = make_float4(__uint_as_float(e0.x), __uint_as_float(e0.y), __uint_as_float(e0.z), 0.0f);
+            hi = make_float4(__uint_as_float(e1.x), __uint_as_float(e1.y), __uint_as_float(e1.z), 0.0f);
+            mask = e0.w;
+            depth = e1.w;
         }
         if (!dead && lane == 0) {
             A.st_cnt[i] = make_uint2(npair, nref);
@@ -2631,23 +2664,25 @@ __global__ void __launch_bounds__(256) k_sub_place(LevelArgs A) {
     }
     const uint32_t nsn = min(c->sc_node_ctr, A.cap_sc_nodes), nsr = min(c->sc_ref_ctr, A.cap_sc_refs);
     for (uint32_t j = t0; j < nsn; j += stride) {
-        const uint2 key = A.sc_key[j];
-        if (key.x >= n) continue;   // an unused slot
-        const uint2 base = A.st_base[key.x];
-        const uint32_t nb = N0 + base.x, g = nb + key.y;
+        const uint4 *rec = reinterpret_cast<const uint4 *>(A.sc_rec + (size_t)j * kWords);
+        const uint4 w0 = rec[0], w1 = rec[1], w2 = rec[2], w3 = rec[3];
+        if (w0.w >= n) continue;  // an unused slot
+        const uint2 base = A.st_base[w0.w];
+        const uint32_t nb = N0 + base.x, g = nb + w1.w;
         if (g >= A.cap_nodes) {
             atomicOr(A.err, 16u);
             continue;
         }
-        A.out_nodes[g] = sub_relocate(A.sc_node[j], nb, R0 + base.y);
-        A.out_cbox[2 * (size_t)g] = A.sc_cbox[2 * (size_t)j];
-        A.out_cbox[2 * (size_t)g + 1] = A.sc_cbox[2 * (size_t)j + 1];
-#pragma unroll
-        for (int f = 0; f < 6; f++) {
-            uint32_t r = A.sc_rope[6 * (size_t)j + f];
-            if (r != kNoSlot && (r & kLocalRope)) r = nb + (r & ~kLocalRope);
-            A.out_ropes[6 * (size_t)g + f] = r;
-        }
+        A.out_nodes[g] = sub_relocate(make_uint2(w3.z, w3.w), nb, R0 + base.y);
+        A.out_cbox[2 * (size_t)g] =
+            make_float4(__uint_as_float(w0.x), __uint_as_float(w0.y), __uint_as_float(w0.z), 0.0f);
+        A.out_cbox[2 * (size_t)g + 1] =
+            make_float4(__uint_as_float(w1.x), __uint_as_float(w1.y), __uint_as_float(w1.z), 0.0f);
+        auto rope = [&](uint32_t r) { return r != kNoSlot && (r & kLocalRope) ? nb + (r & ~kLocalRope) : r; };
+        uint2 *dst = reinterpret_cast<uint2 *>(A.out_ropes + 6 * (size_t)g);   // 24 bytes a node: 8-byte aligned
+        dst[0] = make_uint2(rope(w2.x), rope(w2.y));
+        dst[1] = make_uint2(rope(w2.z), rope(w2.w));
+        dst[2] = make_uint2(rope(w3.x), rope(w3.y));
     }
     for (uint32_t j = t0; j < nsr; j += stride) {
         const uint4 q = A.sc_ref[j];
@@ -2709,7 +2744,7 @@ void build_release(BuildState &S) {
     f(S.ctr); f(S.err);
     f(S.out_nodes); f(S.out_refs); f(S.out_ropes); f(S.out_cbox);
     f(S.d_root); f(S.d_lo); f(S.d_hi); f(S.defer_refs);
-    f(S.sc_key); f(S.sc_node); f(S.sc_cbox); f(S.sc_rope); f(S.sc_ref);
+    f(S.sc_rec); f(S.sc_ref);
     f(S.st_cnt); f(S.st_root); f(S.st_base); f(S.sub_flags); f(S.sub_agg); f(S.sub_incl);
     S.cap_defer = S.cap_sc_nodes = S.cap_sc_refs = S.sub_tiles = 0;
     if (S.ev_fork) cudaEventDestroy(S.ev_fork);
@@ -2805,10 +2840,7 @@ hk_status build_prepare(BuildState &S, const BuildParams &p, uint32_t nt, int sm
     bad |= dalloc(S.d_lo, S.cap_defer) != cudaSuccess;
     bad |= dalloc(S.d_hi, S.cap_defer) != cudaSuccess;
     bad |= dalloc(S.defer_refs, cap_refs) != cudaSuccess;
-    bad |= dalloc(S.sc_key, S.cap_sc_nodes) != cudaSuccess;
-    bad |= dalloc(S.sc_node, S.cap_sc_nodes) != cudaSuccess;
-    bad |= dalloc(S.sc_cbox, (size_t)S.cap_sc_nodes * 2) != cudaSuccess;
-    bad |= dalloc(S.sc_rope, (size_t)S.cap_sc_nodes * 6) != cudaSuccess;
+    bad |= dalloc(S.sc_rec, (size_t)S.cap_sc_nodes * kWords) != cudaSuccess;
     bad |= dalloc(S.sc_ref, S.cap_sc_refs) != cudaSuccess;
     bad |= dalloc(S.st_cnt, S.cap_defer) != cudaSuccess;
     bad |= dalloc(S.st_root, S.cap_defer) != cudaSuccess;
@@ -2920,10 +2952,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     A.d_hi = S.d_hi;
     A.defer_refs = S.defer_refs;
     A.cap_defer = S.cap_defer;
-    A.sc_key = S.sc_key;
-    A.sc_node = S.sc_node;
-    A.sc_cbox = S.sc_cbox;
-    A.sc_rope = S.sc_rope;
+    A.sc_rec = S.sc_rec;
     A.sc_ref = S.sc_ref;
     A.cap_sc_nodes = S.cap_sc_nodes;
     A.cap_sc_refs = S.cap_sc_refs;

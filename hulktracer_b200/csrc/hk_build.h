@@ -150,13 +150,11 @@ struct BuildState {
     uint4 *d_root = nullptr;
     float4 *d_lo = nullptr, *d_hi = nullptr;
     uint32_t *defer_refs = nullptr;
-    // subtree scratch: node slots (subtree, local index), their entries, cells
-    // and ropes; reference slots (subtree, local index, triangle); per subtree
-    // its sizes, root entry and place
+    // subtree scratch: node records of 16 words (cell, ropes, entry, subtree and
+    // local index); reference slots (subtree, local index, triangle); per
+    // subtree its sizes, root entry and place
     uint32_t cap_sc_nodes = 0, cap_sc_refs = 0;
-    uint2 *sc_key = nullptr, *sc_node = nullptr;
-    float4 *sc_cbox = nullptr;
-    uint32_t *sc_rope = nullptr;
+    uint32_t *sc_rec = nullptr;
     uint4 *sc_ref = nullptr;
     uint2 *st_cnt = nullptr, *st_root = nullptr, *st_base = nullptr;
     uint32_t sub_tiles = 0;
