@@ -2075,27 +2075,20 @@ struct RefOp {
     using Ctx = uint32_t;   // the level stopped splitting
     static constexpr int kItems = 4;
     LevelArgs A;
-    // kItems consecutive references from `base` (a multiple of kItems), those
-    // before n: the indices in two 16-byte loads, then every gather together
+    // kItems references, one of each run of 32 from `base`, those before n:
+    // every index load together, then every gather
     __device__ void load(uint32_t base, uint32_t n, const Ctx &stop, Item (&it)[kItems]) const {
-        uint32_t node[4] = {0, 0, 0, 0}, tri[4] = {0, 0, 0, 0};
-        if (base + 4 <= n) {
-            const uint4 a = *reinterpret_cast<const uint4 *>(A.ref_node() + base);
-            const uint4 b = *reinterpret_cast<const uint4 *>(A.refs() + base);
-            node[0] = a.x; node[1] = a.y; node[2] = a.z; node[3] = a.w;
-            tri[0] = b.x; tri[1] = b.y; tri[2] = b.z; tri[3] = b.w;
-        } else {
+        uint32_t node[kItems], tri[kItems];
 #pragma unroll
-            for (int k = 0; k < kItems; k++)
-                if (base + k < n) {
-                    node[k] = A.ref_node()[base + k];
-                    tri[k] = A.refs()[base + k];
-                }
+        for (int k = 0; k < kItems; k++) {
+            const bool in = base + 32u * k < n;
+            node[k] = in ? A.ref_node()[base + 32u * k] : 0u;
+            tri[k] = in ? A.refs()[base + 32u * k] : 0u;
         }
         float4 sp[kItems];
 #pragma unroll
         for (int k = 0; k < kItems; k++)
-            sp[k] = base + k < n ? A.split[node[k]] : make_float4(__int_as_float(-1), 0, 0, 0);
+            sp[k] = base + 32u * k < n ? A.split[node[k]] : make_float4(__int_as_float(-1), 0, 0, 0);
 #pragma unroll
         for (int k = 0; k < kItems; k++) {
             const int ax = stop ? -1 : __float_as_int(sp[k].x);
@@ -2109,8 +2102,8 @@ struct RefOp {
         }
     }
     // R: the reference's rank among its node's below / above references
-    __device__ void apply(uint32_t r, uint2 R, const Item &it, const Ctx &) const {
-        const uint4 sc = __ldcg(A.scat + it.s);   // written by a plan tile of this launch
+    // sc: the node's destinations
+    __device__ void apply(uint32_t r, uint2 R, const Item &it, const uint4 &sc) const {
         if (!(sc.w & 1u)) {
             const uint32_t off = sc.x + r;   // leaf, or a deferred root (w = 2)
             if (off < A.cap_refs) (sc.w & 2u ? A.defer_refs : A.out_refs)[off] = it.tri;
@@ -2147,20 +2140,17 @@ struct SegV {
 __device__ __forceinline__ SegV seg_join(SegV a, SegV b) {   // a before b
     return SegV{b.h ? b.v : vadd(a.v, b.v), a.h | b.h};
 }
-__device__ __forceinline__ SegV seg_shfl_up(SegV x, int d) {
-    return SegV{make_uint2(__shfl_up_sync(0xffffffffu, x.v.x, d), __shfl_up_sync(0xffffffffu, x.v.y, d)),
-                __shfl_up_sync(0xffffffffu, x.h, d)};
-}
 
 struct RefTileSmem {
     SegV w_tot[kScanThreads / 32];
-    uint32_t w_last[kScanThreads / 32];   // node of each warp's last reference
     uint2 carry;                          // the tile's first segment: flags in earlier tiles
     uint32_t first_node, last_node;       // nodes of the tile's references
     uint32_t wait_ok;
 };
 
-// One reference tile (kTile references, kScanItems per thread). The scan is
+// One reference tile (kTile references; a warp's 128 are consecutive, a run of
+// 32 per item, so ranks are ballots and population counts and a warp's stores
+// of an item are runs too). The scan is
 // segmented by node: a tile in which a node starts publishes its last
 // segment's counts as complete (status 2) at once; only its first segment,
 // when it continues a node of earlier tiles, needs the look-back, which ends at
@@ -2173,48 +2163,47 @@ __device__ void ref_tile(const RefOp &R, uint32_t rt, uint32_t nr, uint32_t tag,
     const LevelArgs &A = R.A;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint32_t r0 = rt * kTile;
-    const uint32_t base = r0 + threadIdx.x * kScanItems;
-    const uint32_t first_prev = (threadIdx.x == 0 && r0 > 0) ? A.ref_node()[r0 - 1] : 0xffffffffu;
+    const uint32_t w0 = r0 + wid * (32u * kScanItems), base = w0 + lane;
+    // node of the reference before the warp's first one
+    uint32_t prev = (lane == 0 && w0 > 0 && w0 <= nr) ? A.ref_node()[w0 - 1] : 0xffffffffu;
     RefItem it[kScanItems];
-    bool hd[kScanItems];
     R.load(base, nr, stop, it);
-    // node of the reference before this thread's first one
-    uint32_t prev = __shfl_up_sync(0xffffffffu, it[kScanItems - 1].s, 1);
-    if (lane == 31) sh.w_last[wid] = it[kScanItems - 1].s;
     if (threadIdx.x == 0) sh.first_node = it[0].s;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++)
-        if (base + k == min(nr, r0 + kTile) - 1) sh.last_node = it[k].s;
-    __syncthreads();
-    if (lane == 0) prev = wid ? sh.w_last[wid - 1] : first_prev;
-    SegV t{make_uint2(0, 0), 0u};
+    // rank of each item since the last node start in the warp (seen: there is one)
+    uint2 rank[kScanItems];
+    uint32_t seen = 0, starts = 0;
+    SegV run{make_uint2(0, 0), 0u};
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        const bool valid = base + k < nr;
-        hd[k] = !valid || it[k].s != (k ? it[k - 1].s : prev);
-        t = seg_join(t, SegV{it[k].f, hd[k] ? 1u : 0u});
+        const uint32_t r = base + 32u * k;
+        if (r == min(nr, r0 + kTile) - 1) sh.last_node = it[k].s;
+        const uint32_t up = __shfl_up_sync(0xffffffffu, it[k].s, 1);
+        if (lane) prev = up;
+        const bool hd = r >= nr || it[k].s != prev;
+        if (k == 0) starts = hd ? 1u : 0u;
+        prev = __shfl_sync(0xffffffffu, it[k].s, 31);   // for lane 0 of the next item
+        const uint32_t H = __ballot_sync(0xffffffffu, hd), B = __ballot_sync(0xffffffffu, it[k].f.x != 0);
+        const uint32_t Ab = __ballot_sync(0xffffffffu, it[k].f.y != 0);
+        const uint32_t below = (1u << lane) - 1u, hle = H & (below | (1u << lane));
+        // the lanes before this one, from the last start on
+        const uint32_t span = hle ? below & (0xffffffffu << (31 - __clz(hle))) : below;
+        rank[k] = make_uint2(__popc(B & span), __popc(Ab & span));
+        if (!hle) rank[k] = vadd(rank[k], run.v);
+        if (hle || run.h) seen |= 1u << k;
+        const uint32_t tail = H ? 0xffffffffu << (31 - __clz(H)) : 0xffffffffu;
+        run = seg_join(run, SegV{make_uint2(__popc(B & tail), __popc(Ab & tail)), H ? 1u : 0u});
     }
-    // warp and block segmented scans
-    SegV inc = t;
-    for (int d = 1; d < 32; d <<= 1) {
-        const SegV o = seg_shfl_up(inc, d);
-        if ((int)lane >= d) inc = seg_join(o, inc);
-    }
-    SegV ex = seg_shfl_up(inc, 1);
-    if (lane == 0) ex = SegV{make_uint2(0, 0), 0u};
-    if (lane == 31) sh.w_tot[wid] = inc;
+    if (lane == 0) sh.w_tot[wid] = run;
     __syncthreads();
     SegV wp{make_uint2(0, 0), 0u}, tot{make_uint2(0, 0), 0u};
     for (uint32_t w = 0; w < kScanThreads / 32; w++) {
         if (w < wid) wp = seg_join(wp, sh.w_tot[w]);
         tot = seg_join(tot, sh.w_tot[w]);
     }
-    ex = seg_join(wp, ex);
     if (threadIdx.x == 0) ref_publish(recs + rt, (tag << 2) | (tot.h ? 2u : 1u), tot.v);
     if (wid == 0) {
-        // the tile's first reference starts a node: no earlier tile matters
-        const bool starts = r0 == 0 || first_prev != it[0].s;
-        const uint2 c = __shfl_sync(0xffffffffu, starts ? 1u : 0u, 0)
+        // when the tile's first reference starts a node no earlier tile matters
+        const uint2 c = __shfl_sync(0xffffffffu, starts, 0)
                             ? make_uint2(0, 0)
                             : ref_lookback(recs, rt, tag, A.err, A.spin_limit);
         if (threadIdx.x == 0) {
@@ -2227,13 +2216,15 @@ __device__ void ref_tile(const RefOp &R, uint32_t rt, uint32_t nr, uint32_t tag,
     }
     __syncthreads();
     if (!sh.wait_ok) return;   // uniform: the scatter needs the plan's destinations
-    uint2 run = ex.h ? ex.v : vadd(ex.v, sh.carry);
+    if (!wp.h) wp.v = vadd(wp.v, sh.carry);
+    uint4 sc[kScanItems];   // written by plan tiles of this launch
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        if (hd[k]) run = make_uint2(0, 0);
-        if (base + k < nr) R.apply(base + k, run, it[k], stop);
-        run = vadd(run, it[k].f);
-    }
+    for (int k = 0; k < kScanItems; k++)
+        sc[k] = base + 32u * k < nr ? __ldcg(A.scat + it[k].s) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++)
+        if (base + 32u * k < nr)
+            R.apply(base + 32u * k, (seen >> k) & 1u ? rank[k] : vadd(rank[k], wp.v), it[k], sc[k]);
     __syncthreads();
 }
 
