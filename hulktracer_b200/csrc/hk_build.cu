@@ -272,28 +272,28 @@ __device__ __forceinline__ void hist_ref(uint32_t *H, float4 tlo, float4 thi, fl
     }
 }
 
-// The node's planes p_k (k = 0..31) of each axis in P[a * 32 + k], so the bin
-// corrections read them instead of recomputing them (the same values): one
-// warp (lane k writes plane k of the three axes) or threads 0..95 of a CTA;
-// the caller syncs before reading.
-constexpr uint32_t kPlanes = 3 * kBins;
+// The node's planes p_k (k = 1..31) of each axis in P[a * kPlaneRow + k], so the
+// bin corrections read them instead of recomputing them (the same values),
+// between -inf (k = 0) and +inf (k = 32): one warp or threads of a CTA; the
+// caller syncs before reading.
+constexpr uint32_t kPlaneRow = kBins + 1;
+constexpr uint32_t kPlanes = (3 * kPlaneRow + 3) & ~3u;
 // a warp's scratch for one node: histogram and plane table, or the packed
 // bounds of at most 32 references
 constexpr uint32_t kWarpScratch = kHist + kPlanes;
-__device__ __forceinline__ void node_planes_warp(float *P, float4 blo, float4 bhi) {
+// one axis (a warp)
+__device__ __forceinline__ void node_planes_row(float *P, uint32_t a, float4 blo, float4 bhi) {
     const uint32_t lane = threadIdx.x & 31u;
+    const float l = c3(blo, a);
+    P[a * kPlaneRow + lane] = lane ? plane_k(l, __fsub_rn(c3(bhi, a), l), lane) : -kInf;
+    if (lane == 0) P[a * kPlaneRow + kBins] = kInf;
+}
+__device__ __forceinline__ void node_planes_warp(float *P, float4 blo, float4 bhi) {
 #pragma unroll
-    for (uint32_t a = 0; a < 3; a++) {
-        const float l = c3(blo, a);
-        P[a * 32 + lane] = plane_k(l, __fsub_rn(c3(bhi, a), l), lane);
-    }
+    for (uint32_t a = 0; a < 3; a++) node_planes_row(P, a, blo, bhi);
 }
 __device__ __forceinline__ void node_planes_cta(float *P, float4 blo, float4 bhi) {
-    if (threadIdx.x < kPlanes) {
-        const uint32_t a = threadIdx.x >> 5, k = threadIdx.x & 31u;
-        const float l = c3(blo, a);
-        P[threadIdx.x] = plane_k(l, __fsub_rn(c3(bhi, a), l), k);
-    }
+    if (threadIdx.x < 96) node_planes_row(P, threadIdx.x >> 5, blo, bhi);
 }
 
 // bin_interval with the planes of the axis read from Pa
@@ -310,22 +310,38 @@ __device__ __forceinline__ void bin_interval_tab(float lo, float hi, float blo, 
     on = (lo == hi) && b >= 1 && lo == Pa[b];
 }
 
-// hist_ref with the node's plane table P (node_planes_*)
+// hist_ref with the node's plane table P (node_planes_*). A first guess of a
+// bin is all but always right, so the six bins are checked together, without a
+// branch between their twelve plane reads; a reference with any wrong guess
+// takes the walk.
 __device__ __forceinline__ void hist_ref_tab(uint32_t *H, float4 tlo, float4 thi, float4 blo, float4 bhi, float4 inv3,
                                              const float *P) {
+    int b[3], c[3];
+    bool on[3], good = true;
 #pragma unroll
     for (uint32_t a = 0; a < 3; a++) {
-        float l = c3(blo, a), h = c3(bhi, a);
-        float ext = __fsub_rn(h, l);
-        if (!(ext > 0.0f)) continue;
-        float inv = c3(inv3, a);
-        float lo = mxf(c3(tlo, a), l), hi = mnf(c3(thi, a), h);
-        int b, c;
-        bool on;
-        bin_interval_tab(lo, hi, l, inv, P + a * 32, b, c, on);
-        atomicAdd(&H[a * 96 + b], 1u);
-        atomicAdd(&H[a * 96 + 32 + c], 1u);
-        if (on) atomicAdd(&H[a * 96 + 64 + b], 1u);
+        const float l = c3(blo, a), h = c3(bhi, a), inv = c3(inv3, a);
+        const float lo = mxf(c3(tlo, a), l), hi = mnf(c3(thi, a), h);
+        const float *Pa = P + a * kPlaneRow;
+        b[a] = min(max(__float2int_rz(__fmul_rn(__fsub_rn(lo, l), inv)), 0), (int)kBins - 1);
+        c[a] = min(max(__float2int_rz(__fmul_rn(__fsub_rn(hi, l), inv)), 0), (int)kBins - 1);
+        const float b0 = Pa[b[a]], b1 = Pa[b[a] + 1], c0 = Pa[c[a]], c1 = Pa[c[a] + 1];
+        good = good && (!(__fsub_rn(h, l) > 0.0f) || (lo >= b0 && lo < b1 && hi > c0 && hi <= c1));
+        on[a] = lo == hi && b[a] >= 1 && lo == b0;
+    }
+    if (!good) {
+#pragma unroll
+        for (uint32_t a = 0; a < 3; a++) {
+            const float l = c3(blo, a), h = c3(bhi, a);
+            bin_interval_tab(mxf(c3(tlo, a), l), mnf(c3(thi, a), h), l, c3(inv3, a), P + a * kPlaneRow, b[a], c[a], on[a]);
+        }
+    }
+#pragma unroll
+    for (uint32_t a = 0; a < 3; a++) {
+        if (!(__fsub_rn(c3(bhi, a), c3(blo, a)) > 0.0f)) continue;   // uniform
+        atomicAdd(&H[a * 96 + b[a]], 1u);
+        atomicAdd(&H[a * 96 + 32 + c[a]], 1u);
+        if (on[a]) atomicAdd(&H[a * 96 + 64 + b[a]], 1u);
     }
 }
 
