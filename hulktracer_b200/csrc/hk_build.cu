@@ -582,8 +582,13 @@ __device__ __forceinline__ bool is_medium(const LevelArgs &A, uint32_t c) {
 }
 // large: k_hist's chunked histograms (in learned mode the proposer rows too, so
 // that the proposer's chain needs nothing from k_small)
-__device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c) {
-    return (c > kSmall || is_learn(A, c)) && !is_exact(A, c) && !is_row_warp(A, c);
+// A node of 33..256 references is a warp's work where a level has many of them
+// and a CTA's chunk where it has few: one warp takes 8 us more for it (levels
+// of up to 0 / 32k / 64k / 128k references: a frame of 3.5k triangles 529 / 519 /
+// 519 / 519 us, of 24k 945 / 922 / 917 / 915, of 200k 1,656 / 1,652 / 1,654 / 1,653).
+constexpr uint32_t kFewRefs = 131072;
+__device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c, uint32_t refs) {
+    return (c > (refs <= kFewRefs ? kWarpExact : kSmall) || is_learn(A, c)) && !is_exact(A, c) && !is_row_warp(A, c);
 }
 // References per chunk of a node of more than kChunk references, in a level
 // of `refs` references: small enough that the level's chunks fill k_decide's
@@ -609,7 +614,7 @@ __device__ __forceinline__ bool is_deferred(const LevelArgs &A, uint32_t c) {
 __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
     const bool dec = nt > A.leaf_size && A.max_depth > 0;
     const bool medium = dec && is_medium(A, nt);
-    const bool large = dec && is_large(A, nt);
+    const bool large = dec && is_large(A, nt, nt);
     const uint32_t per = nt <= kChunk ? kChunk : chunk_refs(nt), nch = large ? node_chunks(nt, per) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *A.epoch += 1u;
@@ -1496,7 +1501,7 @@ template <bool WARP_EXACT, bool LEARNED>
 __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXACT && !LEARNED> *WSp, Tally &tally,
                                            uint32_t cta) {
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t nodes = A.lc->nodes;
+    const uint32_t nodes = A.lc->nodes, refs = A.lc->refs;
     const uint32_t ngroups = (nodes + 7) / 8;
     for (uint32_t g = cta; g < ngroups; g += gridDim.x) {
         const uint32_t s = g * 8 + wib;
@@ -1505,7 +1510,7 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];   // (with the record: one round trip)
         const uint32_t cnt = info.y;
         const bool dec = decidable(A, cnt);
-        if (dec && (is_large(A, cnt) || is_medium(A, cnt))) continue;   // k_hist
+        if (dec && (is_large(A, cnt, refs) || is_medium(A, cnt))) continue;   // k_hist
         if (!dec || is_deferred(A, cnt)) {
             // a leaf, or the root of a subtree built after the levels
             if (lane == 0) {
@@ -1913,8 +1918,9 @@ __device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t start, uin
         else atomicOr(A.err, 2u);
         return;
     }
-    if (!(dec && is_large(A, c))) return;
-    const uint32_t per = c <= kChunk ? kChunk : chunk_refs(A.lc->t_childrefs), nch = node_chunks(c, per);
+    const uint32_t refs = A.lc->t_childrefs;
+    if (!(dec && is_large(A, c, refs))) return;
+    const uint32_t per = c <= kChunk ? kChunk : chunk_refs(refs), nch = node_chunks(c, per);
     const uint32_t rank = atomicAdd(&A.nlc->n_large, 1u);
     const uint32_t first = atomicAdd(&A.nlc->n_chunks, nch);
     if (rank >= A.cap_large || first + nch > A.cap_chunks) {
