@@ -1359,7 +1359,7 @@ __device__ __forceinline__ HistStart hist_start(const LevelArgs &A) {
                      MEDIUM ? min(__ldcg(&A.lc->n_medium), A.cap_medium) : 0u, __ldcg(&A.lc->nodes)};
 }
 
-template <bool MEDIUM>
+template <bool MEDIUM, uint32_t NT>
 __device__ __forceinline__ void hist_body(const LevelArgs &A, const HistStart &hs, HistSmem &SH, ExactSmem<256> *XSp,
                                           Tally &tally) {
     uint32_t *H = SH.H;
@@ -1412,15 +1412,15 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, const HistStart &h
         for (uint32_t i = threadIdx.x; i < kHist; i += blockDim.x) H[i] = 0;
         node_planes_cta(SH.P, blo, bhi);
         __syncthreads();
-        {
-            // all of the thread's references and bounds loaded first
-            constexpr int kPer = kChunk / 256;
-            const float4 inv3 = bin_scale(blo, bhi);
+        const float4 inv3 = bin_scale(blo, bhi);
+        for (uint32_t q0 = r0; q0 < r1; q0 += 4 * NT) {
+            // four references a thread, their bounds loaded together
+            constexpr int kPer = 4;
             uint32_t tri[kPer];
             float4 tlo[kPer], thi[kPer];
 #pragma unroll
             for (int k = 0; k < kPer; k++) {
-                const uint32_t r = r0 + threadIdx.x + 256u * k;
+                const uint32_t r = q0 + threadIdx.x + NT * k;
                 tri[k] = r < r1 ? A.refs()[r] : 0xffffffffu;
             }
 #pragma unroll
@@ -1474,8 +1474,8 @@ __global__ void __launch_bounds__(256, MODE == kHistRows ? 4 : 3) k_hist(LevelAr
     const HistStart hs = hist_start<MODE != kHistChunks>(A);
     if (level_aborted(A)) return;
     Tally tally;
-    if constexpr (MODE == kHistExact) hist_body<true>(A, hs, SH.hist, &XS, tally);
-    else hist_body<false>(A, HistStart{hs.ck, hs.nch, 0u, hs.nodes}, SH.hist, nullptr, tally);
+    if constexpr (MODE == kHistExact) hist_body<true, 256>(A, hs, SH.hist, &XS, tally);
+    else hist_body<false, 256>(A, HistStart{hs.ck, hs.nch, 0u, hs.nodes}, SH.hist, nullptr, tally);
     if constexpr (MODE == kHistRows) {
         __syncthreads();
         const uint32_t wib = threadIdx.x >> 5;
@@ -1502,9 +1502,9 @@ __device__ __forceinline__ void small_body(const LevelArgs &A, WarpSmem<WARP_EXA
                                            uint32_t cta) {
     const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nodes = A.lc->nodes, refs = A.lc->refs;
-    const uint32_t ngroups = (nodes + 7) / 8;
+    const uint32_t nw = blockDim.x >> 5, ngroups = (nodes + nw - 1) / nw;
     for (uint32_t g = cta; g < ngroups; g += gridDim.x) {
-        const uint32_t s = g * 8 + wib;
+        const uint32_t s = g * nw + wib;
         if (s >= nodes) continue;
         const uint4 info = A.n_info()[s];
         const float4 blo = A.n_lo()[s], bhi = A.n_hi()[s];   // (with the record: one round trip)
@@ -1555,19 +1555,24 @@ __global__ void __launch_bounds__(256, LEARNED ? 5 : 4) k_small(LevelArgs A) {
 // Binned mode (no medium nodes, no proposer): a level's large-node chunks and
 // small nodes in one launch on the build's stream, PDL-chained to the plan
 // (no second stream, no fork and join per level)
+// (1,024 threads per SM: a CTA's other warps wait while one costs a large
+// node's planes, so the many nodes of large scenes go to CTAs of 128 threads,
+// the few of small ones to CTAs of 256)
+template <uint32_t NT>
 union DecideSmem {
     HistSmem hist;
-    WarpSmem<false> small[8];
+    WarpSmem<false> small[NT / 32];
 };
 
-__global__ void __launch_bounds__(256, 4) k_decide(LevelArgs A) {
-    __shared__ __align__(16) DecideSmem sm;
+template <uint32_t NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_decide(LevelArgs A) {
+    __shared__ __align__(16) DecideSmem<NT> sm;
     __shared__ uint32_t s_tally[kTallies];
     wait_prior_grid();
     const HistStart hs = hist_start<false>(A);
     if (level_aborted(A)) return;
     Tally tally;
-    hist_body<false>(A, hs, sm.hist, nullptr, tally);
+    hist_body<false, NT>(A, hs, sm.hist, nullptr, tally);
     __syncthreads();
     // the last CTAs take the first node groups: the first ones have the chunks
     small_body<false, false>(A, sm.small, tally, gridDim.x - 1 - blockIdx.x);
@@ -3022,7 +3027,8 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         A.nlc = &S.ctr->lvl[L + 1];
         if (binned_only) {
             // one wave (four CTAs per SM resident), grid-stride over the work
-            launch_pdl(k_decide, S.sm_count * 4, 256, 0, st, A);
+            if (nt > kFewRefs) launch_pdl(k_decide<128>, S.sm_count * 8, 128, 0, st, A);
+            else launch_pdl(k_decide<256>, S.sm_count * 4, 256, 0, st, A);
             launch_pdl(k_plan_refs, S.sm_count * kPlanGrid, kScanThreads, 0, st, A, S.plan_flags,
                        static_cast<U7 *>(S.plan_agg), static_cast<U7 *>(S.plan_incl), S.ref_recs, S.plan_done,
                        &A.lc->plan_ticket);
