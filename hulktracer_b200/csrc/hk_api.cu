@@ -128,7 +128,7 @@ struct hk_ctx {
     // shadow rays
     DevBuf<float4> srays;
     DevBuf<hk_hit> shits;
-    DevBuf<uint32_t> slot, spix, scount;
+    DevBuf<uint32_t> slot, scount;
     DevBuf<uint32_t> hleaf;     // per pixel: the leaf its primary ropes traversal ended in
     DevBuf<float4> hit4;
     DevBuf<uint32_t> rgba;
@@ -279,7 +279,7 @@ hk_status hk_destroy(hk_ctx *c) {
     c->box.release(); c->box_ord.release(); c->rec.release(); c->cache_tmp.release();
     c->nodes.release(); c->refs.release(); c->imp_ropes.release(); c->imp_cbox.release(); c->fetch.release(); c->counters.release(); c->errw.release();
     c->rays.release(); c->hits.release(); c->cam.release(); c->lights.release();
-    c->srays.release(); c->shits.release(); c->slot.release(); c->spix.release(); c->scount.release();
+    c->srays.release(); c->shits.release(); c->slot.release(); c->scount.release();
     c->hleaf.release();
     c->hit4.release(); c->rgba.release();
     c->mirror.release(); c->mrays.release(); c->prays.release(); c->mhits.release(); c->phits.release();
@@ -1123,7 +1123,6 @@ static hk_status render_buffers(hk_ctx *c, uint32_t npix, uint32_t nl) {
     HK_CUDA(c, c->srays.ensure(2 * ns));
     HK_CUDA(c, c->shits.ensure(ns));
     HK_CUDA(c, c->slot.ensure(ns));
-    HK_CUDA(c, c->spix.ensure(ns));
     HK_CUDA(c, c->hleaf.ensure(npix));
     HK_CUDA(c, c->hit4.ensure(npix));
     HK_CUDA(c, c->rgba.ensure(npix));
@@ -1174,7 +1173,7 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
         shade_hits = c->phits.p;
     }
     HK_CUDA(c, launch_shadow_rays(shade_rays, shade_hits, c->rec.p, npix, c->lights.p, nl,
-                                  hint ? c->hleaf.p : nullptr, c->srays.p, c->slot.p, c->spix.p, c->scount.p,
+                                  hint ? c->hleaf.p : nullptr, c->srays.p, c->slot.p, c->scount.p,
                                   c->stream));
     s = trace_enqueue(c, c->srays.p, 0, c->scount.p, v, c->shits.p, true, nullptr, kRefillCoherent);
     if (s != HK_OK) return s;

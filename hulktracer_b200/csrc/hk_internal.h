@@ -123,7 +123,7 @@ cudaError_t launch_camera_rays(const float *cam16_dev, uint32_t w, uint32_t h, f
                                bool tiled = false, uint32_t row0 = 0, uint32_t full_h = 0);
 cudaError_t launch_shadow_rays(const float4 *rays, const hk_hit *hits, const TriRec *tris, uint32_t npix,
                                const float *lights_dev, uint32_t nl, const uint32_t *leaf_hint, float4 *srays,
-                               uint32_t *slot, uint32_t *spix, uint32_t *scount, cudaStream_t s);
+                               uint32_t *slot, uint32_t *scount, cudaStream_t s);
 cudaError_t launch_shade_cpu(const float4 *rays, const hk_hit *hits, const TriRec *tris, uint32_t npix,
                              const float *lights_dev, uint32_t nl, const uint32_t *slot, const hk_hit *shits,
                              uint32_t *rgba, cudaStream_t s, uint32_t w = 0, bool tiled = false);

@@ -47,7 +47,7 @@ int g_sm_count[kMaxDevices] = {0};
 size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
 struct Layout {
-    size_t control, box, cam, lights, rays, hits, srays, shits, slot, spix, total;
+    size_t control, box, cam, lights, rays, hits, srays, shits, slot, total;
 };
 
 // control block: [0] ray-batch counter, [1] error word, [2] shadow-ray count,
@@ -65,7 +65,7 @@ Layout layout(uint64_t npix, uint64_t nl, uint64_t npoint) {
     L.srays = o; o = up(o + ns * 32);
     L.shits = o; o = up(o + ns * 8);
     L.slot = o; o = up(o + npix * (nl ? nl : 1) * 4);
-    L.spix = o; o = up(o + ns * 4);
+    o = up(o + ns * 4);   // unused; a call is refused above the documented size
     L.total = o;
     return L;
 }
@@ -127,7 +127,6 @@ extern "C" hk_status hk_render_noalloc(const uint32_t *d_nodes2, const uint32_t 
     float4 *srays = reinterpret_cast<float4 *>(S + Lo.srays);
     hk_hit *shits = reinterpret_cast<hk_hit *>(S + Lo.shits);
     uint32_t *slot = reinterpret_cast<uint32_t *>(S + Lo.slot);
-    uint32_t *spix = reinterpret_cast<uint32_t *>(S + Lo.spix);
 
 #define HK_TRY(x)                                   \
     do {                                            \
@@ -161,8 +160,7 @@ extern "C" hk_status hk_render_noalloc(const uint32_t *d_nodes2, const uint32_t 
     L.n = (uint32_t)npix;
     L.n_dev = nullptr;
     HK_TRY(launch_trace(L, s));
-    HK_TRY(launch_shadow_rays(rays, hits, L.tris, (uint32_t)npix, lights, nl, nullptr, srays, slot, spix, control + 2,
-                              s));
+    HK_TRY(launch_shadow_rays(rays, hits, L.tris, (uint32_t)npix, lights, nl, nullptr, srays, slot, control + 2, s));
     L.rays = srays;
     L.hits = shits;
     L.n = 0;
