@@ -93,7 +93,7 @@ struct hk_ctx {
     DevBuf<uint32_t> part;
     DevBuf<float> mats;
     DevBuf<float> box;          // 8 floats
-    DevBuf<uint32_t> box_ord;   // 8 words
+    DevBuf<uint32_t> box_ord;   // kBoxWords
     float hbox[8] = {0};
     bool box_user = false;
     // triangle records
@@ -255,12 +255,17 @@ hk_status hk_create(hk_ctx **out, const hk_config *cfg) {
     cudaEventCreate(&x->ev0);
     cudaEventCreate(&x->ev1);
     if (x->fetch.ensure(4) || x->counters.ensure(3) || x->errw.ensure(1) || x->box.ensure(8) ||
-        x->box_ord.ensure(8) || x->scount.ensure(1)) {
+        x->box_ord.ensure(kBoxWords) || x->scount.ensure(1)) {
         hk_destroy(x);
         return HK_E_ALLOC;
     }
     cudaMemset(x->errw.p, 0, 4);
     cudaMemset(x->counters.p, 0, 24);
+    if (launch_box_reset(x->box_ord.p, x->own_stream) != cudaSuccess ||
+        cudaStreamSynchronize(x->own_stream) != cudaSuccess) {
+        hk_destroy(x);
+        return HK_E_CUDA;
+    }
     *out = x;
     return HK_OK;
 }
@@ -408,8 +413,8 @@ hk_status hk_scene_set_parts(hk_ctx *c, const uint32_t *part, uint32_t nparts) {
 
 // device part of a frame's transform: mats already in c->mats
 static hk_status transform_device(hk_ctx *c) {
-    HK_CUDA(c, launch_transform(c->rest.p, c->part.p, c->nv, c->mats.p, c->verts.p, c->box_ord.p, c->stream));
-    if (!c->box_user) HK_CUDA(c, launch_box_finish(c->box_ord.p, c->box.p, c->stream));
+    HK_CUDA(c, launch_transform(c->rest.p, c->part.p, c->nv, c->mats.p, c->verts.p, c->box_ord.p,
+                                c->box_user ? nullptr : c->box.p, c->stream));
     HK_CUDA(c, launch_precompute(c->verts.p, c->tris.p, c->nt, c->rec.p, c->stream));
     c->rec_valid = true;
     c->rec_epoch++;

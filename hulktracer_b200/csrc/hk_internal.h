@@ -114,10 +114,12 @@ cudaError_t launch_precompute(const float4 *verts, const uint4 *tris, uint32_t n
 cudaError_t launch_cache_to_rec(const float *cache16, const float4 *verts, const uint4 *tris, uint32_t nt,
                                 TriRec *out, cudaStream_t s);
 cudaError_t launch_rec_to_cache(const TriRec *rec, uint32_t nt, float *cache16, cudaStream_t s);
-cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12,
-                             float4 *out, uint32_t *box_ord, cudaStream_t s);
-cudaError_t launch_box_finish(const uint32_t *box_ord, float *box, cudaStream_t s);
-cudaError_t launch_box(const float4 *verts, uint32_t nv, uint32_t *box_ord, float *box, cudaStream_t s);
+// box_ord: kBoxWords words, set once by launch_box_reset; box: the transformed
+// scene's box, or null (the caller's own box stays)
+constexpr uint32_t kBoxWords = 8;
+cudaError_t launch_box_reset(uint32_t *box_ord, cudaStream_t s);
+cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12, float4 *out,
+                             uint32_t *box_ord, float *box, cudaStream_t s);
 // rays of rows row0 .. row0 + h - 1 of a w x full_h image (full_h 0: h)
 cudaError_t launch_camera_rays(const float *cam16_dev, uint32_t w, uint32_t h, float4 *rays, cudaStream_t s,
                                bool tiled = false, uint32_t row0 = 0, uint32_t full_h = 0);

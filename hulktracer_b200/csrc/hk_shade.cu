@@ -1,6 +1,7 @@
 // hk_shade.cu -- per-frame geometry and shading kernels (sm_100a):
 // rigid transform + scene box, triangle records, primary rays, shadow rays
 // and the two shading semantics of the reference.
+#include <algorithm>
 #include <cfloat>
 
 #include "hk_common.cuh"
@@ -108,21 +109,6 @@ cudaError_t launch_rec_to_cache(const TriRec *rec, uint32_t nt, float *cache16, 
 // rigid transform v' = M[part] (x, y, z, 1) fused with the scene-box
 // reduction (BoundingBoxVisitor, HulkEngine/src/BoundingBoxVisitor.cpp:72-80)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void box_accumulate(float x, float y, float z, uint32_t *box_ord) {
-    // warp-reduce before the atomics
-    uint32_t lo[3] = {f2ord(x), f2ord(y), f2ord(z)}, hi[3] = {lo[0], lo[1], lo[2]};
-    for (int off = 16; off; off >>= 1)
-        for (int k = 0; k < 3; k++) {
-            lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
-            hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
-        }
-    if ((threadIdx.x & 31u) == 0)
-        for (int k = 0; k < 3; k++) {
-            atomicMin(&box_ord[k], lo[k]);
-            atomicMax(&box_ord[4 + k], hi[k]);
-        }
-}
-
 __device__ __forceinline__ float3 xform(const float *m, float4 v) {
     float x = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], v.x), __fmul_rn(m[1], v.y)), __fmul_rn(m[2], v.z)), m[3]);
     float y = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[4], v.x), __fmul_rn(m[5], v.y)), __fmul_rn(m[6], v.z)), m[7]);
@@ -130,53 +116,68 @@ __device__ __forceinline__ float3 xform(const float *m, float4 v) {
     return make_float3(x, y, z);
 }
 
-__global__ void k_transform(const float4 *__restrict__ R, const uint32_t *__restrict__ P, uint32_t nv,
-                            const float *__restrict__ M, float4 *__restrict__ out, uint32_t *box_ord) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    // lanes past the end repeat the block's first vertex (a no-op for min/max)
-    uint32_t j = i < nv ? i : blockIdx.x * blockDim.x;
-    float3 p = xform(M + 12 * (size_t)P[j], R[j]);
-    if (i < nv) out[i] = make_float4(p.x, p.y, p.z, 1.0f);
-    box_accumulate(p.x, p.y, p.z, box_ord);
-}
-
-__global__ void k_box(const float4 *__restrict__ V, uint32_t nv, uint32_t *box_ord) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float4 v = V[i < nv ? i : blockIdx.x * blockDim.x];
-    box_accumulate(v.x, v.y, v.z, box_ord);
-}
-
-__global__ void k_box_init(uint32_t *box_ord) {
-    int k = threadIdx.x;
-    if (k < 8) box_ord[k] = (k < 4) ? 0xffffffffu : 0u;
-}
-
-__global__ void k_box_finish(const uint32_t *box_ord, float *box) {
-    int k = threadIdx.x;
-    if (k < 3) {
-        box[k] = ord2f(box_ord[k]);
-        box[4 + k] = ord2f(box_ord[4 + k]);
-    } else if (k == 3 || k == 7) {
-        box[k] = 1.0f;
+// The box is reduced per CTA, then over the grid's CTAs in box_ord (kBoxWords:
+// minima, a count of finished CTAs, maxima): the last CTA writes it to `box`
+// (unless null) and leaves box_ord as it found it, as launch_box_reset set it.
+// The grid is bounded, so that the atomics on one line are few: six per warp
+// of the whole grid took 17 us of 100k vertices' transform.
+constexpr int kTransformThreads = 256;
+__global__ void __launch_bounds__(kTransformThreads)
+k_transform(const float4 *__restrict__ R, const uint32_t *__restrict__ P, uint32_t nv, const float *__restrict__ M,
+            float4 *__restrict__ out, uint32_t *box_ord, float *box) {
+    __shared__ uint32_t s_lo[3][kTransformThreads / 32], s_hi[3][kTransformThreads / 32];
+    __shared__ bool s_last;
+    uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0, 0, 0};
+    for (uint32_t i = blockIdx.x * kTransformThreads + threadIdx.x; i < nv; i += gridDim.x * kTransformThreads) {
+        const float3 p = xform(M + 12 * (size_t)P[i], R[i]);
+        out[i] = make_float4(p.x, p.y, p.z, 1.0f);
+        const uint32_t o[3] = {f2ord(p.x), f2ord(p.y), f2ord(p.z)};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            lo[k] = min(lo[k], o[k]);
+            hi[k] = max(hi[k], o[k]);
+        }
     }
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        lo[k] = __reduce_min_sync(0xffffffffu, lo[k]);
+        hi[k] = __reduce_max_sync(0xffffffffu, hi[k]);
+        if (lane == 0) {
+            s_lo[k][wib] = lo[k];
+            s_hi[k][wib] = hi[k];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        uint32_t l = s_lo[threadIdx.x][0], h = s_hi[threadIdx.x][0];
+        for (int w = 1; w < kTransformThreads / 32; w++) {
+            l = min(l, s_lo[threadIdx.x][w]);
+            h = max(h, s_hi[threadIdx.x][w]);
+        }
+        atomicMin(&box_ord[threadIdx.x], l);
+        atomicMax(&box_ord[4 + threadIdx.x], h);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&box_ord[3], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last || threadIdx.x >= 8) return;
+    __threadfence();
+    const int k = threadIdx.x;
+    if (box) box[k] = (k & 3) == 3 ? 1.0f : ord2f(__ldcg(box_ord + k));
+    box_ord[k] = k < 3 ? 0xffffffffu : 0u;
 }
 
-cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12,
-                             float4 *out, uint32_t *box_ord, cudaStream_t s) {
-    k_box_init<<<1, 32, 0, s>>>(box_ord);
-    if (nv) k_transform<<<blocks_for(nv, 256), 256, 0, s>>>(rest, part, nv, mats12, out, box_ord);
-    return cudaGetLastError();
+cudaError_t launch_box_reset(uint32_t *box_ord, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(box_ord, 0xff, 3 * sizeof(uint32_t), s);
+    return e == cudaSuccess ? cudaMemsetAsync(box_ord + 3, 0, (kBoxWords - 3) * sizeof(uint32_t), s) : e;
 }
 
-cudaError_t launch_box_finish(const uint32_t *box_ord, float *box, cudaStream_t s) {
-    k_box_finish<<<1, 32, 0, s>>>(box_ord, box);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_box(const float4 *verts, uint32_t nv, uint32_t *box_ord, float *box, cudaStream_t s) {
-    k_box_init<<<1, 32, 0, s>>>(box_ord);
-    if (nv) k_box<<<blocks_for(nv, 256), 256, 0, s>>>(verts, nv, box_ord);
-    k_box_finish<<<1, 32, 0, s>>>(box_ord, box);
+cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12, float4 *out,
+                             uint32_t *box_ord, float *box, cudaStream_t s) {
+    const int grid = std::min(std::max(blocks_for(nv, kTransformThreads), 1), 148 * 4);
+    k_transform<<<grid, kTransformThreads, 0, s>>>(rest, part, nv, mats12, out, box_ord, box);
     return cudaGetLastError();
 }
 
