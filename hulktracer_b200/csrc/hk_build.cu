@@ -537,16 +537,6 @@ __device__ __forceinline__ bool level_aborted(const LevelArgs &A) {
     return __syncthreads_or((int)(__ldcg(A.err) & kErrAbort)) != 0;
 }
 
-__global__ void k_tri_bounds(const float4 *__restrict__ V, const uint4 *__restrict__ T, uint32_t nt, float4 *tb) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nt) return;
-    uint4 t = T[i];
-    float4 a = V[t.x], b = V[t.y], c = V[t.z];
-    tb[2 * (size_t)i] = make_float4(mnf(mnf(a.x, b.x), c.x), mxf(mxf(a.x, b.x), c.x), mnf(mnf(a.y, b.y), c.y),
-                                    mxf(mxf(a.y, b.y), c.y));
-    tb[2 * (size_t)i + 1] = make_float4(mnf(mnf(a.z, b.z), c.z), mxf(mxf(a.z, b.z), c.z), 0.0f, 0.0f);
-}
-
 __device__ __forceinline__ void load_bounds(const LevelArgs &A, uint32_t tri, float4 &lo, float4 &hi) {
     const float4 a = A.tb[2 * (size_t)tri], b = A.tb[2 * (size_t)tri + 1];
     lo = make_float4(a.x, a.z, b.x, 0.0f);
@@ -609,13 +599,21 @@ __device__ __forceinline__ bool is_deferred(const LevelArgs &A, uint32_t c) {
     return c >= 2 && c <= A.defer && A.level >= A.defer_level;
 }
 
-// root node + references of level 0 (the counters were zeroed by a memset);
-// a root with more than 256 references is the first large node
-__global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
+// the build's counters zeroed, the triangles' bounds, and the root node and
+// references of level 0; a root with more than 256 references is the first
+// large node (one launch: a memset and two kernels cost a small scene 5 us more)
+static_assert(sizeof(BuildCounters) % 4 == 0, "cleared word by word");
+__global__ void __launch_bounds__(256) k_root(LevelArgs A, const float *box, const float4 *__restrict__ V,
+                                              const uint4 *__restrict__ T, uint32_t nt, float4 *__restrict__ tb) {
     const bool dec = nt > A.leaf_size && A.max_depth > 0;
     const bool medium = dec && is_medium(A, nt);
     const bool large = dec && is_large(A, nt, nt);
     const uint32_t per = nt <= kChunk ? kChunk : chunk_refs(nt), nch = large ? node_chunks(nt, per) : 0u;
+    if (blockIdx.x == 0) {
+        uint32_t *w = reinterpret_cast<uint32_t *>(A.ctr);
+        for (uint32_t i = threadIdx.x; i < sizeof(BuildCounters) / 4; i += blockDim.x) w[i] = 0;
+        __syncthreads();
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *A.epoch += 1u;
         LevelCounters *l0 = &A.ctr->lvl[0];
@@ -639,6 +637,11 @@ __global__ void k_root(LevelArgs A, const float *box, uint32_t nt) {
         for (int f = 0; f < 6; f++) A.out_ropes[f] = 0xffffffffu;
     }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
+        uint4 t = T[i];
+        float4 a = V[t.x], b = V[t.y], c = V[t.z];
+        tb[2 * (size_t)i] = make_float4(mnf(mnf(a.x, b.x), c.x), mxf(mxf(a.x, b.x), c.x), mnf(mnf(a.y, b.y), c.y),
+                                        mxf(mxf(a.y, b.y), c.y));
+        tb[2 * (size_t)i + 1] = make_float4(mnf(mnf(a.z, b.z), c.z), mxf(mxf(a.z, b.z), c.z), 0.0f, 0.0f);
         A.refs()[i] = i;
         A.ref_node()[i] = 0;
     }
@@ -3002,12 +3005,10 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         const cudaError_t e = build_learn_setup();
         if (e != cudaSuccess) return e;
     }
-    cudaMemsetAsync(S.ctr, 0, sizeof(BuildCounters), st);
     if (A.prop_log) cudaMemsetAsync(A.prop_log, 0xff, (size_t)S.cap_nodes * 8 * sizeof(int32_t), st);
     // the per-rank histograms and done counters are zero here: zeroed at
     // allocation, cleaned by the kernel that used them, and zeroed again by
     // build_read_stats after a build that stopped on an error
-    if (nt) k_tri_bounds<<<(nt + 255) / 256, 256, 0, st>>>(verts, tris, nt, S.tb);
     for (int k = 0; k < 2; k++) {
         A.lo_buf[k] = S.n_lo[k];
         A.hi_buf[k] = S.n_hi[k];
@@ -3016,7 +3017,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         A.ref_node_buf[k] = S.ref_node[k];
     }
     A.level = 0;
-    k_root<<<G, 256, 0, st>>>(A, box, nt);
+    k_root<<<G, 256, 0, st>>>(A, box, verts, tris, nt, S.tb);
     const bool exact_small = A.learned || A.exact_max >= kWarpExact;
     const uint32_t sub_E = sub_stack_entries(S.p.max_depth);
     const size_t sub_smem = kSubWarps * sub_warp_smem(sub_E, exact_small);
