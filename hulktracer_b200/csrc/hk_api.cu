@@ -128,7 +128,7 @@ struct hk_ctx {
     // shadow rays
     DevBuf<float4> srays;
     DevBuf<hk_hit> shits;
-    DevBuf<uint32_t> slot, scount;
+    DevBuf<uint32_t> slot, frame_ctr;   // frame_ctr: kFrameCounters
     DevBuf<uint32_t> hleaf;     // per pixel: the leaf its primary ropes traversal ended in
     DevBuf<float4> hit4;
     DevBuf<uint32_t> rgba;
@@ -137,7 +137,7 @@ struct hk_ctx {
     bool has_mirrors = false;
     DevBuf<float4> mrays, prays;
     DevBuf<hk_hit> mhits, phits;
-    DevBuf<uint32_t> mslot, mcount;
+    DevBuf<uint32_t> mslot;
     // frame graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
@@ -255,7 +255,7 @@ hk_status hk_create(hk_ctx **out, const hk_config *cfg) {
     cudaEventCreate(&x->ev0);
     cudaEventCreate(&x->ev1);
     if (x->fetch.ensure(4) || x->counters.ensure(3) || x->errw.ensure(1) || x->box.ensure(8) ||
-        x->box_ord.ensure(kBoxWords) || x->scount.ensure(1)) {
+        x->box_ord.ensure(kBoxWords) || x->frame_ctr.ensure(kFrameCounters)) {
         hk_destroy(x);
         return HK_E_ALLOC;
     }
@@ -284,11 +284,11 @@ hk_status hk_destroy(hk_ctx *c) {
     c->box.release(); c->box_ord.release(); c->rec.release(); c->cache_tmp.release();
     c->nodes.release(); c->refs.release(); c->imp_ropes.release(); c->imp_cbox.release(); c->fetch.release(); c->counters.release(); c->errw.release();
     c->rays.release(); c->hits.release(); c->cam.release(); c->lights.release();
-    c->srays.release(); c->shits.release(); c->slot.release(); c->scount.release();
+    c->srays.release(); c->shits.release(); c->slot.release(); c->frame_ctr.release();
     c->hleaf.release();
     c->hit4.release(); c->rgba.release();
     c->mirror.release(); c->mrays.release(); c->prays.release(); c->mhits.release(); c->phits.release();
-    c->mslot.release(); c->mcount.release();
+    c->mslot.release();
     build_release(c->build);
     c->resort.release();
     c->ooc.release();
@@ -968,7 +968,7 @@ static hk_status ensure_imported_ropes(hk_ctx *c) {
 
 static hk_status trace_enqueue(hk_ctx *c, const float4 *d_rays, uint32_t n, const uint32_t *n_dev, hk_variant v,
                                hk_hit *d_hits, bool occlusion = false, uint32_t *leaf_out = nullptr,
-                               uint32_t refill = 0) {
+                               uint32_t refill = 0, uint32_t *fetch = nullptr) {
     if ((int)v < HK_TRACE_FULLSTACK || (int)v > HK_TRACE_BRUTE) return fail(c, HK_E_ILLEGAL_INPUT, "variant");
     if (!c->rec_valid) return fail(c, HK_E_STATE, "no triangle cache (hk_precompute or hk_cache_import)");
     if (v != HK_TRACE_BRUTE && !c->tree_valid) return fail(c, HK_E_STATE, "no tree");
@@ -996,7 +996,8 @@ static hk_status trace_enqueue(hk_ctx *c, const float4 *d_rays, uint32_t n, cons
     L.n_dev = n_dev;
     L.ntris = c->nt;
     L.box = c->box.p;
-    L.fetch = c->fetch.p;
+    L.fetch = fetch ? fetch : c->fetch.p;   // (a frame's are clear)
+    L.fetch_clear = fetch != nullptr;
     L.counters = c->counters.p;
     L.err = c->errw.p;
     L.stack_depth = c->cfg.short_stack;
@@ -1139,7 +1140,6 @@ static hk_status render_buffers(hk_ctx *c, uint32_t npix, uint32_t nl) {
         HK_CUDA(c, c->mhits.ensure(npix));
         HK_CUDA(c, c->phits.ensure(npix));
         HK_CUDA(c, c->mslot.ensure(npix));
-        HK_CUDA(c, c->mcount.ensure(1));
     }
     return HK_OK;
 }
@@ -1153,11 +1153,12 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
     c->last_primary = npix;
     c->last_shade = shade;
     const bool tiled = (w % 8u == 0) && (h % 4u == 0);
-    HK_CUDA(c, launch_camera_rays(c->cam.p, w, h, c->rays.p, c->stream, tiled, row0, full_h));
+    uint32_t *const ctr = c->frame_ctr.p;
+    HK_CUDA(c, launch_camera_rays(c->cam.p, w, h, c->rays.p, c->stream, tiled, row0, full_h, ctr));
     // ropes: each pixel's last leaf, where its shadow rays may start
     const bool hint = v == HK_TRACE_ROPES && shade != HK_SHADE_PICTURE;
     hk_status s = trace_enqueue(c, c->rays.p, npix, nullptr, v, c->hits.p, false, hint ? c->hleaf.p : nullptr,
-                                kRefillCoherent);
+                                kRefillCoherent, ctr + kFetchPrimary);
     if (s != HK_OK) return s;
     if (shade == HK_SHADE_PICTURE) {
         HK_CUDA(c, launch_hit4(c->hits.p, c->rec.p, npix, c->hit4.p, c->stream));
@@ -1169,8 +1170,9 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
     if (shade == HK_SHADE_MIRROR) {
         // one mirror bounce: reflected rays, traced, merged into the shading rays
         HK_CUDA(c, launch_mirror_rays(c->rays.p, c->hits.p, c->rec.p, c->mirror.p, npix, c->mrays.p, c->mslot.p,
-                                      c->mcount.p, c->stream));
-        s = trace_enqueue(c, c->mrays.p, 0, c->mcount.p, v, c->mhits.p, false, nullptr, kRefillMirror);
+                                      ctr + kMirrorCount, c->stream));
+        s = trace_enqueue(c, c->mrays.p, 0, ctr + kMirrorCount, v, c->mhits.p, false, nullptr, kRefillMirror,
+                          ctr + kFetchMirror);
         if (s != HK_OK) return s;
         HK_CUDA(c, launch_mirror_merge(c->rays.p, c->hits.p, c->mslot.p, c->mrays.p, c->mhits.p, npix, c->prays.p,
                                        c->phits.p, c->stream));
@@ -1178,9 +1180,10 @@ static hk_status render_enqueue(hk_ctx *c, uint32_t nl, uint32_t w, uint32_t h, 
         shade_hits = c->phits.p;
     }
     HK_CUDA(c, launch_shadow_rays(shade_rays, shade_hits, c->rec.p, npix, c->lights.p, nl,
-                                  hint ? c->hleaf.p : nullptr, c->srays.p, c->slot.p, c->scount.p,
-                                  c->stream));
-    s = trace_enqueue(c, c->srays.p, 0, c->scount.p, v, c->shits.p, true, nullptr, kRefillCoherent);
+                                  hint ? c->hleaf.p : nullptr, c->srays.p, c->slot.p,
+                                  ctr + kShadowCount, c->stream));
+    s = trace_enqueue(c, c->srays.p, 0, ctr + kShadowCount, v, c->shits.p, true, nullptr, kRefillCoherent,
+                      ctr + kFetchShadow);
     if (s != HK_OK) return s;
     HK_CUDA(c, launch_shade_cpu(shade_rays, shade_hits, c->rec.p, npix, c->lights.p, nl, c->slot.p, c->shits.p,
                                 d_rgba, c->stream, w, tiled));
@@ -1356,9 +1359,9 @@ hk_status hk_get_ray_counts(hk_ctx *c, uint64_t *primary, uint64_t *shadow) {
     cudaSetDevice(c->device);
     uint32_t ns = 0, nm = 0;
     if (c->last_shade != HK_SHADE_PICTURE && c->last_primary)
-        HK_CUDA(c, cudaMemcpyAsync(&ns, c->scount.p, 4, cudaMemcpyDeviceToHost, c->stream));
+        HK_CUDA(c, cudaMemcpyAsync(&ns, c->frame_ctr.p + kShadowCount, 4, cudaMemcpyDeviceToHost, c->stream));
     if (c->last_shade == HK_SHADE_MIRROR && c->last_primary)
-        HK_CUDA(c, cudaMemcpyAsync(&nm, c->mcount.p, 4, cudaMemcpyDeviceToHost, c->stream));
+        HK_CUDA(c, cudaMemcpyAsync(&nm, c->frame_ctr.p + kMirrorCount, 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (primary) *primary = c->last_primary;
     if (shadow) *shadow = (uint64_t)ns + nm;   /* secondary rays: shadow + mirror */

@@ -34,6 +34,7 @@ struct TraceLaunch {
     uint32_t ntris;
     const float *box;           // device pointer, 8 floats
     uint32_t *fetch;            // ray-batch counter
+    bool fetch_clear;           // it is zero already (else launch_trace clears it)
     unsigned long long *counters;
     uint32_t *err;
     uint32_t stack_depth;
@@ -120,9 +121,15 @@ constexpr uint32_t kBoxWords = 8;
 cudaError_t launch_box_reset(uint32_t *box_ord, cudaStream_t s);
 cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12, float4 *out,
                              uint32_t *box_ord, float *box, cudaStream_t s);
-// rays of rows row0 .. row0 + h - 1 of a w x full_h image (full_h 0: h)
+// a frame's counters, cleared by its camera-ray launch: the traces' ray-batch
+// counters and the lists' lengths
+enum FrameCounter : uint32_t { kFetchPrimary, kFetchMirror, kFetchShadow, kShadowCount, kMirrorCount, kFrameCounters };
+// rays of rows row0 .. row0 + h - 1 of a w x full_h image (full_h 0: h);
+// counters: kFrameCounters words to clear, or null
 cudaError_t launch_camera_rays(const float *cam16_dev, uint32_t w, uint32_t h, float4 *rays, cudaStream_t s,
-                               bool tiled = false, uint32_t row0 = 0, uint32_t full_h = 0);
+                               bool tiled = false, uint32_t row0 = 0, uint32_t full_h = 0,
+                               uint32_t *counters = nullptr);
+// scount: the list's length, zero before
 cudaError_t launch_shadow_rays(const float4 *rays, const hk_hit *hits, const TriRec *tris, uint32_t npix,
                                const float *lights_dev, uint32_t nl, const uint32_t *leaf_hint, float4 *srays,
                                uint32_t *slot, uint32_t *scount, cudaStream_t s);

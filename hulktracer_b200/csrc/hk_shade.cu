@@ -198,8 +198,9 @@ __device__ __forceinline__ uint32_t pixel_of(uint32_t i, uint32_t w, bool tiled)
 // image when row0 = 0 and full_h = h); ray i belongs to pixel pixel_of(i) of
 // that band.
 __global__ void k_camera_rays(const float *__restrict__ cam, uint32_t w, uint32_t h, float4 *__restrict__ rays,
-                              bool tiled, uint32_t row0, uint32_t full_h) {
+                              bool tiled, uint32_t row0, uint32_t full_h, uint32_t *counters) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (counters && i < kFrameCounters) counters[i] = 0;
     if (i >= w * h) return;
     uint32_t pix = pixel_of(i, w, tiled);
     uint32_t x = pix % w, y = pix / w + row0;
@@ -217,9 +218,11 @@ __global__ void k_camera_rays(const float *__restrict__ cam, uint32_t w, uint32_
 }
 
 cudaError_t launch_camera_rays(const float *cam16_dev, uint32_t w, uint32_t h, float4 *rays, cudaStream_t s,
-                               bool tiled, uint32_t row0, uint32_t full_h) {
+                               bool tiled, uint32_t row0, uint32_t full_h, uint32_t *counters) {
     uint32_t n = w * h;
-    if (n) k_camera_rays<<<blocks_for(n, 256), 256, 0, s>>>(cam16_dev, w, h, rays, tiled, row0, full_h ? full_h : h);
+    if (n)
+        k_camera_rays<<<blocks_for(n, 256), 256, 0, s>>>(cam16_dev, w, h, rays, tiled, row0, full_h ? full_h : h,
+                                                        counters);
     return cudaGetLastError();
 }
 
@@ -310,8 +313,6 @@ k_shadow_rays(const float4 *__restrict__ rays, const hk_hit *__restrict__ hits, 
 cudaError_t launch_shadow_rays(const float4 *rays, const hk_hit *hits, const TriRec *, uint32_t npix,
                                const float *lights_dev, uint32_t nl, const uint32_t *leaf_hint, float4 *srays,
                                uint32_t *slot, uint32_t *scount, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(scount, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
     if (npix)
         k_shadow_rays<<<blocks_for(npix, kShadowThreads), kShadowThreads, 0, s>>>(rays, hits, npix, lights_dev, nl,
                                                                                   leaf_hint, srays, slot, scount);
@@ -521,8 +522,6 @@ __global__ void k_mirror_merge(const float4 *__restrict__ rays, const hk_hit *__
 
 cudaError_t launch_mirror_rays(const float4 *rays, const hk_hit *hits, const TriRec *tris, const uint8_t *mirror,
                                uint32_t npix, float4 *mrays, uint32_t *mslot, uint32_t *mcount, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(mcount, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
     if (npix) k_mirror_rays<<<blocks_for(npix, 256), 256, 0, s>>>(rays, hits, tris, mirror, npix, mrays, mslot, mcount);
     return cudaGetLastError();
 }

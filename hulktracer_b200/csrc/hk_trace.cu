@@ -793,8 +793,10 @@ cudaError_t launch_trace(const TraceLaunch &L, cudaStream_t s) {
     a.remaining = L.remaining;
     a.done_ns = L.done_ns;
     a.start_ns = L.start_ns;
-    cudaError_t e = cudaMemsetAsync(L.fetch, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
+    if (!L.fetch_clear) {
+        const cudaError_t e = cudaMemsetAsync(L.fetch, 0, sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+    }
     if (L.n == 0 && L.n_dev == nullptr) return cudaSuccess;
     int block = L.block;
     // one resident wave: a warp beyond it would find no rays left (batches keep
