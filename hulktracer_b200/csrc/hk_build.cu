@@ -2737,6 +2737,16 @@ __global__ void __launch_bounds__(256) k_sub_place(LevelArgs A) {
 // k_subtree's grid: four CTAs of kSubWarps warps per SM, one wave
 static unsigned sub_grid(int sm_count) { return (unsigned)sm_count * 4u; }
 
+// CTAs of a level kernel: at most per_sm per SM (one resident wave), and no
+// more waves of one per SM than `ctas` fill. Every kernel here takes any grid;
+// CTAs without work still cost their launch and exit (a scene of 3.5k
+// triangles: 592 CTAs per k_decide 504 us a frame, 296 486), and too few cost
+// more (24k triangles: 592 CTAs 910 us, 296 917).
+static unsigned level_grid(int sm_count, unsigned per_sm, uint64_t ctas) {
+    const uint64_t waves = (ctas + sm_count - 1) / sm_count;
+    return (unsigned)sm_count * (unsigned)std::min<uint64_t>(std::max<uint64_t>(waves, 1), per_sm);
+}
+
 // a launch that may start while the stream's previous kernel finishes
 // (programmatic stream serialization); the kernel calls wait_prior_grid()
 // before it reads anything that kernel wrote
@@ -3017,10 +3027,14 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         A.ref_node_buf[k] = S.ref_node[k];
     }
     A.level = 0;
-    k_root<<<G, 256, 0, st>>>(A, box, verts, tris, nt, S.tb);
+    k_root<<<std::min<unsigned>(G, nt / 256 + 1), 256, 0, st>>>(A, box, verts, tris, nt, S.tb);
     const bool exact_small = A.learned || A.exact_max >= kWarpExact;
     const uint32_t sub_E = sub_stack_entries(S.p.max_depth);
     const size_t sub_smem = kSubWarps * sub_warp_smem(sub_E, exact_small);
+    // (a level's references are two to three times the triangles, its nodes of a
+    // CTA each rarely below 64 references; a plan tile is 1,024 references)
+    const unsigned g_nodes3 = level_grid(S.sm_count, 3, nt / 32), g_nodes4 = level_grid(S.sm_count, 4, nt / 32);
+    const unsigned g_plan = level_grid(S.sm_count, kPlanGrid, nt / 256);
     const bool binned_only = !A.learned && A.exact_max == 0 && S.p.level_streams != 2;
     for (uint32_t L = 0; L <= S.p.max_depth; L++) {
         A.level = L;
@@ -3029,8 +3043,8 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         if (binned_only) {
             // one wave (four CTAs per SM resident), grid-stride over the work
             if (nt > kFewRefs) launch_pdl(k_decide<128>, S.sm_count * 8, 128, 0, st, A);
-            else launch_pdl(k_decide<256>, S.sm_count * 4, 256, 0, st, A);
-            launch_pdl(k_plan_refs, S.sm_count * kPlanGrid, kScanThreads, 0, st, A, S.plan_flags,
+            else launch_pdl(k_decide<256>, g_nodes4, 256, 0, st, A);
+            launch_pdl(k_plan_refs, g_plan, kScanThreads, 0, st, A, S.plan_flags,
                        static_cast<U7 *>(S.plan_agg), static_cast<U7 *>(S.plan_incl), S.ref_recs, S.plan_done,
                        &A.lc->plan_ticket);
             continue;
@@ -3041,9 +3055,9 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         cudaEventRecord(S.ev_fork, st);
         cudaStreamWaitEvent(S.aux, S.ev_fork, 0);
         // one wave: three (four) CTAs per SM resident
-        if (A.learned) k_hist<kHistRows><<<S.sm_count * 4, 256, 0, S.aux>>>(A);
-        else if (A.exact_max >= kWarpExact) k_hist<kHistExact><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
-        else k_hist<kHistChunks><<<S.sm_count * 3, 256, 0, S.aux>>>(A);
+        if (A.learned) k_hist<kHistRows><<<g_nodes4, 256, 0, S.aux>>>(A);
+        else if (A.exact_max >= kWarpExact) k_hist<kHistExact><<<g_nodes3, 256, 0, S.aux>>>(A);
+        else k_hist<kHistChunks><<<g_nodes3, 256, 0, S.aux>>>(A);
         if (A.learned) {
             // the proposer's chain on the second stream after the histograms
             // (every proposer row comes from k_hist), beside the small nodes
@@ -3054,21 +3068,21 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
             // stream, beside the CTA-costed ones
             cudaEventRecord(S.ev_learn, S.aux);
             cudaStreamWaitEvent(S.aux2, S.ev_learn, 0);
-            k_refine_warp<<<S.sm_count * 3, 256, 0, S.aux2>>>(A);
+            k_refine_warp<<<g_nodes3, 256, 0, S.aux2>>>(A);
             cudaEventRecord(S.ev_join2, S.aux2);
-            launch_pdl(k_refine_cta, S.sm_count * 3, 256, 0, S.aux, A);
+            launch_pdl(k_refine_cta, g_nodes3, 256, 0, S.aux, A);
         }
         cudaEventRecord(S.ev_join, S.aux);
         if (A.learned) {
-            launch_pdl(k_small<true, true>, S.sm_count * 5, 256, 0, st, A);
+            launch_pdl(k_small<true, true>, level_grid(S.sm_count, 5, nt / 32), 256, 0, st, A);
         } else if (A.exact_max >= kWarpExact) {
-            launch_pdl(k_small<true, false>, S.sm_count * 4, 256, 0, st, A);
+            launch_pdl(k_small<true, false>, g_nodes4, 256, 0, st, A);
         } else {
-            launch_pdl(k_small<false, false>, S.sm_count * 4, 256, 0, st, A);
+            launch_pdl(k_small<false, false>, g_nodes4, 256, 0, st, A);
         }
         cudaStreamWaitEvent(st, S.ev_join, 0);
         if (A.learned) cudaStreamWaitEvent(st, S.ev_join2, 0);
-        launch_pdl(k_plan_refs, S.sm_count * kPlanGrid, kScanThreads, 0, st, A, S.plan_flags, static_cast<U7 *>(S.plan_agg),
+        launch_pdl(k_plan_refs, g_plan, kScanThreads, 0, st, A, S.plan_flags, static_cast<U7 *>(S.plan_agg),
                    static_cast<U7 *>(S.plan_incl), S.ref_recs, S.plan_done, &A.lc->plan_ticket);
     }
     if (A.defer) {
@@ -3078,14 +3092,15 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
         // scan's flags apart from the levels'
         A.lc = &S.ctr->lvl[0];
         A.nlc = &S.ctr->lvl[S.p.max_depth + 1];
+        const unsigned g_sub = std::min(g_nodes4, sub_grid(S.sm_count));
         if (exact_small)
-            launch_pdl(k_subtree<true>, sub_grid(S.sm_count), kSubWarps * 32, sub_smem, st, A, sub_E);
+            launch_pdl(k_subtree<true>, g_sub, kSubWarps * 32, sub_smem, st, A, sub_E);
         else
-            launch_pdl(k_subtree<false>, sub_grid(S.sm_count), kSubWarps * 32, sub_smem, st, A, sub_E);
+            launch_pdl(k_subtree<false>, g_sub, kSubWarps * 32, sub_smem, st, A, sub_E);
         A.level = 63;
         A.lc = &S.ctr->lvl[S.p.max_depth + 1];
-        launch_pdl(k_sub_scan, S.sm_count * 2, kScanThreads, 0, st, A, S.sub_flags, S.sub_agg, S.sub_incl);
-        launch_pdl(k_sub_place, S.sm_count * 8, 256, 0, st, A);
+        launch_pdl(k_sub_scan, std::min<unsigned>(S.sm_count * 2, nt / kTile + 1), kScanThreads, 0, st, A, S.sub_flags, S.sub_agg, S.sub_incl);
+        launch_pdl(k_sub_place, level_grid(S.sm_count, 8, nt / 64), 256, 0, st, A);
     }
     S.active = true;
     S.last_level = S.p.max_depth + 1;
