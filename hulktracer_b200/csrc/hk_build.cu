@@ -7,24 +7,27 @@
 // are deferred subtrees (below; hk_config subtree_max / subtree_depth /
 // level_streams choose the layout). Splits are searched over 32 bins per
 // axis, or, with exact_max (32..1024), over every clipped reference bound for
-// nodes of at most exact_max references (one warp in registers up to 32, one
-// CTA above):
-//   work      large nodes (> 256 references): one CTA per chunk of 1024
-//             references builds shared-memory histograms (3 axes x {lo bin,
-//             hi bin, flat-on-plane}) of the clipped reference bounds and
-//             flushes them with atomics; the CTA that finishes a node's last
-//             chunk runs the SAH (one warp: scans over the 32 bins, exact cost
-//             at the 31 planes per axis, argmin). Small nodes: one warp per
-//             node, warp-private histogram, same SAH. Every decision is also
+// nodes of at most exact_max references (one warp up to 128, one CTA above):
+//   work      large nodes (> 256 references, or > 32 in a level of few
+//             references): one CTA per chunk of up to 1024 references builds
+//             shared-memory histograms (3 axes x {lo bin, hi bin,
+//             flat-on-plane}) of the clipped reference bounds; a node of one
+//             chunk is decided from them (one warp: scans over the 32 bins,
+//             exact cost at the 31 planes per axis, argmin), the chunks of a
+//             larger one are added up in global memory and the CTA that
+//             finishes the last decides. Small nodes: one warp per node,
+//             warp-private histogram, same SAH (up to 32 references counted
+//             plane by plane, without a histogram). Every decision is also
 //             tallied into the level totals (leaf refs, splits, next-level
 //             nodes, child refs) that the capacity guard needs.
 //   [learn]   learned mode: nodes of 33..1024 references get the binned SAH
-//             and their histogram features in the small-node kernel; then
-//             k_learn runs the tensor-core MLP on them (64-node tiles), takes
-//             the top-k (axis, bin) proposals and costs every clipped
-//             reference bound inside the proposed bins exactly (the exact
-//             SAH restricted to those bins); the cheaper of that and the
-//             binned optimum splits the node
+//             and their histogram features in k_hist (a warp each up to 256
+//             references); then k_learn runs the tensor-core MLP on them
+//             (128-row tiles) and takes the top-k (axis, bin) proposals, and
+//             k_refine_warp / k_refine_cta cost every clipped reference bound
+//             inside the proposed bins exactly (the exact SAH restricted to
+//             those bins); the cheaper of that and the binned optimum splits
+//             the node
 //   plan      single-pass scan over nodes (decoupled look-back): leaf
 //             reference offsets, child pairs, next-level slots, child
 //             reference offsets; emits compact node entries, cells and ropes,
@@ -2193,8 +2196,9 @@ struct RefTileSmem {
 
 // One reference tile (kTile references; a warp's 128 are consecutive, a run of
 // 32 per item, so ranks are ballots and population counts and a warp's stores
-// of an item are runs too). The scan is
-// segmented by node: a tile in which a node starts publishes its last
+// of an item are runs too: four consecutive references per thread with shuffle
+// scans took 1,707 us a 200k-triangle frame against 1,688). What bounds it is
+// the chain of dependent loads and waits. The scan is segmented by node: a tile in which a node starts publishes its last
 // segment's counts as complete (status 2) at once; only its first segment,
 // when it continues a node of earlier tiles, needs the look-back, which ends at
 // the tile where that node starts. One warp looks back while another waits
@@ -2350,9 +2354,8 @@ __device__ __forceinline__ void plan_refs_body(const LevelArgs &A, PlanSmem &SM,
 
 // Four CTAs per SM, one resident wave: 64 registers keep the four references
 // of a thread in flight without spills, and fewer CTAs take fewer tickets (six
-// per SM, 40 registers: a 200k-triangle frame 1,950 us; five 1,930; four 1,905;
-// three and two 1,930 and 1,923, and the 1M-triangle frame 3,290 and 3,407
-// against 3,205).
+// per SM: a 200k-triangle frame 1,631 us, a 1M one 2,764; five 1,610 and 2,701;
+// four 1,602 and 2,678; three 1,645 and 2,762).
 constexpr int kPlanGrid = 4;
 __global__ void __launch_bounds__(kScanThreads, kPlanGrid) k_plan_refs(LevelArgs A, uint32_t *pflags, U7 *paggs, U7 *pincls,
                                                                ulonglong2 *rrecs, uint32_t *pdone, uint32_t *ticket) {
@@ -2451,6 +2454,9 @@ __device__ __forceinline__ bool sub_aborted(const LevelArgs &A) {
 // two words of each child's record (its cell's cut side, its rope across the
 // plane), so the pair's records are one 128-byte store, the lower half's the
 // below child, and the above child's stack entry one shared-memory store.
+// Issue-bound (86% of issue slots): about 600 warp instructions per node with
+// 615,571 nodes on the 200k-triangle frame, 409 us (806 and 599 us with a
+// histogram per node and separate entry, cell and rope stores).
 template <bool WARP_EXACT>
 __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint32_t E) {
     extern __shared__ __align__(16) unsigned char sub_smem[];

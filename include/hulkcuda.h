@@ -110,7 +110,8 @@ typedef struct hk_config {
                                  block_size x 8 bytes for the warp-shared leaf test of
                                  every closest-hit variant but BRUTE) exceeds 48 KB is
                                  refused with HK_E_ILLEGAL_INPUT */
-    uint32_t blocks_per_sm;   /* persistent trace grid = SMs * blocks_per_sm */
+    uint32_t blocks_per_sm;   /* persistent trace grid = SMs * blocks_per_sm (0, the default:
+                                 one resident wave) */
     uint32_t max_refs;        /* builder reference arena capacity (0 = 16 x tris) */
     uint32_t topk;            /* learned builder: proposed bins refined per node (1..8, 4) */
     float fallback_ratio;     /* learned builder: the binned SAH's plane splits a node
