@@ -1563,7 +1563,9 @@ __global__ void __launch_bounds__(256, LEARNED ? 5 : 4) k_small(LevelArgs A) {
 // (no second stream, no fork and join per level)
 // (1,024 threads per SM: a CTA's other warps wait while one costs a large
 // node's planes, so the many nodes of large scenes go to CTAs of 128 threads,
-// the few of small ones to CTAs of 256)
+// the few of small ones to CTAs of 256. A frame of 1M triangles 2,714 us with
+// 128, 2,778 with 256, 2,746 with 64; 200k 1,638, 1,640 and 1,661; 24k 935 with
+// 128 and 928 with 256)
 template <uint32_t NT>
 union DecideSmem {
     HistSmem hist;

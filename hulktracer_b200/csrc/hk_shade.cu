@@ -119,8 +119,8 @@ __device__ __forceinline__ float3 xform(const float *m, float4 v) {
 // The box is reduced per CTA, then over the grid's CTAs in box_ord (kBoxWords:
 // minima, a count of finished CTAs, maxima): the last CTA writes it to `box`
 // (unless null) and leaves box_ord as it found it, as launch_box_reset set it.
-// The grid is bounded, so that the atomics on one line are few: six per warp
-// of the whole grid took 17 us of 100k vertices' transform.
+// The grid is bounded, so that the atomics on one line are few: with six per
+// warp of the whole grid 100k vertices took 17 us, now 5.6.
 constexpr int kTransformThreads = 256;
 __global__ void __launch_bounds__(kTransformThreads)
 k_transform(const float4 *__restrict__ R, const uint32_t *__restrict__ P, uint32_t nv, const float *__restrict__ M,
@@ -253,8 +253,10 @@ __device__ __forceinline__ float4 hit_pos(float4 o, float4 d, float t) {
 
 // Writes one shadow ray per (hit pixel, point light) into a compacted list;
 // slot[l * npix + p] = list index or 0xffffffff. A CTA takes its place in the
-// list with one atomic (one per warp and light before, all on one address:
-// 72 us for 2M pixels), light by light so that a light's rays lie together.
+// list with one atomic, light by light so that a light's rays lie together
+// (one atomic per warp and light, all on one address: 24.5 us for 921,600
+// pixels and one light against 13.8 now, where reading and writing the rays
+// bounds it).
 // leaf_hint (optional): per pixel, the leaf the pixel's ropes traversal ended
 // in, passed in the direction's w lane as where the shadow ray may start.
 constexpr int kShadowThreads = 256;
