@@ -2491,8 +2491,8 @@ __device__ __forceinline__ bool sub_aborted(const LevelArgs &A) {
 // two words of each child's record (its cell's cut side, its rope across the
 // plane), so the pair's records are one 128-byte store, the lower half's the
 // below child, and the above child's stack entry one shared-memory store.
-// Issue-bound (86% of issue slots): about 600 warp instructions per node with
-// 615,571 nodes on the 200k-triangle frame, 409 us (806 and 599 us with a
+// Issue-bound (87% of issue slots): 576 warp instructions per SAH evaluation,
+// 615,571 of them on the 200k-triangle frame, 398 us (806 and 599 us with a
 // histogram per node and separate entry, cell and rope stores).
 template <bool WARP_EXACT>
 __global__ void __launch_bounds__(kSubWarps * 32, 4) k_subtree(LevelArgs A, uint32_t E) {

@@ -77,3 +77,26 @@ def test_shadow_lists(hk, oracle, w, h, kinds):
     hits = ctx.trace(rays, hk.SHORTSTACK)
     assert ctx.ray_counts() == (w * h, int((hits["tri"] >= 0).sum()) * kinds.count("p"))
     ctx.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -40, 2.0 ** 40])
+@pytest.mark.parametrize("ct,ci", [(1.0, 1.5), (0.0, 1.0), (500.0, 1.5), (1.0, 1e-3), (0.0, 1e-30), (1.0, 1e30)])
+@pytest.mark.parametrize("lattice", [False, True])
+def test_costs_identical_to_oracle(hk, oracle, lattice, ct, ci, scale):
+    """Costs dominated by either term, and scenes of unusual size, with many
+    equal costs (lattice) or few."""
+    sc = scenes.cluster_soup(4000, seed=21)
+    V = sc.verts.copy()
+    if lattice:
+        V[:, :3] = np.round(V[:, :3] * 0.25)
+    V[:, :3] *= np.float32(scale)
+    box = scenes.scene_box(V)
+    ctx = hk.Context(traverse_cost=ct, intersect_cost=ci, leaf_size=1, subtree_depth=0)
+    ctx.upload(V, sc.tris)
+    ctx.set_box(box)
+    ctx.precompute()
+    ctx.build()
+    cn, cr = ctx.export_compact()
+    on, orf = oracle.build_binned(V, sc.tris, box, ct=ct, ci=ci, leaf_size=1, defer_margin=0)
+    assert np.array_equal(cn, on) and np.array_equal(cr, orf)
+    ctx.close()
