@@ -851,7 +851,7 @@ extern "C" {
 // (hk_build_resort.cu); its tree takes the place of an imported one
 static hk_status build_resort(hk_ctx *c, hk_tree_stats *stats) {
     const ResortParams p{c->cfg.traverse_cost, c->cfg.intersect_cost, c->cfg.max_depth, c->cfg.leaf_size,
-                         c->cfg.sah_sample ? c->cfg.sah_sample : 5u};
+                         c->cfg.sah_sample ? c->cfg.sah_sample : 5u, c->cfg.spin_limit, c->debug_flags};
     float hb[8];
     HK_CUDA(c, cudaMemcpyAsync(hb, c->box.p, 32, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));

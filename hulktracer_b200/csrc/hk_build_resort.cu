@@ -97,32 +97,44 @@ cudaError_t grow_keep(RBuf<T> &b, size_t n, size_t keep, cudaStream_t st) {
 constexpr int kScanNT = 256;    // threads per scan tile
 constexpr int kScanItems = 4;   // elements per thread
 constexpr uint32_t kScanTile = kScanNT * kScanItems;
-constexpr uint32_t kScanSpins = 1u << 22;   // polls before a wait gives up (error word)
+// polls before a wait gives up (error word). A short limit is raised: a tile's
+// predecessor publishes within microseconds of its start, 64K polls are tens of
+// milliseconds
+constexpr uint32_t kScanSpins = 1u << 22, kScanSpinsMin = 1u << 16;
 
 // tile states of a scan and its ticket; every scan of a build has a tag and a
 // ticket of its own
 struct ScanPtrs {
     uint32_t *flags, *ticket, *err;
     uint4 *aggs, *incls;   // uint2 scans use their first half
-    uint32_t tag;
+    uint32_t tag, spin_limit;
+    uint32_t withhold;     // test aid: tile 0 publishes under an old tag, so that no tile sees it
 };
 
 // one scan: op.count() elements, op.load(i) -> Item, op.value(Item) -> T,
-// op.apply(i, exclusive prefix, Item), op.finish(total) by one thread
+// op.apply(i, exclusive prefix, Item), op.finish(total) by one thread.
+// A wait that runs out leaves prefixes that are too small, never too large, so
+// this scan's own stores stay in range; what they index (key ranges, places of
+// nodes and references) no longer fits together, so every later kernel of the
+// build returns at once on the error word, which the host reads at the level's
+// end.
 template <class Op>
 __global__ void __launch_bounds__(kScanNT) k_r_scan(Op op, ScanPtrs sp) {
     using T = typename Op::T;
     __shared__ T sw[kScanNT / 32];
     __shared__ T s_excl;
-    __shared__ uint32_t s_tile;
+    __shared__ uint32_t s_tile, s_err;
     const uint32_t n = op.count();
     const uint32_t ntiles = n ? (n + kScanTile - 1) / kScanTile : 1u;
     T *aggs = reinterpret_cast<T *>(sp.aggs), *incls = reinterpret_cast<T *>(sp.incls);
     for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(sp.ticket, 1u);
+        if (threadIdx.x == 0) {
+            s_err = __ldcg(sp.err);
+            s_tile = atomicAdd(sp.ticket, 1u);
+        }
         __syncthreads();
         const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
+        if (tile >= ntiles || s_err) break;
         const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
         typename Op::Item it[kScanItems];
         T v[kScanItems], s = vzero<T>();
@@ -137,7 +149,8 @@ __global__ void __launch_bounds__(kScanNT) k_r_scan(Op op, ScanPtrs sp) {
         }
         T tot;
         const T ex = block_excl<kScanNT>(s, sw, tot);
-        tile_prefix(tile, tot, sp.tag, sp.flags, aggs, incls, &s_excl, sp.err, kScanSpins);
+        const uint32_t tag = sp.withhold && tile == 0 ? sp.tag - 1u : sp.tag;
+        tile_prefix(tile, tot, tag, sp.flags, aggs, incls, &s_excl, sp.err, sp.spin_limit);
         T pre = vadd(s_excl, ex);
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) {
@@ -157,9 +170,11 @@ constexpr int kRI = 4;                       // keys per thread
 constexpr uint32_t kTile = kRT * kRI;
 
 __global__ void __launch_bounds__(kRT) k_rs_hist(const u64 *__restrict__ keys, const uint32_t *__restrict__ nkeys,
-                                                 int shift, uint32_t ntiles, uint32_t *hist) {
+                                                 int shift, uint32_t ntiles, uint32_t *hist,
+                                                 const uint32_t *__restrict__ err) {
     __shared__ uint32_t h[256];
     const uint32_t n = *nkeys;
+    if (*err) return;   // (uniform: only scans set it)
     h[threadIdx.x] = 0;
     __syncthreads();
     const size_t base = (size_t)blockIdx.x * kTile;
@@ -188,10 +203,12 @@ struct RsScanOp {
 // 256 consecutive keys; warps in order; lanes by __match_any_sync)
 __global__ void __launch_bounds__(kRT) k_rs_scatter(const u64 *__restrict__ in, u64 *__restrict__ out,
                                                     const uint32_t *__restrict__ nkeys, int shift, uint32_t ntiles,
-                                                    const uint32_t *__restrict__ offs) {
+                                                    const uint32_t *__restrict__ offs,
+                                                    const uint32_t *__restrict__ err) {
     __shared__ uint32_t run[256];
     __shared__ uint32_t wc[kRT / 32][256];
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, n = *nkeys;
+    if (*err) return;
     run[threadIdx.x] = 0;
     const size_t base = (size_t)blockIdx.x * kTile;
     for (int r = 0; r < kRI; r++) {
@@ -278,6 +295,10 @@ struct LevelPtrs {
     uint32_t depth;
 };
 
+// a scan of this build gave up waiting (the same for every thread of a kernel
+// that is no scan): the kernel does nothing. Read beside the kernel's first loads.
+__device__ __forceinline__ bool r_aborted(const LevelPtrs &L) { return L.sizes[SK_ERR] != 0; }
+
 __device__ __forceinline__ bool forced_leaf(const LevelPtrs &L, uint32_t c, uint32_t depth) {
     return c == 0 || c <= L.p.leaf_size || depth >= L.p.max_depth;
 }
@@ -301,8 +322,8 @@ struct InitOp {
 
 // KDTreeSAH.cpp:51-82: candidates of the sampled polygons
 __global__ void k_r_emit(LevelPtrs L, const float4 *__restrict__ V, const uint4 *__restrict__ T) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= L.koff[L.n] / 6u) return;
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, Q = L.koff[L.n] / 6u;
+    if (r_aborted(L) || q >= Q) return;
     uint32_t a = 0, b = L.n;   // node: koff[i] / 6 <= q < koff[i + 1] / 6
     while (a < b) {
         const uint32_t m = (a + b) >> 1;
@@ -368,7 +389,7 @@ __global__ void k_seg_sort_warp(LevelPtrs L, uint32_t nseg) {
     uint32_t i, ax, s0, s1;
     seg_range(L, seg, i, ax, s0, s1);
     const uint32_t n = s1 - s0;
-    if (n <= 1 || n > kSegWarpMax) return;
+    if (r_aborted(L) || n <= 1 || n > kSegWarpMax) return;
     uint32_t n2 = 1;
     while (n2 < n) n2 <<= 1;
     const uint32_t nr = (n2 + 31u) >> 5;
@@ -406,6 +427,7 @@ __global__ void k_seg_sort_warp(LevelPtrs L, uint32_t nseg) {
 
 __global__ void __launch_bounds__(256) k_seg_sort_cta(LevelPtrs L, uint32_t nseg) {
     __shared__ u64 sk[kSegCtaMax];
+    if (r_aborted(L)) return;
     for (uint32_t seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
         uint32_t i, ax, s0, s1;
         seg_range(L, seg, i, ax, s0, s1);
@@ -505,6 +527,7 @@ __device__ u64 r_group_cost(const LevelPtrs &L, uint32_t p) {
 __global__ void k_r_cost(LevelPtrs L) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, K = L.koff[L.n];
     const uint32_t lane = threadIdx.x & 31u;
+    if (r_aborted(L)) return;
     u64 packed = ~0ull;
     uint32_t node = 0xffffffffu;
     if (p < K) {
@@ -645,6 +668,7 @@ __device__ __forceinline__ uint32_t r_node(const LevelPtrs &L, uint32_t i) {
 
 __global__ void k_r_nodes(LevelPtrs L) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r_aborted(L)) return;
     // the largest child with candidates
     const uint32_t m = __reduce_max_sync(0xffffffffu, i < L.n ? r_node(L, i) : 0u);
     if (m && (threadIdx.x & 31u) == 0) atomicMax(&L.sizes[SK_MAXCNT], m);
@@ -758,7 +782,8 @@ void ResortState::release() {
     } while (0)
 
 // the tile states of a scan of up to n elements, and its tag and ticket
-static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t &next_ticket, ScanPtrs &sp, cudaStream_t st) {
+static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t spin_limit, bool withhold, uint32_t &next_ticket,
+                              ScanPtrs &sp, cudaStream_t st) {
     const size_t tiles = n / kScanTile + 2;
     if (tiles > S.scan_flags.cap) {
         cudaError_t e = S.scan_flags.ensure(tiles);
@@ -769,14 +794,15 @@ static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t &next_ticket, S
     }
     S.scan_tag = (S.scan_tag + 1u) & 0x3fffffffu;
     sp = ScanPtrs{S.scan_flags.p, S.tickets.p + next_ticket++, S.sizes.p + SK_ERR, S.scan_agg.p, S.scan_incl.p,
-                  S.scan_tag};
+                  S.scan_tag, spin_limit ? std::max(spin_limit, kScanSpinsMin) : kScanSpins, withhold ? 1u : 0u};
     return cudaSuccess;
 }
 
 template <class Op>
-static cudaError_t scan(ResortState &S, const Op &op, size_t n, uint32_t &next_ticket, cudaStream_t st) {
+static cudaError_t scan(ResortState &S, const Op &op, size_t n, uint32_t spin_limit, bool withhold,
+                        uint32_t &next_ticket, cudaStream_t st) {
     ScanPtrs sp;
-    cudaError_t e = scan_begin(S, n, next_ticket, sp, st);
+    cudaError_t e = scan_begin(S, n, spin_limit, withhold, next_ticket, sp, st);
     if (e != cudaSuccess) return e;
     // a CTA per tile up to four per SM
     const unsigned grid = (unsigned)std::min<size_t>(n / kScanTile + 1, 148u * 4u);
@@ -825,6 +851,7 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
     uint32_t maxcnt = (nt <= p.leaf_size || p.max_depth == 0) ? 0u : nt;
     for (uint32_t level = 0; n > 0; level++) {
         const int cur = level & 1, nxt = cur ^ 1;
+        const bool hold = (p.debug_flags & 1u) && level >= 1;
         depth = level;
         // per-node scratch
         RS_CHECK(S.koff.ensure((size_t)n + 1));
@@ -900,7 +927,7 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
         // 1. candidates
         int kc = 0;
         L.keys = S.keys[kc].p;
-        RS_CHECK(scan(S, InitOp{L}, n, next_ticket, st));
+        RS_CHECK(scan(S, InitOp{L}, n, p.spin_limit, hold, next_ticket, st));
         if (K) {
             k_r_emit<<<blocks(K / 6), 256, 0, st>>>(L, verts, tris);
             // 2. sort by (segment, value, marker)
@@ -916,21 +943,23 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
                 const uint32_t ntiles = (K + kTile - 1) / kTile;
                 RS_CHECK(S.hist.ensure(256 * (size_t)ntiles));
                 for (int shift = 0; shift < nbits; shift += 8) {
-                    k_rs_hist<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, L.koff + n, shift, ntiles, S.hist.p);
-                    RS_CHECK(scan(S, RsScanOp{S.hist.p, 256 * ntiles}, 256 * (size_t)ntiles, next_ticket, st));
+                    k_rs_hist<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, L.koff + n, shift, ntiles, S.hist.p,
+                                                     L.sizes + SK_ERR);
+                    RS_CHECK(scan(S, RsScanOp{S.hist.p, 256 * ntiles}, 256 * (size_t)ntiles, p.spin_limit, hold, next_ticket,
+                                  st));
                     k_rs_scatter<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, S.keys[kc ^ 1].p, L.koff + n, shift, ntiles,
-                                                         S.hist.p);
+                                                         S.hist.p, L.sizes + SK_ERR);
                     kc ^= 1;
                 }
             }
             L.keys = S.keys[kc].p;
             // 3. sweep
-            RS_CHECK(scan(S, SweepOp{L}, K, next_ticket, st));
+            RS_CHECK(scan(S, SweepOp{L}, K, p.spin_limit, false, next_ticket, st));
             k_r_cost<<<blocks(K), 256, 0, st>>>(L);
         }
         // 4. decisions, ranks, leaf offsets; classification; cells and nodes
-        RS_CHECK(scan(S, DecideOp{L}, n, next_ticket, st));
-        RS_CHECK(scan(S, ClassifyOp{L, R, verts, tris}, R, next_ticket, st));
+        RS_CHECK(scan(S, DecideOp{L}, n, p.spin_limit, hold, next_ticket, st));
+        RS_CHECK(scan(S, ClassifyOp{L, R, verts, tris}, R, p.spin_limit, false, next_ticket, st));
         k_r_nodes<<<blocks(n), 256, 0, st>>>(L);
         RS_CHECK(cudaGetLastError());
         RS_CHECK(cudaMemcpyAsync(S.host_sizes, S.sizes.p, SK_WORDS * 4, cudaMemcpyDeviceToHost, st));

@@ -362,7 +362,8 @@ class Context:
 
     def set_debug_flags(self, flags):
         """Test aid (hk_set_debug_flags): bit 0 withholds one plan tile's done
-        flag so that the build's bounded waits run out."""
+        flag (BUILD_SAH_RESORT: the first tile's of some scans) so that the
+        build's bounded waits run out."""
         self._check(self.L.hk_set_debug_flags(self.h, int(flags)))
 
     # -- learned split proposer --

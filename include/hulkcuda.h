@@ -126,7 +126,8 @@ typedef struct hk_config {
     uint32_t spin_limit;      /* builder: polls before a bounded device-side wait (a
                                  scan look-back, a reference tile waiting for its
                                  plan tile) gives up; the build then stops and
-                                 returns HK_E_DEVICE_TIMEOUT (0 = 4M polls) */
+                                 returns HK_E_DEVICE_TIMEOUT (0 = 4M polls;
+                                 HK_BUILD_SAH_RESORT: at least 65,536) */
     uint32_t max_steps;       /* traversal: node steps per ray before the trace stops
                                  the ray and returns HK_E_BOUNDS (0 = 2^26) */
     uint32_t sah_sample;      /* HK_BUILD_SAH_RESORT: every sah_sample-th polygon of a
@@ -179,7 +180,10 @@ hk_status hk_set_stream(hk_ctx *ctx, void *cuda_stream);
 /* Test aid for failure detection: bit 0 makes every later build withhold the
  * done flag of the first plan tile of tree level 1, so the reference tiles
  * that wait for it run out of polls (hk_config.spin_limit) and the build
- * returns HK_E_DEVICE_TIMEOUT without hanging; 0 restores normal builds. */
+ * returns HK_E_DEVICE_TIMEOUT without hanging. HK_BUILD_SAH_RESORT: from
+ * level 1 on, the first tile of the radix sort's scans and of the scans over
+ * nodes withholds its flag (a level of more than 1,024 nodes has a tile that
+ * waits for the latter). 0 restores normal builds. */
 hk_status hk_set_debug_flags(hk_ctx *ctx, uint32_t flags);
 /* The builder layout of the next builds (hk_config subtree_max <= 32,
  * subtree_depth, level_streams 0..2), as hk_autotune_build sets it. */
