@@ -93,7 +93,8 @@ __host__ __device__ constexpr bool trace_coop_slots(int variant, bool batch, boo
 // Blocks of kTraceMaxBlock threads that an instantiation is compiled to keep
 // resident on an SM (its __launch_bounds__; smaller blocks in proportion).
 __host__ __device__ constexpr uint32_t trace_resident_blocks(int variant, bool batch, bool any) {
-    return batch ? 4u : (trace_coop_slots(variant, batch, any) ? 5u : 6u);
+    if (batch) return variant == HK_TRACE_BRUTE ? 5u : 4u;
+    return trace_coop_slots(variant, batch, any) ? 5u : 6u;
 }
 
 // dynamic shared memory of one trace launch: the shared-memory ring of

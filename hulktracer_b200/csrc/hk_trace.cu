@@ -31,6 +31,7 @@ struct TraceArgs {
     uint32_t stack_depth;     // ring depth for the short-stack variants
     uint32_t max_steps;       // per-ray iteration bound
     uint32_t refill;          // idle lanes before a warp takes new rays
+    uint32_t warps;           // warps of the launch that are resident together
     const uint32_t *ropes;    // ropes variant: 6 per node
     const float4 *cbox;       // ropes variant: cell min, max per node
     uint32_t rope_nn;         // compact node count (legs bound 4 n + 8) ...
@@ -513,11 +514,12 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
         __syncwarp();
     }
     const uint32_t n = A.n_dev ? *A.n_dev : A.n;
-    // Fewer rays than lanes: every warp takes an even share on its first lanes,
-    // so that the rays spread over all warps, a warp waits for fewer of them at
-    // each step, and its other lanes only share the leaf tests.
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const bool takes = lane < max(1u, min(32u, (n + warps - 1) / warps));
+    // Fewer rays than lanes: every resident warp takes an even share on its first
+    // lanes, so that the rays spread over all of them, a warp waits for fewer of
+    // them at each step, and its other lanes only share the leaf tests. (Shares
+    // of all launched warps leave lanes idle where a caller's blocks_per_sm is
+    // above what fits: 100,000 rays at 128 took 723 us, 259 at 0.)
+    const bool takes = lane < max(1u, min(32u, (n + A.warps - 1) / A.warps));
     if (BATCH && threadIdx.x == 0) atomicMin(A.start_ns, global_ns());
     // scene arrays: launch-uniform for one scene, per lane in a batch
     SceneView V{A.nodes, A.refs, A.tris, A.ropes, A.cbox};
@@ -799,16 +801,18 @@ cudaError_t launch_trace(const TraceLaunch &L, cudaStream_t s) {
     }
     if (L.n == 0 && L.n_dev == nullptr) return cudaSuccess;
     int block = L.block;
-    // one resident wave: a warp beyond it would find no rays left (batches keep
-    // more than their bound's threads resident at 128 a block: as many as an SM
-    // has)
-    const uint32_t threads =
-        L.scenes ? 2048u : trace_resident_blocks(L.variant, false, L.occlusion && !L.count) * kTraceMaxBlock;
-    const int wave = L.sm_count * (int)std::max(1u, threads / (uint32_t)std::max(block, 32));
-    int grid = L.grid > 0 ? L.grid : wave;
     const size_t smem =
         trace_smem_bytes(L.variant, (uint32_t)block, L.stack_depth, L.scenes != nullptr, L.occlusion, L.count);
     if (block < 32 || (uint32_t)block > kTraceMaxBlock || smem > kTraceMaxSmem) return cudaErrorInvalidConfiguration;
+    // one resident wave: a warp beyond it would find no rays left. Blocks per SM
+    // by the registers the instantiation is compiled for, by shared memory (228
+    // KB, 1 KB of them reserved per block) and by the SM's 32 block slots.
+    const uint32_t regs =
+        trace_resident_blocks(L.variant, L.scenes != nullptr, L.occlusion && !L.count) * kTraceMaxBlock / (uint32_t)block;
+    const uint32_t per_sm = std::min({regs, (uint32_t)(228 * 1024 / (smem + 1024)), 32u});
+    const int wave = L.sm_count * (int)per_sm;
+    const int grid = L.grid > 0 ? L.grid : wave;
+    a.warps = (uint32_t)std::min(grid, wave) * ((uint32_t)block / 32u);
     switch (L.variant) {
     case HK_TRACE_FULLSTACK: return launch_v<HK_TRACE_FULLSTACK>(a, L.count, L.occlusion, grid, block, smem, s);
     case HK_TRACE_SHORTSTACK: return launch_v<HK_TRACE_SHORTSTACK>(a, L.count, L.occlusion, grid, block, smem, s);
