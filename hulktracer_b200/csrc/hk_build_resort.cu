@@ -785,11 +785,17 @@ void ResortState::release() {
 static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t spin_limit, bool withhold, uint32_t &next_ticket,
                               ScanPtrs &sp, cudaStream_t st) {
     const size_t tiles = n / kScanTile + 2;
-    if (tiles > S.scan_flags.cap) {
-        cudaError_t e = S.scan_flags.ensure(tiles);
-        if (e == cudaSuccess) e = S.scan_agg.ensure(tiles);
+    if (tiles > std::min({S.scan_flags.cap, S.scan_agg.cap, S.scan_incl.cap})) {
+        // the flags last: while they have a capacity all three stand and they
+        // are cleared, also for the next build after a failure here
+        S.scan_flags.release();
+        cudaError_t e = S.scan_agg.ensure(tiles);
         if (e == cudaSuccess) e = S.scan_incl.ensure(tiles);
-        if (e == cudaSuccess) e = cudaMemsetAsync(S.scan_flags.p, 0, S.scan_flags.cap * 4, st);
+        if (e == cudaSuccess) e = S.scan_flags.ensure(tiles);
+        if (e == cudaSuccess) {
+            e = cudaMemsetAsync(S.scan_flags.p, 0, S.scan_flags.cap * 4, st);
+            if (e != cudaSuccess) S.scan_flags.release();
+        }
         if (e != cudaSuccess) return e;
     }
     S.scan_tag = (S.scan_tag + 1u) & 0x3fffffffu;
