@@ -50,7 +50,8 @@ constexpr uint32_t kMlpKeepRows = 16384;
 
 // buffers of the proposer's forward and training calls, kept by the context
 // from one call to the next (allocating and freeing eleven of them took longer
-// than a 4,096-row step's kernels); trim gives large ones back
+// than a 4,096-row step's kernels); a call that made one larger than that gives
+// them all back at its end, whether it succeeded or not (Lease)
 struct MlpWork {
     DevBuf<float> X, H1, H2, H3, Z4, d1, d2, d3, d4, part, loss;
     DevBuf<int32_t> y;
@@ -73,8 +74,15 @@ struct MlpWork {
         y.release();
     }
     void trim() {
-        if (Z4.cap > (size_t)kMlpKeepRows * kMlpOut) release();
+        bool large = X.cap > (size_t)kMlpKeepRows * kMlpIn || y.cap > kMlpKeepRows;
+        for (DevBuf<float> *b : {&H1, &H2, &H3, &d1, &d2, &d3}) large |= b->cap > (size_t)kMlpKeepRows * kMlpHid;
+        for (DevBuf<float> *b : {&Z4, &d4}) large |= b->cap > (size_t)kMlpKeepRows * kMlpOut;
+        if (large) release();
     }
+    struct Lease {
+        MlpWork &W;
+        ~Lease() { W.trim(); }
+    };
 };
 
 static void batch_detach(hk_batch *b);
@@ -1845,12 +1853,12 @@ hk_status hk_mlp_forward(hk_ctx *c, const float *X, uint32_t n, float *logits) {
     if (!c->learn.have_mlp) return fail(c, HK_E_STATE, "no network");
     cudaSetDevice(c->device);
     MlpWork &W = c->mlp_work;
+    const MlpWork::Lease lease{W};
     HK_CUDA(c, W.ensure_forward(n));
     HK_CUDA(c, cudaMemcpyAsync(W.X.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
     HK_CUDA(c, mlp_infer(c->learn.mlp, W.X.p, nullptr, n, W.Z4.p, c->sm_count, c->stream, c->errw.p));
     HK_CUDA(c, cudaMemcpyAsync(logits, W.Z4.p, (size_t)n * kMlpOut * 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));
-    W.trim();
     uint32_t w = 0;
     HK_CUDA(c, cudaMemcpy(&w, c->errw.p, 4, cudaMemcpyDeviceToHost));
     if (w) {
@@ -1889,6 +1897,7 @@ hk_status hk_mlp_grad(hk_ctx *c, const float *X, const int32_t *y, uint32_t n, f
         if (y[i] < 0 || y[i] >= kMlpOut) return fail(c, HK_E_ILLEGAL_INPUT, "label out of range");
     cudaSetDevice(c->device);
     MlpWork &W = c->mlp_work;
+    const MlpWork::Lease lease{W};
     HK_CUDA(c, W.ensure(n));
     HK_CUDA(c, cudaMemcpyAsync(W.X.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, c->stream));
     HK_CUDA(c, cudaMemcpyAsync(W.y.p, y, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
@@ -1900,7 +1909,6 @@ hk_status hk_mlp_grad(hk_ctx *c, const float *X, const int32_t *y, uint32_t n, f
     HK_CUDA(c, cudaMemcpyAsync(&ls, W.loss.p, 4, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (loss) *loss = ls / (float)n;
-    W.trim();
     return HK_OK;
 }
 
@@ -1961,6 +1969,7 @@ hk_status hk_mlp_train(hk_ctx *c, uint32_t epochs, uint32_t batch, float lr, uin
     if (rows < batch) return fail(c, HK_E_STATE, "fewer recorded rows than one batch");
     DevBuf<uint32_t> perm;
     MlpWork &W = c->mlp_work;
+    const MlpWork::Lease lease{W};
     HK_CUDA(c, perm.ensure(rows));
     HK_CUDA(c, W.ensure(batch));
     std::vector<uint32_t> idx(rows);
@@ -1986,7 +1995,6 @@ hk_status hk_mlp_train(hk_ctx *c, uint32_t epochs, uint32_t batch, float lr, uin
         if (epoch_loss) epoch_loss[e] = ls / (float)(nb * batch);
     }
     perm.release();
-    W.trim();
     return mlp_pack(c);
 }
 

@@ -78,3 +78,31 @@ def test_resort_build_after_each_failed_allocation(fake):
         assert L.fake_bad_launches() == 0, "scan workspaces after allocation %d failed" % k
         L.hk_destroy(h)
     assert L.fake_live_bytes() == 0
+
+
+@pytest.mark.parametrize("call", ["forward", "grad"])
+def test_proposer_calls_give_large_buffers_back(fake, call):
+    """Rows beyond the bound that a context keeps: nothing is held after the
+    call, whether it succeeded or one of its allocations failed."""
+    L = fake
+    rows = 16_384 + 1
+    x, y = np.zeros((rows, 200), np.float32), np.zeros(rows, np.int32)
+    logits, grads = np.zeros((rows, 96), np.float32), np.zeros(1 << 20, np.float32)
+
+    def run(h):
+        if call == "forward":
+            return L.hk_mlp_forward(h, p(x), C.c_uint32(rows), p(logits))
+        return L.hk_mlp_grad(h, p(x), p(y), C.c_uint32(rows), p(grads), None)
+    h = context(L)
+    assert L.hk_mlp_init(h, C.c_uint64(1)) == 0
+    held, before = L.fake_live_bytes(), L.fake_allocs()
+    assert run(h) == 0
+    n = L.fake_allocs() - before
+    assert n >= 2 and L.fake_live_bytes() == held
+    for k in range(1, n + 1):
+        L.fake_fail_at(k)
+        assert run(h) != 0
+        L.fake_fail_at(0)
+        assert L.fake_live_bytes() == held, "allocation %d" % k
+    assert run(h) == 0
+    L.hk_destroy(h)
