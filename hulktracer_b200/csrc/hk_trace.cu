@@ -1,9 +1,9 @@
 // hk_trace.cu -- KD-tree traversal kernels (sm_100a).
 //
-// One persistent kernel per traversal variant. Each warp takes 32 rays at a
-// time from a global counter (atomicAdd by lane 0, broadcast with
-// __shfl_sync), so the grid is sized to the SM count rather than the ray
-// count and uneven ray batches balance themselves. Traversal semantics follow
+// One persistent kernel per traversal variant. Each warp refills its idle lanes
+// from a global ray counter (atomicAdd by lane 0, broadcast with __shfl_sync),
+// so the grid is sized to the SM count rather than the ray count and uneven ray
+// batches balance themselves. Traversal semantics follow
 // the reference kernels exactly (comparison operators, near/far rule, the
 // "child 0" sentinel, strict < between hits in leaf order); see the comments
 // at each variant. Most launches test the leaves of a whole warp together
@@ -124,10 +124,11 @@ struct LaneState {
     uint32_t ray;
 };
 
-// A leg run with DEFER leaves its leaf test to the warp (coop_leaf): it
+// A leg of a stack variant leaves its leaf test to the warp (coop_leaf): it
 // records the leaf's reference run and what follows the test -- kDoneIfCloser:
 // finished when the closest hit precedes tmax; kGoOn: not finished; kDone:
-// finished.
+// finished. Only a batch's shared-memory ring, without DEFER, tests the leaf
+// itself.
 enum : int { kNoTest = 0, kDoneIfCloser = 2, kGoOn = 3, kDone = 4 };
 struct Defer {
     uint32_t start, cnt;
@@ -137,7 +138,7 @@ struct Defer {
 // one leg of the ring short stack (KDTreeCPU::searchKDTreeStackless,
 // KDTreeCPU.cpp:363-447; GPUTrace_shortStack.cl:6-105; GPUTrace_LDSshortStack.cl:
 // 7-105 with the ring in shared memory, one column per thread); true = finished
-template <bool SMEM, bool COUNT, bool ANY, bool DEFER = false>
+template <bool SMEM, bool COUNT, bool DEFER>
 __device__ __forceinline__ bool leg_shortstack(const TraceArgs &A, const SceneView &V, LaneState &L, uint2 root, float *s_s, float *s_e,
                                                uint32_t *s_n, float *l_s, float *l_e, uint32_t *l_n,
                                                uint32_t &c_nodes, uint32_t &c_refs, uint32_t &steps, Defer *df = nullptr) {
@@ -170,7 +171,7 @@ __device__ __forceinline__ bool leg_shortstack(const TraceArgs &A, const SceneVi
             return true;
         }
         uint32_t axis = L.node.x & 3u, pair = L.node.x >> 2;
-            const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
+        const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
         float pl = __int_as_float(L.node.y);
         float rs = comp(L.o, axis), dc = comp(L.d, axis);
         float split = __fmul_rn(__fsub_rn(pl, rs), comp(L.inv, axis));
@@ -204,19 +205,19 @@ __device__ __forceinline__ bool leg_shortstack(const TraceArgs &A, const SceneVi
             *df = Defer{L.node.x >> 2, L.node.y, kDoneIfCloser};
             return false;
         }
-        test_leaf<COUNT, ANY>(V, L.node, L.o, L.d, L.best, L.best_id, c_refs, L.lim);
-        if (L.best < L.tmax || (ANY && L.best < L.lim)) return true;
+        test_leaf<COUNT, false>(V, L.node, L.o, L.d, L.best, L.best_id, c_refs);
+        if (L.best < L.tmax) return true;
     }
     return false;
 }
 
 // one leg of the full stack (KDTreeCPU::searchKDTree, KDTreeCPU.cpp:285-361 ==
 // GPUTrace.cl:6-90; far children pushed only when they exist), run until a leaf
-// has been tested; true = finished
-template <bool COUNT, bool ANY, bool DEFER = false>
+// is to be tested; true = finished
+template <bool COUNT>
 __device__ __forceinline__ bool leg_fullstack(const TraceArgs &A, const SceneView &V, LaneState &L, uint2 root, float *st_s, float *st_e,
-                                              uint32_t *st_n, int max_stack, uint32_t &c_nodes, uint32_t &c_refs,
-                                              uint32_t &steps, Defer *df = nullptr) {
+                                              uint32_t *st_n, int max_stack, uint32_t &c_nodes, uint32_t &steps,
+                                              Defer *df) {
     while (true) {
         if (L.best < L.tmin) return true;
         if (COUNT) c_nodes++;
@@ -226,13 +227,8 @@ __device__ __forceinline__ bool leg_fullstack(const TraceArgs &A, const SceneVie
         }
         bool tested = false;
         if (is_leaf(L.node)) {
-            if constexpr (DEFER) {
-                // the stack pop below does not depend on the test's outcome
-                *df = Defer{L.node.x >> 2, L.node.y, kGoOn};
-            } else {
-                test_leaf<COUNT, ANY>(V, L.node, L.o, L.d, L.best, L.best_id, c_refs, L.lim);
-                if (ANY && L.best < L.lim) return true;
-            }
+            // the stack pop below does not depend on the test's outcome
+            *df = Defer{L.node.x >> 2, L.node.y, kGoOn};
             L.cur = 0;
             tested = true;
         } else {
@@ -266,7 +262,7 @@ __device__ __forceinline__ bool leg_fullstack(const TraceArgs &A, const SceneVie
             L.node = V.nodes[L.cur];
         }
         if (L.cur == 0) {
-            if (DEFER && tested) df->after = kDone;
+            if (tested) df->after = kDone;
             return true;
         }
         if (tested) return false;
@@ -275,9 +271,9 @@ __device__ __forceinline__ bool leg_fullstack(const TraceArgs &A, const SceneVie
 
 // one leg of kd-restart (GPUTrace_stackless.cl:53-117 with every leaf resident;
 // EARLY adds the resume path's exit once the closest hit precedes tmax); true = finished
-template <bool EARLY, bool COUNT, bool ANY, bool DEFER = false>
+template <bool EARLY, bool COUNT>
 __device__ __forceinline__ bool leg_restart(const TraceArgs &A, const SceneView &V, LaneState &L, uint2 root, uint32_t &c_nodes,
-                                            uint32_t &c_refs, uint32_t &steps, Defer *df = nullptr) {
+                                            uint32_t &steps, Defer *df) {
     if (!(L.tmax < L.te)) return true;
     L.tmin = L.tmax;
     L.tmax = L.te;
@@ -290,7 +286,7 @@ __device__ __forceinline__ bool leg_restart(const TraceArgs &A, const SceneView 
             return true;
         }
         uint32_t axis = L.node.x & 3u, pair = L.node.x >> 2;
-            const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
+        const uint2 nb = V.nodes[pair], na = V.nodes[pair + 1];
         float pl = __int_as_float(L.node.y);
         float rs = comp(L.o, axis), dc = comp(L.d, axis);
         float split = __fmul_rn(__fsub_rn(pl, rs), comp(L.inv, axis));
@@ -307,12 +303,7 @@ __device__ __forceinline__ bool leg_restart(const TraceArgs &A, const SceneView 
     }
     if (is_leaf(L.node)) {
         if (COUNT) c_nodes++;
-        if constexpr (DEFER) {
-            *df = Defer{L.node.x >> 2, L.node.y, EARLY ? kDoneIfCloser : kGoOn};
-            return false;
-        }
-        test_leaf<COUNT, ANY>(V, L.node, L.o, L.d, L.best, L.best_id, c_refs, L.lim);
-        if ((EARLY && L.best < L.tmax) || (ANY && L.best < L.lim)) return true;
+        *df = Defer{L.node.x >> 2, L.node.y, EARLY ? kDoneIfCloser : kGoOn};
     }
     return false;
 }
@@ -387,15 +378,15 @@ __device__ __forceinline__ bool ropes_advance(LaneState &L, uint32_t lcnt, float
     return false;
 }
 
-// the whole leg with the in-order leaf test (occlusion rays, batches)
-template <bool COUNT, bool ANY>
-__device__ __forceinline__ bool leg_ropes(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
-                                          uint32_t &c_refs) {
+// the whole leg with the in-order leaf test (occlusion rays)
+template <bool COUNT>
+__device__ __forceinline__ bool leg_ropes_any(const SceneView &A, LaneState &L, uint32_t legs_max, uint32_t &c_nodes,
+                                              uint32_t &c_refs) {
     uint32_t lstart, lcnt, rope;
     float texit;
     if (ropes_locate<COUNT>(A, L, legs_max, c_nodes, lstart, lcnt, texit, rope)) return true;
-    if (lcnt) test_leaf<COUNT, ANY>(A, make_uint2(lstart << 2, lcnt), L.o, L.d, L.best, L.best_id, c_refs, L.lim);
-    return ropes_advance<ANY>(L, lcnt, texit, rope);
+    if (lcnt) test_leaf<COUNT, true>(A, make_uint2(lstart << 2, lcnt), L.o, L.d, L.best, L.best_id, c_refs, L.lim);
+    return ropes_advance<true>(L, lcnt, texit, rope);
 }
 
 // The leaf tests of a whole warp shared out over its 32 lanes (all lanes call
@@ -665,15 +656,14 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
             if (active) {
                 if (BATCH) look_up();
                 if (VARIANT == HK_TRACE_FULLSTACK)
-                    fin = leg_fullstack<COUNT, ANY, true>(A, V, L, root, l_s, l_e, l_n, kLocal, c_nodes, c_refs,
-                                                          steps, &df);
+                    fin = leg_fullstack<COUNT>(A, V, L, root, l_s, l_e, l_n, kLocal, c_nodes, steps, &df);
                 else if (VARIANT == HK_TRACE_RESTART)
-                    fin = leg_restart<false, COUNT, ANY, true>(A, V, L, root, c_nodes, c_refs, steps, &df);
+                    fin = leg_restart<false, COUNT>(A, V, L, root, c_nodes, steps, &df);
                 else if (VARIANT == HK_TRACE_RESTART_EARLY)
-                    fin = leg_restart<true, COUNT, ANY, true>(A, V, L, root, c_nodes, c_refs, steps, &df);
+                    fin = leg_restart<true, COUNT>(A, V, L, root, c_nodes, steps, &df);
                 else
-                    fin = leg_shortstack<smem_ring, COUNT, ANY, true>(A, V, L, root, s_s, s_e, s_n, l_s, l_e, l_n,
-                                                                      c_nodes, c_refs, steps, &df);
+                    fin = leg_shortstack<smem_ring, COUNT, true>(A, V, L, root, s_s, s_e, s_n, l_s, l_e, l_n, c_nodes,
+                                                                 c_refs, steps, &df);
             }
             const uint32_t work = (active && df.after != kNoTest) ? df.cnt : 0u;
             coop_leaf<BATCH>(V, A.scenes, scene, L, df.start, work, slot);
@@ -687,6 +677,7 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
             }
             continue;
         }
+        // brute force, a batch's shared-memory ring, ropes occlusion rays
         if (BATCH) look_up();
         bool done;
         if (VARIANT == HK_TRACE_BRUTE) {
@@ -701,21 +692,14 @@ __global__ void __launch_bounds__(kTraceMaxBlock, trace_resident_blocks(VARIANT,
             }
             if (COUNT) c_refs += ntris;
             done = true;
-        } else if (VARIANT == HK_TRACE_FULLSTACK) {
-            done = leg_fullstack<COUNT, ANY>(A, V, L, root, l_s, l_e, l_n, kLocal, c_nodes, c_refs, steps);
         } else if (VARIANT == HK_TRACE_ROPES) {
-            done = leg_ropes<COUNT, ANY>(V, L, legs_max, c_nodes, c_refs);
-        } else if (VARIANT == HK_TRACE_RESTART) {
-            done = leg_restart<false, COUNT, ANY>(A, V, L, root, c_nodes, c_refs, steps);
-        } else if (VARIANT == HK_TRACE_RESTART_EARLY) {
-            done = leg_restart<true, COUNT, ANY>(A, V, L, root, c_nodes, c_refs, steps);
+            done = leg_ropes_any<COUNT>(V, L, legs_max, c_nodes, c_refs);
         } else {
-            done = leg_shortstack<smem_ring, COUNT, ANY>(A, V, L, root, s_s, s_e, s_n, l_s, l_e, l_n, c_nodes, c_refs,
-                                                    steps);
+            done = leg_shortstack<true, COUNT, false>(A, V, L, root, s_s, s_e, s_n, l_s, l_e, l_n, c_nodes, c_refs,
+                                                      steps);
         }
         if (done) {
             A.hits[L.ray] = hk_hit{L.best, L.best_id};
-            if (VARIANT == HK_TRACE_ROPES && !BATCH && A.leaf_out) A.leaf_out[L.ray] = L.cur;
             active = false;
             if (BATCH && atomicSub(&A.remaining[scene], 1u) == 1u) A.done_ns[scene] = global_ns();
         }
