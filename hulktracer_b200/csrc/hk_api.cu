@@ -422,7 +422,7 @@ hk_status hk_scene_set_parts(hk_ctx *c, const uint32_t *part, uint32_t nparts) {
 // device part of a frame's transform: mats already in c->mats
 static hk_status transform_device(hk_ctx *c) {
     HK_CUDA(c, launch_transform(c->rest.p, c->part.p, c->nv, c->mats.p, c->verts.p, c->box_ord.p,
-                                c->box_user ? nullptr : c->box.p, c->stream));
+                                c->box_user ? nullptr : c->box.p, c->sm_count, c->stream));
     HK_CUDA(c, launch_precompute(c->verts.p, c->tris.p, c->nt, c->rec.p, c->stream));
     c->rec_valid = true;
     c->rec_epoch++;
@@ -859,7 +859,8 @@ extern "C" {
 // (hk_build_resort.cu); its tree takes the place of an imported one
 static hk_status build_resort(hk_ctx *c, hk_tree_stats *stats) {
     const ResortParams p{c->cfg.traverse_cost, c->cfg.intersect_cost, c->cfg.max_depth, c->cfg.leaf_size,
-                         c->cfg.sah_sample ? c->cfg.sah_sample : 5u, c->cfg.spin_limit, c->debug_flags};
+                         c->cfg.sah_sample ? c->cfg.sah_sample : 5u, (uint32_t)c->sm_count, c->cfg.spin_limit,
+                         c->debug_flags};
     float hb[8];
     HK_CUDA(c, cudaMemcpyAsync(hb, c->box.p, 32, cudaMemcpyDeviceToHost, c->stream));
     HK_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -459,6 +459,7 @@ struct LevelArgs {
     // triangle bounds, 32 bytes (one memory sector) each: {lo.x, hi.x, lo.y,
     // hi.y}, {lo.z, hi.z, -, -}
     const float4 *tb;
+    uint32_t wave;          // four CTAs per SM
     // the level's nodes and references, ping-pong by level parity: level L
     // reads buffer L & 1 and writes the other (the accessors below)
     float4 *lo_buf[2], *hi_buf[2];
@@ -585,11 +586,11 @@ __device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c, uint32_
 }
 // References per chunk of a node of more than kChunk references, in a level
 // of `refs` references: small enough that the level's chunks fill k_decide's
-// one wave of four CTAs per SM (148 SMs), since a chunk of 256 takes 1.5 us less
+// one wave of four CTAs per SM (A.wave), since a chunk of 256 takes 1.5 us less
 // than one of 1024 and the levels of small scenes have few of them. A node of
 // up to kChunk is one chunk: it then needs no sum in global memory.
-__device__ __forceinline__ uint32_t chunk_refs(uint32_t refs) {
-    const uint32_t per = refs / (4u * 148u);
+__device__ __forceinline__ uint32_t chunk_refs(const LevelArgs &A, uint32_t refs) {
+    const uint32_t per = refs / A.wave;
     return per <= kChunkMin ? kChunkMin : (per <= 2 * kChunkMin ? 2 * kChunkMin : kChunk);
 }
 __device__ __forceinline__ uint32_t node_chunks(uint32_t c, uint32_t per) {
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(256) k_root(LevelArgs A, const float *box, con
     const bool dec = nt > A.leaf_size && A.max_depth > 0;
     const bool medium = dec && is_medium(A, nt);
     const bool large = dec && is_large(A, nt, nt);
-    const uint32_t per = nt <= kChunk ? kChunk : chunk_refs(nt), nch = large ? node_chunks(nt, per) : 0u;
+    const uint32_t per = nt <= kChunk ? kChunk : chunk_refs(A, nt), nch = large ? node_chunks(nt, per) : 0u;
     if (blockIdx.x == 0) {
         uint32_t *w = reinterpret_cast<uint32_t *>(A.ctr);
         for (uint32_t i = threadIdx.x; i < sizeof(BuildCounters) / 4; i += blockDim.x) w[i] = 0;
@@ -1484,7 +1485,7 @@ __device__ __forceinline__ void hist_body(const LevelArgs &A, const HistStart &h
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) {
-            const uint32_t nchunks = node_chunks(info.y, chunk_refs(A.lc->refs));
+            const uint32_t nchunks = node_chunks(info.y, chunk_refs(A, A.lc->refs));
             s_last = (atomicAdd(&A.done[rank], 1u) == nchunks - 1) ? 1 : 0;
         }
         __syncthreads();
@@ -1968,7 +1969,7 @@ __device__ void child_setup(const LevelArgs &A, uint32_t ns, uint32_t start, uin
     }
     const uint32_t refs = A.lc->t_childrefs;
     if (!(dec && is_large(A, c, refs))) return;
-    const uint32_t per = c <= kChunk ? kChunk : chunk_refs(refs), nch = node_chunks(c, per);
+    const uint32_t per = c <= kChunk ? kChunk : chunk_refs(A, refs), nch = node_chunks(c, per);
     const uint32_t rank = atomicAdd(&A.nlc->n_large, 1u);
     const uint32_t first = atomicAdd(&A.nlc->n_chunks, nch);
     if (rank >= A.cap_large || first + nch > A.cap_chunks) {
@@ -2991,6 +2992,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     LevelArgs A;
     memset(&A, 0, sizeof(A));
     A.tb = S.tb;
+    A.wave = (uint32_t)G;
     A.axis = S.d_axis;
     A.plane = S.d_plane;
     A.cnt = S.d_cnt;

@@ -782,7 +782,7 @@ void ResortState::release() {
     } while (0)
 
 // the tile states of a scan of up to n elements, and its tag and ticket
-static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t spin_limit, bool withhold, uint32_t &next_ticket,
+static cudaError_t scan_begin(ResortState &S, const ResortParams &p, size_t n, bool withhold, uint32_t &next_ticket,
                               ScanPtrs &sp, cudaStream_t st) {
     const size_t tiles = n / kScanTile + 2;
     if (tiles > std::min({S.scan_flags.cap, S.scan_agg.cap, S.scan_incl.cap})) {
@@ -800,18 +800,18 @@ static cudaError_t scan_begin(ResortState &S, size_t n, uint32_t spin_limit, boo
     }
     S.scan_tag = (S.scan_tag + 1u) & 0x3fffffffu;
     sp = ScanPtrs{S.scan_flags.p, S.tickets.p + next_ticket++, S.sizes.p + SK_ERR, S.scan_agg.p, S.scan_incl.p,
-                  S.scan_tag, spin_limit ? std::max(spin_limit, kScanSpinsMin) : kScanSpins, withhold ? 1u : 0u};
+                  S.scan_tag, p.spin_limit ? std::max(p.spin_limit, kScanSpinsMin) : kScanSpins, withhold ? 1u : 0u};
     return cudaSuccess;
 }
 
 template <class Op>
-static cudaError_t scan(ResortState &S, const Op &op, size_t n, uint32_t spin_limit, bool withhold,
+static cudaError_t scan(ResortState &S, const ResortParams &p, const Op &op, size_t n, bool withhold,
                         uint32_t &next_ticket, cudaStream_t st) {
     ScanPtrs sp;
-    cudaError_t e = scan_begin(S, n, spin_limit, withhold, next_ticket, sp, st);
+    cudaError_t e = scan_begin(S, p, n, withhold, next_ticket, sp, st);
     if (e != cudaSuccess) return e;
     // a CTA per tile up to four per SM
-    const unsigned grid = (unsigned)std::min<size_t>(n / kScanTile + 1, 148u * 4u);
+    const unsigned grid = (unsigned)std::min<size_t>(n / kScanTile + 1, (size_t)p.sm_count * 4);
     k_r_scan<Op><<<grid, kScanNT, 0, st>>>(op, sp);
     return cudaGetLastError();
 }
@@ -933,7 +933,7 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
         // 1. candidates
         int kc = 0;
         L.keys = S.keys[kc].p;
-        RS_CHECK(scan(S, InitOp{L}, n, p.spin_limit, hold, next_ticket, st));
+        RS_CHECK(scan(S, p, InitOp{L}, n, hold, next_ticket, st));
         if (K) {
             k_r_emit<<<blocks(K / 6), 256, 0, st>>>(L, verts, tris);
             // 2. sort by (segment, value, marker)
@@ -941,7 +941,7 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
             if (maxseg <= kSegCtaMax) {
                 const uint32_t nseg = 3 * n;
                 k_seg_sort_warp<<<(unsigned)(((size_t)nseg * 32 + 255) / 256), 256, 0, st>>>(L, nseg);
-                if (maxseg > kSegWarpMax) k_seg_sort_cta<<<std::min<uint32_t>(nseg, 148u * 8u), 256, 0, st>>>(L, nseg);
+                if (maxseg > kSegWarpMax) k_seg_sort_cta<<<std::min<uint32_t>(nseg, p.sm_count * 8u), 256, 0, st>>>(L, nseg);
             } else {
                 uint32_t segbits = 1;
                 while (segbits < 30 && (1ull << segbits) < 3ull * n) segbits++;
@@ -951,8 +951,7 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
                 for (int shift = 0; shift < nbits; shift += 8) {
                     k_rs_hist<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, L.koff + n, shift, ntiles, S.hist.p,
                                                      L.sizes + SK_ERR);
-                    RS_CHECK(scan(S, RsScanOp{S.hist.p, 256 * ntiles}, 256 * (size_t)ntiles, p.spin_limit, hold, next_ticket,
-                                  st));
+                    RS_CHECK(scan(S, p, RsScanOp{S.hist.p, 256 * ntiles}, 256 * (size_t)ntiles, hold, next_ticket, st));
                     k_rs_scatter<<<ntiles, kRT, 0, st>>>(S.keys[kc].p, S.keys[kc ^ 1].p, L.koff + n, shift, ntiles,
                                                          S.hist.p, L.sizes + SK_ERR);
                     kc ^= 1;
@@ -960,12 +959,12 @@ hk_status resort_build(ResortState &S, const ResortParams &p, const float4 *vert
             }
             L.keys = S.keys[kc].p;
             // 3. sweep
-            RS_CHECK(scan(S, SweepOp{L}, K, p.spin_limit, false, next_ticket, st));
+            RS_CHECK(scan(S, p, SweepOp{L}, K, false, next_ticket, st));
             k_r_cost<<<blocks(K), 256, 0, st>>>(L);
         }
         // 4. decisions, ranks, leaf offsets; classification; cells and nodes
-        RS_CHECK(scan(S, DecideOp{L}, n, p.spin_limit, hold, next_ticket, st));
-        RS_CHECK(scan(S, ClassifyOp{L, R, verts, tris}, R, p.spin_limit, false, next_ticket, st));
+        RS_CHECK(scan(S, p, DecideOp{L}, n, hold, next_ticket, st));
+        RS_CHECK(scan(S, p, ClassifyOp{L, R, verts, tris}, R, false, next_ticket, st));
         k_r_nodes<<<blocks(n), 256, 0, st>>>(L);
         RS_CHECK(cudaGetLastError());
         RS_CHECK(cudaMemcpyAsync(S.host_sizes, S.sizes.p, SK_WORDS * 4, cudaMemcpyDeviceToHost, st));

@@ -121,7 +121,7 @@ cudaError_t launch_rec_to_cache(const TriRec *rec, uint32_t nt, float *cache16, 
 constexpr uint32_t kBoxWords = 8;
 cudaError_t launch_box_reset(uint32_t *box_ord, cudaStream_t s);
 cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12, float4 *out,
-                             uint32_t *box_ord, float *box, cudaStream_t s);
+                             uint32_t *box_ord, float *box, int sm_count, cudaStream_t s);
 // a frame's counters, cleared by its camera-ray launch: the traces' ray-batch
 // counters and the lists' lengths
 enum FrameCounter : uint32_t { kFetchPrimary, kFetchMirror, kFetchShadow, kShadowCount, kMirrorCount, kFrameCounters };

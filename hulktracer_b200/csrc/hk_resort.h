@@ -14,6 +14,7 @@ struct ResortParams {
     uint32_t max_depth;   // a node at this depth is a leaf
     uint32_t leaf_size;   // a node of at most this many references is a leaf
     uint32_t sample;      // every sample-th reference of a node makes candidates
+    uint32_t sm_count;
     uint32_t spin_limit;  // polls before a scan's wait gives up (0: the default)
     uint32_t debug_flags; // test aid (hk_set_debug_flags)
 };

@@ -175,8 +175,8 @@ cudaError_t launch_box_reset(uint32_t *box_ord, cudaStream_t s) {
 }
 
 cudaError_t launch_transform(const float4 *rest, const uint32_t *part, uint32_t nv, const float *mats12, float4 *out,
-                             uint32_t *box_ord, float *box, cudaStream_t s) {
-    const int grid = std::min(std::max(blocks_for(nv, kTransformThreads), 1), 148 * 4);
+                             uint32_t *box_ord, float *box, int sm_count, cudaStream_t s) {
+    const int grid = std::min(std::max(blocks_for(nv, kTransformThreads), 1), sm_count * 4);
     k_transform<<<grid, kTransformThreads, 0, s>>>(rest, part, nv, mats12, out, box_ord, box);
     return cudaGetLastError();
 }
