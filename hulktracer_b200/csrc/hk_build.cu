@@ -604,8 +604,7 @@ __device__ __forceinline__ bool is_deferred(const LevelArgs &A, uint32_t c) {
 }
 
 // the build's counters zeroed, the triangles' bounds, and the root node and
-// references of level 0; a root with more than 256 references is the first
-// large node (one launch: a memset and two kernels cost a small scene 5 us more)
+// references of level 0; a root that is a large node is the first of them (one launch: a memset and two kernels cost a small scene 5 us more)
 static_assert(sizeof(BuildCounters) % 4 == 0, "cleared word by word");
 __global__ void __launch_bounds__(256) k_root(LevelArgs A, const float *box, const float4 *__restrict__ V,
                                               const uint4 *__restrict__ T, uint32_t nt, float4 *__restrict__ tb) {
@@ -766,9 +765,8 @@ __device__ __forceinline__ int32_t exact_label(int axis, float p, float4 blo, fl
 // reference bound on every axis with a positive extent is a candidate plane p
 // (+0.0f turns a -0 bound into +0), with
 //   below = #(lo < p) + #(flat at p),  above = #(hi > p) + #(flat at p)
-// -- the partition's own classification -- from sorted copies of the lower
-// bounds, upper bounds and flat references' bounds; the lowest cost wins,
-// ties to the lower axis, then the lower plane, as in the oracle's loop.
+// -- the partition's own classification; the lowest cost wins, ties to the lower
+// axis, then the lower plane, as in the oracle's loop.
 // ---------------------------------------------------------------------------
 // Nodes of at most 32 references, one warp, one reference per lane. A plane p
 // strictly inside the node needs no clipped bounds (lo < p says the same of
@@ -1299,9 +1297,6 @@ __device__ Decision sah_exact_group(const LevelArgs &A, uint4 info, float4 blo, 
     return best;
 }
 
-// Large nodes, binned mode: one CTA per chunk of 1024 references builds the
-// chunk's histograms in shared memory and adds them to the node's global
-// histogram; the CTA that finishes the node's last chunk evaluates the SAH.
 // the binned SAH of a large node from its complete histogram (one warp): a
 // proposer row keeps the binned decision and the features for k_refine_cta /
 // k_refine_warp, every other node is decided here
@@ -1624,10 +1619,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_decide(LevelArgs A) {
 }
 
 constexpr int kLearnMaxK = 8;
-constexpr uint32_t kLearnScratch = 2048;   // floats of list space per warp
-
-// list capacity per (proposal, list): the largest power of two with 3 k of
-// them in one warp's space (128 for k = 4), so a list sorts in place
+// list capacity per (proposal, list): the largest power of two whose 3 k-fold
+// is at most 2,048 (128 for k = 4). A bin with a longer list is not costed, so
+// the rule is part of the result (the oracle has the same)
+constexpr uint32_t kLearnScratch = 2048;
 __host__ __device__ constexpr uint32_t learn_list_cap(uint32_t K) {
     uint32_t c = 1;
     while (2 * c * 3 * K <= kLearnScratch) c *= 2;
@@ -2406,8 +2401,8 @@ __global__ void __launch_bounds__(kScanThreads, kPlanGrid) k_plan_refs(LevelArgs
 // deferred subtrees. After the levels, one warp builds each subtree rooted at
 // a recorded node of at most kDeferMax references, depth first, with one
 // reference per lane (a node's references are a mask of the warp's lanes, in
-// the root's order), deciding every node with the levels' SAH (the binned
-// histograms, or the exact search in registers). Nodes are numbered locally:
+// the root's order), deciding every node with the levels' SAH of at most 32
+// references (sah_lanes_binned, or sah_lanes_exact). Nodes are numbered locally:
 // a split takes the next pair of local indices (below, above); the below
 // child is built next and the above child waits on a stack in shared memory.
 // Nodes go to 64-byte scratch records (cell, ropes, entry, subtree and local
@@ -3077,7 +3072,7 @@ cudaError_t build_launch(BuildState &S, const float4 *verts, const uint4 *tris, 
     const uint32_t sub_E = sub_stack_entries(S.p.max_depth);
     const size_t sub_smem = kSubWarps * sub_warp_smem(sub_E, exact_small);
     // (a level's references are two to three times the triangles, its nodes of a
-    // CTA each rarely below 64 references; a plan tile is 1,024 references)
+    // CTA each rarely below 64 references; a reference tile is 1,024 references)
     const unsigned g_nodes3 = level_grid(S.sm_count, 3, nt / 32), g_nodes4 = level_grid(S.sm_count, 4, nt / 32);
     const unsigned g_plan = level_grid(S.sm_count, kPlanGrid, nt / 256);
     const bool binned_only = !A.learned && A.exact_max == 0 && S.p.level_streams != 2;

@@ -108,8 +108,9 @@ typedef struct hk_config {
                                  kernel's launch bound). A trace whose shared memory
                                  (SMEMSTACK: short_stack x block_size x 12 bytes, plus
                                  block_size x 8 bytes for the warp-shared leaf test of
-                                 every closest-hit variant but BRUTE) exceeds 48 KB is
-                                 refused with HK_E_ILLEGAL_INPUT */
+                                 every launch but BRUTE, shadow rays by ROPES and
+                                 batches by SMEMSTACK) exceeds 48 KB is refused with
+                                 HK_E_ILLEGAL_INPUT */
     uint32_t blocks_per_sm;   /* persistent trace grid = SMs * blocks_per_sm (0, the default:
                                  one resident wave) */
     uint32_t max_refs;        /* builder reference arena capacity (0 = 16 x tris) */
