@@ -590,8 +590,9 @@ __device__ __forceinline__ bool is_large(const LevelArgs &A, uint32_t c, uint32_
 // than one of 1024 and the levels of small scenes have few of them. A node of
 // up to kChunk is one chunk: it then needs no sum in global memory.
 __device__ __forceinline__ uint32_t chunk_refs(const LevelArgs &A, uint32_t refs) {
-    const uint32_t per = refs / A.wave;
-    return per <= kChunkMin ? kChunkMin : (per <= 2 * kChunkMin ? 2 * kChunkMin : kChunk);
+    // (refs / A.wave up to 256, up to 512)
+    return refs < (kChunkMin + 1) * A.wave ? kChunkMin
+                                           : (refs < (2 * kChunkMin + 1) * A.wave ? 2 * kChunkMin : kChunk);
 }
 __device__ __forceinline__ uint32_t node_chunks(uint32_t c, uint32_t per) {
     return c <= kChunk ? 1u : (c + per - 1) / per;
