@@ -436,7 +436,9 @@ hk_status hk_mlp_load(hk_ctx *ctx, const char *path);
  * W stored in x out row-major; n = 207712 */
 hk_status hk_mlp_get_params(hk_ctx *ctx, float *params, uint32_t n);
 hk_status hk_mlp_set_params(hk_ctx *ctx, const float *params, uint32_t n);
-/* tensor-core inference: logits[n][96] of X[n][200] (host arrays) */
+/* tensor-core inference: logits[n][96] of X[n][200] (host arrays). This call and
+ * the next keep their device buffers in the context for later calls, those of
+ * up to 16,384 rows (139 MB with the gradients'), until hk_destroy. */
 hk_status hk_mlp_forward(hk_ctx *ctx, const float *X, uint32_t n, float *logits);
 /* FP32 training kernels: mean softmax cross-entropy of labels y and its
  * gradient with respect to every parameter (flat layout above) */
